@@ -46,3 +46,21 @@ def test_prune_component_tiles(port, sizes):
             out, err = mg.simplify(idx, pos, target, error, opt)
             assert np.array_equal(out, ref)
             assert err == ref_err
+
+
+@pytest.mark.parametrize("order", ["rows", "reversed", "shuffled"])
+@pytest.mark.parametrize("amp,ratio", [(0.02, 1.0), (0.02, 0.4), (0.2, 0.6)])
+def test_update_vertex_orders(port, order, amp, ratio):
+    """The position solve depends on vertex order: long index-ordered chains, forwards and backwards, and none."""
+    idx, pos = W.heightfield(67, seed=21, amp=amp)
+    n = len(pos)
+    new = {"rows": np.arange(n), "reversed": np.arange(n)[::-1], "shuffled": np.random.default_rng(4).permutation(n)}[order]
+    p = np.empty_like(pos)
+    p[new] = pos
+    i = new[idx].astype(np.uint32)
+    target = W.target_count(len(i), ratio)
+    ref = port.simplify_with_update("port", i, p, target, 1.0, 0)
+    got = mg.simplify_with_update(i, p, target, 1.0, 0)
+    assert np.array_equal(got[0], ref[0])
+    assert _same(got[1], ref[1])
+    assert not _same(got[1], p)
