@@ -1615,9 +1615,8 @@ struct PerformArgs
 //    test runs against the one-ring as moved by earlier commits only (moving commit < k).
 
 // the commit of a decided candidate: r0 moves to its target and both endpoints lock
-__device__ __forceinline__ void commitOne(const PerformArgs& a, unsigned int c, unsigned int k, unsigned int r0, unsigned int r1)
+__device__ __forceinline__ void commitOne(const PerformArgs& a, const uint4& cd, unsigned int k, unsigned int r0, unsigned int r1)
 {
-	const uint4 cd = __ldg(a.crec + c);
 	const unsigned int i0 = cd.x, i1 = cd.y;
 	const unsigned char kd = (unsigned char)cd.w;
 	unsigned int target;
@@ -1645,9 +1644,14 @@ __device__ __forceinline__ void commitOne(const PerformArgs& a, unsigned int c, 
 // (ringDecide) for the waits, the flip test and the commit; and last the candidates that still
 // wait: locked at once if a commit of this round took an endpoint, else marked for the next round.
 
+#ifndef MO_RING_LANES
+#define MO_RING_LANES 4
+#endif
 #ifndef MO_RING_BATCH
 #define MO_RING_BATCH 2
 #endif
+constexpr unsigned int kRingLanes = MO_RING_LANES; // lanes that walk one candidate's one-ring
+constexpr unsigned int kRingBatch = MO_RING_BATCH; // corners per lane in one batch of loads
 
 enum
 {
@@ -1656,28 +1660,42 @@ enum
 	kRingCommit = 2,
 };
 
-// One walk over the one-ring of r0. If an undecided earlier candidate moves a vertex of it, the
-// candidate waits. Otherwise the flip test (hasTriangleFlips :1201-1232) sees the one-ring as
-// moved by earlier commits only, and the candidate is rejected or commits. The whole ring is
-// checked for waits before a flip decides anything: a wait means an earlier decision is still
-// open that may move a vertex the test reads.
-__device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, unsigned int k, const uint4& rec, unsigned int round)
+// One walk over the one-ring of r0, by kRingLanes lanes together (all of `mask`; lane sub == 0 of them
+// records the decision). If an undecided earlier candidate moves a vertex of the ring, the candidate
+// waits. Otherwise the flip test (hasTriangleFlips :1201-1232) sees the one-ring as moved by earlier
+// commits only, and the candidate is rejected or commits. The whole ring is checked for waits before
+// a flip decides anything: a wait means an earlier decision is still open that may move a vertex the
+// test reads.
+// Bound by dependent L2 round trips: a ring of up to kRingLanes * kRingBatch corners is two of them
+// (its corners, then their marks and positions), and its corners are read side by side. One lane per
+// candidate, two corners at a time, took three or four batches of both: 4 lanes x 2 corners against
+// it, whole calls: 256^2 heightfield 0.92 -> 0.81 ms, 2M attribute sphere 4.36 -> 4.17, 20M terrain
+// 40.4 -> 38.5. 8 x 1: 0.81, 4.22, 39.0; 4 x 1: 0.84, 4.26, 39.2; 2 x 2: 0.87, 4.29, 39.4; 2 x 4
+// (spills): 0.88, 4.61, 43.7.
+__device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, unsigned int k, const uint4& rec, unsigned int round, unsigned int sub,
+    unsigned int mask)
 {
 	const unsigned int r0 = rec.x, r1 = rec.y, b = rec.z, e = rec.w;
 	const unsigned long long tag = roundTag(round);
 	const unsigned int p = round & 1;
+	const uint4 cd = sub == 0 ? __ldg(a.crec + c) : make_uint4(0, 0, 0, 0); // in flight during the walk
 	const V3 v0 = ldpos(a.pos, r0), v1 = ldpos(a.pos, r1);
 	bool flip = false;
-	constexpr int FB = MO_RING_BATCH;
-	for (unsigned int j = b; j < e; j += FB)
+	constexpr unsigned int FB = kRingBatch;
+	for (unsigned int j0 = b; j0 < e; j0 += FB * kRingLanes)
 	{
 		uint2 ed[FB];
 		ulonglong2 sx[FB], sy[FB];
 		float4 px[FB], py[FB];
 #pragma unroll
-		for (int q = 0; q < FB; ++q)
+		for (unsigned int q = 0; q < FB; ++q)
 		{
-			ed[q] = j + q < e ? __ldg(a.adj + j + q) : make_uint2(r1, r1); // r1 is in the ring already
+			const unsigned int j = j0 + q * kRingLanes + sub;
+			ed[q] = j < e ? __ldg(a.adj + j) : make_uint2(r1, r1); // r1 is in the ring already
+		}
+#pragma unroll
+		for (unsigned int q = 0; q < FB; ++q)
+		{
 			sx[q] = __ldcg(reinterpret_cast<const ulonglong2*>(a.minS) + ed[q].x);
 			sy[q] = __ldcg(reinterpret_cast<const ulonglong2*>(a.minS) + ed[q].y);
 			px[q] = __ldg(a.pos + ed[q].x);
@@ -1685,14 +1703,12 @@ __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, 
 		}
 		bool wait = false;
 #pragma unroll
-		for (int q = 0; q < FB; ++q)
+		for (unsigned int q = 0; q < FB; ++q)
 			wait |= earlierThan(p ? sx[q].y : sx[q].x, tag, k) | earlierThan(p ? sy[q].y : sy[q].x, tag, k);
-		if (wait)
+		if (__any_sync(mask, wait))
 			return kRingWaits;
-		if (flip)
-			continue;
 #pragma unroll
-		for (int q = 0; q < FB; ++q)
+		for (unsigned int q = 0; q < FB; ++q)
 		{
 			// moved by an earlier commit: the pair holds {commit, target} with tag 0
 			const bool mvx = (sx[q].x >> 32) == 0 && (unsigned int)sx[q].x < k;
@@ -1706,13 +1722,15 @@ __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, 
 			flip |= triFlip(pa, pb, v0, v1);
 		}
 	}
-	if (flip)
+	flip = __any_sync(mask, flip);
+	if (sub == 0)
 	{
-		a.status[k] = kSkipFlip;
-		return kRingFlip;
+		if (flip)
+			a.status[k] = kSkipFlip;
+		else
+			commitOne(a, cd, k, r0, r1);
 	}
-	commitOne(a, c, k, r0, r1);
-	return kRingCommit;
+	return flip ? kRingFlip : kRingCommit;
 }
 
 __device__ __forceinline__ void markCandidate(const PerformArgs& a, unsigned int k, const uint4& rec, unsigned int round)
@@ -1985,6 +2003,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	const unsigned int G = gridDim.x;
 	const size_t gthreads = (size_t)G * blockDim.x;
 	const unsigned int lane = threadIdx.x & 31;
+	const unsigned int sub = lane & (kRingLanes - 1), ring_mask = (~0u >> (32 - kRingLanes)) << (lane - sub);
 
 	// per-pass scalars: the launch parameters, or the device-resident loop's live state
 	unsigned int count = a.count, tris = a.tris, first_window = a.first_window, round_base = a.round_base, prev_err = a.prev_err_bits;
@@ -2144,18 +2163,18 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 				__syncthreads();
 				// stage B: the one-ring's marks, the flip test and the commit, in one walk
 				const unsigned int nB = s_app[1];
-				for (unsigned int base = 0; base < nB; base += blockDim.x)
+				for (unsigned int base = 0; base < nB; base += blockDim.x / kRingLanes)
 				{
-					const unsigned int x = base + threadIdx.x;
+					const unsigned int x = base + threadIdx.x / kRingLanes;
 					int r = kRingFlip;
 					unsigned int c = 0;
 					if (x < nB)
 					{
 						c = s_stage[0][x];
-						r = ringDecide(a, c, __ldg(a.rank + c), __ldg(a.cring + c), round);
+						r = ringDecide(a, c, __ldg(a.rank + c), __ldg(a.cring + c), round, sub, ring_mask);
 					}
-					append(r == kRingWaits, c, &s_app[3], s_stage[1]);
-					append(r == kRingCommit, c, &s_commits, commits);
+					append(sub == 0 && r == kRingWaits, c, &s_app[3], s_stage[1]);
+					append(sub == 0 && r == kRingCommit, c, &s_commits, commits);
 				}
 				__syncthreads();
 				// stage C: the candidates that wait. A commit of this round (this block's, or another's
