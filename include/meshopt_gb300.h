@@ -287,7 +287,8 @@ typedef struct meshoptgpu_ServerConfig
 	int max_batch;            /* requests per batch launch at most (0: 2048) */
 	int batch_threads;        /* threads per CTA of the batch kernel (0: 256) */
 	int plain;                /* 1: no batching, one request at a time on the single-mesh path */
-	int perform_blocks;       /* cap on the cooperative pass kernel's grid per single-mesh request, so
+	int perform_blocks;       /* cap on the cooperative pass kernel's grid (in blocks of 256 threads) per
+	                             single-mesh request, so
 	                             that concurrent requests share the GPU (0: 64; plain mode: no cap) */
 } meshoptgpu_ServerConfig;
 

@@ -60,6 +60,61 @@ __device__ __forceinline__ void gridBarrier(unsigned int* bar, unsigned int* err
 	__syncthreads();
 }
 
+// A grid barrier that also adds up one value per block, in the arrival itself, so that the total is
+// there when the wait ends and costs no round trip of its own. word[0] and word[1] (zero before the
+// launch) serve alternate barriers: arrivals in the low half, the running sum in the high half. No
+// block can arrive at the next barrier of the same word before every block has left this one, so the
+// high half a waiting block reads holds this barrier's values and no later ones.
+struct GridSum
+{
+	unsigned long long* word; // global, two words
+	unsigned int* err;
+	unsigned int* s;    // shared: [0], [1] the words' sums so far, [2] this barrier's total, [3] the error flag
+	unsigned int phase; // barriers passed
+
+	__device__ void start(unsigned long long* w, unsigned int* e, unsigned int* sh)
+	{
+		word = w, err = e, s = sh, phase = 0;
+		if (threadIdx.x == 0)
+			s[0] = s[1] = s[2] = s[3] = 0;
+	}
+	__device__ __forceinline__ unsigned int wait(unsigned int add = 0, unsigned int limit = kBarrierSpinLimit)
+	{
+		__syncthreads();
+		if (threadIdx.x == 0)
+		{
+			unsigned long long* w = word + (phase & 1);
+			unsigned long long v;
+			asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;" : "=l"(v) : "l"(w), "l"(1ull | (unsigned long long)add << 32) : "memory");
+			const unsigned int target = ((unsigned int)v / gridDim.x + 1) * gridDim.x;
+			const unsigned int failed = __ldcg(err); // another block's, seen one barrier later at most
+			unsigned int spins = 0, out = 0;
+			for (;;)
+			{
+				asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
+				if ((int)((unsigned int)v - target) >= 0)
+					break;
+				if (++spins > limit)
+				{
+					atomicOr(err, 1u);
+					out = 1;
+					break;
+				}
+				if (kBarrierSleepNs)
+					__nanosleep(kBarrierSleepNs);
+			}
+			const unsigned int sum = (unsigned int)(v >> 32);
+			s[2] = sum - s[phase & 1];
+			s[phase & 1] = sum;
+			s[3] = failed | out;
+		}
+		++phase;
+		__syncthreads();
+		return s[2];
+	}
+	__device__ __forceinline__ bool failed() const { return s[3] != 0; }
+};
+
 // A grid barrier that a cooperative launch passes once, leaving its two words zero for the next
 // launch: bar[0] counts arrivals, bar[1] departures, and the last block to depart clears both
 // (by then no block polls bar[0] any more). A launch whose wait ran out leaves them nonzero: the

@@ -104,12 +104,10 @@ struct Scalars
 	unsigned int invalid;
 	unsigned int result_error_bits;
 	unsigned int vertex_error_bits;
-	unsigned int bar[2];          // grid barrier (arrivals, generation)
+	alignas(8) unsigned int bar[4]; // grid barrier words (the pass kernel: two of 64 bits; the position solve: the first)
 	unsigned int grid_error;      // a grid barrier gave up waiting
 	unsigned int rounds;          // decision rounds of the last pass
-	unsigned int act_count[3];    // appended candidates, rotating by round (round r appends to [(r+1)%3])
 	unsigned long long active_sum; // candidates processed by the rounds of the last pass
-	unsigned int carry[3];        // stop-rule prefix (triangles, flips, max error) after a window
 	unsigned int windows;         // sorted-order windows the last pass needed
 	unsigned long long phase_cycles[8]; // kPerform phases, SM cycles of block 0, summed over the run
 	unsigned int trace_count;           // decision rounds traced so far in the run
@@ -1645,10 +1643,10 @@ __device__ __forceinline__ void commitOne(const PerformArgs& a, const uint4& cd,
 // wait: locked at once if a commit of this round took an endpoint, else marked for the next round.
 
 #ifndef MO_RING_LANES
-#define MO_RING_LANES 4
+#define MO_RING_LANES 8
 #endif
 #ifndef MO_RING_BATCH
-#define MO_RING_BATCH 2
+#define MO_RING_BATCH 1
 #endif
 constexpr unsigned int kRingLanes = MO_RING_LANES; // lanes that walk one candidate's one-ring
 constexpr unsigned int kRingBatch = MO_RING_BATCH; // corners per lane in one batch of loads
@@ -1668,10 +1666,11 @@ enum
 // test reads.
 // Bound by dependent L2 round trips: a ring of up to kRingLanes * kRingBatch corners is two of them
 // (its corners, then their marks and positions), and its corners are read side by side. One lane per
-// candidate, two corners at a time, took three or four batches of both: 4 lanes x 2 corners against
-// it, whole calls: 256^2 heightfield 0.92 -> 0.81 ms, 2M attribute sphere 4.36 -> 4.17, 20M terrain
-// 40.4 -> 38.5. 8 x 1: 0.81, 4.22, 39.0; 4 x 1: 0.84, 4.26, 39.2; 2 x 2: 0.87, 4.29, 39.4; 2 x 4
-// (spills): 0.88, 4.61, 43.7.
+// candidate, two corners at a time, took three or four batches of both. Whole calls, 256^2
+// heightfield / 2M attribute sphere / 20M terrain, in ms: one lane 0.92 / 4.36 / 40.4; 8 lanes x 1
+// corner 0.81 / 4.22 / 39.0; 4 x 2 0.82 / 4.20 / 38.5; 4 x 1 0.84 / 4.26 / 39.2; 2 x 4 (spills)
+// 0.88 / 4.61 / 43.7. With the candidates' lists in shared memory and blocks of 512: 8 x 1
+// 0.75 / 4.06 / 38.3, 4 x 2 0.77 / 4.12 / 38.3.
 __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, unsigned int k, const uint4& rec, unsigned int round, unsigned int sub,
     unsigned int mask)
 {
@@ -1981,7 +1980,10 @@ struct PhaseClock
 };
 
 #ifndef MO_PERFORM_THREADS
-#define MO_PERFORM_THREADS 256 // threads per block of the pass kernel
+// threads per block of the pass kernel: fewer blocks arrive at each grid barrier. 256^2 heightfield /
+// 2M attribute sphere / 20M terrain in ms: 256 threads 0.76 / 4.04 / 38.7, 512 0.75 / 4.06 / 38.3,
+// 1024 (4 lanes x 2 corners) 0.81 / 4.33 / 38.7
+#define MO_PERFORM_THREADS 512
 #endif
 #ifndef MO_PERFORM_MIN_BLOCKS
 #define MO_PERFORM_MIN_BLOCKS (1024 / MO_PERFORM_THREADS) // resident blocks per SM the pass kernel is compiled for (64 registers)
@@ -1992,7 +1994,9 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 {
 	__shared__ unsigned int s_app[4];
 	__shared__ unsigned int s_stage[2][kStageChunk]; // candidates passed to stage B, and kept for stage C (wait)
+	__shared__ unsigned int s_list[kStageChunk];     // the block's undecided candidates, once they fit
 	__shared__ unsigned int s_commits;               // this block's commits so far
+	__shared__ unsigned int s_grid[4];
 	__shared__ long long s_clock[10];
 	PhaseClock pc{s_clock};
 	const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
@@ -2027,6 +2031,9 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 		error_limit = lv->error_limit;
 	}
 
+	GridSum grid;
+	grid.start(reinterpret_cast<unsigned long long*>(sc->bar), &sc->grid_error, s_grid);
+
 	// per-vertex state of the pass, streamed: collapse_remap, and both parities of both marks (the
 	// marks the window's candidates set below come after the barrier)
 	for (size_t i = gtid(); i < a.vcount; i += gthreads)
@@ -2036,7 +2043,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 		a.minT[1][i] = ~0ull;
 		reinterpret_cast<ulonglong2*>(a.minS)[i] = make_ulonglong2(~0ull, ~0ull);
 	}
-	gridBarrier(sc->bar, &sc->grid_error);
+	grid.wait();
 
 	unsigned int round = round_base;
 	unsigned long long active_sum = 0;
@@ -2077,34 +2084,31 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 			if (k >= K0 && k < K1)
 				markCandidate(a, k, __ldg(a.cring + c), round + 1);
 		}
-		if (gtid() == 0)
-			sc->act_count[(round + 2) % 3] = 0; // appended to by the window's first round
-		gridBarrier(sc->bar, &sc->grid_error);
+		grid.wait();
 		if (timer)
 			pc.lap(windows == 1 ? kPhInit : kPhMarks);
 
-		// the first round walks the block's tiles and takes the window's candidates among them;
-		// the block keeps the candidates it left undecided in its region of the lists, compacted
-		// with shared-memory atomics, and walks that region in the later rounds; only the
-		// per-round total crosses blocks (one global add per block, read after the barrier)
+		// the first round walks the block's tiles and takes the window's candidates among them; the
+		// block keeps the candidates it left undecided, compacted with shared-memory atomics, in its
+		// region of the lists, or in shared memory once they fit there, and walks those in the later
+		// rounds; only the per-round total crosses blocks, with the round's barrier. The lists in shared
+		// memory and the total in the arrival take three L2 round trips out of a round, and every block
+		// adding up the block totals (below) two barriers out of a pass: 256^2 heightfield 0.82 ->
+		// 0.77 ms, 2M attribute sphere 4.20 -> 4.07.
 		unsigned int nb = tiles * blockDim.x; // this block's undecided candidates (slots in the first round)
 		unsigned int n = K1 - K0;             // all blocks'
-		bool first = true;
+		bool first = true, listed = false;    // listed: the candidates are in s_list
 		unsigned int guard = 0;
-		unsigned int gerr = __ldcg(&sc->grid_error); // read again with each round's total, in one round trip
 		while (n)
 		{
 			++round;
-			if (++guard > count + 1 || gerr)
+			if (++guard > count + 1 || grid.failed())
 				break;
 			active_sum += n;
 			const unsigned int* cur = a.list[round & 1] + region;
-			unsigned int* next = a.list[(round + 1) & 1] + region;
-			unsigned int* next_total = &sc->act_count[(round + 1) % 3];
-			// the total round+1 adds to; every thread read it (as round-2's result) before the
-			// barrier that ended round-1
-			if (gtid() == 0)
-				sc->act_count[(round + 2) % 3] = 0;
+			// survivors go to s_list when one chunk takes all (its old content is read by then)
+			const bool list_next = nb <= kStageChunk;
+			unsigned int* next = list_next ? s_list : a.list[(round + 1) & 1] + region;
 			if (threadIdx.x == 0)
 				s_app[0] = 0;
 			for (unsigned int c0 = 0; c0 < nb; c0 += kStageChunk)
@@ -2126,7 +2130,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 						const unsigned int x = base + q * blockDim.x + threadIdx.x;
 						const unsigned int g = (x - threadIdx.x) * G + blockIdx.x * blockDim.x + threadIdx.x;
 						ok[q] = x < c1 && (!first || g < count);
-						cc[q] = ok[q] ? (first ? g : __ldcg(cur + x)) : 0u;
+						cc[q] = ok[q] ? (first ? g : (listed ? s_list[x] : __ldcg(cur + x))) : 0u;
 					}
 					uint2 ends[kStageItems];
 #pragma unroll
@@ -2223,9 +2227,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 			}
 			__syncthreads(); // the counter's reset is seen when the block had no candidates
 			nb = s_app[0];
-			if (threadIdx.x == 0 && nb)
-				atomicAdd(next_total, nb);
-			gridBarrier(sc->bar, &sc->grid_error);
+			const unsigned int nn = grid.wait(nb);
 			if (timer)
 			{
 				long long before = pc.last();
@@ -2239,19 +2241,18 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 					s_clock[9] = tc + 1;
 				}
 			}
-			const unsigned int nn = __ldcg(next_total);
-			gerr = __ldcg(&sc->grid_error);
 			if (nn >= n)
 			{
 				if (gtid() == 0)
 					atomicOr(&sc->grid_error, 2u);
-				break;
+				return;
 			}
 			n = nn;
 			first = false;
+			listed = list_next;
 		}
-		if (__ldcg(&sc->grid_error))
-			break;
+		if (grid.failed())
+			return;
 
 		// ---- stop rules over [K0, K1): block chunks, thread sub-chunks, carried prefix
 		const unsigned int len = K1 - K0;
@@ -2270,29 +2271,22 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 		uint3 tot = blockScan3(eT, eF, eM, sm);
 		if (threadIdx.x == 0)
 			a.blk[blockIdx.x] = make_uint4(tot.x, tot.y, tot.z, 0);
-		gridBarrier(sc->bar, &sc->grid_error);
-		if (blockIdx.x == 0)
+		grid.wait();
+		// every block adds up the block totals itself: those before it (with the carry of earlier
+		// windows) and, for the next window's carry, all of them
+		unsigned int bT = 0, bF = 0, bM = carryM, wT = 0, wF = 0, wM = carryM;
+		for (unsigned int q = threadIdx.x; q < G; q += blockDim.x)
 		{
-			// exclusive prefix over the block totals with the carry of earlier windows
-			unsigned int rT = carryT, rF = carryF, rM = carryM;
-			for (unsigned int q0 = 0; q0 < G; q0 += blockDim.x)
-			{
-				unsigned int q = q0 + threadIdx.x;
-				uint4 v = q < G ? __ldcg(a.blk + q) : make_uint4(0, 0, 0, 0);
-				unsigned int x = v.x, y = v.y, z = v.z;
-				uint3 ct = blockScan3(x, y, z, sm);
-				if (q < G)
-					a.blk[q] = make_uint4(rT + x, rF + y, max(rM, z), 0);
-				rT += ct.x, rF += ct.y, rM = max(rM, ct.z);
-			}
-			if (threadIdx.x == 0)
-				sc->carry[0] = rT, sc->carry[1] = rF, sc->carry[2] = rM;
+			const uint4 v = __ldcg(a.blk + q);
+			wT += v.x, wF += v.y, wM = max(wM, v.z);
+			if (q < blockIdx.x)
+				bT += v.x, bF += v.y, bM = max(bM, v.z);
 		}
-		gridBarrier(sc->bar, &sc->grid_error);
+		const uint3 bb = blockScan3(bT, bF, bM, sm);
+		const uint3 ww = blockScan3(wT, wF, wM, sm);
 		{
-			uint4 bb = __ldcg(a.blk + blockIdx.x);
-			unsigned long long T = (unsigned long long)bb.x + eT;
-			unsigned long long F = (unsigned long long)bb.y + eF;
+			unsigned long long T = (unsigned long long)carryT + bb.x + eT;
+			unsigned long long F = (unsigned long long)carryF + bb.y + eF;
 			unsigned int M = max(bb.z, eM);
 			const unsigned long long egoal0 = goal / 2;
 			// the error goal moves with the flip count only: the last one read is kept with its
@@ -2328,18 +2322,18 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 				T += tt, F += ff, M = max(M, ee);
 			}
 		}
-		gridBarrier(sc->bar, &sc->grid_error);
+		grid.wait();
 		if (timer)
 			pc.lap(kPhStop);
-		if (__ldcg(&sc->cut) != ~0ull || K1 == count || __ldcg(&sc->grid_error))
+		if (__ldcg(&sc->cut) != ~0ull || K1 == count || grid.failed())
 			break;
-		carryT = __ldcg(&sc->carry[0]);
-		carryF = __ldcg(&sc->carry[1]);
-		carryM = __ldcg(&sc->carry[2]);
+		carryT += ww.x;
+		carryF += ww.y;
+		carryM = ww.z;
 		K0 = K1;
 		K1 = (unsigned int)min((unsigned long long)count, 2ull * K1);
 	}
-	if (__ldcg(&sc->grid_error))
+	if (grid.failed())
 		return;
 
 	// ---- apply the committed prefix. Commits are independent (no two share an endpoint), so
@@ -2386,10 +2380,10 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 				atomicMax(&sc->vertex_error_bits, t2.z);
 		}
 	}
-	gridBarrier(sc->bar, &sc->grid_error);
+	grid.wait();
 	if (timer)
 		pc.lap(kPhApply);
-	if (__ldcg(&sc->done) == 0 || __ldcg(&sc->grid_error))
+	if (__ldcg(&sc->done) == 0 || grid.failed())
 	{
 		if (timer)
 			for (int i = 0; i < 8; ++i)
@@ -2437,34 +2431,26 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	uint3 ktot = blockScan3(ek, d1, d2, sm);
 	if (threadIdx.x == 0)
 		a.blk[blockIdx.x] = make_uint4(ktot.x, 0, 0, 0);
-	gridBarrier(sc->bar, &sc->grid_error);
+	grid.wait();
 	if (timer)
 		pc.lap(kPhLoops);
-	if (blockIdx.x == 0)
+	if (grid.failed())
+		return;
 	{
-		unsigned int run = 0;
-		for (unsigned int q0 = 0; q0 < G; q0 += blockDim.x)
+		unsigned int before = 0, z1 = 0, z2 = 0; // triangles the blocks before this one keep
+		for (unsigned int q = threadIdx.x; q < blockIdx.x; q += blockDim.x)
+			before += __ldcg(&a.blk[q].x);
+		before = blockScan3(before, z1, z2, sm).x;
+		if (threadIdx.x == 0 && blockIdx.x == G - 1)
 		{
-			unsigned int q = q0 + threadIdx.x;
-			unsigned int x = q < G ? __ldcg(&a.blk[q].x) : 0u, y = 0, z = 0;
-			uint3 ct = blockScan3(x, y, z, sm);
-			if (q < G)
-				a.blk[q].y = run + x;
-			run += ct.x;
-		}
-		if (threadIdx.x == 0)
-		{
-			sc->tri_total = run;
+			sc->tri_total = before + ktot.x;
 			sc->rounds = round - round_base;
 			sc->active_sum = active_sum;
 			sc->windows = windows;
 		}
-	}
-	gridBarrier(sc->bar, &sc->grid_error);
-	if (timer)
-		pc.lap(kPhScan);
-	{
-		unsigned int w = __ldcg(&a.blk[blockIdx.x].y) + ek;
+		if (timer)
+			pc.lap(kPhScan);
+		unsigned int w = before + ek;
 		for (unsigned int t = tt0; t < tt1; ++t)
 		{
 			uint3 o;
@@ -2791,8 +2777,8 @@ __global__ void kPassPrep(Scalars* sc)
 	lv.goal = goal;
 	double wf = lv.window_factor * double(goal / 2) + 4096.0;
 	lv.first_window = unsigned(double(C) < wf ? double(C) : wf);
-	sc->bar[0] = 0;
-	sc->bar[1] = 0;
+	for (int i = 0; i < 4; ++i)
+		sc->bar[i] = 0;
 	sc->grid_error = 0;
 	sc->cut = ~0ull;
 	sc->done = 0;
@@ -3296,6 +3282,11 @@ Simplifier::Simplifier(int device) : device_(device)
 	coopScanCapacity(); // cached now: the pass loop's scans may first run while it is recorded
 }
 
+unsigned int Simplifier::performGridCap() const
+{
+	return std::max(1u, unsigned(tuning_.perform_grid_cap) * 256u / kPerformThreads);
+}
+
 void Simplifier::dropLoopGraph()
 {
 	if (loop_.exec)
@@ -3754,7 +3745,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		// grid of the pass kernel
 		unsigned int blocks = std::max(1u, std::min(perform_blocks_, gridFor(std::max(std::max(capn, V), T0), kPerformThreads)));
 		if (tuning_.perform_grid_cap > 0)
-			blocks = std::min(blocks, unsigned(tuning_.perform_grid_cap));
+			blocks = std::min(blocks, performGridCap());
 		if (size_t(blocks) * kPerformThreads > kListSlack)
 			throw std::runtime_error("kPerform grid exceeds the candidate list slack");
 
@@ -3982,14 +3973,14 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 			pa.blk = w.blk;
 			pa.live = nullptr;
 			pa.sc = w.sc;
-			MO_CUDA_CHECK(cudaMemsetAsync(w.sc->bar, 0, sizeof(unsigned int) * 3, stream));
+			MO_CUDA_CHECK(cudaMemsetAsync(w.sc->bar, 0, sizeof(unsigned int) * 5, stream));
 			MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->cut, 0xFF, 8, stream));
 			MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->done, 0, 12, stream));
 			MO_CUDA_CHECK(cudaMemcpyAsync(&w.sc->result_error_bits, &result_error_bits, 4, cudaMemcpyHostToDevice, stream));
 			unsigned int want = gridFor(std::max(std::max(C, V), T), kPerformThreads);
 			unsigned int blocks = std::max(1u, std::min(perform_blocks_, want));
 			if (tuning_.perform_grid_cap > 0)
-				blocks = std::min(blocks, unsigned(tuning_.perform_grid_cap));
+				blocks = std::min(blocks, performGridCap());
 			if (size_t(blocks) * kPerformThreads > kListSlack)
 				throw std::runtime_error("kPerform grid exceeds the candidate list slack");
 			void* params[] = {&pa};
@@ -4106,7 +4097,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 			// co-resident blocks of this kernel (its own register count), as many as the pass kernel's at most
 			unsigned int resident = unsigned(std::max(1, solve_per_sm_ * sms_));
 			unsigned int blocks = std::max(1u, std::min(std::min(perform_blocks_, resident), gV));
-			MO_CUDA_CHECK(cudaMemsetAsync(w.sc->bar, 0, sizeof(unsigned int) * 3, stream));
+			MO_CUDA_CHECK(cudaMemsetAsync(w.sc->bar, 0, sizeof(unsigned int) * 5, stream));
 			void* params[] = {&sa};
 			cudaEvent_t e0 = probeBegin("kSolvePositions", stream);
 			MO_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kSolvePositions, dim3(blocks), dim3(kThreads), params, 0, stream));

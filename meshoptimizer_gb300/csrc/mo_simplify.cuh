@@ -116,10 +116,10 @@ private:
 // MESHOPTGPU_PERFORM_BLOCKS_PER_SM, MESHOPTGPU_WINDOW_FACTOR and MESHOPTGPU_DEVICE_LOOP).
 struct Tuning
 {
-	int perform_blocks_per_sm = 4;  // resident blocks per SM of the cooperative pass kernel
+	int perform_blocks_per_sm = 2;  // resident blocks (512 threads) per SM of the cooperative pass kernel
 	double window_factor = 2.0;     // first decision window = factor * (triangle goal / 2) + 4096
-	int perform_grid_cap = 0;       // at most this many blocks for the pass kernel (0: no cap); lets
-	                                // concurrent simplifications share the GPU
+	int perform_grid_cap = 0;       // at most this many blocks of 256 threads for the pass kernel and the
+	                                // scans (0: no cap); lets concurrent simplifications share the GPU
 	bool device_loop = true;        // run the pass loop as a device-resident CUDA graph (off: one host
 	                                // round trip per pass, needed for per-kernel event timing)
 	static Tuning fromEnvironment();
@@ -179,6 +179,7 @@ private:
 		cudaGraphExec_t exec = nullptr;
 	} loop_;
 	void dropLoopGraph();
+	unsigned int performGridCap() const; // perform_grid_cap in blocks of the pass kernel
 
 public:
 	void setTuning(const Tuning& t)
