@@ -598,7 +598,6 @@ size_t updateHost(unsigned int* indices, size_t index_count, float* vertex_posit
 // ---------------------------------------------------------------- batched path
 
 const size_t kBatchSmemDefault = 104 * 1024;    // shared-memory budget per CTA (two CTAs per SM)
-const unsigned int kMeshletPoolDefault = 0;      // re-clusterization: all per-group arrays in global scratch
 const size_t kBatchSlabTotal = size_t(16) << 30; // global slabs for meshes beyond the budget
 
 struct BatchTuner
@@ -1538,18 +1537,6 @@ int meshoptgpu_simplifyGroups(unsigned int* destination, const unsigned int* ind
 	}
 }
 
-// shared memory per warp of the re-clusterization kernel (MESHOPTGPU_MESHLET_POOL bytes, at
-// most 48 KiB; default below)
-static unsigned int meshletPoolBytes()
-{
-	static const unsigned int bytes = [] {
-		const char* v = getenv("MESHOPTGPU_MESHLET_POOL");
-		long n = v ? atol(v) : long(kMeshletPoolDefault);
-		return unsigned(std::min(std::max(n, 0L), 48L * 1024) & ~15L);
-	}();
-	return bytes;
-}
-
 int meshoptgpu_buildMeshletsFlexGroups(unsigned int* meshlets, unsigned int* meshlet_vertices, unsigned char* meshlet_triangles,
     const size_t* meshlet_offsets, size_t* meshlet_counts, const unsigned int* indices, const size_t* group_offsets, size_t group_count,
     const float* vertex_positions, size_t vertex_count, size_t vertex_positions_stride, size_t max_vertices, size_t min_triangles, size_t max_triangles,
@@ -1602,13 +1589,17 @@ int meshoptgpu_buildMeshletsFlexGroups(unsigned int* meshlets, unsigned int* mes
 		const size_t G = group_count;
 		std::vector<unsigned long long> host((G + 1) * 3, 0);
 		unsigned long long scratch = 0;
+		unsigned int max_index_count = 0;
 		for (size_t g = 0; g <= G; ++g)
 		{
 			host[g] = group_offsets[g];
 			host[(G + 1) + g] = meshlet_offsets[g];
 			host[2 * (G + 1) + g] = scratch;
 			if (g < G)
+			{
 				scratch += meshletScratchBytes(group_offsets[g + 1] - group_offsets[g]);
+				max_index_count = std::max(max_index_count, unsigned(group_offsets[g + 1] - group_offsets[g]));
+			}
 		}
 		const size_t meta = ((host.size() * 8 + 255) / 256) * 256, words = ((G + 1) * 4 + 255) / 256 * 256;
 		char* base = static_cast<char*>(s.meshlet_scratch.ensure(meta + words + scratch + 256));
@@ -1640,7 +1631,7 @@ int meshoptgpu_buildMeshletsFlexGroups(unsigned int* meshlets, unsigned int* mes
 		b.scratch = d_scratch;
 		b.scratch_off = d_meta + 2 * (G + 1);
 		b.error = d_err;
-		b.pool_bytes = meshletPoolBytes();
+		b.max_index_count = max_index_count;
 		b.optimize_level = optimize_level;
 		b.rows = meshlet_offsets[G];
 		buildMeshletsBatch(b, st);

@@ -10,20 +10,33 @@
 //  - group-local vertex ids in first-use order (a hash table keyed by vertex, a warp scan);
 //  - every vertex's triangle list in face order (ranks among equal vertices from match_any, so
 //    corners enter their lists in corner order, as the reference's fill loop does);
-//  - the triangle cones;
-//  - the neighbour search of every step: lanes scan the lists of different meshlet vertices and
-//    a warp reduction picks the smallest (priority, score, scan position), which is the
-//    reference's first best triangle in its scan order. A NaN score breaks that ordering, so a
-//    step that meets one is scanned again by lane 0 alone, in the reference's order;
+//  - the triangle cones; the kd-tree, built only when a step first needs it;
+//  - the neighbour search of every step. The reference scans the live triangle lists of all
+//    meshlet vertices; here the distinct triangles in them are kept as a frontier, and the lanes
+//    score those. The smallest (priority, score) is the reference's first best triangle unless
+//    two tie exactly; then the tied ones' scan positions (meshlet vertex, list entry) decide. A
+//    NaN score breaks that ordering, so a step that meets one is scanned again by lane 0 alone,
+//    in the reference's order;
+//  - the list removals and frontier insertions of the appended triangle;
 //  - each meshlet vertex's best seed neighbour when a meshlet ends.
 // The reference keys its per-vertex arrays by the caller's vertex index; nothing in its result
 // depends on that numbering, only on vertex identity and on the order vertices enter a meshlet,
 // so group-local ids give the same meshlets.
+//
+// A step is a chain of dependent instructions (one issue in 7 cycles per warp, three warps per
+// scheduler), and a level takes about one group's chain, so what counts is the instructions of a
+// step and that every group of a level is resident: the arrays that steps write are packed into
+// shared memory (16-bit ids in groups below 65,535 corners: 13 KB for 512 triangles, 14 groups per
+// SM). 2,048 simplified groups of 512 triangles with the reorder, whole call: 5.84 ms with all
+// meshlet vertices' lists scanned at every step, lane 0 doing the appends and the tree built for
+// every group; 1.48 ms now (1.92 with the lists and the reorder's shifts still on lane 0; 0.1 more
+// with every array in the group's scratch).
 #include "mo_meshlets.cuh"
 #include "mo_common.cuh"
 #include "mo_prims.cuh"
 #include "mo_probe.cuh"
 
+#include <algorithm>
 #include <float.h>
 #include <type_traits>
 
@@ -37,7 +50,14 @@ constexpr unsigned int kMaxSeeds = 256; // kMeshletMaxSeeds, :27
 constexpr unsigned int kAddSeeds = 4;   // kMeshletAddSeeds, :28
 constexpr int kMaxDepth = 50;           // kMeshletMaxTreeDepth, :31
 constexpr unsigned int kLeafSize = 8;   // :1090
-constexpr int kMaxWarpsPerBlock = 4;
+#ifndef MO_FLEX_POOL_MAX
+#define MO_FLEX_POOL_MAX 40960
+#endif
+constexpr size_t kPoolMax = MO_FLEX_POOL_MAX; // shared memory of one group at most
+#ifndef MO_FLEX_TABLE_MAX
+#define MO_FLEX_TABLE_MAX 16384
+#endif
+constexpr size_t kPoolTableMax = MO_FLEX_TABLE_MAX; // ... of its vertex table
 
 struct Cone
 {
@@ -66,45 +86,122 @@ __host__ __device__ inline unsigned int tableSize(unsigned int I)
 	return h;
 }
 
-// one group's scratch, carved from its base in a fixed order (host and device agree)
-struct Scratch
+// per-triangle and per-vertex words of a group, in 16 bits where every id and count fits
+struct Narrow
 {
-	unsigned int *hkey, *hpos, *hid, *slot, *lidx, *gid, *cnt, *off, *fill, *adj, *mvl, *kdidx, *vbest, *seeds;
-	short* used;
-	unsigned char* emitted;
-	Cone* cones;
-	float* area;
-	KDNode* nodes;
+	typedef unsigned short Id;
+	typedef ushort2 Vertex;
+	typedef ushort4 Triangle;
 };
 
-__host__ __device__ inline size_t carve(Scratch& s, char* base, unsigned int I)
+struct Wide
 {
+	typedef unsigned int Id;
+	typedef uint2 Vertex;
+	typedef uint4 Triangle;
+};
+
+// states of a triangle
+enum : unsigned char
+{
+	kTriFree = 0,     // live, not next to the current meshlet
+	kTriFrontier = 1, // live, in the frontier
+	kTriEmitted = 2,
+};
+
+// one group's scratch, carved from its base in a fixed order (host and device agree)
+template <class K>
+struct Scratch
+{
+	typedef typename K::Id Id;
+	unsigned int *hkey, *gid, *vbest, *seeds, *kdrank;
+	Id *hid, *hcnt, *lid, *lpos; // hash table: local id per slot; corners per vertex; per corner: vertex, place in its list
+	Id *adj, *off, *kdidx, *kdtmp;
+	typename K::Vertex* vert;  // {live triangles, index in the current meshlet (all ones: none)}
+	typename K::Triangle* tri; // {vertices}
+	unsigned char* state;      // of each triangle
+	// the frontier, its first kFrontSlots triangles and the others: {vertices, triangle} and apex
+	typename K::Triangle *front, *front_more;
+	float *apex, *apex_more; // apex x of every slot, then y, then z
+	unsigned int more;       // stride of apex_more
+	float *cent, *norm;      // cone apex and axis, 3 floats per triangle
+	float* area;
+	KDNode* nodes;
+	Id* mvl;             // the current meshlet's vertices
+	unsigned char* mtri; // and its triangles, as places among them
+
+	static __device__ __forceinline__ Id none() { return Id(~0u); }
+};
+
+constexpr unsigned int kFrontSlots = 128; // a multiple of the warp; a 128-triangle meshlet's frontier is 20 to 60
+
+// the arrays that steps write, for shared memory (a line of L1 that is stored to is read again from
+// L2, while the arrays that only setup writes stay in L1)
+template <class K>
+__host__ __device__ inline size_t carveHot(Scratch<K>& s, char* base, unsigned int F, unsigned int U)
+{
+	size_t o = 0;
+	auto take = [&](auto*& ptr, size_t count) {
+		if (base)
+			ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(base + o);
+		o += (count * sizeof(*ptr) + 15) & ~size_t(15);
+	};
+	take(s.front, kFrontSlots);
+	take(s.apex, kFrontSlots * 3);
+	take(s.vert, U);
+	take(s.adj, size_t(F) * 3);
+	take(s.tri, F);
+	take(s.state, F);
+	take(s.off, U);
+	return o;
+}
+
+// slots of the vertex table in shared memory, where it fits there before the arrays above
+__host__ __device__ inline unsigned int sharedTableSize(unsigned int I)
+{
+	unsigned int h = 64;
+	while (h < I + I / 4)
+		h *= 2;
+	return h;
+}
+
+template <class K>
+__host__ __device__ inline size_t carve(Scratch<K>& s, char* base, unsigned int I)
+{
+	typedef typename K::Id Id;
 	const unsigned int F = I / 3, H = tableSize(I);
 	size_t o = 0;
-	auto take = [&](size_t bytes) {
-		char* p = base ? base + o : nullptr;
-		o += (bytes + 15) & ~size_t(15);
-		return p;
+	auto take = [&](auto*& ptr, size_t count) {
+		ptr = base ? reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(base + o) : nullptr;
+		o += (count * sizeof(*ptr) + 15) & ~size_t(15);
 	};
-	s.hkey = reinterpret_cast<unsigned int*>(take(size_t(H) * 4));
-	s.hpos = reinterpret_cast<unsigned int*>(take(size_t(H) * 4));
-	s.hid = reinterpret_cast<unsigned int*>(take(size_t(H) * 4));
-	s.slot = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.lidx = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.gid = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.cnt = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.off = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.fill = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.adj = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.mvl = reinterpret_cast<unsigned int*>(take(size_t(I) * 4));
-	s.kdidx = reinterpret_cast<unsigned int*>(take(size_t(F) * 4));
-	s.vbest = reinterpret_cast<unsigned int*>(take(256 * 3 * 4));
-	s.seeds = reinterpret_cast<unsigned int*>(take(kMaxSeeds * 4));
-	s.used = reinterpret_cast<short*>(take(size_t(I) * 2));
-	s.emitted = reinterpret_cast<unsigned char*>(take(F));
-	s.cones = reinterpret_cast<Cone*>(take(size_t(F) * sizeof(Cone)));
-	s.area = reinterpret_cast<float*>(take(size_t(F) * 4));
-	s.nodes = reinterpret_cast<KDNode*>(take(size_t(F) * 2 * sizeof(KDNode)));
+	take(s.hkey, H);
+	take(s.hid, H);
+	take(s.hcnt, I);
+	take(s.lid, I);
+	take(s.lpos, I);
+	take(s.gid, I);
+	take(s.vbest, 256 * 3);
+	take(s.seeds, kMaxSeeds);
+	take(s.kdrank, F);
+	take(s.adj, I);
+	take(s.off, I);
+	take(s.kdidx, F);
+	take(s.kdtmp, F);
+	take(s.vert, I);
+	take(s.tri, F);
+	take(s.state, F);
+	take(s.front, kFrontSlots);
+	take(s.front_more, F);
+	take(s.apex, kFrontSlots * 3);
+	take(s.apex_more, size_t(F) * 3);
+	s.more = F;
+	take(s.cent, size_t(F) * 3);
+	take(s.norm, size_t(F) * 3);
+	take(s.area, F);
+	take(s.nodes, size_t(F) * 2);
+	take(s.mvl, 256);
+	take(s.mtri, 512 * 3);
 	return o;
 }
 
@@ -133,11 +230,13 @@ __device__ __forceinline__ float meshletScore(float distance, float spread, floa
 }
 
 // topology priority of a candidate triangle (:318-335)
-__device__ __forceinline__ int neighborPriority(const Scratch& s, unsigned int t)
+template <class K>
+__device__ __forceinline__ int neighborPriority(const Scratch<K>& s, const typename K::Triangle& t)
 {
-	unsigned int a = s.lidx[t * 3 + 0], b = s.lidx[t * 3 + 1], c = s.lidx[t * 3 + 2];
-	int extra = (s.used[a] < 0) + (s.used[b] < 0) + (s.used[c] < 0);
-	unsigned int la = s.cnt[a], lb = s.cnt[b], lc = s.cnt[c];
+	const typename K::Vertex a = s.vert[t.x], b = s.vert[t.y], c = s.vert[t.z];
+	const typename K::Id no = Scratch<K>::none();
+	int extra = (a.y == no) + (b.y == no) + (c.y == no);
+	unsigned int la = a.x, lb = b.x, lc = c.x;
 	if (extra == 0)
 		return 0;
 	if (la == 1 || lb == 1 || lc == 1)
@@ -147,32 +246,77 @@ __device__ __forceinline__ int neighborPriority(const Scratch& s, unsigned int t
 	return 2 + extra;
 }
 
-__device__ __forceinline__ float neighborScore(const Scratch& s, unsigned int t, const Cone& mc, float cone_weight, float radius)
+// what a step scores triangles with. With a cone weight of 0 the axes cancel out of the score
+// (1 - spread * 0 is 1 for any finite spread), so they are read only otherwise, or where one of the
+// group's is not finite.
+struct ScoreArgs
 {
-	const Cone& tc = s.cones[t];
-	float distance = dist3(tc.px, tc.py, tc.pz, mc.px, mc.py, mc.pz);
-	float spread = tc.nx * mc.nx + tc.ny * mc.ny + tc.nz * mc.nz;
-	return meshletScore(distance, spread, cone_weight, radius);
+	Cone mc;
+	float cone_weight, radius;
+	bool axes;
+};
+
+template <class K>
+__device__ __forceinline__ float neighborScore(const Scratch<K>& s, unsigned int t, float x, float y, float z, const ScoreArgs& a)
+{
+	float distance = dist3(x, y, z, a.mc.px, a.mc.py, a.mc.pz);
+	float spread = 0.f;
+	if (a.axes)
+	{
+		const float* n = s.norm + (size_t)t * 3;
+		spread = n[0] * a.mc.nx + n[1] * a.mc.ny + n[2] * a.mc.nz;
+	}
+	return meshletScore(distance, spread, a.cone_weight, a.radius);
+}
+
+// slot i of the frontier
+template <class K>
+__device__ __forceinline__ typename K::Triangle frontAt(const Scratch<K>& s, unsigned int i, float& x, float& y, float& z)
+{
+	if (i < kFrontSlots)
+	{
+		x = s.apex[i], y = s.apex[kFrontSlots + i], z = s.apex[2 * kFrontSlots + i];
+		return s.front[i];
+	}
+	const float* m = s.apex_more + (i - kFrontSlots);
+	x = m[0], y = m[s.more], z = m[2 * (size_t)s.more];
+	return s.front_more[i - kFrontSlots];
+}
+
+template <class K>
+__device__ __forceinline__ void frontSet(const Scratch<K>& s, unsigned int i, const typename K::Triangle& f, float x, float y, float z)
+{
+	if (i < kFrontSlots)
+	{
+		s.apex[i] = x, s.apex[kFrontSlots + i] = y, s.apex[2 * kFrontSlots + i] = z;
+		s.front[i] = f;
+		return;
+	}
+	float* m = s.apex_more + (i - kFrontSlots);
+	m[0] = x, m[s.more] = y, m[2 * (size_t)s.more] = z;
+	s.front_more[i - kFrontSlots] = f;
 }
 
 // getNeighborTriangle, :302-362, in the reference's scan order (lane 0 only)
-__device__ unsigned int neighborSerial(const Scratch& s, unsigned int voff, unsigned int vcount, const Cone& mc, float cone_weight, float radius)
+template <class K>
+__device__ unsigned int neighborSerial(const Scratch<K>& s, unsigned int vcount, const ScoreArgs& a)
 {
 	unsigned int best = ~0u;
 	int best_priority = 5;
 	float best_score = FLT_MAX;
 	for (unsigned int i = 0; i < vcount; ++i)
 	{
-		unsigned int v = s.mvl[voff + i];
-		const unsigned int* list = s.adj + s.off[v];
-		const unsigned int n = s.cnt[v];
+		unsigned int v = s.mvl[i];
+		const typename K::Id* list = s.adj + s.off[v];
+		const unsigned int n = s.vert[v].x;
 		for (unsigned int j = 0; j < n; ++j)
 		{
 			unsigned int t = list[j];
-			int priority = neighborPriority(s, t);
+			int priority = neighborPriority(s, s.tri[t]);
 			if (priority > best_priority)
 				continue;
-			float score = neighborScore(s, t, mc, cone_weight, radius);
+			const float* c = s.cent + (size_t)t * 3;
+			float score = neighborScore(s, t, c[0], c[1], c[2], a);
 			if (priority < best_priority || score < best_score)
 			{
 				best = t;
@@ -184,63 +328,119 @@ __device__ unsigned int neighborSerial(const Scratch& s, unsigned int voff, unsi
 	return best;
 }
 
-// the same choice by the whole warp: lane l scans the lists of meshlet vertices l, l + 32, ...,
-// then the warp takes the smallest (priority, score, scan position); *nan is set when a score
-// was NaN (the warp's answer is then not the reference's)
-__device__ unsigned int neighborWarp(const Scratch& s, unsigned int voff, unsigned int vcount, const Cone& mc, float cone_weight, float radius, bool* nan)
+// floats (no NaN, no -0) as unsigned integers of the same order
+__device__ __forceinline__ unsigned int orderedBits(float f)
 {
-	const unsigned int lane = threadIdx.x & 31;
-	unsigned int best = ~0u;
-	unsigned long long key = ~0ull; // scan position: (meshlet vertex, list entry)
-	int bp = 5;
-	float bs = FLT_MAX;
-	bool sawnan = false;
-	for (unsigned int i = lane; i < vcount; i += 32)
-	{
-		unsigned int v = s.mvl[voff + i];
-		const unsigned int* list = s.adj + s.off[v];
-		const unsigned int n = s.cnt[v];
-		for (unsigned int j = 0; j < n; ++j)
-		{
-			unsigned int t = list[j];
-			int priority = neighborPriority(s, t);
-			if (priority > bp)
-				continue;
-			float score = neighborScore(s, t, mc, cone_weight, radius);
-			sawnan |= score != score;
-			if (priority < bp || score < bs)
-			{
-				best = t;
-				bp = priority;
-				bs = score;
-				key = ((unsigned long long)i << 32) | j;
-			}
-		}
-	}
-	for (int o = 16; o > 0; o >>= 1)
-	{
-		unsigned int ob = __shfl_xor_sync(0xffffffffu, best, o);
-		unsigned long long ok = __shfl_xor_sync(0xffffffffu, key, o);
-		int op = __shfl_xor_sync(0xffffffffu, bp, o);
-		float os = __shfl_xor_sync(0xffffffffu, bs, o);
-		bool take = op < bp || (op == bp && (os < bs || (os == bs && ok < key)));
-		if (take)
-		{
-			best = ob;
-			bp = op;
-			bs = os;
-			key = ok;
-		}
-	}
-	*nan = __any_sync(0xffffffffu, sawnan);
-	return __shfl_sync(0xffffffffu, best, 0);
+	const unsigned int u = __float_as_uint(f);
+	return u ^ ((unsigned int)((int)u >> 31) | 0x80000000u);
 }
 
-// kdtreeBuild, :532-581, depth first on an explicit stack (lane 0): a subtree's nodes start
-// where the previous one in that order ended, and a right subtree records its distance from its
-// parent when it starts, which is after the whole left subtree
-__device__ void kdBuild(const Scratch& s, unsigned int F, unsigned int* err)
+// The same choice from the frontier by the whole warp; *slot is its place there. *nan is set when a
+// score was NaN (the warp's answer is then not the reference's).
+template <class K>
+__device__ unsigned int neighborWarp(const Scratch<K>& s, unsigned int fn, const ScoreArgs& a, unsigned int* slot, bool* nan)
 {
+	const unsigned int lane = threadIdx.x & 31;
+	unsigned int best = ~0u, at = 0;
+	int bp = 6;
+	float bs = FLT_MAX;
+	bool sawnan = false, tie = false;
+	for (unsigned int i = lane; i < fn; i += 32)
+	{
+		float x, y, z;
+		const typename K::Triangle f = frontAt(s, i, x, y, z);
+		const int priority = neighborPriority(s, f);
+		if (priority > bp)
+			continue;
+		const float score = neighborScore(s, f.w, x, y, z, a) + 0.f;
+		sawnan |= score != score;
+		if (priority < bp || score < bs)
+		{
+			best = f.w;
+			at = i;
+			bp = priority;
+			bs = score;
+			tie = false;
+		}
+		else
+			tie |= score == bs;
+	}
+	// one reduction where the best scores are all in [1, 2^64): then (priority, score) fits a word
+	const unsigned int from1 = __float_as_uint(bs) - 0x3f800000u;
+	unsigned int win;
+	int P;
+	if (__any_sync(0xffffffffu, sawnan || (best != ~0u && from1 >> 29)))
+	{
+		*nan = __any_sync(0xffffffffu, sawnan);
+		P = (int)__reduce_min_sync(0xffffffffu, (unsigned int)bp);
+		const unsigned int key = bp == P && best != ~0u ? orderedBits(bs) : ~0u;
+		const unsigned int least = __reduce_min_sync(0xffffffffu, key);
+		win = __ballot_sync(0xffffffffu, best != ~0u && key == least);
+	}
+	else
+	{
+		*nan = false;
+		const unsigned int key = best != ~0u ? (unsigned int)bp << 29 | from1 : ~0u;
+		const unsigned int least = __reduce_min_sync(0xffffffffu, key);
+		win = __ballot_sync(0xffffffffu, key == least);
+		P = (int)(least >> 29);
+	}
+	if ((win & (win - 1)) || (fn > 32 && __any_sync(0xffffffffu, tie && (win >> lane & 1u))))
+	{
+		const unsigned int Kmin = orderedBits(__shfl_sync(0xffffffffu, bs, __ffs(win) - 1));
+		// several are equally good: the first one in scan order
+		unsigned long long first = ~0ull;
+		for (unsigned int i = lane; i < fn; i += 32)
+		{
+			float px, py, pz;
+			const typename K::Triangle tr = frontAt(s, i, px, py, pz);
+			const unsigned int t = tr.w;
+			if (neighborPriority(s, tr) != P || orderedBits(neighborScore(s, t, px, py, pz, a) + 0.f) != Kmin)
+				continue;
+			const typename K::Vertex va = s.vert[tr.x], vb = s.vert[tr.y], vc = s.vert[tr.z];
+			unsigned int v = tr.x, y = va.y;
+			if (vb.y < y)
+				v = tr.y, y = vb.y;
+			if (vc.y < y)
+				v = tr.z, y = vc.y;
+			const typename K::Id* list = s.adj + s.off[v];
+			unsigned int j = 0;
+			for (const unsigned int n = s.vert[v].x; j < n && list[j] != t; ++j)
+				;
+			const unsigned long long key64 = (unsigned long long)y << 32 | j;
+			if (key64 < first)
+			{
+				first = key64;
+				best = t;
+				at = i;
+			}
+		}
+		unsigned long long m = first;
+		for (int o = 16; o > 0; o >>= 1)
+		{
+			const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
+			m = x < m ? x : m;
+		}
+		const unsigned int w = __ffs(__ballot_sync(0xffffffffu, first == m)) - 1;
+		*slot = __shfl_sync(0xffffffffu, at, w);
+		return __shfl_sync(0xffffffffu, best, w);
+	}
+	const unsigned int w = __ffs(win) - 1;
+	*slot = __shfl_sync(0xffffffffu, at, w);
+	return __shfl_sync(0xffffffffu, best, w);
+}
+
+// kdtreeBuild, :532-581, depth first on an explicit stack, by the whole warp: a subtree's nodes
+// start where the previous one in that order ended, and a right subtree records its distance from
+// its parent when it starts, which is after the whole left subtree. Every lane holds the stack.
+// The statistics run in point order, one axis per lane, on points the warp loads 32 at a time.
+template <class K>
+__device__ void kdBuild(const Scratch<K>& s, unsigned int F, unsigned int* err)
+{
+	typedef typename K::Id Id;
+	// the points in the frontier's memory where they fit: it is empty when the tree is built
+	Id* const points = size_t(F) * sizeof(Id) <= kFrontSlots * sizeof(typename K::Triangle) ? reinterpret_cast<Id*>(s.front) : s.kdidx;
+	const unsigned int lane = threadIdx.x & 31, below = (1u << lane) - 1u;
 	struct Task
 	{
 		unsigned int start, count, parent;
@@ -248,74 +448,136 @@ __device__ void kdBuild(const Scratch& s, unsigned int F, unsigned int* err)
 	} stack[kMaxDepth + 8];
 	int top = 0;
 	stack[top++] = Task{0, F, ~0u, 0};
+	for (unsigned int i = lane; i < F; i += 32)
+		points[i] = Id(i);
+	__syncwarp();
 	unsigned int next = 0;
 	while (top > 0)
 	{
-		Task t = stack[--top];
+		const Task t = stack[--top];
 		const unsigned int offset = next;
-		if (t.parent != ~0u)
+		if (t.parent != ~0u && lane == 0)
 			s.nodes[t.parent].children = offset - t.parent - 1;
-		unsigned int* idx = s.kdidx + t.start;
+		Id* idx = points + t.start;
 		bool leaf = t.count <= kLeafSize;
 		float split = 0.f;
-		int axis = 0;
-		unsigned int middle = 0;
+		unsigned int axis = 0, middle = 0;
 		if (!leaf)
 		{
-			float mean[3] = {0.f, 0.f, 0.f}, vars[3] = {0.f, 0.f, 0.f};
-			float runc = 1, runs = 1;
-			for (unsigned int i = 0; i < t.count; ++i, runc += 1.f, runs = 1.f / runc)
+			// Welford's mean and sum of squares, :544-560: lane k (mod 3) runs axis k
+			const unsigned int k = lane % 3;
+			float mean = 0.f, var = 0.f;
+			for (unsigned int base = 0; base < t.count; base += 32)
 			{
-				const Cone& c = s.cones[idx[i]];
-				const float p[3] = {c.px, c.py, c.pz};
-				for (int k = 0; k < 3; ++k)
+				const unsigned int i = base + lane;
+				const float* c = s.cent + (size_t)(i < t.count ? idx[i] : idx[0]) * 3;
+				const float px = c[0], py = c[1], pz = c[2];
+				const float runs = 1.f / float(i + 1);
+				const unsigned int m = min(32u, t.count - base);
+#pragma unroll 8
+				for (unsigned int j = 0; j < m; ++j)
 				{
-					float delta = p[k] - mean[k];
-					mean[k] += delta * runs;
-					vars[k] += delta * (p[k] - mean[k]);
+					const float x = __shfl_sync(0xffffffffu, px, j), y = __shfl_sync(0xffffffffu, py, j), z = __shfl_sync(0xffffffffu, pz, j);
+					const float r = __shfl_sync(0xffffffffu, runs, j);
+					const float p = k == 0 ? x : (k == 1 ? y : z);
+					float delta = p - mean;
+					mean += delta * r;
+					var += delta * (p - mean);
 				}
 			}
-			axis = (vars[0] >= vars[1] && vars[0] >= vars[2]) ? 0 : (vars[1] >= vars[2] ? 1 : 2);
-			split = mean[axis];
-			// kdtreePartition, :487-506
-			unsigned int m = 0;
-			for (unsigned int i = 0; i < t.count; ++i)
+			const float v0 = __shfl_sync(0xffffffffu, var, 0), v1 = __shfl_sync(0xffffffffu, var, 1), v2 = __shfl_sync(0xffffffffu, var, 2);
+			axis = (v0 >= v1 && v0 >= v2) ? 0 : (v1 >= v2 ? 1 : 2);
+			split = __shfl_sync(0xffffffffu, mean, axis);
+			// kdtreePartition, :487-506, swaps point i with the first point not below the split, for i
+			// in order. Points below it end up in front in order. For the others, let f(j) be the point
+			// at the boundary before step j: step i leaves f(i) in place i and makes f(i + 1) point i
+			// itself, or, when that one is below the split, what step m + 1 left in place m + 1, where m
+			// is the number of points below the split before i: f(i + 1) = f(m + 1).
+			if (t.count <= 32)
 			{
-				const Cone& c = s.cones[idx[i]];
-				float v = axis == 0 ? c.px : (axis == 1 ? c.py : c.pz);
-				unsigned int tmp = idx[m];
-				idx[m] = idx[i];
-				idx[i] = tmp;
-				m += v < split;
+				const bool valid = lane < t.count;
+				const Id x = valid ? idx[lane] : Id(0);
+				const bool less = valid && s.cent[(size_t)x * 3 + axis] < split;
+				const unsigned int bal = __ballot_sync(0xffffffffu, less);
+				middle = __popc(bal);
+				unsigned int j = lane == middle ? t.count : lane;
+				if (lane >= middle && valid)
+					while (bal >> (j - 1) & 1u)
+						j = __popc(bal & ((1u << (j - 1)) - 1u)) + 1;
+				const Id y = Id(__shfl_sync(0xffffffffu, (unsigned int)x, (j - 1) & 31));
+				__syncwarp();
+				if (less)
+					idx[__popc(bal & below)] = x;
+				if (valid && lane >= middle)
+					idx[lane] = y;
+				__syncwarp();
 			}
-			middle = m;
+			else
+			{
+				unsigned int m = 0;
+				for (unsigned int base = 0; base < t.count; base += 32)
+				{
+					const unsigned int i = base + lane;
+					const bool valid = i < t.count;
+					const Id x = valid ? idx[i] : Id(0);
+					const bool less = valid && s.cent[(size_t)x * 3 + axis] < split;
+					const unsigned int bal = __ballot_sync(0xffffffffu, less);
+					const unsigned int rank = m + __popc(bal & below);
+					if (valid)
+						s.kdrank[i] = rank << 1 | (less ? 1u : 0u);
+					if (less)
+						s.kdtmp[rank] = x;
+					m += __popc(bal);
+				}
+				middle = m;
+				__syncwarp();
+				for (unsigned int q = middle + lane; q < t.count; q += 32)
+				{
+					unsigned int j = q == middle ? t.count : q; // the last boundary point, or f(q)
+					for (unsigned int guard = 0; guard <= t.count; ++guard)
+					{
+						const unsigned int r = s.kdrank[j - 1];
+						if (!(r & 1u))
+							break;
+						j = (r >> 1) + 1;
+					}
+					s.kdtmp[q] = idx[j - 1];
+				}
+				__syncwarp();
+				for (unsigned int i = lane; i < t.count; i += 32)
+					idx[i] = s.kdtmp[i];
+				__syncwarp();
+			}
 			leaf = middle <= kLeafSize / 2 || middle >= t.count - kLeafSize / 2 || t.depth >= kMaxDepth;
 		}
 		if (leaf)
 		{
 			// kdtreeBuildLeaf, :508-530
-			s.nodes[offset] = KDNode{idx[0], 3u, t.count};
-			for (unsigned int i = 1; i < t.count; ++i)
-				s.nodes[offset + i] = KDNode{idx[i], 3u, ~0u >> 2};
+			for (unsigned int i = lane; i < t.count; i += 32)
+				s.nodes[offset + i] = KDNode{idx[i], 3u, i ? ~0u >> 2 : t.count};
 			next = offset + t.count;
 			continue;
 		}
-		s.nodes[offset] = KDNode{__float_as_uint(split), unsigned(axis), 0u};
+		if (lane == 0)
+			s.nodes[offset] = KDNode{__float_as_uint(split), axis, 0u};
 		next = offset + 1;
 		if (top + 2 > kMaxDepth + 8)
 		{
-			atomicOr(err, 2u);
-			return;
+			if (lane == 0)
+				atomicOr(err, 2u);
+			break;
 		}
 		stack[top++] = Task{t.start + middle, t.count - middle, offset, t.depth + 1};
 		stack[top++] = Task{t.start, middle, ~0u, t.depth + 1};
 	}
+	__syncwarp();
 }
 
 // kdtreeNearest, :583-639, on an explicit stack in the recursion's order (lane 0): a branch
 // leaves "its second child, if the split is within the best distance then" under its first
 // child; emptied leaves and branches are switched off on the way
-__device__ void kdNearest(const Scratch& s, const float* pos, unsigned int* result, float* limit)
+template <class K>
+__device__ void kdNearest(const Scratch<K>& s, const float* pos, unsigned int* result, float* limit)
 {
 	struct Frame
 	{
@@ -339,11 +601,11 @@ __device__ void kdNearest(const Scratch& s, const float* pos, unsigned int* resu
 			for (unsigned int i = 0; i < node.children; ++i)
 			{
 				unsigned int index = s.nodes[root + i].word;
-				if (s.emitted[index])
+				if (s.state[index] == kTriEmitted)
 					continue;
 				inactive = false;
-				const Cone& c = s.cones[index];
-				float d = dist3(c.px, c.py, c.pz, pos[0], pos[1], pos[2]);
+				const float* c = s.cent + (size_t)index * 3;
+				float d = dist3(c[0], c[1], c[2], pos[0], pos[1], pos[2]);
 				if (d < *limit)
 				{
 					*result = index;
@@ -369,47 +631,98 @@ __device__ void kdNearest(const Scratch& s, const float* pos, unsigned int* resu
 	}
 }
 
-// meshopt_optimizeMeshletLevel (src/meshletutils.cpp:366-554) on one meshlet, by one warp: at
-// every position the scan over the remaining triangles runs 32 at a time (the stop after the
-// level-th edge match found with a ballot, then the first best score up to it), the shift and
-// the bookkeeping on lane 0; 8-bit timestamps and valences wrap as the reference's do
+// kdtreeNearest without the tree: the nearest live triangle, by the whole warp. The search finds a
+// triangle at the smallest distance: a subtree it skips lies beyond a plane further away than the
+// best so far, and rounding keeps that order (no distance is below its own axis difference, which
+// is not below the plane's) while no square over- or underflows. So a single nearest triangle is the
+// search's result; with several equally near ones, or values outside that range (*sure = false),
+// its order decides.
+// A tree cost 0.65M cycles per group of 512 triangles and its search 0.15M; a scan takes 5k.
+constexpr unsigned int kNearestScan = 4096; // triangles of a group at most: above, the tree's search is shorter
+template <class K>
+__device__ unsigned int nearestScan(const Scratch<K>& s, unsigned int F, const Cone& mc, float* distance, bool* sure)
+{
+	const unsigned int lane = threadIdx.x & 31;
+	unsigned int best = ~0u;
+	float bd = FLT_MAX;
+	bool tie = false;
+#pragma unroll 4
+	for (unsigned int t = lane; t < F; t += 32)
+	{
+		if (s.state[t] == kTriEmitted)
+			continue;
+		const float* c = s.cent + (size_t)t * 3;
+		const float d = dist3(c[0], c[1], c[2], mc.px, mc.py, mc.pz);
+		tie = d < bd ? false : (tie || d == bd);
+		if (d < bd)
+		{
+			bd = d;
+			best = t;
+		}
+	}
+	const unsigned int key = __float_as_uint(bd); // not negative
+	const unsigned int least = __reduce_min_sync(0xffffffffu, key);
+	const unsigned int win = __ballot_sync(0xffffffffu, key == least && best != ~0u);
+	*distance = __uint_as_float(least);
+	*sure = (win & (win - 1)) == 0 && !__any_sync(0xffffffffu, tie && (win >> lane & 1u)) && *distance > 1e-15f && fabsf(mc.px) <= 1e15f &&
+	        fabsf(mc.py) <= 1e15f && fabsf(mc.pz) <= 1e15f && win;
+	return win ? __shfl_sync(0xffffffffu, best, __ffs(win) - 1) : ~0u;
+}
+
+// meshopt_optimizeMeshletLevel (src/meshletutils.cpp:366-554) on one meshlet, by one warp. At every
+// position the scan over the remaining triangles runs 32 at a time (the stop after the level-th edge
+// match found with a ballot, then the first best score up to it), and the triangles before the
+// chosen one shift up together; 8-bit timestamps and valences wrap as the reference's do. The
+// rotations and the renumbering need only each vertex's first use, so every triangle is done at once.
 struct MeshletOpt
 {
-	unsigned char idx[512 * 3];
-	unsigned char cache[256];
+	unsigned int tri[512]; // three 8-bit corners
 	unsigned int valence[256];
-	short remap[256];
-	unsigned int order[256];
+	unsigned int first[256];
+	unsigned char cache[256];
 };
+
+__device__ __forceinline__ unsigned int packCorners(unsigned int a, unsigned int b, unsigned int c)
+{
+	return a | b << 8 | c << 16;
+}
 
 __device__ void optimizeMeshletWarp(unsigned int* verts, unsigned char* tris, unsigned int vc, unsigned int tc, int level, MeshletOpt& o)
 {
-	const unsigned int lane = threadIdx.x & 31;
+	const unsigned int lane = threadIdx.x & 31, below = (1u << lane) - 1u;
 	const unsigned char cutoff = 3;
-	for (unsigned int k = lane; k < tc * 3; k += 32)
-		o.idx[k] = tris[k];
 	for (unsigned int v = lane; v < vc; v += 32)
 	{
 		o.cache[v] = 0;
 		o.valence[v] = 0;
+		o.first[v] = ~0u;
 	}
 	__syncwarp();
-	for (unsigned int k = lane; k < tc * 3; k += 32)
-		atomicAdd(&o.valence[o.idx[k]], 1u);
+	for (unsigned int j = lane; j < tc; j += 32)
+	{
+		const unsigned int a = tris[j * 3], b = tris[j * 3 + 1], c = tris[j * 3 + 2];
+		o.tri[j] = packCorners(a, b, c);
+		atomicAdd(&o.valence[a], 1u);
+		atomicAdd(&o.valence[b], 1u);
+		atomicAdd(&o.valence[c], 1u);
+	}
 	__syncwarp();
 	unsigned char cache_last = 128;
 	for (unsigned int i = 0; i < tc; ++i)
 	{
-		int next = -1, next_score = -1, edges = 0;
+		unsigned int next = 0, word = 0;
+		int next_score = -1, edges = 0;
 		bool done = false;
 		for (unsigned int j0 = i; j0 < tc && !done; j0 += 32)
 		{
 			const unsigned int j = j0 + lane;
 			const bool valid = j < tc;
 			int score = -2, match = 0;
+			unsigned int w = 0;
 			if (valid)
 			{
-				unsigned char a = o.idx[j * 3 + 0], b = o.idx[j * 3 + 1], c = o.idx[j * 3 + 2];
+				w = o.tri[j];
+				const unsigned int a = w & 255u, b = w >> 8 & 255u, c = w >> 16;
 				unsigned char ad = (unsigned char)(cache_last - o.cache[a]);
 				unsigned char bd = (unsigned char)(cache_last - o.cache[b]);
 				unsigned char cd = (unsigned char)(cache_last - o.cache[c]);
@@ -438,30 +751,30 @@ __device__ void optimizeMeshletWarp(unsigned int* verts, unsigned char* tris, un
 			}
 			edges += __popc(em & (last == 31 ? 0xffffffffu : ((2u << last) - 1u)));
 			// the first best score among the scanned ones
-			int bs = (valid && lane <= last) ? score : -2;
-			unsigned int bj = (valid && lane <= last) ? j : ~0u;
-			for (int off = 16; off > 0; off >>= 1)
-			{
-				int os = __shfl_xor_sync(0xffffffffu, bs, off);
-				unsigned int oj = __shfl_xor_sync(0xffffffffu, bj, off);
-				if (os > bs || (os == bs && oj < bj))
-					bs = os, bj = oj;
-			}
+			const int mine = valid && lane <= last ? score : -2;
+			const int bs = __reduce_max_sync(0xffffffffu, mine);
 			if (bs > next_score)
 			{
-				next = int(bj);
+				const unsigned int at = __ffs(__ballot_sync(0xffffffffu, mine == bs)) - 1;
+				next = j0 + at;
 				next_score = bs;
+				word = __shfl_sync(0xffffffffu, w, at);
 			}
+		}
+		for (unsigned int top = next; top > i; top = top > i + 32 ? top - 32 : i)
+		{
+			// place p takes the triangle before it
+			const bool moves = top >= lane && top - lane > i;
+			const unsigned int x = moves ? o.tri[top - lane - 1] : 0u;
+			__syncwarp();
+			if (moves)
+				o.tri[top - lane] = x;
+			__syncwarp();
 		}
 		if (lane == 0)
 		{
-			const unsigned int n = unsigned(next);
-			unsigned char a = o.idx[n * 3 + 0], b = o.idx[n * 3 + 1], c = o.idx[n * 3 + 2];
-			for (unsigned int k = n * 3; k > i * 3; --k) // the triangles before it shift forward
-				o.idx[k + 2] = o.idx[k - 1];
-			o.idx[i * 3 + 0] = a;
-			o.idx[i * 3 + 1] = b;
-			o.idx[i * 3 + 2] = c;
+			const unsigned int a = word & 255u, b = word >> 8 & 255u, c = word >> 16;
+			o.tri[i] = word;
 			unsigned char stamp = (unsigned char)(cache_last + 1);
 			o.cache[a] = o.cache[b] = o.cache[c] = stamp;
 			o.valence[a] = (o.valence[a] - 1) & 0xFF;
@@ -471,215 +784,204 @@ __device__ void optimizeMeshletWarp(unsigned int* verts, unsigned char* tris, un
 		cache_last++;
 		__syncwarp();
 	}
-	if (lane == 0)
+	if (level >= 1)
 	{
-		if (level >= 1)
+		// a vertex is seen from its first triangle on; the edges compared below are the same whichever
+		// corner a triangle starts at
+		for (unsigned int i = lane; i < tc; i += 32)
 		{
-			for (unsigned int v = 0; v < vc; ++v)
-				o.cache[v] = 0;
-			for (unsigned int i = 0; i < tc; ++i)
+			const unsigned int w = o.tri[i];
+			atomicMin(&o.first[w & 255u], i);
+			atomicMin(&o.first[w >> 8 & 255u], i);
+			atomicMin(&o.first[w >> 16], i);
+		}
+		__syncwarp();
+		for (unsigned int base = 0; base < tc; base += 32)
+		{
+			const unsigned int i = base + lane;
+			unsigned int w = 0;
+			if (i < tc)
 			{
-				unsigned char a = o.idx[i * 3 + 0], b = o.idx[i * 3 + 1], c = o.idx[i * 3 + 2];
-				if (!o.cache[a] && o.cache[b] && !o.cache[c])
-				{
-					unsigned char t = a;
-					a = b, b = c, c = t;
-				}
-				else if (!o.cache[a] && !o.cache[b] && !o.cache[c])
+				w = o.tri[i];
+				const unsigned int a = w & 255u, b = w >> 8 & 255u, c = w >> 16;
+				const bool sa = o.first[a] < i, sb = o.first[b] < i, sc = o.first[c] < i;
+				if (!sa && sb && !sc)
+					w = packCorners(b, c, a);
+				else if (!sa && !sb && !sc)
 				{
 					bool ab = false, bc = false, ca = false;
 					for (unsigned int j = i + 1; j < tc && j <= i + cutoff; ++j)
 					{
-						unsigned char oa = o.idx[j * 3 + 0], ob = o.idx[j * 3 + 1], oc = o.idx[j * 3 + 2];
+						const unsigned int x = o.tri[j];
+						const unsigned int oa = x & 255u, ob = x >> 8 & 255u, oc = x >> 16;
 						ab |= (oa == b && ob == a) || (ob == b && oc == a) || (oc == b && oa == a);
 						bc |= (oa == c && ob == b) || (ob == c && oc == b) || (oc == c && oa == b);
 						ca |= (oa == a && ob == c) || (ob == a && oc == c) || (oc == a && oa == c);
 					}
 					if (ab && !bc)
-					{
-						unsigned char t = a;
-						a = b, b = c, c = t;
-					}
+						w = packCorners(b, c, a);
 					else if ((ab && !ca) || (!ab && bc && !ca))
-					{
-						unsigned char t = c;
-						c = b, b = a, a = t;
-					}
+						w = packCorners(c, a, b);
 				}
-				o.idx[i * 3 + 0] = a, o.idx[i * 3 + 1] = b, o.idx[i * 3 + 2] = c;
-				o.cache[a] = o.cache[b] = o.cache[c] = 1;
 			}
+			__syncwarp(); // the next triangles of this step were read above
+			if (i < tc)
+				o.tri[i] = w;
+			__syncwarp();
 		}
-		// vertices renumbered in first-use order
-		for (unsigned int v = 0; v < vc; ++v)
-			o.remap[v] = -1;
-		unsigned int n = 0;
-		for (unsigned int k = 0; k < tc * 3; ++k)
-		{
-			short r = o.remap[o.idx[k]];
-			if (r < 0)
-			{
-				r = short(n);
-				o.remap[o.idx[k]] = r;
-				o.order[n++] = verts[o.idx[k]];
-			}
-			o.idx[k] = (unsigned char)r;
-		}
-		for (unsigned int v = 0; v < n; ++v)
-			verts[v] = o.order[v];
 	}
+	// vertices renumbered in first-use order; the valence words now hold the new numbers
+	for (unsigned int v = lane; v < vc; v += 32)
+		o.first[v] = ~0u;
 	__syncwarp();
 	for (unsigned int k = lane; k < tc * 3; k += 32)
-		tris[k] = o.idx[k];
+		atomicMin(&o.first[o.tri[k / 3] >> (k % 3 * 8) & 255u], k);
+	__syncwarp();
+	unsigned int n = 0;
+	unsigned int moved[8]; // this lane's vertices by new number, at most 256 / 32
+#pragma unroll
+	for (int q = 0; q < 8; ++q)
+		moved[q] = 0;
+	for (unsigned int base = 0; base < tc * 3; base += 32)
+	{
+		const unsigned int k = base + lane;
+		const unsigned int v = k < tc * 3 ? o.tri[k / 3] >> (k % 3 * 8) & 255u : 0u;
+		const bool first = k < tc * 3 && o.first[v] == k;
+		const unsigned int m = __ballot_sync(0xffffffffu, first);
+		if (first)
+			o.valence[v] = n + __popc(m & below);
+		n += __popc(m);
+	}
+	__syncwarp();
+#pragma unroll
+	for (int q = 0; q < 8; ++q)
+	{
+		const unsigned int v = q * 32 + lane;
+		if (v < vc && o.first[v] != ~0u)
+			moved[q] = verts[v];
+	}
+	__syncwarp();
+#pragma unroll
+	for (int q = 0; q < 8; ++q)
+	{
+		const unsigned int v = q * 32 + lane;
+		if (v < vc && o.first[v] != ~0u)
+			verts[o.valence[v]] = moved[q];
+	}
+	for (unsigned int k = lane; k < tc * 3; k += 32)
+		tris[k] = (unsigned char)o.valence[o.tri[k / 3] >> (k % 3 * 8) & 255u];
 	__syncwarp();
 }
 
-__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kMeshletsFlex(MeshletBatch b)
+// Group-local vertex ids in first-use order, each corner's id and its place in its vertex's triangle
+// list, and the corners of every vertex; false if there are more than `cap` vertices. A step takes 32
+// corners: the first of each vertex among them finds or enters it in the table.
+template <class K>
+__device__ __forceinline__ bool assignIds(const MeshletBatch& b, const Scratch<K>& s, const unsigned int* indices, unsigned int I, unsigned int* hkey,
+    typename K::Id* hid, typename K::Id* hcnt, unsigned int H, unsigned int cap, unsigned int& U)
 {
-	const unsigned int lane = threadIdx.x & 31;
-	const unsigned int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-	if (g >= b.groups)
-		return;
-	const unsigned long long i0 = b.offsets[g], i1 = b.offsets[g + 1];
-	const unsigned int I = unsigned(i1 - i0) / 3 * 3, F = I / 3;
-	const unsigned int* indices = b.indices + i0;
-	if (F == 0)
+	typedef typename K::Id Id;
+	const unsigned int lane = threadIdx.x, below = (1u << lane) - 1u;
+	for (unsigned int h = lane; h < H; h += 32)
+		hkey[h] = ~0u;
+	__syncwarp();
+	U = 0;
+	unsigned int ahead = lane < I ? indices[lane] : 0u;
+	for (unsigned int base = 0; base < I; base += 32)
 	{
-		if (lane == 0)
-			b.counts[g] = 0;
-		return;
+		const unsigned int p = base + lane;
+		const bool valid = p < I;
+		unsigned int v = ahead;
+		ahead = p + 32 < I ? indices[p + 32] : 0u;
+		if (valid && v >= b.vertex_count)
+		{
+			atomicOr(b.error, 1u);
+			v = 0;
+		}
+		const unsigned int peers = __match_any_sync(0xffffffffu, valid ? v : ~0u); // no vertex is ~0
+		const unsigned int leader = __ffs(peers) - 1;
+		unsigned int h = hashVertex(v) & (H - 1), k = ~0u;
+		if (valid && lane == leader)
+			for (unsigned int probe = 0; probe < H; ++probe)
+			{
+				k = atomicCAS(&hkey[h], ~0u, v);
+				if (k == ~0u || k == v)
+					break;
+				h = (h + 1) & (H - 1);
+			}
+		const bool fresh = valid && lane == leader && k == ~0u;
+		const unsigned int m = __ballot_sync(0xffffffffu, fresh);
+		if (U + __popc(m) > cap)
+			return false;
+		unsigned int id = 0, count = 0;
+		if (valid && lane == leader)
+		{
+			if (fresh)
+			{
+				id = U + __popc(m & below);
+				hid[h] = Id(id);
+				s.gid[id] = v;
+			}
+			else
+			{
+				id = hid[h];
+				count = hcnt[id];
+			}
+			hcnt[id] = Id(count + __popc(peers));
+		}
+		U += __popc(m);
+		id = __shfl_sync(0xffffffffu, id, leader);
+		count = __shfl_sync(0xffffffffu, count, leader);
+		if (valid)
+		{
+			s.lid[p] = Id(id);
+			s.lpos[p] = Id(count + __popc(peers & below));
+		}
+		__syncwarp();
 	}
-	Scratch s;
-	carve(s, b.scratch + b.scratch_off[g], I);
-	const unsigned int H = tableSize(I);
+	return true;
+}
+
+// one group with its ids assigned: everything after
+template <class K>
+__device__ __forceinline__ void buildGroup(const MeshletBatch& b, const Scratch<K>& s, const unsigned long long g, unsigned int I, unsigned int U)
+{
+	typedef typename K::Id Id;
+	typedef typename K::Vertex Vertex;
+	typedef typename K::Triangle Triangle;
+	const unsigned int lane = threadIdx.x;
+	const unsigned int below = (1u << lane) - 1u;
+	const unsigned int F = I / 3;
+	const unsigned long long i0 = b.offsets[g];
 	unsigned int* out = b.meshlets + b.meshlet_base[g] * 4;
 	const unsigned long long out_rows = b.meshlet_base[g + 1] - b.meshlet_base[g];
 	unsigned int* mverts = b.mverts + i0;
 	unsigned char* mtris = b.mtris + i0;
 
-	// ---- group-local vertex ids in first-use order
-	for (unsigned int h = lane; h < H; h += 32)
-	{
-		s.hkey[h] = ~0u;
-		s.hpos[h] = ~0u;
-	}
-	__syncwarp();
-	for (unsigned int p = lane; p < I; p += 32)
-	{
-		unsigned int v = indices[p];
-		if (v >= b.vertex_count)
-		{
-			atomicOr(b.error, 1u);
-			v = 0;
-		}
-		unsigned int h = hashVertex(v) & (H - 1);
-		for (unsigned int probe = 0; probe < H; ++probe)
-		{
-			unsigned int k = atomicCAS(&s.hkey[h], ~0u, v);
-			if (k == ~0u || k == v)
-			{
-				atomicMin(&s.hpos[h], p);
-				s.slot[p] = h;
-				break;
-			}
-			h = (h + 1) & (H - 1);
-		}
-	}
-	__syncwarp();
-	unsigned int U = 0;
-	for (unsigned int base = 0; base < I; base += 32)
-	{
-		const unsigned int p = base + lane;
-		const bool first = p < I && s.hpos[s.slot[p]] == p;
-		const unsigned int m = __ballot_sync(0xffffffffu, first);
-		if (first)
-		{
-			unsigned int id = U + __popc(m & ((1u << lane) - 1u));
-			s.hid[s.slot[p]] = id;
-			unsigned int v = indices[p];
-			s.gid[id] = v < b.vertex_count ? v : 0u;
-		}
-		U += __popc(m);
-	}
-	// the arrays the greedy loop reads at every step move to this warp's shared memory, in the
-	// order of their use per step, while they fit (U is known now)
-	{
-		extern __shared__ __align__(16) char pool[];
-		char* base = pool + (threadIdx.x >> 5) * b.pool_bytes;
-		size_t used_bytes = 0;
-		auto promote = [&](auto*& ptr, size_t bytes) {
-			bytes = (bytes + 15) & ~size_t(15);
-			if (used_bytes + bytes <= b.pool_bytes)
-			{
-				ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(base + used_bytes);
-				used_bytes += bytes;
-			}
-		};
-		promote(s.cnt, size_t(U) * 4);
-		promote(s.off, size_t(U) * 4);
-		promote(s.used, size_t(U) * 2);
-		promote(s.lidx, size_t(I) * 4);
-		promote(s.adj, size_t(I) * 4);
-		promote(s.mvl, size_t(I) * 4);
-		promote(s.emitted, F);
-		promote(s.cones, size_t(F) * sizeof(Cone));
-	}
-	__syncwarp();
-	for (unsigned int p = lane; p < I; p += 32)
-		s.lidx[p] = s.hid[s.slot[p]];
-	for (unsigned int v = lane; v < U; v += 32)
-	{
-		s.cnt[v] = 0;
-		s.fill[v] = 0;
-		s.used[v] = -1;
-	}
-	for (unsigned int t = lane; t < F; t += 32)
-		s.emitted[t] = 0;
-	__syncwarp();
-
 	// ---- triangle lists per vertex, in face order (corner order)
+	const Id none = Scratch<K>::none();
+	bool degenerate = false; // a triangle that names a vertex twice
+	for (unsigned int t = lane; t < F; t += 32)
+	{
+		Triangle tr;
+		tr.x = s.lid[t * 3], tr.y = s.lid[t * 3 + 1], tr.z = s.lid[t * 3 + 2], tr.w = Id(t);
+		s.tri[t] = tr;
+		s.state[t] = kTriFree;
+		degenerate |= tr.x == tr.y || tr.x == tr.z || tr.y == tr.z;
+	}
+	degenerate = __any_sync(0xffffffffu, degenerate);
+	__syncwarp();
 	for (unsigned int p = lane; p < I; p += 32)
-		atomicAdd(&s.cnt[s.lidx[p]], 1u);
-	__syncwarp();
-	{
-		unsigned int run = 0;
-		for (unsigned int base = 0; base < U; base += 32)
-		{
-			const unsigned int v = base + lane;
-			unsigned int c = v < U ? s.cnt[v] : 0u, x = c;
-			for (int o = 1; o < 32; o <<= 1)
-			{
-				unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
-				if (lane >= (unsigned)o)
-					x += y;
-			}
-			if (v < U)
-				s.off[v] = run + x - c;
-			run += __shfl_sync(0xffffffffu, x, 31);
-		}
-	}
-	__syncwarp();
-	for (unsigned int base = 0; base < I; base += 32)
-	{
-		const unsigned int p = base + lane;
-		const bool valid = p < I;
-		const unsigned int v = valid ? s.lidx[p] : (0x80000000u | lane);
-		const unsigned int peers = __match_any_sync(0xffffffffu, v);
-		const unsigned int leader = __ffs(peers) - 1;
-		unsigned int o = 0;
-		if (valid && lane == leader)
-			o = atomicAdd(&s.fill[v], __popc(peers));
-		o = __shfl_sync(0xffffffffu, o, leader);
-		if (valid)
-			s.adj[s.off[v] + o + __popc(peers & ((1u << lane) - 1u))] = p / 3;
-	}
+		s.adj[s.off[s.lid[p]] + s.lpos[p]] = Id(p / 3);
 
 	// ---- triangle cones (computeTriangleCones, :201-241)
+	bool finite = true, small = F <= kNearestScan;
 	for (unsigned int t = lane; t < F; t += 32)
 	{
-		const float* p0 = b.positions + size_t(b.stride_f) * s.gid[s.lidx[t * 3 + 0]];
-		const float* p1 = b.positions + size_t(b.stride_f) * s.gid[s.lidx[t * 3 + 1]];
-		const float* p2 = b.positions + size_t(b.stride_f) * s.gid[s.lidx[t * 3 + 2]];
+		const Triangle tr = s.tri[t];
+		const float* p0 = b.positions + size_t(b.stride_f) * s.gid[tr.x];
+		const float* p1 = b.positions + size_t(b.stride_f) * s.gid[tr.y];
+		const float* p2 = b.positions + size_t(b.stride_f) * s.gid[tr.z];
 		float p10[3] = {p1[0] - p0[0], p1[1] - p0[1], p1[2] - p0[2]};
 		float p20[3] = {p2[0] - p0[0], p2[1] - p0[1], p2[2] - p0[2]};
 		float nx = p10[1] * p20[2] - p10[2] * p20[1];
@@ -687,88 +989,128 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kMeshletsFlex(MeshletB
 		float nz = p10[0] * p20[1] - p10[1] * p20[0];
 		float area = sqrtf(nx * nx + ny * ny + nz * nz);
 		float inv = (area == 0.f) ? 0.f : 1.f / area;
-		Cone c;
-		c.px = (p0[0] + p1[0] + p2[0]) / 3.f;
-		c.py = (p0[1] + p1[1] + p2[1]) / 3.f;
-		c.pz = (p0[2] + p1[2] + p2[2]) / 3.f;
-		c.nx = nx * inv;
-		c.ny = ny * inv;
-		c.nz = nz * inv;
-		s.cones[t] = c;
+		float* c = s.cent + size_t(t) * 3;
+		float* n = s.norm + size_t(t) * 3;
+		c[0] = (p0[0] + p1[0] + p2[0]) / 3.f;
+		c[1] = (p0[1] + p1[1] + p2[1]) / 3.f;
+		c[2] = (p0[2] + p1[2] + p2[2]) / 3.f;
+		n[0] = nx * inv;
+		n[1] = ny * inv;
+		n[2] = nz * inv;
+		finite = finite && fabsf(n[0]) <= FLT_MAX && fabsf(n[1]) <= FLT_MAX && fabsf(n[2]) <= FLT_MAX;
+		small = small && fabsf(c[0]) <= 1e15f && fabsf(c[1]) <= 1e15f && fabsf(c[2]) <= 1e15f;
 		s.area[t] = area;
-		s.kdidx[t] = t;
 	}
+	ScoreArgs sa;
+	sa.cone_weight = b.cone_weight;
+	sa.axes = b.cone_weight != 0.f || __any_sync(0xffffffffu, !finite);
+	const bool tame = __all_sync(0xffffffffu, small); // nearestScan's answers hold
 	__syncwarp();
 
-	// ---- serial setup (lane 0): mesh area in face order, the kd-tree, the corner, the first seed
-	float radius = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-	unsigned int initial = ~0u;
+	// ---- mesh area in face order (lane 0), the corner, the first seed
+	float mesh_area = 0.f;
 	if (lane == 0)
 	{
-		float mesh_area = 0.f;
+#pragma unroll 8
 		for (unsigned int t = 0; t < F; ++t)
 			mesh_area += s.area[t];
 		float tri_area_avg = mesh_area / float(F) * 0.5f;
-		radius = sqrtf(tri_area_avg * float(b.max_triangles)) * 0.5f;
-		kdBuild(s, F, b.error);
-		cx = FLT_MAX, cy = FLT_MAX, cz = FLT_MAX;
-		for (unsigned int t = 0; t < F; ++t)
+		sa.radius = sqrtf(tri_area_avg * float(b.max_triangles)) * 0.5f;
+	}
+	sa.radius = __shfl_sync(0xffffffffu, sa.radius, 0);
+	const float radius = sa.radius;
+	// the smallest of each coordinate, NaN skipped (the sign of a zero does not reach the distances)
+	float cx = FLT_MAX, cy = FLT_MAX, cz = FLT_MAX;
+	for (unsigned int t = lane; t < F; t += 32)
+	{
+		const float* c = s.cent + size_t(t) * 3;
+		cx = cx > c[0] ? c[0] : cx;
+		cy = cy > c[1] ? c[1] : cy;
+		cz = cz > c[2] ? c[2] : cz;
+	}
+	for (int o = 16; o > 0; o >>= 1)
+	{
+		const float x = __shfl_xor_sync(0xffffffffu, cx, o), y = __shfl_xor_sync(0xffffffffu, cy, o), z = __shfl_xor_sync(0xffffffffu, cz, o);
+		cx = cx > x ? x : cx;
+		cy = cy > y ? y : cy;
+		cz = cz > z ? z : cz;
+	}
+	// the first triangle with the smallest distance to it; a NaN first distance keeps triangle 0
+	unsigned int initial = ~0u;
+	{
+		float bd = 0.f;
+		bool nan0 = false;
+		for (unsigned int t = lane; t < F; t += 32)
 		{
-			const Cone& c = s.cones[t];
-			cx = cx > c.px ? c.px : cx;
-			cy = cy > c.py ? c.py : cy;
-			cz = cz > c.pz ? c.pz : cz;
-		}
-		float initial_score = FLT_MAX;
-		for (unsigned int t = 0; t < F; ++t)
-		{
-			const Cone& c = s.cones[t];
-			float d = dist3(c.px, c.py, c.pz, cx, cy, cz);
-			if (initial == ~0u || d < initial_score)
+			const float* c = s.cent + size_t(t) * 3;
+			const float d = dist3(c[0], c[1], c[2], cx, cy, cz);
+			nan0 |= t == 0 && d != d;
+			if (d == d && (initial == ~0u || d < bd))
 			{
 				initial = t;
-				initial_score = d;
+				bd = d;
 			}
 		}
+		const unsigned int key = initial == ~0u ? ~0u : orderedBits(bd);
+		const unsigned int m = __reduce_min_sync(0xffffffffu, key);
+		initial = __reduce_min_sync(0xffffffffu, key == m && initial != ~0u ? initial : ~0u);
+		if (__any_sync(0xffffffffu, nan0) || initial == ~0u)
+			initial = 0;
 	}
-	radius = __shfl_sync(0xffffffffu, radius, 0);
-	cx = __shfl_sync(0xffffffffu, cx, 0);
-	cy = __shfl_sync(0xffffffffu, cy, 0);
-	cz = __shfl_sync(0xffffffffu, cz, 0);
-	initial = __shfl_sync(0xffffffffu, initial, 0);
 	__syncwarp();
 
 	// ---- the greedy loop (:1125-1216); every lane holds the same meshlet state
 	unsigned int m_voff = 0, m_toff = 0, m_vc = 0, m_tc = 0; // the current meshlet
 	unsigned int offset = 0, seed_count = 0;
+	unsigned int fn = 0; // triangles in the frontier
+	bool tree = false;   // the kd-tree is built
 	Cone acc = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-	for (unsigned int step = 0; step <= F; ++step)
+	// the current meshlet's row, vertices and triangles
+	auto writeMeshlet = [&]() {
+		if (offset >= out_rows || m_voff + m_vc > I || m_toff + m_tc * 3 > I)
+		{
+			if (lane == 0)
+				atomicOr(b.error, 4u);
+			return;
+		}
+		if (lane < 4)
+			out[offset * 4 + lane] = lane == 0 ? m_voff : (lane == 1 ? m_toff : (lane == 2 ? m_vc : m_tc));
+		for (unsigned int j = lane; j < m_vc; j += 32)
+			mverts[m_voff + j] = s.gid[s.mvl[j]];
+		for (unsigned int j = lane; j < m_tc * 3; j += 32)
+			mtris[m_toff + j] = s.mtri[j];
+	};
+	for (unsigned int step = 0; step < F; ++step) // with every triangle emitted there is no next one
 	{
 		// getMeshletCone, :181-199
-		Cone mc = acc;
+		sa.mc = acc;
 		{
 			float center_scale = m_tc == 0 ? 0.f : 1.f / float(m_tc);
-			mc.px *= center_scale;
-			mc.py *= center_scale;
-			mc.pz *= center_scale;
-			float len = mc.nx * mc.nx + mc.ny * mc.ny + mc.nz * mc.nz;
-			float axis_scale = len == 0.f ? 0.f : 1.f / sqrtf(len);
-			mc.nx *= axis_scale;
-			mc.ny *= axis_scale;
-			mc.nz *= axis_scale;
+			sa.mc.px *= center_scale;
+			sa.mc.py *= center_scale;
+			sa.mc.pz *= center_scale;
+			if (sa.axes)
+			{
+				float len = sa.mc.nx * sa.mc.nx + sa.mc.ny * sa.mc.ny + sa.mc.nz * sa.mc.nz;
+				float axis_scale = len == 0.f ? 0.f : 1.f / sqrtf(len);
+				sa.mc.nx *= axis_scale;
+				sa.mc.ny *= axis_scale;
+				sa.mc.nz *= axis_scale;
+			}
 		}
-		unsigned int best;
+		unsigned int best = ~0u, slot = ~0u;
 		if (offset == 0 && m_tc == 0)
 			best = initial;
-		else
+		else if (fn)
 		{
 			bool nan = false;
-			best = neighborWarp(s, m_voff, m_vc, mc, b.cone_weight, radius, &nan);
+			best = neighborWarp(s, fn, sa, &slot, &nan);
 			if (nan)
 			{
 				if (lane == 0)
-					best = neighborSerial(s, m_voff, m_vc, mc, b.cone_weight, radius);
+					best = neighborSerial(s, m_vc, sa);
 				best = __shfl_sync(0xffffffffu, best, 0);
+				slot = ~0u;
 			}
 		}
 		bool split = false;
@@ -776,33 +1118,47 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kMeshletsFlex(MeshletB
 		{
 			// no adjacent triangle: the nearest unemitted one (kdtreeNearest)
 			float distance = FLT_MAX;
-			if (lane == 0)
+			bool sure = false;
+			if (tame)
+				best = nearestScan(s, F, sa.mc, &distance, &sure);
+			if (!sure)
 			{
-				const float pos[3] = {mc.px, mc.py, mc.pz};
-				kdNearest(s, pos, &best, &distance);
+				if (!tree)
+					kdBuild(s, F, b.error);
+				tree = true;
+				best = ~0u;
+				distance = FLT_MAX;
+				if (lane == 0)
+				{
+					const float pos[3] = {sa.mc.px, sa.mc.py, sa.mc.pz};
+					kdNearest(s, pos, &best, &distance);
+				}
+				best = __shfl_sync(0xffffffffu, best, 0);
+				distance = __shfl_sync(0xffffffffu, distance, 0);
 			}
-			best = __shfl_sync(0xffffffffu, best, 0);
-			distance = __shfl_sync(0xffffffffu, distance, 0);
 			split = m_tc >= b.min_triangles && b.split_factor > 0 && distance > radius * b.split_factor;
 		}
 		if (best == ~0u)
 			break;
 		__syncwarp();
-		const int best_extra = (s.used[s.lidx[best * 3 + 0]] < 0) + (s.used[s.lidx[best * 3 + 1]] < 0) + (s.used[s.lidx[best * 3 + 2]] < 0);
-		if (split || m_vc + best_extra > b.max_vertices || m_tc >= b.max_triangles)
+		Triangle bt = s.tri[best];
+		Id y0 = s.vert[bt.x].y, y1 = s.vert[bt.y].y, y2 = s.vert[bt.z].y;
+		int extra = (y0 == none) + (y1 == none) + (y2 == none);
+		if (split || m_vc + extra > b.max_vertices || m_tc >= b.max_triangles)
 		{
 			// each meshlet vertex's neighbour with the smallest live count (appendSeedTriangles,
 			// :364-430, inner loop), then the seed bookkeeping in vertex order on lane 0
 			for (unsigned int i = lane; i < m_vc; i += 32)
 			{
-				unsigned int v = s.mvl[m_voff + i];
-				const unsigned int* list = s.adj + s.off[v];
-				const unsigned int n = s.cnt[v];
+				unsigned int v = s.mvl[i];
+				const Id* list = s.adj + s.off[v];
+				const unsigned int n = s.vert[v].x;
 				unsigned int bn = ~0u, bn_live = ~0u;
 				for (unsigned int j = 0; j < n; ++j)
 				{
 					unsigned int t = list[j];
-					unsigned int l = s.cnt[s.lidx[t * 3 + 0]] + s.cnt[s.lidx[t * 3 + 1]] + s.cnt[s.lidx[t * 3 + 2]];
+					const Triangle tr = s.tri[t];
+					unsigned int l = s.vert[tr.x].x + s.vert[tr.y].x + s.vert[tr.z].x;
 					if (l < bn_live)
 					{
 						bn = t;
@@ -812,8 +1168,8 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kMeshletsFlex(MeshletB
 				float score = 0.f;
 				if (bn != ~0u)
 				{
-					const Cone& c = s.cones[bn];
-					score = dist3(c.px, c.py, c.pz, cx, cy, cz);
+					const float* c = s.cent + size_t(bn) * 3;
+					score = dist3(c[0], c[1], c[2], cx, cy, cz);
 				}
 				s.vbest[i * 3 + 0] = bn;
 				s.vbest[i * 3 + 1] = bn_live;
@@ -828,7 +1184,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kMeshletsFlex(MeshletB
 				{
 					unsigned int sd = s.seeds[i];
 					s.seeds[r] = sd;
-					r += s.emitted[sd] == 0;
+					r += s.state[sd] != kTriEmitted;
 				}
 				seed_count = (r + kAddSeeds <= kMaxSeeds) ? r : kMaxSeeds - kAddSeeds;
 				unsigned int bs[kAddSeeds], bl[kAddSeeds];
@@ -864,9 +1220,10 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kMeshletsFlex(MeshletB
 				for (unsigned int i = 0; i < seed_count; ++i)
 				{
 					unsigned int sd = s.seeds[i];
-					unsigned int live = s.cnt[s.lidx[sd * 3 + 0]] + s.cnt[s.lidx[sd * 3 + 1]] + s.cnt[s.lidx[sd * 3 + 2]];
-					const Cone& c = s.cones[sd];
-					float score = dist3(c.px, c.py, c.pz, cx, cy, cz);
+					const Triangle tr = s.tri[sd];
+					unsigned int live = s.vert[tr.x].x + s.vert[tr.y].x + s.vert[tr.z].x;
+					const float* c = s.cent + size_t(sd) * 3;
+					float score = dist3(c[0], c[1], c[2], cx, cy, cz);
 					if (live < blive || (live == blive && score < bscore))
 					{
 						bseed = sd;
@@ -874,137 +1231,297 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kMeshletsFlex(MeshletB
 						bscore = score;
 					}
 				}
-				best = bseed != ~0u ? bseed : best;
+				if (bseed != ~0u && bseed != best)
+				{
+					best = bseed;
+					slot = ~0u;
+				}
 			}
 			best = __shfl_sync(0xffffffffu, best, 0);
+			slot = __shfl_sync(0xffffffffu, slot, 0);
 			seed_count = __shfl_sync(0xffffffffu, seed_count, 0);
+			bt = s.tri[best];
+			y0 = s.vert[bt.x].y, y1 = s.vert[bt.y].y, y2 = s.vert[bt.z].y;
+			extra = (y0 == none) + (y1 == none) + (y2 == none);
 		}
 
-		// appendMeshlet (:243-300), the list removal (:1177-1199) and the emitted flag on lane 0
-		unsigned int reset = 0;
-		if (lane == 0)
+		bool in_front = s.state[best] == kTriFrontier;
+		// appendMeshlet, :243-300
+		if (m_vc + extra > b.max_vertices || m_tc >= b.max_triangles || split)
 		{
-			const unsigned int v3[3] = {s.lidx[best * 3 + 0], s.lidx[best * 3 + 1], s.lidx[best * 3 + 2]};
-			const int extra = (s.used[v3[0]] < 0) + (s.used[v3[1]] < 0) + (s.used[v3[2]] < 0);
-			if (m_vc + extra > b.max_vertices || m_tc >= b.max_triangles || split)
+			writeMeshlet();
+			for (unsigned int j = lane; j < m_vc; j += 32)
+				s.vert[s.mvl[j]].y = none;
+			for (unsigned int i = lane; i < fn; i += 32)
 			{
-				if (offset < out_rows)
-				{
-					out[offset * 4 + 0] = m_voff;
-					out[offset * 4 + 1] = m_toff;
-					out[offset * 4 + 2] = m_vc;
-					out[offset * 4 + 3] = m_tc;
-				}
-				else
-					atomicOr(b.error, 4u);
-				for (unsigned int j = 0; j < m_vc; ++j)
-					s.used[s.mvl[m_voff + j]] = -1;
-				m_voff += m_vc;
-				m_toff += m_tc * 3;
-				m_vc = 0;
-				m_tc = 0;
-				reset = 1;
+				float x, y, z;
+				s.state[frontAt(s, i, x, y, z).w] = kTriFree;
 			}
-			for (int k = 0; k < 3; ++k)
-				if (s.used[v3[k]] < 0)
-				{
-					s.used[v3[k]] = short(m_vc);
-					if (m_voff + m_vc < I)
-					{
-						s.mvl[m_voff + m_vc] = v3[k];
-						mverts[m_voff + m_vc] = s.gid[v3[k]];
-					}
-					else
-						atomicOr(b.error, 4u);
-					m_vc++;
-				}
-			if (m_toff + m_tc * 3 + 2 < I)
-				for (int k = 0; k < 3; ++k)
-					mtris[m_toff + m_tc * 3 + k] = (unsigned char)s.used[v3[k]];
-			else
-				atomicOr(b.error, 4u);
-			m_tc++;
-			// the emitted triangle leaves its vertices' lists (swap with the last)
-			for (int k = 0; k < 3; ++k)
-			{
-				const unsigned int v = v3[k];
-				unsigned int* list = s.adj + s.off[v];
-				const unsigned int n = s.cnt[v];
-				for (unsigned int i = 0; i < n; ++i)
-					if (list[i] == best)
-					{
-						list[i] = list[n - 1];
-						s.cnt[v] = n - 1;
-						break;
-					}
-			}
-			s.emitted[best] = 1;
-			offset += reset;
-		}
-		m_voff = __shfl_sync(0xffffffffu, m_voff, 0);
-		m_toff = __shfl_sync(0xffffffffu, m_toff, 0);
-		m_vc = __shfl_sync(0xffffffffu, m_vc, 0);
-		m_tc = __shfl_sync(0xffffffffu, m_tc, 0);
-		offset = __shfl_sync(0xffffffffu, offset, 0);
-		reset = __shfl_sync(0xffffffffu, reset, 0);
-		if (reset)
+			fn = 0;
+			in_front = false;
+			y0 = y1 = y2 = none;
+			m_voff += m_vc;
+			m_toff += m_tc * 3;
+			m_vc = 0;
+			m_tc = 0;
+			offset++;
 			acc = Cone{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-		const Cone& c = s.cones[best];
-		acc.px += c.px;
-		acc.py += c.py;
-		acc.pz += c.pz;
-		acc.nx += c.nx;
-		acc.ny += c.ny;
-		acc.nz += c.nz;
+			__syncwarp();
+		}
+		const unsigned int v0 = bt.x, v1 = bt.y, v2 = bt.z;
+		const bool n0 = y0 == none, n1 = y1 == none && v1 != v0, n2 = y2 == none && v2 != v0 && v2 != v1;
+		const unsigned int l0 = n0 ? m_vc : y0;
+		const unsigned int l1 = n1 ? m_vc + n0 : (v1 == v0 ? l0 : y1);
+		const unsigned int l2 = n2 ? m_vc + n0 + n1 : (v2 == v0 ? l0 : (v2 == v1 ? l1 : y2));
+		__syncwarp(); // every lane has read the words written below
+		if (lane < 3)
+		{
+			const unsigned int v = lane == 0 ? v0 : (lane == 1 ? v1 : v2), l = lane == 0 ? l0 : (lane == 1 ? l1 : l2);
+			if (lane == 0 ? n0 : (lane == 1 ? n1 : n2))
+			{
+				s.vert[v].y = Id(l);
+				s.mvl[l] = Id(v);
+			}
+			s.mtri[m_tc * 3 + lane] = (unsigned char)l;
+		}
+		m_vc += n0 + n1 + n2;
+		m_tc++;
+		// its place in the frontier: the first triangle that joins takes it, else the last one does
+		if (in_front)
+			for (unsigned int base = 0; base < fn && slot == ~0u; base += 32)
+			{
+				float x, y, z;
+				const unsigned int hit = __ballot_sync(0xffffffffu, base + lane < fn && frontAt(s, base + lane, x, y, z).w == best);
+				if (hit)
+					slot = base + __ffs(hit) - 1;
+			}
+		if (lane == 0)
+			s.state[best] = kTriEmitted;
+		// and its vertices' lists (swap with the last, :1177-1199), and the other live triangles of
+		// vertices new to the meshlet join the frontier: eight lanes per vertex, every entry read once
+		if (!degenerate)
+		{
+			const unsigned int k = lane >> 3;
+			const unsigned int v = k == 0 ? v0 : (k == 1 ? v1 : v2);
+			const bool fresh = k == 0 ? n0 : (k == 1 ? n1 : n2 && k == 2);
+			const unsigned int n = k < 3 ? s.vert[v].x : 0u;
+			Id* list = s.adj + s.off[v];
+			__syncwarp();
+			for (unsigned int j = lane & 7; __any_sync(0xffffffffu, j < n); j += 8)
+			{
+				bool add = false;
+				unsigned int t = 0;
+				Triangle tr;
+				float x = 0.f, y = 0.f, z = 0.f;
+				if (j < n)
+				{
+					t = list[j];
+					if (t == best)
+					{
+						list[j] = list[n - 1];
+						s.vert[v].x = Id(n - 1);
+					}
+					else if (fresh)
+					{
+						// a triangle of two new vertices joins with the first
+						const float* c = s.cent + size_t(t) * 3;
+						tr = s.tri[t];
+						x = c[0], y = c[1], z = c[2];
+						add = s.state[t] == kTriFree && !(k >= 1 && n0 && (tr.x == v0 || tr.y == v0 || tr.z == v0)) &&
+						      !(k == 2 && n1 && (tr.x == v1 || tr.y == v1 || tr.z == v1));
+					}
+				}
+				const unsigned int m = __ballot_sync(0xffffffffu, add);
+				if (m)
+				{
+					const unsigned int r = __popc(m & below);
+					if (add)
+					{
+						frontSet(s, in_front ? (r ? fn + r - 1 : slot) : fn + r, tr, x, y, z);
+						s.state[t] = kTriFrontier;
+					}
+					fn += __popc(m) - in_front;
+					in_front = false;
+				}
+			}
+		}
+		else
+		{
+			// a triangle may name a vertex twice, and its list then holds it twice: in order, one lane
+			__syncwarp();
+			if (lane == 0)
+				for (int k = 0; k < 3; ++k)
+				{
+					const unsigned int v = k == 0 ? v0 : (k == 1 ? v1 : v2);
+					Id* list = s.adj + s.off[v];
+					const unsigned int n = s.vert[v].x;
+					for (unsigned int i = 0; i < n; ++i)
+						if (list[i] == best)
+						{
+							list[i] = list[n - 1];
+							s.vert[v].x = Id(n - 1);
+							break;
+						}
+				}
+			__syncwarp();
+			if (lane == 0)
+				for (int k = 0; k < 3; ++k)
+				{
+					const unsigned int v = k == 0 ? v0 : (k == 1 ? v1 : v2);
+					const Id* list = s.adj + s.off[v];
+					for (unsigned int j = 0, n = (k == 0 ? n0 : (k == 1 ? n1 : n2)) ? s.vert[v].x : 0u; j < n; ++j)
+						if (s.state[list[j]] == kTriFree)
+						{
+							const float* c = s.cent + size_t(list[j]) * 3;
+							frontSet(s, fn++, s.tri[list[j]], c[0], c[1], c[2]);
+							s.state[list[j]] = kTriFrontier;
+						}
+				}
+			fn = __shfl_sync(0xffffffffu, fn, 0);
+		}
+		if (in_front)
+		{
+			--fn;
+			if (lane == 0 && slot != fn)
+			{
+				float x, y, z;
+				const Triangle f = frontAt(s, fn, x, y, z);
+				frontSet(s, slot, f, x, y, z);
+			}
+		}
 		__syncwarp();
+		const float* c = s.cent + size_t(best) * 3;
+		acc.px += c[0];
+		acc.py += c[1];
+		acc.pz += c[2];
+		if (sa.axes)
+		{
+			const float* n = s.norm + size_t(best) * 3;
+			acc.nx += n[0];
+			acc.ny += n[1];
+			acc.nz += n[2];
+		}
+	}
+	if (m_tc)
+	{
+		writeMeshlet();
+		offset++;
 	}
 	if (lane == 0)
-	{
-		if (m_tc)
-		{
-			if (offset < out_rows)
-			{
-				out[offset * 4 + 0] = m_voff;
-				out[offset * 4 + 1] = m_toff;
-				out[offset * 4 + 2] = m_vc;
-				out[offset * 4 + 3] = m_tc;
-			}
-			else
-				atomicOr(b.error, 4u);
-			offset++;
-		}
 		b.counts[g] = offset;
+}
+
+template <class K>
+__global__ void __launch_bounds__(32) kMeshletsFlex(MeshletBatch b, unsigned int pool_bytes)
+{
+	typedef typename K::Id Id;
+	extern __shared__ __align__(16) char pool[];
+	__shared__ Id mvl[256];
+	__shared__ unsigned char mtri[512 * 3];
+	const unsigned int lane = threadIdx.x;
+	const unsigned int g = blockIdx.x;
+	const unsigned long long i0 = b.offsets[g];
+	const unsigned int I = unsigned(b.offsets[g + 1] - i0) / 3 * 3, F = I / 3;
+	const unsigned int* indices = b.indices + i0;
+	if (F == 0)
+	{
+		if (lane == 0)
+			b.counts[g] = 0;
+		return;
+	}
+	Scratch<K> s;
+	carve(s, b.scratch + b.scratch_off[g], I);
+	s.mvl = mvl;
+	s.mtri = mtri;
+
+	// the vertex table in shared memory, before the hot arrays need it, or in the scratch
+	unsigned int U = 0;
+	bool done = false;
+	const unsigned int HS = sharedTableSize(I);
+	if (size_t(HS) * (4 + sizeof(Id)) < pool_bytes)
+	{
+		unsigned int* hkey = reinterpret_cast<unsigned int*>(pool);
+		Id* hid = reinterpret_cast<Id*>(hkey + HS);
+		Id* count = hid + HS;
+		const unsigned int cap = unsigned((pool_bytes - size_t(HS) * (4 + sizeof(Id))) / sizeof(Id));
+		done = assignIds(b, s, indices, I, hkey, hid, count, HS, cap, U);
+		if (done)
+		{
+			__syncwarp();
+			for (unsigned int v = lane; v < U; v += 32)
+				s.hcnt[v] = count[v];
+		}
+		__syncwarp();
+	}
+	if (!done)
+		assignIds(b, s, indices, I, s.hkey, s.hid, s.hcnt, tableSize(I), ~0u, U);
+	__syncwarp();
+	// list offsets and live counts, then the rest, with the arrays a step reads in shared memory
+	// where they fit
+	auto vertices = [&](const Scratch<K>& a) {
+		unsigned int run = 0;
+		for (unsigned int base = 0; base < U; base += 32)
+		{
+			const unsigned int v = base + lane;
+			unsigned int c = v < U ? s.hcnt[v] : 0u, x = c;
+			for (int o = 1; o < 32; o <<= 1)
+			{
+				unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
+				if (lane >= (unsigned)o)
+					x += y;
+			}
+			if (v < U)
+			{
+				a.off[v] = Id(run + x - c);
+				typename K::Vertex w;
+				w.x = Id(c), w.y = Scratch<K>::none();
+				a.vert[v] = w;
+			}
+			run += __shfl_sync(0xffffffffu, x, 31);
+		}
+		__syncwarp();
+	};
+	Scratch<K> hot = s;
+	if (carveHot(hot, pool, F, U) <= pool_bytes)
+	{
+		vertices(hot);
+		buildGroup(b, hot, g, I, U);
+	}
+	else
+	{
+		vertices(s);
+		buildGroup(b, s, g, I, U);
 	}
 }
 
 // meshopt_optimizeMeshletLevel on every meshlet, as clusterize runs it (demo/clusterlod.h:292-300):
 // one warp per meshlet row of the batch; a row past its group's meshlet count has nothing to do
-__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32) kOptimizeMeshlets(MeshletBatch b, unsigned long long rows)
+__global__ void __launch_bounds__(32) kOptimizeMeshlets(MeshletBatch b, unsigned long long rows)
 {
-	__shared__ MeshletOpt opt[kMaxWarpsPerBlock];
-	const unsigned long long r = (unsigned long long)blockIdx.x * kMaxWarpsPerBlock + (threadIdx.x >> 5);
-	if (r >= rows)
-		return;
-	// the group whose rows hold r: the last g with meshlet_base[g] <= r
-	unsigned int lo = 0, hi = b.groups;
-	while (hi - lo > 1)
+	__shared__ MeshletOpt opt;
+	for (unsigned long long r = blockIdx.x; r < rows; r += gridDim.x)
 	{
-		unsigned int mid = (lo + hi) / 2;
-		if (b.meshlet_base[mid] <= r)
-			lo = mid;
-		else
-			hi = mid;
+		// the group whose rows hold r: the last g with meshlet_base[g] <= r
+		unsigned int lo = 0, hi = b.groups;
+		while (hi - lo > 1)
+		{
+			unsigned int mid = (lo + hi) / 2;
+			if (b.meshlet_base[mid] <= r)
+				lo = mid;
+			else
+				hi = mid;
+		}
+		const unsigned int g = lo;
+		const unsigned long long k = r - b.meshlet_base[g];
+		if (k >= b.counts[g])
+			continue;
+		const unsigned long long i0 = b.offsets[g];
+		const unsigned int I = unsigned(b.offsets[g + 1] - i0) / 3 * 3;
+		const unsigned int* row = b.meshlets + r * 4;
+		const unsigned int vo = row[0], to = row[1], vc = row[2], tc = row[3];
+		if (vc <= 256 && tc <= 512 && vo + vc <= I && to + tc * 3 <= I)
+			optimizeMeshletWarp(b.mverts + i0 + vo, b.mtris + i0 + to, vc, tc, b.optimize_level, opt);
 	}
-	const unsigned int g = lo;
-	const unsigned long long k = r - b.meshlet_base[g];
-	if (k >= b.counts[g])
-		return;
-	const unsigned long long i0 = b.offsets[g];
-	const unsigned int I = unsigned(b.offsets[g + 1] - i0) / 3 * 3;
-	const unsigned int* row = b.meshlets + r * 4;
-	const unsigned int vo = row[0], to = row[1], vc = row[2], tc = row[3];
-	if (vc <= 256 && tc <= 512 && vo + vc <= I && to + tc * 3 <= I)
-		optimizeMeshletWarp(b.mverts + i0 + vo, b.mtris + i0 + to, vc, tc, b.optimize_level, opt[threadIdx.x >> 5]);
 }
 
 } // namespace
@@ -1019,20 +1536,40 @@ size_t meshletBound(size_t index_count, size_t max_vertices, size_t max_triangle
 
 size_t meshletScratchBytes(size_t index_count)
 {
-	Scratch s;
+	// the wide layout's, which holds either
+	Scratch<Wide> s;
 	return align256(carve(s, nullptr, unsigned(index_count / 3 * 3)));
+}
+
+template <class K>
+void launchFlex(const MeshletBatch& b, unsigned int pool, cudaStream_t stream)
+{
+	MO_LAUNCH((kMeshletsFlex<K>), b.groups, 32, pool, stream, b, pool);
 }
 
 void buildMeshletsBatch(const MeshletBatch& b, cudaStream_t stream)
 {
 	if (!b.groups)
 		return;
-	// with a shared pool, one warp per block (the pool sets how many fit on an SM); without, four
-	const unsigned int warps = b.pool_bytes ? 1 : kMaxWarpsPerBlock;
-	const unsigned int blocks = (b.groups + warps - 1) / warps;
-	MO_LAUNCH(kMeshletsFlex, blocks, warps * 32, warps * b.pool_bytes, stream, b);
+	const unsigned int F = b.max_index_count / 3;
+	const bool narrow = b.max_index_count < 65535;
+	// shared memory for the largest group's hot arrays, with 3 vertices for 4 triangles (a patch of a
+	// surface has about one for two; a group with more keeps them in its scratch), and for its vertex
+	// table where that is small. Above kPoolMax too few groups would fit an SM.
+	const unsigned int U = F - F / 4 + 3;
+	Scratch<Narrow> sn;
+	Scratch<Wide> sw;
+	size_t want = narrow ? carveHot(sn, nullptr, F, U) : carveHot(sw, nullptr, F, U);
+	const size_t table = sharedTableSize(b.max_index_count) * (narrow ? 6 : 8) + U * (narrow ? 2 : 4) + 16;
+	if (table <= kPoolTableMax)
+		want = std::max(want, table);
+	const unsigned int pool = want <= kPoolMax ? unsigned(want) : 0u;
+	if (narrow)
+		launchFlex<Narrow>(b, pool, stream);
+	else
+		launchFlex<Wide>(b, pool, stream);
 	if (b.optimize_level >= 0 && b.rows)
-		MO_LAUNCH(kOptimizeMeshlets, unsigned((b.rows + kMaxWarpsPerBlock - 1) / kMaxWarpsPerBlock), kMaxWarpsPerBlock * 32, 0, stream, b, b.rows);
+		MO_LAUNCH(kOptimizeMeshlets, unsigned(std::min(b.rows, 0x7fffffffull)), 32, 0, stream, b, b.rows);
 	MO_CUDA_CHECK(cudaGetLastError());
 }
 

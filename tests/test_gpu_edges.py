@@ -64,3 +64,58 @@ def test_update_vertex_orders(port, order, amp, ratio):
     assert np.array_equal(got[0], ref[0])
     assert _same(got[1], ref[1])
     assert not _same(got[1], p)
+
+
+def _meshlet_groups(case):
+    """Groups of the sphere's triangles in file order and the parameters they are cut with."""
+    idx, pos, _, _ = W.octa_sphere(6, seed=9)
+    tri = idx.reshape(-1, 3)
+    if case == "frontier":  # whole strips: frontiers beyond the 128 slots kept in shared memory
+        h, p = W.heightfield(120, seed=3, amp=0.02)
+        return [h[: 3 * 6000], h], p, (256, 100, 512, 0.0, 2.0)
+    if case == "ties":  # a flat lattice: scores and distances tie
+        h, p = W.heightfield(33, seed=3, amp=0.0)
+        return [h, h[::-1].copy()], p, (64, 16, 64, 0.0, 1.0)
+    if case == "islands":  # separate triangles: every step asks for the nearest one
+        pick = tri[np.random.default_rng(3).permutation(len(tri))[:1100]].reshape(-1)
+        return [pick, pick[: 3 * 33], pick[: 3 * 31]], pos, (64, 8, 64, 0.5, 0.0)
+    if case == "doubled":  # each triangle twice, and some that name a vertex twice
+        t = tri[:300].copy()
+        t[::7, 1] = t[::7, 0]
+        return [np.repeat(t, 2, axis=0).reshape(-1)], pos, (96, 20, 96, 0.25, 2.0)
+    if case == "hubs":  # one vertex with hundreds of triangles; more vertices than 3 per 4 triangles
+        n = 700
+        p = np.stack([np.cos(np.arange(n + 1)), np.sin(np.arange(n + 1)), 0.1 * np.cos(3.0 * np.arange(n + 1))], 1).astype(np.float32)
+        fan = np.stack([np.full(n - 1, n), np.arange(n - 1), np.arange(1, n)], 1).astype(np.uint32).reshape(-1)
+        loose = np.arange(699, dtype=np.uint32)
+        return [fan, loose], p, (64, 16, 126, 0.0, 2.0)
+    # "sizes": around the warp, the 128-triangle meshlet, the table and the largest group kept in shared memory
+    cuts = [1, 31, 32, 33, 127, 128, 129, 340, 342, 511, 513, 1023, 1700, 4095, 4097]
+    return [tri[: n].reshape(-1) for n in cuts], pos, (128, 42, 128, 0.0, 2.0)
+
+
+@pytest.mark.parametrize("level", [-1, 0, 1, 9])
+@pytest.mark.parametrize("case", ["frontier", "ties", "islands", "doubled", "hubs", "sizes"])
+def test_meshlet_edges(case, level):
+    import meshlets as ML
+
+    groups, pos, params = _meshlet_groups(case)
+    got = mg.build_meshlets_flex_groups(groups, pos, *params, optimize_level=level)
+    for g, idx in enumerate(groups):
+        m, v, t = ML.build_meshlets_flex(idx, pos, *params, kind="port")
+        if level >= 0:
+            v, t = ML.optimize_meshlets(m, v, t, level, kind="port")
+        for a, b in zip(got[g], (m, v, t)):
+            assert np.array_equal(a, b), f"group {g}"
+
+
+def test_meshlets_wide_group():
+    """One group of more corners than 16-bit ids hold."""
+    import meshlets as ML
+
+    idx, pos = W.heightfield(107, seed=5, amp=0.05)
+    assert len(idx) > 65535
+    (m, v, t), = mg.build_meshlets_flex_groups([idx], pos, 128, 42, 128, 0.0, 2.0, optimize_level=1)
+    rm, rv, rt = ML.build_meshlets_flex(idx, pos, 128, 42, 128, 0.0, 2.0, kind="port")
+    rv, rt = ML.optimize_meshlets(rm, rv, rt, 1, kind="port")
+    assert np.array_equal(m, rm) and np.array_equal(v, rv) and np.array_equal(t, rt)
