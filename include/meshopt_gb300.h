@@ -240,26 +240,25 @@ MESHOPTGPU_API void meshoptgpu_setBatchConfig(int threads, unsigned int smem_byt
  * kernel, above 98304 the single-mesh path, and in between whichever the first repeatable call
  * of the size class timed faster on its own mesh. 0 sends every call to the single-mesh path.
  *
- * The single-mesh path's launch shape (pass-kernel blocks per SM, the pass sort's tile) is
- * autotuned the same way, per size class of the mesh: the first repeatable call (destination
- * not aliasing indices, no update mode, Prune or debug bit) times the candidates on its own
- * mesh. MESHOPTGPU_AUTOTUNE=0 in the environment turns both tuners off (fixed defaults). */
+ * The single-mesh path's launch shape (pass-kernel blocks per SM) is autotuned the same way, per
+ * size class of the mesh: the first repeatable call (destination not aliasing indices, no update
+ * mode, Prune or debug bit) times the candidates on its own mesh. MESHOPTGPU_AUTOTUNE=0 in the
+ * environment turns both tuners off (fixed defaults). */
 MESHOPTGPU_API void meshoptgpu_setDropinBatchLimit(size_t max_index_count);
 
 /* The autotuner's choices for meshes of index_count indices (with attributes or not), on the
- * current device: out4[0] pass-kernel blocks per SM, out4[1] pass sort candidates per thread
- * (0: chosen by count), out4[2] drop-in route (1 batch kernel, 0 single-mesh path, -1 not
+ * current device: out4[0] pass-kernel blocks per SM, out4[1] 0 (the pass sort's tile follows the
+ * candidate count), out4[2] drop-in route (1 batch kernel, 0 single-mesh path, -1 not
  * tuned), out4[3] the batch kernel's shared-memory budget (KiB) for the largest size class
  * tuned so far (0: none). Returns 1 if the single-mesh shape is tuned for that size class. */
 MESHOPTGPU_API int meshoptgpu_getTuning(size_t index_count, size_t attribute_count, int* out4);
 
-/* The single-mesh path runs its pass loop (src/simplifier.cpp:2493-2541) on the device: one
- * pass is recorded into a CUDA graph as the body of a WHILE conditional node and replayed
- * until the loop ends, with no host round trip between passes. enabled = 0 switches the
- * calling thread to the host-driven loop (one host read per pass), which per-launch kernel
- * timing (meshoptgpu_setKernelProfile) needs. Pruning, the debug bit and
- * meshoptgpu_setTiming(1) always use the host loop. Results are identical. Returns a
- * meshoptgpu_Status* value. */
+/* The single-mesh path runs its pass loop (src/simplifier.cpp:2493-2541) on the device, in one
+ * cooperative launch whose phases grid barriers separate, with no host round trip between passes
+ * (one per pruning, which the host runs between passes). enabled = 0 switches the calling thread
+ * to the host-driven loop (a launch per phase, two host reads per pass), which per-launch kernel
+ * timing (meshoptgpu_setKernelProfile) needs. The debug bit and meshoptgpu_setTiming(1) always
+ * use the host loop. Results are identical. Returns a meshoptgpu_Status* value. */
 MESHOPTGPU_API int meshoptgpu_setDeviceLoop(int enabled);
 MESHOPTGPU_API int meshoptgpu_getBatchThreads(void);
 

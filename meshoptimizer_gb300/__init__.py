@@ -319,8 +319,8 @@ def last_pass_phase_times():
 
 
 def tuning(index_count, attribute_count=0):
-    """The autotuner's choices for meshes of index_count indices: pass-kernel blocks per SM, pass
-    sort candidates per thread (0: by count), drop-in route (batch / single / None) and the batch
+    """The autotuner's choices for meshes of index_count indices: pass-kernel blocks per SM, 0 (the
+    pass sort's tile follows the count), drop-in route (batch / single / None) and the batch
     kernel's shared-memory budget in KiB (largest size class tuned so far); None if untuned."""
     out = (C.c_int * 4)()
     found = load().meshoptgpu_getTuning(int(index_count), int(attribute_count), C.cast(out, C.c_void_p))
@@ -611,7 +611,7 @@ def probe_barrier_wait(once=False, blocks=8, wait_limit=4096):
 
 
 def set_device_loop(enabled=True):
-    """Pass loop of the single-mesh path on the device (CUDA graph, default) or driven by the host."""
+    """Pass loop of the single-mesh path on the device (one launch, default) or driven by the host."""
     return int(load().meshoptgpu_setDeviceLoop(1 if enabled else 0))
 
 

@@ -852,8 +852,7 @@ bool smallMeshOnBatch(ThreadState& s, const MeshDesc& m, unsigned int* d_out, cu
 // Prune or debug bit) times the candidates on the call's own mesh and keeps the fastest for the
 // class; the results are identical whatever the choice, so the call returns the last candidate's.
 // Later calls of the class take the choice. Tuned:
-//  * the pass kernels' launch shape: pass-kernel blocks per SM (the resident maximum and one and
-//    two fewer), then the pass sort's tile (4, 8 or 16 candidates per thread) at the best;
+//  * the pass kernels' launch shape: blocks per SM, one or two;
 //  * the drop-in route for meshes between kDropinBatchAlways and kDropinSingleAlways indices: the
 //    batch kernel (one CTA does the whole mesh) or the single-mesh path (multi-CTA pass loop).
 constexpr size_t kTuneMinIndices = 3000;       // below: the default shape (nothing to gain)
@@ -864,7 +863,7 @@ constexpr size_t kDropinDefault = 15000;       // the route of calls that cannot
 struct ShapeTuner
 {
 	std::mutex lock;
-	std::map<std::tuple<int, int, int>, std::pair<int, unsigned int>> shape; // -> (blocks per SM, sort items)
+	std::map<std::tuple<int, int, int>, int> shape;  // -> blocks per SM
 	std::map<std::tuple<int, int, int>, bool> batch;                         // -> batch kernel faster
 } g_shapes;
 
@@ -915,41 +914,30 @@ void runSingle(ThreadState& s, const MeshDesc& m, unsigned int* d_out, cudaStrea
 		auto it = g_shapes.shape.find(key);
 		if (it != g_shapes.shape.end())
 		{
-			sp.setPassShape(it->second.first, it->second.second);
+			sp.setPassShape(it->second);
 			s.last = sp.run(m, d_out, st, s.timing ? &s.times : nullptr);
 			return;
 		}
 	}
-	const int top = std::max(1, sp.performBlocksPerSMMax());
 	if (!repeatable(s, m, d_out) || m.index_count < kTuneMinIndices)
 	{
-		sp.setPassShape(top, 0);
+		sp.setPassShape(0);
 		s.last = sp.run(m, d_out, st, s.timing ? &s.times : nullptr);
 		return;
 	}
 	const int reps = 2; // the faster of two runs per candidate
-	auto trial = [&](int bps, unsigned int items) {
-		sp.setPassShape(bps, items);
-		return timedMs(st, [&]() { s.last = sp.run(m, d_out, st); }, reps);
-	};
-	int best_bps = top;
+	int best_bps = 1;
 	float best = 1e30f;
-	for (int bps = top; bps >= std::max(1, top - 2); --bps)
+	for (int bps = std::max(1, sp.performBlocksPerSMMax()); bps >= 1; --bps)
 	{
-		const float ms = trial(bps, 0);
+		sp.setPassShape(bps);
+		const float ms = timedMs(st, [&]() { s.last = sp.run(m, d_out, st); }, reps);
 		if (ms < best)
 			best = ms, best_bps = bps;
 	}
-	unsigned int best_items = 0;
-	for (unsigned int items : {4u, 8u, 16u})
-	{
-		const float ms = trial(best_bps, items);
-		if (ms < best)
-			best = ms, best_items = items;
-	}
-	sp.setPassShape(best_bps, best_items);
+	sp.setPassShape(best_bps);
 	std::lock_guard<std::mutex> g(g_shapes.lock);
-	g_shapes.shape[key] = std::make_pair(best_bps, best_items);
+	g_shapes.shape[key] = best_bps;
 }
 
 size_t singlePathAbove(const ThreadState& s)
@@ -1186,10 +1174,6 @@ void largeWorker(ServerImpl* S)
 		ts.ensure();
 		Tuning t = ts.simplifier->tuning();
 		t.perform_grid_cap = S->cfg.perform_blocks;
-		// requests come in every shape, so a recorded pass graph is never replayed for a second
-		// request, and concurrent workers instantiating graphs contend in the driver: the
-		// single-mesh workers drive their pass loops from the host
-		t.device_loop = false;
 		ts.simplifier->setTuning(t);
 	}
 	catch (const std::exception& e)
@@ -1961,8 +1945,8 @@ int meshoptgpu_getTuning(size_t index_count, size_t attribute_count, int* out4)
 		auto it = g_shapes.shape.find(key);
 		if (it != g_shapes.shape.end())
 		{
-			out4[0] = it->second.first;
-			out4[1] = int(it->second.second);
+			out4[0] = it->second;
+			out4[1] = 0;
 			found = 1;
 		}
 		auto jt = g_shapes.batch.find(key);

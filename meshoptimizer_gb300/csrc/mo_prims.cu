@@ -43,11 +43,9 @@ __global__ void __launch_bounds__(kScanThreads) kScanReduce(const unsigned int* 
 }
 
 __global__ void __launch_bounds__(kScanThreads) kScanApply(const unsigned int* in, unsigned int* out, size_t n, const unsigned int* __restrict__ tileoffs,
-    unsigned int* total, bool aligned, const unsigned int* n_dev = nullptr)
+    unsigned int* total, bool aligned)
 {
 	__shared__ unsigned int smem[kScanThreads / 32 + 1];
-	if (n_dev && *n_dev < n)
-		n = *n_dev;
 	size_t i = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
 	uint4 v = loadTile4(in, n, i, aligned);
 	unsigned int s = v.x + v.y + v.z + v.w;
@@ -81,11 +79,9 @@ __global__ void __launch_bounds__(kScanThreads) kScanApply(const unsigned int* i
 // sums[b]; after the grid barrier each block adds up the sums before it and scans its tiles
 // again, writing the prefixes. in and out may alias: a block writes only elements it has read.
 __global__ void __launch_bounds__(kScanThreads) kScanCoop(const unsigned int* in, unsigned int* out, size_t n, unsigned int* total,
-    unsigned int* sums, unsigned int* bar, unsigned int* err, bool aligned, const unsigned int* n_dev)
+    unsigned int* sums, unsigned int* bar, unsigned int* err, bool aligned)
 {
 	__shared__ unsigned int smem[kScanThreads / 32 + 1];
-	if (n_dev && *n_dev < n)
-		n = *n_dev; // the live count; the grid covers n
 	const size_t tiles = (n + kScanTile - 1) / kScanTile;
 	const size_t per = (tiles + gridDim.x - 1) / gridDim.x;
 	const size_t t0 = min(tiles, (size_t)blockIdx.x * per), t1 = min(tiles, t0 + per);
@@ -149,14 +145,12 @@ void scanLevel(const unsigned int* in, unsigned int* out, size_t n, unsigned int
 	bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
 	if (tiles <= 1)
 	{
-		MO_LAUNCH(kScanApply, 1, kScanThreads, 0, stream, in, out, n, nullptr, total, aligned, sync.n_dev);
+		MO_LAUNCH(kScanApply, 1, kScanThreads, 0, stream, in, out, n, nullptr, total, aligned);
 		return;
 	}
 	unsigned int cap = sync.bar ? coopScanCapacity() : 0u;
 	if (cap && sync.max_blocks)
 		cap = std::min(cap, sync.max_blocks);
-	if (sync.n_dev && !cap)
-		throw std::invalid_argument("scanExclusive: a device-side count needs the single-launch mode");
 	if (cap)
 	{
 		// consecutive tiles per block, then as few blocks as that needs
@@ -164,8 +158,7 @@ void scanLevel(const unsigned int* in, unsigned int* out, size_t n, unsigned int
 		const unsigned int blocks = unsigned((tiles + per - 1) / per);
 		unsigned int* sums = scratch;
 		cudaEvent_t e0 = probeBegin("kScanCoop", stream);
-		void* params[] = {(void*)&in, (void*)&out, (void*)&n, (void*)&total, (void*)&sums, (void*)&sync.bar, (void*)&sync.err, (void*)&aligned,
-		                  (void*)&sync.n_dev};
+		void* params[] = {(void*)&in, (void*)&out, (void*)&n, (void*)&total, (void*)&sums, (void*)&sync.bar, (void*)&sync.err, (void*)&aligned};
 		MO_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kScanCoop, dim3(blocks), dim3(kScanThreads), params, 0, stream));
 		probeEnd(e0, stream);
 		return;
@@ -176,20 +169,10 @@ void scanLevel(const unsigned int* in, unsigned int* out, size_t n, unsigned int
 	MO_LAUNCH(kScanApply, (unsigned)tiles, kScanThreads, 0, stream, in, out, n, sums, total, aligned);
 }
 
-// n_dev (optional): the live element count on the device, at most n; the grid covers n
-__device__ __forceinline__ size_t liveCount(size_t n, const unsigned int* n_dev)
-{
-	if (!n_dev)
-		return n;
-	size_t d = *n_dev;
-	return d < n ? d : n;
-}
-
-__global__ void __launch_bounds__(kSortThreads) kRadixHist(const unsigned int* __restrict__ keys, size_t n, const unsigned int* n_dev, int shift,
+__global__ void __launch_bounds__(kSortThreads) kRadixHist(const unsigned int* __restrict__ keys, size_t n, int shift,
     unsigned int* __restrict__ hist, unsigned int tiles)
 {
 	__shared__ unsigned int sh[kSortBins];
-	n = liveCount(n, n_dev);
 	sh[threadIdx.x] = 0;
 	__syncthreads();
 	size_t base = (size_t)blockIdx.x * kSortTile + threadIdx.x;
@@ -215,11 +198,10 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortWarpSpan = kSortTile / kSortWarps; // consecutive elements per warp
 
 __global__ void __launch_bounds__(kSortThreads, 5) kRadixScatter(const unsigned int* __restrict__ kin, const unsigned int* __restrict__ vin,
-    unsigned int* __restrict__ kout, unsigned int* __restrict__ vout, size_t n, const unsigned int* n_dev, int shift, const unsigned int* __restrict__ hist,
+    unsigned int* __restrict__ kout, unsigned int* __restrict__ vout, size_t n, int shift, const unsigned int* __restrict__ hist,
     unsigned int tiles)
 {
 	// vin == nullptr stands for the identity values 0..n-1
-	n = liveCount(n, n_dev);
 	__shared__ unsigned int lbase[kSortBins];              // tile-local start per digit
 	__shared__ unsigned int gbase[kSortBins];              // global position of the tile's first element per digit
 	__shared__ unsigned int wcnt[kSortWarps][kSortBins];   // per warp and digit: count, then offset within the digit
@@ -440,21 +422,18 @@ __global__ void __launch_bounds__(kSmallSortThreads) kSmallSortPairs(const unsig
 }
 
 void radixSortPairs(const unsigned int* keys_in, const unsigned int* vals_in, unsigned int* keys_out, unsigned int* vals_out,
-    unsigned int* keys_tmp, unsigned int* vals_tmp, size_t n, int bits, unsigned int* scratch, cudaStream_t stream, const unsigned int* n_dev,
-    ScanSync sync)
+    unsigned int* keys_tmp, unsigned int* vals_tmp, size_t n, int bits, unsigned int* scratch, cudaStream_t stream, ScanSync sync)
 {
 	if (n == 0)
 		return;
 	int passes = (bits + 7) / 8;
 	if (passes == 0)
 	{
-		if (n_dev)
-			throw std::invalid_argument("radixSortPairs: a device count needs at least one digit pass");
 		MO_CUDA_CHECK(cudaMemcpyAsync(keys_out, keys_in, n * 4, cudaMemcpyDeviceToDevice, stream));
 		MO_CUDA_CHECK(cudaMemcpyAsync(vals_out, vals_in, n * 4, cudaMemcpyDeviceToDevice, stream));
 		return;
 	}
-	if (!n_dev && n <= kSmallSortMax)
+	if (n <= kSmallSortMax)
 	{
 		const unsigned int mask = passes >= 4 ? ~0u : (1u << (8 * passes)) - 1u;
 		MO_LAUNCH(kSmallSortPairs, 1, kSmallSortThreads, 0, stream, keys_in, vals_in, keys_out, vals_out, (unsigned int)n, mask);
@@ -473,9 +452,9 @@ void radixSortPairs(const unsigned int* keys_in, const unsigned int* vals_in, un
 		unsigned int* kd = to_out ? keys_out : keys_tmp;
 		unsigned int* vd = to_out ? vals_out : vals_tmp;
 		int shift = p * 8;
-		MO_LAUNCH(kRadixHist, tiles, kSortThreads, 0, stream, ks, n, n_dev, shift, hist, tiles);
+		MO_LAUNCH(kRadixHist, tiles, kSortThreads, 0, stream, ks, n, shift, hist, tiles);
 		scanExclusive(hist, hist, size_t(tiles) * kSortBins, nullptr, sscratch, stream, sync);
-		MO_LAUNCH(kRadixScatter, tiles, kSortThreads, 0, stream, ks, vs, kd, vd, n, n_dev, shift, hist, tiles);
+		MO_LAUNCH(kRadixScatter, tiles, kSortThreads, 0, stream, ks, vs, kd, vd, n, shift, hist, tiles);
 		ks = kd;
 		vs = vd;
 	}

@@ -88,8 +88,6 @@ struct ScanSync
 	unsigned int* err = nullptr;
 	unsigned int max_blocks = 0; // at most this many blocks (0: as many as are resident at once), so
 	                             // concurrent callers on other streams can be resident beside it
-	const unsigned int* n_dev = nullptr; // optional: the live element count on the device (at most n),
-	                                     // read by the kernels; needs the single-launch mode
 };
 
 // Runs the grid barrier (once != 0: the single-use one) with one of `blocks` blocks never
@@ -98,7 +96,7 @@ struct ScanSync
 unsigned int probeBarrierWait(int once, unsigned int blocks, unsigned int limit, cudaStream_t stream);
 
 // Blocks a single-launch scan may use on the current device (all resident at once); queried
-// once per device and cached. Call it outside stream capture before the first such scan.
+// once per device and cached.
 unsigned int coopScanCapacity();
 
 // out[i] = sum(in[0..i)) for i < n; if total != nullptr, *total (device) = sum(in[0..n)).
@@ -113,13 +111,11 @@ size_t radixScratchWords(size_t n);
 // the values 0..n-1. Sorted result ends in
 // (keys_out, vals_out); keys_tmp/vals_tmp are ping-pong buffers of n elements. Input
 // arrays are left unchanged only when the pass count is even; callers treat them as scratch.
-// n_dev (optional): the live count on the device (<= n), read by the kernels, so that the
-// launches can be recorded once and replayed for any count up to n. Up to 4,096 pairs with a
-// host count sort in one single-block launch instead of the digit passes (the same order).
+// Up to 4,096 pairs sort in one single-block launch instead of the digit passes (the same order).
 // The outputs must not alias the inputs.
 void radixSortPairs(const unsigned int* keys_in, const unsigned int* vals_in, unsigned int* keys_out, unsigned int* vals_out,
     unsigned int* keys_tmp, unsigned int* vals_tmp, size_t n, int bits, unsigned int* scratch, cudaStream_t stream,
-    const unsigned int* n_dev = nullptr, ScanSync sync = ScanSync());
+    ScanSync sync = ScanSync());
 
 inline unsigned int gridFor(size_t n, int threads)
 {

@@ -45,27 +45,16 @@ constexpr size_t kPinnedBytes = 16384; // host readback buffer of the scalars bl
 constexpr unsigned int kStageChunk = MO_STAGE_CHUNK; // candidates of a block taken through the decision stages at a time
 constexpr unsigned int kStageItems = MO_STAGE_ITEMS; // candidates per thread in the first decision stage
 
-// State of the device-resident pass loop: the counts each pass's kernels read instead of
-// launch parameters, so that one recorded pass can be replayed until the loop ends.
-struct PassLive
+// Where kPassLoop left the pass loop.
+struct LoopState
 {
-	const unsigned int* res;  // current index buffer
-	unsigned int* res_next;   // the next pass's
-	unsigned int indices;     // current index count
-	unsigned int tris;
-	unsigned int count;       // candidates of the pass
-	unsigned int stop;        // nonzero: the loop has ended; the pass's kernels return at once
-	unsigned long long goal;  // triangle goal of the pass
-	unsigned int first_window;
-	unsigned int round_base;
+	const unsigned int* res; // current index buffer
+	unsigned int* res_next;  // the next pass's
+	unsigned int indices;    // current index count
+	unsigned int stop;       // why it ended
 	unsigned int passes;
-	unsigned int iterations;
-	unsigned int target;      // target_index_count
-	unsigned int sort_items;  // candidates per thread of the sort's tiles
-	unsigned int sort_cells;  // cells of the pass's live sort histogram matrix
-	float error_limit;        // squared, in the rescaled space (:2489-2491)
-	double window_factor;     // this pass's first decision window, in units of the triangle goal / 2
-	double window_base;       // its smallest value
+	unsigned int round_base;
+	double window_factor;    // the next pass's first decision window, in units of the triangle goal / 2
 };
 
 // The sorted positions a pass decides before its stop rules cut grow from pass to pass relative to
@@ -96,6 +85,7 @@ struct Scalars
 	unsigned long long dual;
 	unsigned int pick_total;
 	unsigned int pick_trunc;
+	unsigned int list_end;        // adjacency entries handed out so far in the pass (kPassLoop)
 	unsigned int active_count;
 	unsigned int tri_total;
 	unsigned long long cut;
@@ -112,13 +102,12 @@ struct Scalars
 	unsigned long long phase_cycles[8]; // kPerform phases, SM cycles of block 0, summed over the run
 	unsigned int trace_count;           // decision rounds traced so far in the run
 	unsigned int trace[2 * 512];        // per round: active candidates, SM cycles / 16
-	PassLive live;                      // device-resident pass loop
+	LoopState live;                     // the one-launch pass loop's end
 	PassStats pstats[kMaxPassStats];    // its per-pass counters
 	unsigned int solve_pending[3];      // update mode: vertices queued for a round, rotating by round
 	unsigned int solve_rounds;
 	unsigned int max_degree;            // corners of the busiest vertex
 	unsigned int scan_bar[2];           // the single-launch scans' barrier words (left zero by each scan)
-	unsigned int scan_bar2[2];          // those of the scans on the pass loop's second branch (the pick)
 	unsigned int scan_error;            // a single-launch scan's barrier gave up waiting
 };
 
@@ -1110,19 +1099,10 @@ __global__ void kCapacity(size_t index_count, Scalars* sc)
 // ---------------------------------------------------------------- pass: adjacency
 
 // corners per vertex of the current index buffer, welded by remap; each corner keeps the count
-// before it as its slot in its vertex's list, so the fill below needs no atomics. lv: the live
-// pass's buffer and count, and the slots go to its next buffer (free until the compaction)
+// before it as its slot in its vertex's list, so the fill below needs no atomics.
 __global__ void kCountCorners(const unsigned int* __restrict__ res, size_t n, const unsigned int* __restrict__ remap, unsigned int* __restrict__ cnt,
-    unsigned int* __restrict__ slot, const PassLive* lv)
+    unsigned int* __restrict__ slot)
 {
-	if (lv)
-	{
-		if (lv->stop)
-			return;
-		res = lv->res;
-		n = lv->indices;
-		slot = lv->res_next;
-	}
 	const size_t i = gtid();
 	if (i - (threadIdx.x & 31) >= n)
 		return; // the whole warp is past the corners
@@ -1145,16 +1125,8 @@ __global__ void kCountCorners(const unsigned int* __restrict__ res, size_t n, co
 // half-edges {next, prev} of every vertex in its list (the order within a list is arbitrary: the
 // flip test and the one-ring checks do not depend on it)
 __global__ void kAdjFill(const unsigned int* __restrict__ res, size_t tris, const unsigned int* __restrict__ remap, const unsigned int* __restrict__ off,
-    const unsigned int* __restrict__ slot, uint2* __restrict__ adj, const PassLive* lv, size_t adj_cap)
+    const unsigned int* __restrict__ slot, uint2* __restrict__ adj, size_t adj_cap)
 {
-	if (lv)
-	{
-		if (lv->stop)
-			return;
-		res = lv->res;
-		tris = lv->tris;
-		slot = lv->res_next;
-	}
 	size_t t = gtid();
 	if (t >= tris)
 		return;
@@ -1171,8 +1143,8 @@ __global__ void kAdjFill(const unsigned int* __restrict__ res, size_t tris, cons
 // ---------------------------------------------------------------- pass: pick
 
 // pickEdgeCollapses :1323-1368 for edge e of one triangle; returns false if not a candidate
-__device__ __forceinline__ bool pickEdge(unsigned int i0, unsigned int i1, const unsigned int* __restrict__ remap, const unsigned char* __restrict__ kind,
-    const unsigned int* __restrict__ loop, const unsigned int* __restrict__ loopback, unsigned int& v0, unsigned int& v1, unsigned int& bidi)
+__device__ __forceinline__ bool pickEdge(unsigned int i0, unsigned int i1, const unsigned int* remap, const unsigned char* kind, const unsigned int* loop,
+    const unsigned int* loopback, unsigned int& v0, unsigned int& v1, unsigned int& bidi)
 {
 	unsigned int r0 = remap[i0], r1 = remap[i1];
 	if (r0 == r1)
@@ -1202,8 +1174,8 @@ __device__ __forceinline__ bool pickEdge(unsigned int i0, unsigned int i1, const
 
 // a triangle's picked edges as 3 bits each (bit 0: a candidate, bit 1: bidirectional, bit 2:
 // from the edge's second vertex), so the emit needs no vertex gathers
-__device__ __forceinline__ unsigned int pickCode(const unsigned int a[3], const unsigned int* __restrict__ remap, const unsigned char* __restrict__ kind,
-    const unsigned int* __restrict__ loop, const unsigned int* __restrict__ loopback)
+__device__ __forceinline__ unsigned int pickCode(const unsigned int a[3], const unsigned int* remap, const unsigned char* kind, const unsigned int* loop,
+    const unsigned int* loopback)
 {
 	unsigned int code = 0;
 #pragma unroll
@@ -1217,21 +1189,12 @@ __device__ __forceinline__ unsigned int pickCode(const unsigned int a[3], const 
 }
 
 // candidates per block of kThreads triangles (the scan runs over blocks, not triangles) and
-// each triangle's pick code. lv: counts of the live pass; the grid covers the first pass's
-// triangles and blocks past the live count write zero, so the scan over the full range is the
-// scan of the live one
+// each triangle's pick code
 __global__ void __launch_bounds__(kThreads) kPickCount(const unsigned int* __restrict__ res, size_t tris, const unsigned int* __restrict__ remap,
     const unsigned char* __restrict__ kind, const unsigned int* __restrict__ loop, const unsigned int* __restrict__ loopback,
-    unsigned int* __restrict__ bcnt, unsigned short* __restrict__ codes, const PassLive* lv)
+    unsigned int* __restrict__ bcnt, unsigned short* __restrict__ codes)
 {
 	__shared__ unsigned int sm[kThreads / 32 + 1];
-	if (lv)
-	{
-		if (lv->stop)
-			return;
-		res = lv->res;
-		tris = lv->tris;
-	}
 	const size_t t = gtid();
 	unsigned int c = 0;
 	if (t < tris)
@@ -1251,16 +1214,9 @@ __global__ void __launch_bounds__(kThreads) kPickCount(const unsigned int* __res
 // (the capacity check at :1319-1320 stops at the first triangle that does not); a triangle's
 // prefix is its block's scanned count plus the block-local prefix
 __global__ void __launch_bounds__(kThreads) kPickEmit(const unsigned int* __restrict__ res, size_t tris, const unsigned short* __restrict__ codes,
-    const unsigned int* __restrict__ boffs, Scalars* sc, uint4* __restrict__ crec, const PassLive* lv)
+    const unsigned int* __restrict__ boffs, Scalars* sc, uint4* __restrict__ crec)
 {
 	__shared__ unsigned int sm[kThreads / 32 + 1];
-	if (lv)
-	{
-		if (lv->stop)
-			return;
-		res = lv->res;
-		tris = lv->tris;
-	}
 	const size_t t = gtid();
 	const unsigned int code = t < tris ? codes[t] : 0u;
 	unsigned int total;
@@ -1299,22 +1255,10 @@ constexpr unsigned int kRankThreads = MO_RANK_THREADS; // threads per block of k
 // beside it. Candidates stay in pick (triangle) order from here on: the sort only gives each
 // its sorted position, and the decision rounds walk pick order, where neighbouring candidates
 // share vertices.
-__global__ void kRank(size_t count, uint4* __restrict__ crec, uint4* __restrict__ cring, unsigned int* __restrict__ cerr, unsigned char* __restrict__ ckind,
-    const float4* __restrict__ pos, const Quadric* __restrict__ vq, const unsigned int* __restrict__ remap, const unsigned int* __restrict__ wedge,
-    const unsigned char* __restrict__ kind, const unsigned int* __restrict__ loop, const unsigned int* __restrict__ loopback,
-    const unsigned int* __restrict__ adj_off, const float* __restrict__ attr, const Quadric* __restrict__ aq, const float4* __restrict__ ag, int ac,
-    const PassLive* lv)
+__device__ __forceinline__ void rankCandidate(const uint4& cand, const float4* pos, const Quadric* vq, const unsigned int* remap, const unsigned int* wedge,
+    const unsigned char* kind, const unsigned int* loop, const unsigned int* loopback, const unsigned int* adj_off, const float* attr, const Quadric* aq,
+    const float4* ag, int ac, uint4& rec, uint4& ring, const unsigned int* cnt = nullptr)
 {
-	if (lv)
-	{
-		if (lv->stop)
-			return;
-		count = lv->count;
-	}
-	size_t c = gtid();
-	if (c >= count)
-		return;
-	const uint4 cand = crec[c];
 	const unsigned int i0 = cand.x, i1 = cand.y;
 	const bool bidi = cand.z != 0;
 	const unsigned int ra = remap[i0], rb = remap[i1];
@@ -1360,10 +1304,25 @@ __global__ void kRank(size_t count, uint4* __restrict__ crec, uint4* __restrict_
 	float err = ej < ei ? ej : ei;
 	unsigned int bits = __float_as_uint(err);
 	const unsigned char ks = kind[s0];
-	crec[c] = make_uint4(s0, s1, bits, ks);
-	cring[c] = make_uint4(r0, r1, adj_off[r0], adj_off[r0 + 1]);
-	cerr[c] = bits;
-	ckind[c] = ks;
+	rec = make_uint4(s0, s1, bits, ks);
+	const unsigned int b = adj_off[r0]; // with cnt, lists are in no order
+	ring = make_uint4(r0, r1, b, cnt ? b + cnt[r0] : adj_off[r0 + 1]);
+}
+
+__global__ void kRank(size_t count, uint4* __restrict__ crec, uint4* __restrict__ cring, unsigned int* __restrict__ cerr, unsigned char* __restrict__ ckind,
+    const float4* __restrict__ pos, const Quadric* __restrict__ vq, const unsigned int* __restrict__ remap, const unsigned int* __restrict__ wedge,
+    const unsigned char* __restrict__ kind, const unsigned int* __restrict__ loop, const unsigned int* __restrict__ loopback,
+    const unsigned int* __restrict__ adj_off, const float* __restrict__ attr, const Quadric* __restrict__ aq, const float4* __restrict__ ag, int ac)
+{
+	size_t c = gtid();
+	if (c >= count)
+		return;
+	uint4 rec, ring;
+	rankCandidate(crec[c], pos, vq, remap, wedge, kind, loop, loopback, adj_off, attr, aq, ag, ac, rec, ring);
+	crec[c] = rec;
+	cring[c] = ring;
+	cerr[c] = rec.z;
+	ckind[c] = (unsigned char)rec.w;
 }
 
 // ---------------------------------------------------------------- pass: sort
@@ -1402,15 +1361,9 @@ size_t keySortScratchWords(size_t n)
 }
 
 template <unsigned int ITEMS>
-__global__ void __launch_bounds__(kThreads) kKeyHist(const unsigned int* __restrict__ cerr, size_t n, unsigned int* __restrict__ hist, const PassLive* lv)
+__global__ void __launch_bounds__(kThreads) kKeyHist(const unsigned int* __restrict__ cerr, size_t n, unsigned int* __restrict__ hist)
 {
 	__shared__ unsigned int sh[kKeyBins];
-	if (lv)
-	{
-		if (lv->stop)
-			return;
-		n = lv->count;
-	}
 	const unsigned int tiles = keySortTiles(n, ITEMS);
 	if (blockIdx.x >= tiles)
 		return;
@@ -1442,18 +1395,11 @@ __global__ void __launch_bounds__(kThreads) kKeyHist(const unsigned int* __restr
 // order, as the reference's counting sort keeps collapse order.
 template <unsigned int ITEMS>
 __global__ void __launch_bounds__(kThreads) kKeyScatter(const unsigned int* __restrict__ cerr, const unsigned char* __restrict__ ckind, size_t n,
-    const unsigned int* __restrict__ hist, unsigned int* __restrict__ rank, unsigned int* __restrict__ serr, unsigned char* __restrict__ skind,
-    const PassLive* lv)
+    const unsigned int* __restrict__ hist, unsigned int* __restrict__ rank, unsigned int* __restrict__ serr, unsigned char* __restrict__ skind)
 {
 	extern __shared__ __align__(16) unsigned char key_smem[];
 	unsigned int* gbase = reinterpret_cast<unsigned int*>(key_smem);               // sorted position of the tile's first candidate per key
 	unsigned short* wcnt = reinterpret_cast<unsigned short*>(gbase + kKeyBins);   // per warp and key: count, then offset in the tile
-	if (lv)
-	{
-		if (lv->stop)
-			return;
-		n = lv->count;
-	}
 	const unsigned int tiles = keySortTiles(n, ITEMS);
 	if (blockIdx.x >= tiles)
 		return;
@@ -1599,9 +1545,6 @@ struct PerformArgs
 	unsigned int tris;
 	uint4* blk;
 	Scalars* sc;
-	// device-resident pass loop (else nullptr): count, goal, first_window, round_base, tris, res,
-	// res_next and the previous result error come from here instead of the fields above
-	const PassLive* live;
 };
 
 // Decision rule: candidate k is decided once nothing earlier in sorted order can change its
@@ -1611,6 +1554,15 @@ struct PerformArgs
 //  * otherwise it waits until it is the earliest undecided candidate on both endpoints (minT)
 //    and no undecided earlier candidate moves a vertex of its one-ring (minS); then the flip
 //    test runs against the one-ring as moved by earlier commits only (moving commit < k).
+
+// A load of data that is constant in one pass. LOOP (kPassLoop): another pass of the same launch
+// wrote it, so it goes through L1, which the grid barriers' acquire clears; else through the
+// read-only path, which keeps it across barriers (2M attribute sphere 4.06 ms, 4.22 without).
+template <bool LOOP, class T>
+__device__ __forceinline__ T ld(const T* p)
+{
+	return LOOP ? *p : __ldg(p);
+}
 
 // the commit of a decided candidate: r0 moves to its target and both endpoints lock
 __device__ __forceinline__ void commitOne(const PerformArgs& a, const uint4& cd, unsigned int k, unsigned int r0, unsigned int r1)
@@ -1671,13 +1623,14 @@ enum
 // corner 0.81 / 4.22 / 39.0; 4 x 2 0.82 / 4.20 / 38.5; 4 x 1 0.84 / 4.26 / 39.2; 2 x 4 (spills)
 // 0.88 / 4.61 / 43.7. With the candidates' lists in shared memory and blocks of 512: 8 x 1
 // 0.75 / 4.06 / 38.3, 4 x 2 0.77 / 4.12 / 38.3.
+template <bool LOOP>
 __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, unsigned int k, const uint4& rec, unsigned int round, unsigned int sub,
     unsigned int mask)
 {
 	const unsigned int r0 = rec.x, r1 = rec.y, b = rec.z, e = rec.w;
 	const unsigned long long tag = roundTag(round);
 	const unsigned int p = round & 1;
-	const uint4 cd = sub == 0 ? __ldg(a.crec + c) : make_uint4(0, 0, 0, 0); // in flight during the walk
+	const uint4 cd = sub == 0 ? ld<LOOP>(a.crec + c) : make_uint4(0, 0, 0, 0); // in flight during the walk
 	const V3 v0 = ldpos(a.pos, r0), v1 = ldpos(a.pos, r1);
 	bool flip = false;
 	constexpr unsigned int FB = kRingBatch;
@@ -1690,7 +1643,7 @@ __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, 
 		for (unsigned int q = 0; q < FB; ++q)
 		{
 			const unsigned int j = j0 + q * kRingLanes + sub;
-			ed[q] = j < e ? __ldg(a.adj + j) : make_uint2(r1, r1); // r1 is in the ring already
+			ed[q] = j < e ? ld<LOOP>(a.adj + j) : make_uint2(r1, r1); // r1 is in the ring already
 		}
 #pragma unroll
 		for (unsigned int q = 0; q < FB; ++q)
@@ -1784,7 +1737,7 @@ __device__ __forceinline__ uint3 blockScan3(unsigned int& t, unsigned int& f, un
 	return tot;
 }
 
-__device__ __forceinline__ bool keepTriangle(const unsigned int* __restrict__ res, size_t t, const unsigned int* cr, const unsigned int* __restrict__ remap,
+__device__ __forceinline__ bool keepTriangle(const unsigned int* res, size_t t, const unsigned int* cr, const unsigned int* remap,
     uint3& out)
 {
 	unsigned int v0 = __ldcg(cr + res[t * 3 + 0]), v1 = __ldcg(cr + res[t * 3 + 1]), v2 = __ldcg(cr + res[t * 3 + 2]);
@@ -1793,16 +1746,24 @@ __device__ __forceinline__ bool keepTriangle(const unsigned int* __restrict__ re
 	return r0 != r1 && r0 != r2 && r1 != r2;
 }
 
+// rows that an earlier pass of the same launch may have written, read once: through L2
+__device__ __forceinline__ Quadric ldquadricL2(const Quadric* q, unsigned int i)
+{
+	const float4* p = reinterpret_cast<const float4*>(q + i);
+	const float4 a = __ldcg(p), b = __ldcg(p + 1), c = __ldcg(p + 2);
+	return Quadric{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, 0.f};
+}
+
 // attribute quadric and gradient rows of vertex v added into those of vertex t (t != v)
 __device__ __forceinline__ void mergeRows(const Quadric* __restrict__ vq, Quadric* __restrict__ tq, const float4* __restrict__ vg, float4* __restrict__ tg,
     int ac)
 {
-	Quadric A = ldquadric(tq, 0);
-	qadd(A, ldquadric(vq, 0));
+	Quadric A = ldquadricL2(tq, 0);
+	qadd(A, ldquadricL2(vq, 0));
 	stquadric(tq, 0, A);
 	for (int q = 0; q < ac; ++q)
 	{
-		float4 g = tg[q], h = vg[q];
+		float4 g = __ldcg(tg + q), h = __ldcg(vg + q);
 		g.x += h.x, g.y += h.y, g.z += h.z, g.w += h.w;
 		tg[q] = g;
 	}
@@ -1810,13 +1771,13 @@ __device__ __forceinline__ void mergeRows(const Quadric* __restrict__ vq, Quadri
 
 __device__ __forceinline__ void mergeAttributes(const PerformArgs& a, unsigned int v, unsigned int t)
 {
-	Quadric A = ldquadric(a.aq, t);
-	qadd(A, ldquadric(a.aq, v));
+	Quadric A = ldquadricL2(a.aq, t);
+	qadd(A, ldquadricL2(a.aq, v));
 	stquadric(a.aq, t, A);
 	const int ac = a.ac;
 	for (int q = 0; q < ac; ++q)
 	{
-		float4 g = a.ag[(size_t)t * ac + q], h = a.ag[(size_t)v * ac + q];
+		float4 g = __ldcg(a.ag + (size_t)t * ac + q), h = __ldcg(a.ag + (size_t)v * ac + q);
 		g.x += h.x, g.y += h.y, g.z += h.z, g.w += h.w;
 		a.ag[(size_t)t * ac + q] = g;
 	}
@@ -1829,8 +1790,8 @@ __device__ __forceinline__ void mergeAttributes(const PerformArgs& a, unsigned i
 // commit of the pass writes.
 __device__ void applyComplexCommit(const PerformArgs& a, unsigned int r0, unsigned int r1, unsigned int i0, unsigned int i1, unsigned int& derrbits)
 {
-	Quadric Q1 = ldquadric(a.vq, r1);
-	Quadric Q0 = ldquadric(a.vq, r0);
+	Quadric Q1 = ldquadricL2(a.vq, r1);
+	Quadric Q0 = ldquadricL2(a.vq, r0);
 	unsigned int v = i0;
 	do
 	{
@@ -1841,8 +1802,8 @@ __device__ void applyComplexCommit(const PerformArgs& a, unsigned int r0, unsign
 	stquadric(a.vq, r1, Q1);
 	if (a.vg)
 	{
-		float4 g = a.vg[r1];
-		gadd(g, a.vg[r0]);
+		float4 g = __ldcg(a.vg + r1);
+		gadd(g, __ldcg(a.vg + r0));
 		a.vg[r1] = g;
 	}
 	if (a.ac)
@@ -1872,10 +1833,11 @@ __device__ void applyComplexCommit(const PerformArgs& a, unsigned int r0, unsign
 }
 
 // the commit of candidate c (pick order)
+template <bool LOOP>
 __device__ void applyCommit(const PerformArgs& a, unsigned int c, unsigned int& errbits, unsigned int& derrbits)
 {
-	const uint4 rec = __ldg(a.cring + c);
-	const uint4 cd = __ldg(a.crec + c);
+	const uint4 rec = ld<LOOP>(a.cring + c);
+	const uint4 cd = ld<LOOP>(a.crec + c);
 	const unsigned int r0 = rec.x, r1 = rec.y, i0 = cd.x, i1 = cd.y;
 	const unsigned char kd = (unsigned char)cd.w;
 	const float e = __uint_as_float(cd.z);
@@ -1913,16 +1875,16 @@ __device__ void applyCommit(const PerformArgs& a, unsigned int c, unsigned int& 
 		const unsigned int tr = r0 == s0 ? s1 : (r0 == i0 ? i1 : __ldcg(a.cr + r0));
 		pr = ldpos(a.pos, __ldg(a.remap + tr));
 	}
-	Quadric Q1 = ldquadric(q1, 0);
-	Quadric Q0 = ldquadric(q0, 0);
+	Quadric Q1 = ldquadricL2(q1, 0);
+	Quadric Q0 = ldquadricL2(q0, 0);
 	qadd(Q1, Q0);
 	stquadric(q1, 0, Q1);
 	if (a.vg)
 	{
 		const float4* __restrict__ g0 = a.vg + r0;
 		float4* __restrict__ g1 = a.vg + r1;
-		float4 g = *g1;
-		gadd(g, *g0);
+		float4 g = __ldcg(g1);
+		gadd(g, __ldcg(g0));
 		*g1 = g;
 	}
 	if (ac)
@@ -1977,6 +1939,10 @@ struct PhaseClock
 		s[phase] += t - s[8];
 		s[8] = t;
 	}
+	__device__ void skip() // the time since the last lap belongs to no phase
+	{
+		s[8] = clock64();
+	}
 };
 
 #ifndef MO_PERFORM_THREADS
@@ -1990,52 +1956,31 @@ struct PhaseClock
 #endif
 constexpr unsigned int kPerformThreads = MO_PERFORM_THREADS;
 
-__global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerform(PerformArgs a)
+// the shared memory of performPass
+struct PassShared
 {
-	__shared__ unsigned int s_app[4];
-	__shared__ unsigned int s_stage[2][kStageChunk]; // candidates passed to stage B, and kept for stage C (wait)
-	__shared__ unsigned int s_list[kStageChunk];     // the block's undecided candidates, once they fit
-	__shared__ unsigned int s_commits;               // this block's commits so far
-	__shared__ unsigned int s_grid[4];
-	__shared__ long long s_clock[10];
-	PhaseClock pc{s_clock};
-	const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
-	if (timer)
-		pc.start(a.sc);
-	__shared__ unsigned int sm[3][33];
-	Scalars* sc = a.sc;
-	const unsigned int G = gridDim.x;
-	const size_t gthreads = (size_t)G * blockDim.x;
-	const unsigned int lane = threadIdx.x & 31;
-	const unsigned int sub = lane & (kRingLanes - 1), ring_mask = (~0u >> (32 - kRingLanes)) << (lane - sub);
+	unsigned int* stage[2]; // kStageChunk each: candidates passed to stage B, and kept for stage C (wait)
+	unsigned int* list;     // kStageChunk: the block's undecided candidates, once they fit
+	unsigned int* app;      // 5 words: the stages' counters, and the block's commits so far
+	long long* clock;       // 10
+	unsigned int (*sm)[33]; // 3 rows
+};
 
-	// per-pass scalars: the launch parameters, or the device-resident loop's live state
-	unsigned int count = a.count, tris = a.tris, first_window = a.first_window, round_base = a.round_base, prev_err = a.prev_err_bits;
-	unsigned long long goal = a.goal;
-	float error_limit = a.error_limit;
-	const unsigned int* res = a.res;
-	unsigned int* res_next = a.res_next;
-	if (a.live)
-	{
-		const PassLive* lv = a.live;
-		if (lv->stop)
-			return;
-		count = lv->count;
-		tris = lv->tris;
-		first_window = lv->first_window;
-		round_base = lv->round_base;
-		goal = lv->goal;
-		res = lv->res;
-		res_next = lv->res_next;
-		prev_err = sc->result_error_bits;
-		error_limit = lv->error_limit;
-	}
+// what a pass starts from, the same in every block
+struct PassIn
+{
+	unsigned int count, tris, first_window, round_base, prev_err;
+	unsigned long long goal;
+	float error_limit;
+	const unsigned int* res;
+	unsigned int* res_next;
+};
 
-	GridSum grid;
-	grid.start(reinterpret_cast<unsigned long long*>(sc->bar), &sc->grid_error, s_grid);
-
-	// per-vertex state of the pass, streamed: collapse_remap, and both parities of both marks (the
-	// marks the window's candidates set below come after the barrier)
+// per-vertex state of a pass, streamed: collapse_remap, and both parities of both marks (the marks
+// the window's candidates set come after a barrier)
+__device__ __forceinline__ void resetVertices(const PerformArgs& a)
+{
+	const size_t gthreads = (size_t)gridDim.x * blockDim.x;
 	for (size_t i = gtid(); i < a.vcount; i += gthreads)
 	{
 		a.cr[i] = (unsigned int)i;
@@ -2043,12 +1988,115 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 		a.minT[1][i] = ~0ull;
 		reinterpret_cast<ulonglong2*>(a.minS)[i] = make_ulonglong2(~0ull, ~0ull);
 	}
-	grid.wait();
+}
+
+enum
+{
+	kPassFailed = 0, // a wait ran out or a round made no progress: the error flag is set
+	kPassEmpty = 1,  // nothing committed
+	kPassDone = 2,
+};
+
+// kPassLoop's arguments
+struct PassLoopArgs
+{
+	PerformArgs p;
+	unsigned int* cnt;         // V: corners per vertex; zero before the launch
+	unsigned int* slot;        // each corner's place in its vertex's list
+	unsigned int* adj_off;     // V: where a vertex's list starts (lists are in no order)
+	uint2* adj;
+	size_t adj_cap;
+	unsigned short* codes;     // per triangle
+	uint4* crec;
+	uint4* cring;
+	unsigned int* rank;
+	unsigned int* serr;
+	unsigned char* skind;
+	const unsigned char* kind;
+	const float* attr;
+	unsigned int* hist;        // key histograms, one row of kKeyBins per sorting block; then the bins' totals
+	unsigned int index_count;  // of the first pass
+	unsigned int target;       // target_index_count
+	unsigned int max_passes;
+	unsigned int passes;       // done before this launch, and their decision rounds
+	unsigned int round_base;
+	double window_factor;      // of this launch's first pass
+	double window_base;
+	float target_error;
+	int absolute;              // target_error is absolute
+	const unsigned int* res;
+	unsigned int* res_next;
+	int prune;                 // leave the loop after a pass whose vertex error reaches prune_error
+	float prune_error;
+};
+
+// the run of triangles a block has in a pass of kPassLoop
+struct BlockTriangles
+{
+	unsigned int begin, end;
+	unsigned int picked; // candidates among them
+};
+
+// the corner counts and pick codes of a warp's triangles (corners' primaries r) at places t of their
+// buffer; returns the candidates of this lane's. Corners of one vertex among the lanes (neighbouring
+// triangles share vertices) take their places with one add. The whole warp calls it.
+__device__ __forceinline__ unsigned int countTriangles(const PassLoopArgs& l, bool valid, unsigned int t, const unsigned int v[3], const unsigned int r[3])
+{
+	const unsigned int lane = threadIdx.x & 31;
+	unsigned int peers[3], at[3];
+#pragma unroll
+	for (int c = 0; c < 3; ++c)
+	{
+		peers[c] = __match_any_sync(0xffffffffu, valid ? r[c] : ~0u); // no vertex is ~0
+		at[c] = 0;
+		if (valid && lane == (unsigned int)(__ffs(peers[c]) - 1))
+			at[c] = atomicAdd(l.cnt + r[c], __popc(peers[c]));
+	}
+	const unsigned int code = valid ? pickCode(v, l.p.remap, l.kind, l.p.loop, l.p.loopback) : 0u;
+#pragma unroll
+	for (int c = 0; c < 3; ++c)
+	{
+		at[c] = __shfl_sync(0xffffffffu, at[c], __ffs(peers[c]) - 1) + __popc(peers[c] & ((1u << lane) - 1u));
+		if (valid)
+			l.slot[(size_t)t * 3 + c] = at[c];
+	}
+	if (valid)
+		l.codes[t] = (unsigned short)code;
+	return __popc(code & 0x49u);
+}
+
+// one pass from its ranked and sorted candidates to the next index buffer, by the whole grid;
+// kept: the triangles of that buffer; cutv: where the stop rules cut (position and rule). LOOP (kPassLoop): the first window's candidates are marked
+// already, and the next pass's counting (countTriangle) is done as the triangles are written: mine
+// becomes the block's run of them.
+template <bool LOOP>
+__device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopArgs* loop, const PassIn& in, GridSum& grid, const PassShared& sh,
+    unsigned int& rounds, unsigned int& kept_total, unsigned long long& cutv, BlockTriangles& mine)
+{
+	Scalars* sc = a.sc;
+	PhaseClock pc{sh.clock};
+	long long* const s_clock = sh.clock;
+	unsigned int (*const sm)[33] = sh.sm;
+	unsigned int* const s_app = sh.app;
+	unsigned int* const s_stage[2] = {sh.stage[0], sh.stage[1]};
+	unsigned int* const s_list = sh.list;
+	unsigned int& s_commits = sh.app[4];
+	const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
+	const unsigned int G = gridDim.x;
+	const size_t gthreads = (size_t)G * blockDim.x;
+	const unsigned int lane = threadIdx.x & 31;
+	const unsigned int sub = lane & (kRingLanes - 1), ring_mask = (~0u >> (32 - kRingLanes)) << (lane - sub);
+	const unsigned int count = in.count, tris = in.tris, round_base = in.round_base;
+	const unsigned long long goal = in.goal;
+	const float error_limit = in.error_limit;
+	const unsigned int* const res = in.res;
+	unsigned int* const res_next = in.res_next;
+
 
 	unsigned int round = round_base;
 	unsigned long long active_sum = 0;
-	unsigned int K0 = 0, K1 = min(count, first_window);
-	unsigned int carryT = 0, carryF = 0, carryM = prev_err;
+	unsigned int K0 = 0, K1 = min(count, in.first_window);
+	unsigned int carryT = 0, carryF = 0, carryM = in.prev_err;
 	unsigned int windows = 0;
 
 	// block b's candidates are the pick-order tiles b, b + G, b + 2G, ... of blockDim each; its
@@ -2078,13 +2126,16 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	{
 		// ---- decision rounds over the sorted window [K0, K1)
 		++windows;
-		for (size_t c = gtid(); c < count; c += gthreads)
+		if (!LOOP || windows > 1)
 		{
-			const unsigned int k = __ldg(a.rank + c);
-			if (k >= K0 && k < K1)
-				markCandidate(a, k, __ldg(a.cring + c), round + 1);
+			for (size_t c = gtid(); c < count; c += gthreads)
+			{
+				const unsigned int k = ld<LOOP>(a.rank + c);
+				if (k >= K0 && k < K1)
+					markCandidate(a, k, ld<LOOP>(a.cring + c), round + 1);
+			}
+			grid.wait();
 		}
-		grid.wait();
 		if (timer)
 			pc.lap(windows == 1 ? kPhInit : kPhMarks);
 
@@ -2136,8 +2187,8 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 #pragma unroll
 					for (unsigned int q = 0; q < kStageItems; ++q)
 					{
-						kk[q] = ok[q] ? __ldg(a.rank + cc[q]) : 0u;
-						const uint4 rec = ok[q] ? __ldg(a.cring + cc[q]) : make_uint4(0, 0, 0, 0);
+						kk[q] = ok[q] ? ld<LOOP>(a.rank + cc[q]) : 0u;
+						const uint4 rec = ok[q] ? ld<LOOP>(a.cring + cc[q]) : make_uint4(0, 0, 0, 0);
 						ends[q] = make_uint2(rec.x, rec.y);
 					}
 #pragma unroll
@@ -2175,7 +2226,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 					if (x < nB)
 					{
 						c = s_stage[0][x];
-						r = ringDecide(a, c, __ldg(a.rank + c), __ldg(a.cring + c), round, sub, ring_mask);
+						r = ringDecide<LOOP>(a, c, ld<LOOP>(a.rank + c), ld<LOOP>(a.cring + c), round, sub, ring_mask);
 					}
 					append(sub == 0 && r == kRingWaits, c, &s_app[3], s_stage[1]);
 					append(sub == 0 && r == kRingCommit, c, &s_commits, commits);
@@ -2195,8 +2246,8 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 					{
 						const unsigned int x = base + q * blockDim.x + threadIdx.x;
 						cc[q] = x < nD ? s_stage[1][x] : ~0u;
-						kk[q] = cc[q] != ~0u ? __ldg(a.rank + cc[q]) : 0u;
-						const uint4 rec = cc[q] != ~0u ? __ldg(a.cring + cc[q]) : make_uint4(0, 0, 0, 0);
+						kk[q] = cc[q] != ~0u ? ld<LOOP>(a.rank + cc[q]) : 0u;
+						const uint4 rec = cc[q] != ~0u ? ld<LOOP>(a.cring + cc[q]) : make_uint4(0, 0, 0, 0);
 						ends[q] = make_uint2(rec.x, rec.y);
 					}
 					unsigned long long m0[kStageItems], m1[kStageItems];
@@ -2245,14 +2296,14 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 			{
 				if (gtid() == 0)
 					atomicOr(&sc->grid_error, 2u);
-				return;
+				return kPassFailed;
 			}
 			n = nn;
 			first = false;
 			listed = list_next;
 		}
 		if (grid.failed())
-			return;
+			return kPassFailed;
 
 		// ---- stop rules over [K0, K1): block chunks, thread sub-chunks, carried prefix
 		const unsigned int len = K1 - K0;
@@ -2264,7 +2315,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 		for (unsigned int k = t0; k < t1; ++k)
 		{
 			unsigned int tt, ff, ee;
-			stopTerms(__ldcg(a.status + k), __ldg(a.skind + k), __ldg(a.serr + k), tt, ff, ee);
+			stopTerms(__ldcg(a.status + k), ld<LOOP>(a.skind + k), ld<LOOP>(a.serr + k), tt, ff, ee);
 			sT += tt, sF += ff, sM = max(sM, ee);
 		}
 		unsigned int eT = sT, eF = sF, eM = sM;
@@ -2295,7 +2346,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 			float error_goal = FLT_MAX;
 			for (unsigned int k = t0; k < t1; ++k)
 			{
-				float e = __uint_as_float(__ldg(a.serr + k));
+				float e = __uint_as_float(ld<LOOP>(a.serr + k));
 				unsigned int reason = 0;
 				if (e > error_limit)
 					reason = 1;
@@ -2307,7 +2358,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 					if (eg != goal_at)
 					{
 						goal_at = eg;
-						error_goal = eg < count ? 1.5f * __uint_as_float(__ldg(a.serr + eg)) : FLT_MAX;
+						error_goal = eg < count ? 1.5f * __uint_as_float(ld<LOOP>(a.serr + eg)) : FLT_MAX;
 					}
 					if (e > error_goal)
 						reason = 3;
@@ -2318,7 +2369,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 					break;
 				}
 				unsigned int tt, ff, ee;
-				stopTerms(__ldcg(a.status + k), __ldg(a.skind + k), __ldg(a.serr + k), tt, ff, ee);
+				stopTerms(__ldcg(a.status + k), ld<LOOP>(a.skind + k), ld<LOOP>(a.serr + k), tt, ff, ee);
 				T += tt, F += ff, M = max(M, ee);
 			}
 		}
@@ -2334,13 +2385,13 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 		K1 = (unsigned int)min((unsigned long long)count, 2ull * K1);
 	}
 	if (grid.failed())
-		return;
+		return kPassFailed;
 
 	// ---- apply the committed prefix. Commits are independent (no two share an endpoint), so
 	// any order gives the same result: each block applies its own commits (pick order, so their
 	// quadric rows are near one another) whose sorted position is inside the prefix. The
 	// decisions of the prefix are counted over sorted order.
-	const unsigned long long cutv = __ldcg(&sc->cut);
+	cutv = __ldcg(&sc->cut);
 	const unsigned int cut = cutv == ~0ull ? count : (unsigned int)(cutv >> 2);
 	unsigned int nd = 0, ns = 0, ni = 0, em = 0, dm = 0;
 	for (size_t k = gtid(); k < cut; k += gthreads)
@@ -2353,10 +2404,10 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 		for (unsigned int x = threadIdx.x; x < mc; x += blockDim.x)
 		{
 			const unsigned int c = commits[x];
-			if (__ldg(a.rank + c) < cut)
+			if (ld<LOOP>(a.rank + c) < cut)
 			{
 				unsigned int eb = 0, db = 0;
-				applyCommit(a, c, eb, db);
+				applyCommit<LOOP>(a, c, eb, db);
 				em = max(em, eb), dm = max(dm, db);
 			}
 		}
@@ -2383,21 +2434,22 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	grid.wait();
 	if (timer)
 		pc.lap(kPhApply);
-	if (__ldcg(&sc->done) == 0 || grid.failed())
+	rounds = round - round_base;
+	if (gtid() == 0)
 	{
-		if (timer)
-			for (int i = 0; i < 8; ++i)
-				atomicAdd(&sc->phase_cycles[i], (unsigned long long)s_clock[i]);
-		if (gtid() == 0)
-		{
-			sc->rounds = round - round_base;
-			sc->active_sum = active_sum;
-			sc->windows = windows;
-		}
-		return;
+		sc->rounds = rounds;
+		sc->active_sum = active_sum;
+		sc->windows = windows;
 	}
+	if (grid.failed())
+		return kPassFailed;
+	if (__ldcg(&sc->done) == 0)
+		return kPassEmpty;
 
 	// ---- loop remap (in place: targets are fixed points of collapse_remap) and kept-triangle counts
+	if (LOOP)
+		for (size_t i = gtid(); i < a.vcount; i += gthreads)
+			loop->cnt[i] = 0; // for the next pass, counted below
 	for (size_t i = gtid(); i < a.vcount; i += gthreads)
 	{
 		unsigned int* arrs[2] = {a.loop, a.loopback};
@@ -2419,10 +2471,8 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	}
 	const unsigned int tper_block = (tris + G - 1) / G;
 	const unsigned int tb0 = min(tris, blockIdx.x * tper_block), tb1 = min(tris, tb0 + tper_block);
-	const unsigned int tper_thread = (tb1 - tb0 + blockDim.x - 1) / blockDim.x;
-	const unsigned int tt0 = min(tb1, tb0 + threadIdx.x * tper_thread), tt1 = min(tb1, tt0 + tper_thread);
 	unsigned int kept = 0;
-	for (unsigned int t = tt0; t < tt1; ++t)
+	for (unsigned int t = tb0 + threadIdx.x; t < tb1; t += blockDim.x)
 	{
 		uint3 o;
 		kept += keepTriangle(res, t, a.cr, a.remap, o);
@@ -2435,39 +2485,528 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	if (timer)
 		pc.lap(kPhLoops);
 	if (grid.failed())
-		return;
+		return kPassFailed;
 	{
-		unsigned int before = 0, z1 = 0, z2 = 0; // triangles the blocks before this one keep
-		for (unsigned int q = threadIdx.x; q < blockIdx.x; q += blockDim.x)
-			before += __ldcg(&a.blk[q].x);
-		before = blockScan3(before, z1, z2, sm).x;
-		if (threadIdx.x == 0 && blockIdx.x == G - 1)
+		// triangles the blocks before this one keep, and all of them
+		unsigned int before = 0, all = 0, z = 0;
+		for (unsigned int q = threadIdx.x; q < G; q += blockDim.x)
 		{
-			sc->tri_total = before + ktot.x;
-			sc->rounds = round - round_base;
-			sc->active_sum = active_sum;
-			sc->windows = windows;
+			const unsigned int x = __ldcg(&a.blk[q].x);
+			all += x;
+			before += q < blockIdx.x ? x : 0u;
 		}
+		const uint3 sums = blockScan3(before, all, z, sm);
+		before = sums.x;
+		kept_total = sums.y;
 		if (timer)
 			pc.lap(kPhScan);
-		unsigned int w = before + ek;
-		for (unsigned int t = tt0; t < tt1; ++t)
+		// tile by tile, so that a warp reads and writes neighbouring triangles
+		unsigned int run = before, picked = 0;
+		for (unsigned int base = tb0; base < tb1; base += blockDim.x)
 		{
-			uint3 o;
-			if (keepTriangle(res, t, a.cr, a.remap, o))
+			const unsigned int t = base + threadIdx.x;
+			uint3 o = make_uint3(0, 0, 0);
+			const bool keep = t < tb1 && keepTriangle(res, t, a.cr, a.remap, o);
+			const unsigned int m = __ballot_sync(0xffffffffu, keep);
+			if (lane == 0)
+				sm[0][threadIdx.x >> 5] = __popc(m);
+			__syncthreads();
+			unsigned int warps = lane < blockDim.x / 32 ? sm[0][lane] : 0u;
+			const unsigned int mine_at = __reduce_add_sync(0xffffffffu, lane < (threadIdx.x >> 5) ? warps : 0u);
+			warps = __reduce_add_sync(0xffffffffu, warps);
+			const unsigned int w = run + mine_at + __popc(m & ((1u << lane) - 1u));
+			run += warps;
+			if (keep)
 			{
 				res_next[(size_t)w * 3 + 0] = o.x;
 				res_next[(size_t)w * 3 + 1] = o.y;
 				res_next[(size_t)w * 3 + 2] = o.z;
-				w++;
 			}
+			if (LOOP)
+			{
+				const unsigned int v[3] = {o.x, o.y, o.z};
+				const unsigned int r[3] = {__ldg(a.remap + o.x), __ldg(a.remap + o.y), __ldg(a.remap + o.z)};
+				picked += countTriangles(*loop, keep, w, v, r);
+			}
+			__syncthreads(); // sm is read
+		}
+		if (LOOP)
+		{
+			unsigned int z1 = 0, z2 = 0;
+			mine.begin = before;
+			mine.end = before + ktot.x;
+			mine.picked = blockScan3(picked, z1, z2, sm).x;
+		}
+	}
+	if (timer)
+		pc.lap(kPhEmit);
+	return kPassDone;
+}
+
+// adds the phase clock's times to the run's (block 0's first thread)
+__device__ __forceinline__ void reportPhases(Scalars* sc, const long long* clock)
+{
+	for (int i = 0; i < 8; ++i)
+		atomicAdd(&sc->phase_cycles[i], (unsigned long long)clock[i]);
+}
+
+__global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerform(PerformArgs a)
+{
+	__shared__ unsigned int s_app[5];
+	__shared__ unsigned int s_stage[2][kStageChunk];
+	__shared__ unsigned int s_list[kStageChunk];
+	__shared__ unsigned int s_grid[4];
+	__shared__ long long s_clock[10];
+	__shared__ unsigned int sm[3][33];
+	Scalars* sc = a.sc;
+	const PassShared sh = {{s_stage[0], s_stage[1]}, s_list, s_app, s_clock, sm};
+	const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
+	if (timer)
+		PhaseClock{s_clock}.start(sc);
+	const PassIn in = {a.count, a.tris, a.first_window, a.round_base, a.prev_err_bits, a.goal, a.error_limit, a.res, a.res_next};
+	GridSum grid;
+	grid.start(reinterpret_cast<unsigned long long*>(sc->bar), &sc->grid_error, s_grid);
+	resetVertices(a);
+	grid.wait();
+	unsigned int rounds = 0, kept = 0;
+	unsigned long long cutv;
+	BlockTriangles none;
+	const int r = performPass<false>(a, nullptr, in, grid, sh, rounds, kept, cutv, none);
+	if (r == kPassDone && gtid() == 0)
+		sc->tri_total = kept;
+	if (timer && r != kPassFailed)
+		reportPhases(sc, s_clock);
+}
+
+// ---------------------------------------------------------------- the pass loop in one launch
+//
+// kPassLoop runs the whole pass loop (src/simplifier.cpp:2493-2541) as one cooperative kernel: each
+// pass's adjacency, pick, rank, sort and perform are phases between grid barriers, over contiguous
+// runs of triangles, vertices and candidates per block:
+//   1 corner counts, pick codes and counts (with the last pass's compaction, but for the first)
+//   2 a place for every vertex's list; candidates emitted in triangle order
+//   3 adjacency, rank, key histograms (one row per sorting block)
+//   4 every bin's prefixes over the rows
+//   5 sorted positions, and the first window's marks
+// then performPass. A pass of a mesh of some 100k triangles is bound by latency: a barrier costs 2 to
+// 3 us where the boundary between kernels of a recorded graph costs 4 to 5 with the next one's ramp.
+// It also needs no recording, and no host round trip per pass where the host must look at a pass's
+// result now and then (pruning) or many callers share the GPU (the server).
+
+// why kPassLoop ended (live.stop)
+enum
+{
+	kLoopEnded = 1,
+	kLoopPrune = 2, // more passes to run after the host has pruned
+};
+
+// candidates per thread of one step of the sort's scatter: a warp's counts of a key fit 8 bits
+constexpr unsigned int kLoopItems = 4;
+constexpr unsigned int kLoopWarps = kPerformThreads / 32;
+static_assert(kLoopWarps == 16 && kLoopItems * 32 < 256, "a key's warp counts are 16 bytes");
+constexpr size_t kLoopSmem = kKeyBins * 4 + size_t(kKeyBins) * kLoopWarps;
+static_assert(kLoopSmem >= 3 * kStageChunk * 4, "performPass's lists share the sort's memory");
+
+constexpr unsigned int kLoopRowsMax = 1024;
+
+// histogram rows and bin totals of passes of up to n candidates
+inline size_t loopHistWords(size_t n)
+{
+	return (std::min<size_t>(kLoopRowsMax, n / kPerformThreads + 1) + 1) * kKeyBins;
+}
+
+// sum of the first n of 16 bytes
+__device__ __forceinline__ unsigned int sumBytes(const uint4& v, unsigned int n)
+{
+	const unsigned int w[4] = {v.x, v.y, v.z, v.w};
+	unsigned int s = 0;
+#pragma unroll
+	for (unsigned int q = 0; q < 4; ++q)
+	{
+		const unsigned int m = n >= 4 * (q + 1) ? 0x01010101u : (n > 4 * q ? 0x01010101u >> (8 * (4 * (q + 1) - n)) : 0u);
+		s = __dp4a(w[q], m, s);
+	}
+	return s;
+}
+
+// block-wide exclusive scan; red: 33 words
+__device__ __forceinline__ unsigned int loopScan(unsigned int v, unsigned int* red, unsigned int& total)
+{
+	unsigned int t;
+	const unsigned int r = blockExclusiveScan<int(kPerformThreads)>(v, red, &t);
+	__syncthreads();
+	total = t;
+	return r;
+}
+
+// Phase 1 of the first pass: even runs of triangles.
+__device__ __forceinline__ BlockTriangles countFirst(const PassLoopArgs& a, const unsigned int* res, unsigned int tris, unsigned int (*sm)[33])
+{
+	const unsigned int per = (tris + gridDim.x - 1) / gridDim.x;
+	BlockTriangles mine;
+	mine.begin = min(tris, blockIdx.x * per);
+	mine.end = min(tris, mine.begin + per);
+	unsigned int picked = 0;
+	for (unsigned int base = mine.begin; base < mine.end; base += kPerformThreads)
+	{
+		const unsigned int t = base + threadIdx.x;
+		const bool valid = t < mine.end;
+		unsigned int v[3] = {0, 0, 0}, r[3] = {0, 0, 0};
+#pragma unroll
+		for (int c = 0; c < 3; ++c)
+			if (valid)
+				v[c] = ld<true>(res + (size_t)t * 3 + c), r[c] = __ldg(a.p.remap + v[c]);
+		picked += countTriangles(a, valid, t, v, r);
+	}
+	unsigned int z1 = 0, z2 = 0;
+	mine.picked = blockScan3(picked, z1, z2, sm).x;
+	return mine;
+}
+
+// phases 2 to 5: the pass's ranked, sorted candidates and its first window; false when there are none
+// (in.count is 0 then) or the grid failed
+__device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTriangles& mine, double window_factor, PassIn& in, GridSum& grid,
+    unsigned char* smem, unsigned int (*sm)[33])
+{
+	const PerformArgs& p = a.p;
+	Scalars* sc = p.sc;
+	const unsigned int* const res = in.res;
+	const unsigned int G = gridDim.x, B = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const unsigned int below = (1u << lane) - 1u;
+
+	if (tid == 0)
+		p.blk[B].z = mine.picked;
+	if (gtid() == 0)
+	{
+		sc->pick_trunc = ~0u;
+		sc->list_end = 0;
+		sc->cut = ~0ull;
+		sc->done = 0;
+		sc->skipped = 0;
+		sc->invalid = 0;
+	}
+	grid.wait();
+
+	// ---- 2: the block's vertices' lists, at a place taken with one add; its candidates
+	const unsigned int vper = (p.vcount + G - 1) / G;
+	const unsigned int vb0 = min(p.vcount, B * vper), vb1 = min(p.vcount, vb0 + vper);
+	unsigned int before = 0, all = 0, z = 0, run = 0, here = 0;
+	for (unsigned int q = tid; q < G; q += kPerformThreads)
+	{
+		const unsigned int x = __ldcg(&p.blk[q].z);
+		all += x;
+		before += q < B ? x : 0u;
+	}
+	unsigned int corners = 0;
+	for (unsigned int v = vb0 + tid; v < vb1; v += kPerformThreads)
+		corners += __ldcg(a.cnt + v);
+	const uint3 sums = blockScan3(before, all, z, sm);
+	loopScan(corners, sm[0], here);
+	__shared__ unsigned int s_lists;
+	if (tid == 0)
+		s_lists = here ? atomicAdd(&sc->list_end, here) : 0u;
+	resetVertices(p);
+	__syncthreads();
+	run = s_lists;
+	for (unsigned int base = vb0; base < vb1; base += kPerformThreads)
+	{
+		const unsigned int v = base + tid;
+		const unsigned int o = loopScan(v < vb1 ? __ldcg(a.cnt + v) : 0u, sm[0], here);
+		if (v < vb1)
+			a.adj_off[v] = run + o;
+		run += here;
+	}
+	run = sums.x;
+	const unsigned int capacity = __ldcg(&sc->capacity);
+	for (unsigned int base = mine.begin; base < mine.end; base += kPerformThreads)
+	{
+		const unsigned int t = base + tid;
+		const unsigned int code = t < mine.end ? a.codes[t] : 0u;
+		unsigned int o = run + loopScan(__popc(code & 0x49u), sm[0], here);
+		run += here;
+		// the capacity check at :1319-1320 stops at the first triangle that has no room for three
+		if (t < mine.end && (size_t)o + 3 > capacity)
+			atomicMin(&sc->pick_trunc, o);
+		else if (code)
+		{
+			const unsigned int tri[3] = {ld<true>(res + (size_t)t * 3), ld<true>(res + (size_t)t * 3 + 1), ld<true>(res + (size_t)t * 3 + 2)};
+#pragma unroll
+			for (int e = 0; e < 3; ++e)
+			{
+				const unsigned int f = (code >> (3 * e)) & 7u;
+				if (f & 1u)
+				{
+					const unsigned int x = tri[e], y = tri[e == 2 ? 0 : e + 1];
+					a.crec[o++] = (f & 4u) ? make_uint4(y, x, 0u, 0u) : make_uint4(x, y, (f >> 1) & 1u, 0u);
+				}
+			}
+		}
+	}
+	grid.wait();
+	const unsigned int C = min(sums.y, __ldcg(&sc->pick_trunc));
+	in.count = C;
+	if (C == 0 || grid.failed())
+		return false;
+	const double wf = window_factor * double(in.goal / 2) + 4096.0;
+	in.first_window = unsigned(double(C) < wf ? double(C) : wf);
+
+	// ---- 3: adjacency; the candidates ranked; the sorting blocks' key histograms
+	for (unsigned int t = mine.begin + tid; t < mine.end; t += kPerformThreads)
+	{
+		const size_t t3 = (size_t)t * 3;
+		const unsigned int v[3] = {__ldg(p.remap + ld<true>(res + t3)), __ldg(p.remap + ld<true>(res + t3 + 1)), __ldg(p.remap + ld<true>(res + t3 + 2))};
+#pragma unroll
+		for (int c = 0; c < 3; ++c)
+		{
+			const size_t at = size_t(ld<true>(a.adj_off + v[c])) + ld<true>(a.slot + t3 + c);
+			if (at < a.adj_cap) // in range whenever the counts are complete
+				a.adj[at] = make_uint2(v[c == 2 ? 0 : c + 1], v[c == 0 ? 2 : c - 1]);
+		}
+	}
+	const unsigned int rows = min(min(G, kLoopRowsMax), (C + kPerformThreads - 1) / kPerformThreads);
+	const unsigned int cper = (C + rows - 1) / rows;
+	const unsigned int cb0 = min(C, B * cper), cb1 = B < rows ? min(C, cb0 + cper) : cb0;
+	unsigned int* const bins = reinterpret_cast<unsigned int*>(smem);
+	if (B < rows)
+	{
+		for (unsigned int b = tid; b < kKeyBins; b += kPerformThreads)
+			bins[b] = 0;
+		__syncthreads();
+		for (unsigned int c = cb0 + tid; c < cb1; c += kPerformThreads)
+		{
+			uint4 rec, ring;
+			rankCandidate(ld<true>(a.crec + c), p.pos, p.vq, p.remap, p.wedge, a.kind, p.loop, p.loopback, a.adj_off, a.attr, p.aq, p.ag, p.ac, rec, ring, a.cnt);
+			a.crec[c] = rec;
+			a.cring[c] = ring;
+			atomicAdd(&bins[sortKey(rec.z)], 1u);
+		}
+		__syncthreads();
+		for (unsigned int b = tid; b < kKeyBins; b += kPerformThreads)
+			a.hist[(size_t)B * kKeyBins + b] = bins[b];
+	}
+	grid.wait();
+
+	// ---- 4: every bin's counts as prefixes over the rows, and its total: 32 bins per block, a run of
+	// rows per warp
+	unsigned int* const totals = a.hist + (size_t)rows * kKeyBins;
+	for (unsigned int g = B; g < kKeyBins / 32; g += G)
+	{
+		unsigned int* const part = reinterpret_cast<unsigned int*>(smem); // kLoopWarps x 32
+		const unsigned int rper = (rows + kLoopWarps - 1) / kLoopWarps;
+		const unsigned int r0 = min(rows, warp * rper), r1 = min(rows, r0 + rper);
+		unsigned int* const col = a.hist + g * 32 + lane;
+		unsigned int s = 0;
+#pragma unroll 4
+		for (unsigned int r = r0; r < r1; ++r)
+			s += __ldcg(col + (size_t)r * kKeyBins);
+		__syncthreads();
+		part[warp * 32 + lane] = s;
+		__syncthreads();
+		unsigned int at = 0, sum = 0;
+		for (unsigned int w = 0; w < kLoopWarps; ++w)
+		{
+			const unsigned int x = part[w * 32 + lane];
+			at += w < warp ? x : 0u;
+			sum += x;
+		}
+		if (warp == 0)
+			totals[g * 32 + lane] = sum;
+#pragma unroll 4
+		for (unsigned int r = r0; r < r1; ++r)
+		{
+			const unsigned int x = __ldcg(col + (size_t)r * kKeyBins);
+			col[(size_t)r * kKeyBins] = at;
+			at += x;
+		}
+	}
+	grid.wait();
+
+	// ---- 5: sorted positions, as kKeyScatter gives them; the first window's candidates mark their
+	// endpoints for the first decision round
+	if (B < rows)
+	{
+		unsigned int* const gbase = reinterpret_cast<unsigned int*>(smem);
+		unsigned char* const wcnt = smem + kKeyBins * 4; // per key, 16 warps: the step's count
+		constexpr unsigned int kPer = kKeyBins / kPerformThreads;
+		static_assert(kPer * kPerformThreads == kKeyBins, "bins divide among the threads");
+		unsigned int tot[kPer], s = 0;
+#pragma unroll
+		for (unsigned int q = 0; q < kPer; ++q)
+			tot[q] = __ldcg(totals + tid * kPer + q), s += tot[q];
+		unsigned int dummy, o = loopScan(s, sm[0], dummy);
+#pragma unroll
+		for (unsigned int q = 0; q < kPer; ++q)
+		{
+			gbase[tid * kPer + q] = o + __ldcg(a.hist + (size_t)B * kKeyBins + tid * kPer + q);
+			o += tot[q];
+		}
+		// a step's candidates per thread: as few as keep every warp busy
+		const unsigned int items = min(kLoopItems, (cb1 - cb0 + kPerformThreads - 1) / kPerformThreads);
+		for (unsigned int base = cb0; base < cb1; base += kPerformThreads * items)
+		{
+			uint4* const zero = reinterpret_cast<uint4*>(wcnt);
+			for (unsigned int b = tid; b < kKeyBins; b += kPerformThreads)
+				zero[b] = make_uint4(0, 0, 0, 0);
+			__syncthreads();
+			const unsigned int w0 = base + warp * 32 * items + lane;
+			unsigned int eb[kLoopItems], kd[kLoopItems], rk[kLoopItems];
+#pragma unroll
+			for (unsigned int q = 0; q < kLoopItems; ++q)
+			{
+				const unsigned int c = w0 + q * 32;
+				const uint2 zw = q < items && c < cb1 ? ld<true>(reinterpret_cast<const uint2*>(a.crec + c) + 1) : make_uint2(0, 0);
+				eb[q] = zw.x, kd[q] = zw.y;
+			}
+#pragma unroll
+			for (unsigned int q = 0; q < kLoopItems; ++q)
+				if (q < items)
+				{
+					const bool valid = w0 + q * 32 < cb1;
+					const unsigned int key = valid ? sortKey(eb[q]) : kKeyBins + lane;
+					const unsigned int peers = __match_any_sync(0xffffffffu, key);
+					const unsigned int leader = __ffs(peers) - 1;
+					unsigned int first = 0;
+					if (valid && lane == leader)
+					{
+						first = wcnt[key * kLoopWarps + warp];
+						wcnt[key * kLoopWarps + warp] = (unsigned char)(first + __popc(peers));
+					}
+					first = __shfl_sync(0xffffffffu, first, leader);
+					rk[q] = first + __popc(peers & below);
+					__syncwarp();
+				}
+			__syncthreads();
+#pragma unroll
+			for (unsigned int q = 0; q < kLoopItems; ++q)
+			{
+				const unsigned int c = w0 + q * 32;
+				if (q < items && c < cb1)
+				{
+					const unsigned int key = sortKey(eb[q]);
+					const unsigned int at = gbase[key] + sumBytes(reinterpret_cast<const uint4*>(wcnt)[key], warp) + rk[q];
+					a.rank[c] = at;
+					if (at < C) // in range whenever the histograms are complete
+					{
+						a.serr[at] = eb[q];
+						a.skind[at] = (unsigned char)kd[q];
+					}
+					if (at < in.first_window)
+						markCandidate(p, at, ld<true>(a.cring + c), in.round_base + 1);
+				}
+			}
+			__syncthreads();
+			if (base + kPerformThreads * items < cb1)
+				for (unsigned int b = tid; b < kKeyBins; b += kPerformThreads)
+					gbase[b] += sumBytes(reinterpret_cast<const uint4*>(wcnt)[b], kLoopWarps);
+		}
+	}
+	grid.wait();
+	return !grid.failed();
+}
+
+// PER_SM: resident blocks per SM it is compiled for (1: 128 registers, no spills; 2: twice the warps).
+// Whole calls with 1 / 2, in ms: heightfields of 40^2 0.56 / 0.58, 256^2 0.66 / 0.69, 400^2 0.84 / 0.84,
+// 560^2 1.15 / 1.08, 1100^2 3.25 / 2.61; attribute spheres of 131k triangles 1.18 / 1.21, 524k 2.25 /
+// 2.20, 2M 5.26 / 3.96; 20M terrain 46.3 / 35.9. A graph of per-phase kernels (recorded once, looping
+// on the device) took 0.63, 0.75, 0.90, 1.16, 2.64; 1.30, 2.36, 4.02; 36.4.
+template <int PER_SM>
+__global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArgs a)
+{
+	extern __shared__ __align__(16) unsigned char loop_smem[];
+	__shared__ unsigned int s_app[5];
+	__shared__ unsigned int s_grid[4];
+	__shared__ long long s_clock[10];
+	__shared__ unsigned int sm[3][33];
+	Scalars* sc = a.p.sc;
+	unsigned int* const lists = reinterpret_cast<unsigned int*>(loop_smem);
+	const PassShared sh = {{lists, lists + kStageChunk}, lists + 2 * kStageChunk, s_app, s_clock, sm};
+	const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
+	if (timer)
+		PhaseClock{s_clock}.start(sc);
+	GridSum grid;
+	grid.start(reinterpret_cast<unsigned long long*>(sc->bar), &sc->grid_error, s_grid);
+
+	const float scale = a.absolute ? __ldcg(&sc->extent) : 1.f;
+	const float error_limit = (a.target_error * a.target_error) / (scale * scale);
+	unsigned int indices = a.index_count, passes = a.passes, round_base = a.round_base;
+	const unsigned int* res = a.res;
+	unsigned int* res_next = a.res_next;
+	double window_factor = a.window_factor;
+	unsigned int stop = kLoopEnded;
+	BlockTriangles mine;
+	while (indices > a.target)
+	{
+		const unsigned int tris = indices / 3;
+		PassIn in;
+		in.tris = tris;
+		in.round_base = round_base;
+		in.prev_err = __ldcg(&sc->result_error_bits);
+		in.goal = (unsigned long long)(indices - a.target) / 3;
+		in.error_limit = error_limit;
+		in.res = res;
+		in.res_next = res_next;
+		if (passes == a.passes)
+			mine = countFirst(a, res, tris, sm);
+		if (!preparePass(a, mine, window_factor, in, grid, loop_smem, sm))
+			break;
+		const unsigned int C = in.count;
+		const unsigned long long goal = in.goal;
+		if (timer)
+			PhaseClock{s_clock}.skip();
+		unsigned int rounds = 0, kept = 0;
+		unsigned long long cutv = 0;
+		const int r = performPass<true>(a.p, &a, in, grid, sh, rounds, kept, cutv, mine);
+		if (r == kPassFailed)
+			break;
+		const unsigned int cut = cutv == ~0ull ? C : (unsigned int)(cutv >> 2);
+		const unsigned int evaluated = cut < C ? cut + 1 : C;
+		if (timer && passes < kMaxPassStats)
+		{
+			PassStats& ps = sc->pstats[passes];
+			ps.triangles = tris;
+			ps.candidates = C;
+			ps.evaluated = evaluated;
+			ps.done = sc->done;
+			ps.skipped = sc->skipped;
+			ps.invalid = sc->invalid;
+			ps.stop = cutv == ~0ull ? 0u : (unsigned int)(cutv & 3);
+			ps.rounds = rounds;
+			ps.active = (unsigned int)sc->active_sum;
+			ps.windows = sc->windows;
+		}
+		window_factor = nextWindowFactor(a.window_base, goal, evaluated);
+		round_base += rounds;
+		passes++;
+		if (r == kPassEmpty)
+			break;
+		indices = kept * 3;
+		const unsigned int* t = res;
+		res = res_next;
+		res_next = const_cast<unsigned int*>(t);
+		if (passes >= a.max_passes && indices > a.target)
+		{
+			if (timer)
+				atomicOr(&sc->grid_error, 4u);
+			break;
+		}
+		const unsigned int verr = a.p.ac ? __ldcg(&sc->vertex_error_bits) : __ldcg(&sc->result_error_bits);
+		if (a.prune && indices > a.target && a.prune_error <= __uint_as_float(verr))
+		{
+			stop = kLoopPrune;
+			break;
 		}
 	}
 	if (timer)
 	{
-		pc.lap(kPhEmit);
-		for (int i = 0; i < 8; ++i)
-			atomicAdd(&sc->phase_cycles[i], (unsigned long long)s_clock[i]);
+		reportPhases(sc, s_clock);
+		LoopState& lv = sc->live;
+		lv.res = res;
+		lv.res_next = res_next;
+		lv.indices = indices;
+		lv.passes = passes;
+		lv.round_base = round_base;
+		lv.window_factor = window_factor;
+		lv.stop = stop;
 	}
 }
 
@@ -2742,105 +3281,6 @@ __global__ void kFinalizeVertices(size_t n, const unsigned char* __restrict__ up
 		attributes[vi * astride_f + am.src[k]] = attr[vi * am.count + k] / am.weight[k];
 }
 
-// ---------------------------------------------------------------- device-resident pass loop
-//
-// The pass loop (src/simplifier.cpp:2493-2541) recorded once into a CUDA graph as the body of
-// a WHILE conditional node: every kernel of a pass reads the pass's counts from PassLive, the
-// grids cover the first (largest) pass, and kPassEnd decides on the device whether another
-// pass runs, so the loop needs no host round trip.
-
-// After the pick: the pass's candidate count, triangle goal and first window (the host loop's
-// arithmetic), and the per-pass resets of kPerform's scalars. No candidate ends the loop (the
-// host loop's break at C == 0).
-// the pass loop's squared error limit (:2489-2491) from the extent kMinMaxFinal left, with the
-// host's operations: target_error^2 / scale^2, scale = the extent for ErrorAbsolute, else 1
-__global__ void kErrorLimit(Scalars* sc, float target_error, int absolute)
-{
-	const float s = absolute ? sc->extent : 1.f;
-	sc->live.error_limit = (target_error * target_error) / (s * s);
-}
-
-__global__ void kPassPrep(Scalars* sc)
-{
-	PassLive& lv = sc->live;
-	if (lv.stop)
-		return;
-	unsigned int C = min(sc->pick_total, sc->pick_trunc);
-	lv.count = C;
-	if (C == 0)
-	{
-		lv.stop = 1;
-		return;
-	}
-	lv.sort_cells = keySortTiles(C, lv.sort_items) * kKeyBins;
-	unsigned long long goal = (unsigned long long)(lv.indices - lv.target) / 3;
-	lv.goal = goal;
-	double wf = lv.window_factor * double(goal / 2) + 4096.0;
-	lv.first_window = unsigned(double(C) < wf ? double(C) : wf);
-	for (int i = 0; i < 4; ++i)
-		sc->bar[i] = 0;
-	sc->grid_error = 0;
-	sc->cut = ~0ull;
-	sc->done = 0;
-	sc->skipped = 0;
-	sc->invalid = 0;
-}
-
-// After kPerform: the pass's counters (as the host loop records them), the next pass's index
-// buffer and counts, and the loop condition.
-__global__ void kPassEnd(Scalars* sc, cudaGraphConditionalHandle handle, unsigned int max_passes)
-{
-	PassLive& lv = sc->live;
-	lv.iterations++;
-	if (!lv.stop)
-	{
-		if (sc->grid_error || sc->scan_error)
-			lv.stop = 1; // reported by the host after the loop
-		else
-		{
-			const unsigned long long cutv = sc->cut;
-			const unsigned int C = lv.count;
-			const unsigned int cut = cutv == ~0ull ? C : (unsigned int)(cutv >> 2);
-			if (lv.passes < kMaxPassStats)
-			{
-				PassStats& ps = sc->pstats[lv.passes];
-				ps.triangles = lv.tris;
-				ps.candidates = C;
-				ps.evaluated = cut < C ? cut + 1 : C;
-				ps.done = sc->done;
-				ps.skipped = sc->skipped;
-				ps.invalid = sc->invalid;
-				ps.stop = cutv == ~0ull ? 0u : (unsigned int)(cutv & 3);
-				ps.rounds = sc->rounds;
-				ps.active = (unsigned int)sc->active_sum;
-				ps.windows = sc->windows;
-			}
-			lv.window_factor = nextWindowFactor(lv.window_base, lv.goal, cut < C ? cut + 1 : C);
-			lv.round_base += sc->rounds;
-			lv.passes++;
-			if (sc->done == 0)
-				lv.stop = 1;
-			else
-			{
-				lv.tris = sc->tri_total;
-				lv.indices = sc->tri_total * 3;
-				const unsigned int* r = lv.res;
-				lv.res = lv.res_next;
-				lv.res_next = const_cast<unsigned int*>(r);
-				if (lv.indices <= lv.target)
-					lv.stop = 1;
-				else if (lv.passes >= max_passes)
-				{
-					lv.stop = 1;
-					sc->grid_error |= 4u;
-				}
-			}
-		}
-	}
-	cudaGraphSetConditional(handle, lv.stop ? 0u : 1u);
-}
-
-
 // a component's root is its smallest primary vertex, as the reference's union-find leaves it
 __global__ void kUnionEdges(const unsigned int* __restrict__ idx, size_t tris, const unsigned int* __restrict__ remap, unsigned int* parent)
 {
@@ -3077,7 +3517,6 @@ struct Work
 	uint4* blk;
 	unsigned int* blkcnt;
 	unsigned int* scratch;
-	unsigned int* scratch2; // the pick's block-count scan, beside the adjacency scan in the pass loop
 	unsigned int hash_mask;
 	// the update mode only
 	float4* vg;              // volume gradients (with attributes)
@@ -3165,9 +3604,8 @@ size_t layout(Work& w, char* base, size_t I, size_t V, size_t ac, bool solve = f
 	w.cr = c.take<unsigned int>(Vp);
 	w.blk = c.take<uint4>(std::max<size_t>(cap / kStopTile + 2, 8192)); // >= blocks of any cooperative launch
 	w.blkcnt = c.take<unsigned int>(T / kThreads + 2);
-	size_t sw = std::max(std::max(scanScratchWords(I + Vp + 2), radixScratchWords(big)), std::max(scanScratchWords(T + 2), keySortScratchWords(cap)));
+	size_t sw = std::max(std::max(scanScratchWords(I + Vp + 2), radixScratchWords(big)), std::max(std::max(scanScratchWords(T + 2), keySortScratchWords(cap)), loopHistWords(cap)));
 	w.scratch = c.take<unsigned int>(sw);
-	w.scratch2 = c.take<unsigned int>(scanScratchWords(T / kThreads + 2));
 	const size_t Vs = solve ? Vp : 0;
 	w.vg = (solve && ac) ? c.take<float4>(Vp) : nullptr;
 	w.pos_new = c.take<float4>(Vs);
@@ -3186,12 +3624,10 @@ int bitsFor(size_t maxval)
 	return b;
 }
 
-// The pass's counting sort (kKeyHist, scan, kKeyScatter) of up to n candidates, in tiles of
-// items * 256 (items: 4, 8 or 16): their sorted positions into w.rank, the error bits and kinds by
-// sorted position into w.serr and w.skind. lv: the device-resident loop's live state (the grids
-// cover n; the kernels and the scan take the live count from it, whose sort_items must equal
-// items), else nullptr.
-void sortCandidates(const Work& w, size_t n, cudaStream_t stream, const PassLive* lv, ScanSync ss, unsigned int items)
+// The pass's counting sort (kKeyHist, scan, kKeyScatter) of n candidates, in tiles of items * 256
+// (items: 4, 8 or 16): their sorted positions into w.rank, the error bits and kinds by sorted position
+// into w.serr and w.skind.
+void sortCandidates(const Work& w, size_t n, cudaStream_t stream, ScanSync ss, unsigned int items)
 {
 	if (n == 0)
 		return;
@@ -3199,21 +3635,19 @@ void sortCandidates(const Work& w, size_t n, cudaStream_t stream, const PassLive
 	const size_t m = size_t(tiles) * kKeyBins;
 	unsigned int* hist = w.scratch;
 	unsigned int* sscratch = w.scratch + ((m + 63) & ~size_t(63));
-	if (lv)
-		ss.n_dev = &lv->sort_cells;
 	if (items == 4)
-		MO_LAUNCH(kKeyHist<4>, tiles, kThreads, 0, stream, w.cerr, n, hist, lv);
+		MO_LAUNCH(kKeyHist<4>, tiles, kThreads, 0, stream, w.cerr, n, hist);
 	else if (items == 8)
-		MO_LAUNCH(kKeyHist<8>, tiles, kThreads, 0, stream, w.cerr, n, hist, lv);
+		MO_LAUNCH(kKeyHist<8>, tiles, kThreads, 0, stream, w.cerr, n, hist);
 	else
-		MO_LAUNCH(kKeyHist<16>, tiles, kThreads, 0, stream, w.cerr, n, hist, lv);
+		MO_LAUNCH(kKeyHist<16>, tiles, kThreads, 0, stream, w.cerr, n, hist);
 	scanExclusive(hist, hist, m, nullptr, sscratch, stream, ss);
 	if (items == 4)
-		MO_LAUNCH(kKeyScatter<4>, tiles, kThreads, kKeyScatterSmem, stream, w.cerr, w.ckind, n, hist, w.rank, w.serr, w.skind, lv);
+		MO_LAUNCH(kKeyScatter<4>, tiles, kThreads, kKeyScatterSmem, stream, w.cerr, w.ckind, n, hist, w.rank, w.serr, w.skind);
 	else if (items == 8)
-		MO_LAUNCH(kKeyScatter<8>, tiles, kThreads, kKeyScatterSmem, stream, w.cerr, w.ckind, n, hist, w.rank, w.serr, w.skind, lv);
+		MO_LAUNCH(kKeyScatter<8>, tiles, kThreads, kKeyScatterSmem, stream, w.cerr, w.ckind, n, hist, w.rank, w.serr, w.skind);
 	else
-		MO_LAUNCH(kKeyScatter<16>, tiles, kThreads, kKeyScatterSmem, stream, w.cerr, w.ckind, n, hist, w.rank, w.serr, w.skind, lv);
+		MO_LAUNCH(kKeyScatter<16>, tiles, kThreads, kKeyScatterSmem, stream, w.cerr, w.ckind, n, hist, w.rank, w.serr, w.skind);
 }
 
 } // namespace
@@ -3263,13 +3697,14 @@ Simplifier::Simplifier(int device) : device_(device)
 {
 	MO_CUDA_CHECK(cudaSetDevice(device));
 	MO_CUDA_CHECK(cudaMallocHost(&pinned_, kPinnedBytes));
-	MO_CUDA_CHECK(cudaStreamCreateWithFlags(&capture_, cudaStreamNonBlocking));
-	MO_CUDA_CHECK(cudaStreamCreateWithFlags(&capture2_, cudaStreamNonBlocking));
-	MO_CUDA_CHECK(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
-	MO_CUDA_CHECK(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
 	int sms = 0, per_sm = 0;
 	MO_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
 	MO_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kPerform, kPerformThreads, 0));
+	MO_CUDA_CHECK(cudaFuncSetAttribute(kPassLoop<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kLoopSmem)));
+	MO_CUDA_CHECK(cudaFuncSetAttribute(kPassLoop<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kLoopSmem)));
+	int loop_per_sm = 0;
+	MO_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&loop_per_sm, kPassLoop<2>, kPerformThreads, kLoopSmem));
+	per_sm = std::min(per_sm, loop_per_sm);
 	MO_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&solve_per_sm_, kSolvePositions, kThreads, 0));
 	MO_CUDA_CHECK(cudaFuncSetAttribute(kKeyScatter<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKeyScatterSmem)));
 	MO_CUDA_CHECK(cudaFuncSetAttribute(kKeyScatter<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKeyScatterSmem)));
@@ -3278,8 +3713,17 @@ Simplifier::Simplifier(int device) : device_(device)
 	sms_ = sms;
 	coop_blocks_ = unsigned(std::max(1, sms * std::max(per_sm, 1)));
 	tuning_ = Tuning::fromEnvironment();
-	perform_blocks_ = std::min(coop_blocks_, unsigned(std::max(1, sms * tuning_.perform_blocks_per_sm)));
-	coopScanCapacity(); // cached now: the pass loop's scans may first run while it is recorded
+}
+
+// Up to here the pass loop runs one block per SM where nothing says otherwise: the sides are measured at
+// kPassLoop.
+constexpr size_t kOnePerSmMax = 1000000;
+
+int Simplifier::passBlocksPerSM(size_t index_count) const
+{
+	if (tuning_.perform_blocks_per_sm > 0)
+		return std::min(tuning_.perform_blocks_per_sm, performBlocksPerSMMax());
+	return index_count <= kOnePerSmMax && tuning_.perform_grid_cap == 0 ? 1 : performBlocksPerSMMax();
 }
 
 unsigned int Simplifier::performGridCap() const
@@ -3287,26 +3731,8 @@ unsigned int Simplifier::performGridCap() const
 	return std::max(1u, unsigned(tuning_.perform_grid_cap) * 256u / kPerformThreads);
 }
 
-void Simplifier::dropLoopGraph()
-{
-	if (loop_.exec)
-		cudaGraphExecDestroy(loop_.exec);
-	if (loop_.graph)
-		cudaGraphDestroy(loop_.graph);
-	loop_ = LoopGraph{};
-}
-
 Simplifier::~Simplifier()
 {
-	dropLoopGraph();
-	if (capture_)
-		cudaStreamDestroy(capture_);
-	if (capture2_)
-		cudaStreamDestroy(capture2_);
-	if (fork_)
-		cudaEventDestroy(fork_);
-	if (join_)
-		cudaEventDestroy(join_);
 	if (pinned_)
 		cudaFreeHost(pinned_);
 }
@@ -3527,7 +3953,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		// rebuild the dup flags (the scan consumed them) into cnt, then compact
 		MO_LAUNCH(kHashRemap, gV, kThreads, 0, stream, w.table, w.slot, V, w.remap, w.wedge, w.cnt);
 		MO_LAUNCH(kCompactFlagged, gV, kThreads, 0, stream, w.cnt, w.flags, w.remap, V, w.keys_b, w.vals_b);
-		radixSortPairs(w.keys_b, w.vals_b, w.keys_a, w.vals_a, w.cerr, reinterpret_cast<unsigned int*>(w.crec), D, bitsFor(V), w.scratch, stream, nullptr, ss);
+		radixSortPairs(w.keys_b, w.vals_b, w.keys_a, w.vals_a, w.cerr, reinterpret_cast<unsigned int*>(w.crec), D, bitsFor(V), w.scratch, stream, ss);
 		MO_LAUNCH(kWedgeLink, gridFor(D, kThreads), kThreads, 0, stream, w.keys_a, w.vals_a, D, w.wedge);
 	}
 
@@ -3544,7 +3970,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	else
 	{
 		// a vertex with many corners: a stable radix sort by vertex
-		radixSortPairs(w.res0, nullptr, w.keys_a, w.csr_raw, w.keys_b, w.vals_b, I, vbits, w.scratch, stream, nullptr, ss);
+		radixSortPairs(w.res0, nullptr, w.keys_a, w.csr_raw, w.keys_b, w.vals_b, I, vbits, w.scratch, stream, ss);
 	}
 
 	// classification
@@ -3612,7 +4038,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		MO_CUDA_CHECK(cudaMemsetAsync(w.cnt, 0, (comp_count + 1) * 4, stream));
 		MO_LAUNCH(kCountKeys, gV, kThreads, 0, stream, w.comp, nullptr, V, w.cnt);
 		scanExclusive(w.cnt, w.comp_off, comp_count + 1, nullptr, w.scratch, stream, ss);
-		radixSortPairs(w.comp, nullptr, w.keys_a, w.vals_a, w.keys_b, w.vals_b, V, bitsFor(comp_count ? comp_count - 1 : 0), w.scratch, stream, nullptr, ss);
+		radixSortPairs(w.comp, nullptr, w.keys_a, w.vals_a, w.keys_b, w.vals_b, V, bitsFor(comp_count ? comp_count - 1 : 0), w.scratch, stream, ss);
 		MO_LAUNCH(kMeasureComponents, gridFor(comp_count, kMeasureWarps), kMeasureWarps * 32, 0, stream, comp_count, w.comp_off, w.vals_a, w.pos, w.comp_err);
 	}
 	if (V)
@@ -3620,11 +4046,9 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	MO_LAUNCH(kCapacity, 1, 32, 0, stream, I, w.sc);
 	MO_CUDA_CHECK(cudaGetLastError());
 
-	// The device-resident pass loop (below) takes no host values from setup: its graph is
-	// recorded and instantiated while the setup kernels run, and the extent is read after it.
-	// Pruning, the debug bit and per-phase event timing need the host between passes.
-	const bool device_loop =
-	    tuning_.device_loop && !timed && !dump && !(m.options & (kOptPrune | kOptInternalDebug)) && I > m.target_index_count;
+	// The one-launch pass loop (below) takes no host values from setup, so it is queued behind it and the
+	// extent is read afterwards. The debug bit and per-phase event timing need the host between passes.
+	const bool one_launch = tuning_.device_loop && !timed && !dump && !(m.options & kOptInternalDebug) && I > m.target_index_count;
 	float vertex_scale = 0.f, error_scale = 1.f, error_limit = 0.f;
 	auto takeScale = [&]() {
 		vertex_scale = hs->extent;
@@ -3632,7 +4056,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		error_scale = (m.options & kOptErrorAbsolute) ? vertex_scale : 1.f;
 		error_limit = (m.target_error * m.target_error) / (error_scale * error_scale);
 	};
-	if (!device_loop)
+	if (!one_launch || (m.options & kOptPrune))
 	{
 		readScalars();
 		takeScale();
@@ -3717,183 +4141,118 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	else if (m.options & kOptPrune)
 		comp_next = FLT_MAX;
 	int passes = 0;
-	double window_factor = tuning_.window_factor; // the host loop's first-window factor, as kPassEnd adapts it
+	double window_factor = tuning_.window_factor; // the first window of the next pass
 	unsigned int round_base = 0; // decision rounds are numbered across the run (mark tags never repeat)
 
-	// ---- the pass loop on the device: one pass recorded into the body of a WHILE conditional
-	// node, replayed until kPassEnd ends it
-	if (device_loop)
-	{
-		// grids cover the capacity bound (boundEdgeCollapses <= I + 3); the kernels stop at the
-		// live counts
-		const size_t T0 = I / 3, capn = I + 3;
-		PassLive init{};
-		init.res = w.res0;
-		init.res_next = w.res1;
-		init.indices = unsigned(I);
-		init.tris = unsigned(T0);
-		init.target = unsigned(m.target_index_count);
-		const unsigned int sort_items = sort_items_ ? sort_items_ : keySortItems(capn);
-		init.sort_items = sort_items;
-		init.window_factor = tuning_.window_factor;
-		init.window_base = tuning_.window_factor;
-		MO_CUDA_CHECK(cudaMemcpyAsync(&w.sc->live, &init, sizeof(init), cudaMemcpyHostToDevice, stream));
-		MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->result_error_bits, 0, 4, stream));
-		MO_LAUNCH(kErrorLimit, 1, 1, 0, stream, w.sc, m.target_error, (m.options & kOptErrorAbsolute) ? 1 : 0);
-		const PassLive* lv = &w.sc->live;
-
-		// grid of the pass kernel
-		unsigned int blocks = std::max(1u, std::min(perform_blocks_, gridFor(std::max(std::max(capn, V), T0), kPerformThreads)));
+	// the pass kernel's arguments but for the pass's own values
+	auto performArgs = [&]() {
+		PerformArgs pa{};
+		pa.crec = w.crec;
+		pa.cring = w.cring;
+		pa.rank = w.rank;
+		pa.skind = w.skind;
+		pa.serr = w.serr;
+		pa.status = w.status;
+		pa.vcount = unsigned(V);
+		pa.minT[0] = w.minT;
+		pa.minT[1] = w.minT + (V + 1);
+		pa.minS = w.minS;
+		pa.cr = w.cr;
+		pa.list[0] = w.act0;
+		pa.list[1] = w.act1;
+		pa.commits = w.commits;
+		pa.adj_off = w.adj_off;
+		pa.adj = w.adj;
+		pa.pos = w.pos;
+		pa.remap = w.remap;
+		pa.wedge = w.wedge;
+		pa.loop = w.loop;
+		pa.loopback = w.loopback;
+		pa.vq = w.vq;
+		pa.aq = w.aq;
+		pa.ag = w.ag;
+		pa.ac = ac;
+		pa.vg = (solve && ac) ? w.vg : nullptr;
+		pa.blk = w.blk;
+		pa.sc = w.sc;
+		return pa;
+	};
+	// the grid of the pass kernels for up to n items in a phase
+	const int per_sm = passBlocksPerSM(I);
+	auto performGrid = [&](size_t n) {
+		unsigned int blocks = std::max(1u, std::min(unsigned(per_sm * sms_), gridFor(n, kPerformThreads)));
 		if (tuning_.perform_grid_cap > 0)
 			blocks = std::min(blocks, performGridCap());
 		if (size_t(blocks) * kPerformThreads > kListSlack)
 			throw std::runtime_error("kPerform grid exceeds the candidate list slack");
+		return blocks;
+	};
 
-		LaunchProbe& lp = probe();
-		const bool reuse = loop_.exec && loop_.base == arena_.base() && loop_.I == I && loop_.V == V && loop_.ac == ac && loop_.solve == solve &&
-		                   loop_.blocks == blocks && loop_.sort_items == sort_items && loop_.scan_blocks == ss.max_blocks;
-		if (!reuse)
+	// ---- the pass loop in one launch (several with pruning, which the host runs between passes)
+	if (one_launch)
+	{
+		PassLoopArgs la{};
+		la.p = performArgs();
+		la.cnt = w.cnt;
+		la.slot = w.csr_raw; // setup is done with it
+		la.adj_off = w.adj_off;
+		la.adj = w.adj;
+		la.adj_cap = I;
+		la.codes = pick_codes;
+		la.crec = w.crec;
+		la.cring = w.cring;
+		la.rank = w.rank;
+		la.serr = w.serr;
+		la.skind = w.skind;
+		la.kind = w.kind;
+		la.attr = w.attr;
+		la.hist = w.scratch;
+		la.target = unsigned(m.target_index_count);
+		la.max_passes = unsigned(I / 3 + 1);
+		la.window_base = tuning_.window_factor;
+		la.target_error = m.target_error;
+		la.absolute = (m.options & kOptErrorAbsolute) ? 1 : 0;
+		la.prune = (m.options & kOptPrune) ? 1 : 0;
+		MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->result_error_bits, 0, 4, stream));
+		while (result_count > m.target_index_count)
 		{
-			dropLoopGraph();
-			// the new graph and its executable are released if recording or instantiation fails
-			struct GraphGuard
-			{
-				cudaGraph_t graph = nullptr;
-				cudaGraphExec_t exec = nullptr;
-				~GraphGuard()
-				{
-					if (exec)
-						cudaGraphExecDestroy(exec);
-					if (graph)
-						cudaGraphDestroy(graph);
-				}
-			} guard;
-			MO_CUDA_CHECK(cudaGraphCreate(&guard.graph, 0));
-			cudaGraph_t graph = guard.graph;
-			cudaGraphConditionalHandle handle;
-			MO_CUDA_CHECK(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
-			cudaGraphNodeParams cp = {};
-			cp.type = cudaGraphNodeTypeConditional;
-			cp.conditional.handle = handle;
-			cp.conditional.type = cudaGraphCondTypeWhile;
-			cp.conditional.size = 1;
-			cudaGraphNode_t loop_node;
-			MO_CUDA_CHECK(cudaGraphAddNode(&loop_node, graph, nullptr, nullptr, 0, &cp));
-			cudaGraph_t body = cp.conditional.phGraph_out[0];
-
-			const unsigned long long launches0 = lp.launches;
-			cudaStream_t cs = capture_; // recording only: nothing runs on it
-			MO_CUDA_CHECK(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-			lp.capturing = true;
-			try
-			{
-				const unsigned int gI = gridFor(I, kThreads), gT0 = gridFor(T0, kThreads);
-				// the pick (its own scan scratch and barrier words) and the adjacency are independent:
-				// two branches of the body, joined before the rank
-				cudaStream_t cs2 = capture2_;
-				ScanSync ss2 = ss;
-				ss2.bar = w.sc->scan_bar2;
-				MO_CUDA_CHECK(cudaEventRecord(fork_, cs));
-				MO_CUDA_CHECK(cudaStreamWaitEvent(cs2, fork_, 0));
-				MO_LAUNCH(kPickCount, gT0, kThreads, 0, cs2, nullptr, T0, w.remap, w.kind, w.loop, w.loopback, w.tcnt, pick_codes, lv);
-				scanExclusive(w.tcnt, w.tcnt, gT0, &w.sc->pick_total, w.scratch2, cs2, ss2);
-				MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->pick_trunc, 0xFF, 4, cs2));
-				MO_LAUNCH(kPickEmit, gT0, kThreads, 0, cs2, nullptr, T0, pick_codes, w.tcnt, w.sc, w.crec, lv);
-				MO_CUDA_CHECK(cudaEventRecord(join_, cs2));
-				MO_CUDA_CHECK(cudaMemsetAsync(w.cnt, 0, (V + 1) * 4, cs));
-				MO_LAUNCH(kCountCorners, gI, kThreads, 0, cs, nullptr, I, w.remap, w.cnt, nullptr, lv);
-				scanExclusive(w.cnt, w.adj_off, V + 1, nullptr, w.scratch, cs, ss);
-				MO_LAUNCH(kAdjFill, gT0, kThreads, 0, cs, nullptr, T0, w.remap, w.adj_off, nullptr, w.adj, lv, I);
-				MO_CUDA_CHECK(cudaStreamWaitEvent(cs, join_, 0));
-				MO_LAUNCH(kPassPrep, 1, 1, 0, cs, w.sc);
-				MO_LAUNCH(kRank, gridFor(capn, kRankThreads), kRankThreads, 0, cs, capn, w.crec, w.cring, w.cerr, w.ckind, w.pos, w.vq, w.remap, w.wedge, w.kind, w.loop, w.loopback,
-				    w.adj_off, w.attr, w.aq, w.ag, ac, lv);
-				sortCandidates(w, capn, cs, lv, ss, sort_items);
-				PerformArgs pa;
-				pa.count = 0;
-				pa.crec = w.crec;
-				pa.cring = w.cring;
-				pa.rank = w.rank;
-				pa.skind = w.skind;
-				pa.serr = w.serr;
-				pa.status = w.status;
-				pa.vcount = unsigned(V);
-				pa.minT[0] = w.minT;
-				pa.minT[1] = w.minT + (V + 1);
-				pa.minS = w.minS;
-				pa.cr = w.cr;
-				pa.list[0] = w.act0;
-				pa.list[1] = w.act1;
-				pa.commits = w.commits;
-				pa.adj_off = w.adj_off;
-				pa.adj = w.adj;
-				pa.pos = w.pos;
-				pa.remap = w.remap;
-				pa.wedge = w.wedge;
-				pa.loop = w.loop;
-				pa.loopback = w.loopback;
-				pa.vq = w.vq;
-				pa.aq = w.aq;
-				pa.ag = w.ag;
-				pa.ac = ac;
-				pa.vg = (solve && ac) ? w.vg : nullptr;
-				pa.prev_err_bits = 0;
-				pa.error_limit = 0.f; // the live state's
-				pa.goal = 0;
-				pa.first_window = 0;
-				pa.round_base = 0;
-				pa.res = nullptr;
-				pa.res_next = nullptr;
-				pa.tris = 0;
-				pa.blk = w.blk;
-				pa.sc = w.sc;
-				pa.live = lv;
-				void* params[] = {&pa};
-				lp.launches++;
-				MO_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kPerform, dim3(blocks), dim3(kPerformThreads), params, 0, cs));
-				MO_LAUNCH(kPassEnd, 1, 1, 0, cs, w.sc, handle, unsigned(T0 + 1));
-			}
-			catch (...)
-			{
-				lp.capturing = false;
-				cudaGraph_t dead = nullptr;
-				cudaStreamEndCapture(cs, &dead);
-				throw;
-			}
-			lp.capturing = false;
-			cudaGraph_t captured = nullptr;
-			MO_CUDA_CHECK(cudaStreamEndCapture(cs, &captured));
-			MO_CUDA_CHECK(cudaGraphInstantiate(&guard.exec, graph, 0));
-			loop_.body_launches = lp.launches - launches0;
-			lp.launches = launches0; // counted below, once per replay
-			loop_.graph = guard.graph;
-			loop_.exec = guard.exec;
-			guard.graph = nullptr;
-			guard.exec = nullptr;
-			loop_.base = arena_.base();
-			loop_.I = I;
-			loop_.V = V;
-			loop_.ac = ac;
-			loop_.solve = solve;
-			loop_.blocks = blocks;
-			loop_.sort_items = sort_items;
-			loop_.scan_blocks = ss.max_blocks;
+			la.index_count = unsigned(result_count);
+			la.passes = unsigned(passes);
+			la.round_base = round_base;
+			la.window_factor = window_factor;
+			la.res = res;
+			la.res_next = res_next;
+			la.prune_error = comp_next;
+			MO_CUDA_CHECK(cudaMemsetAsync(w.cnt, 0, (V + 1) * 4, stream));
+			MO_CUDA_CHECK(cudaMemsetAsync(w.sc->bar, 0, sizeof(unsigned int) * 5, stream));
+			void* params[] = {&la};
+			cudaEvent_t e0 = probeBegin("kPassLoop", stream);
+			MO_CUDA_CHECK(cudaLaunchCooperativeKernel(per_sm == 1 ? (const void*)kPassLoop<1> : (const void*)kPassLoop<2>, dim3(performGrid(std::max(result_count, V))),
+			    dim3(kPerformThreads), params, kLoopSmem, stream));
+			probeEnd(e0, stream);
+			readScalars();
+			if (!(m.options & kOptPrune))
+				takeScale();
+			if (hs->grid_error)
+				throw std::runtime_error(hs->grid_error & 4 ? "pass loop did not converge"
+				                                            : (hs->grid_error & 2 ? "collapse decision round made no progress" : "grid barrier wait limit reached"));
+			passes = int(hs->live.passes);
+			round_base = hs->live.round_base;
+			window_factor = hs->live.window_factor;
+			result_count = hs->live.indices;
+			res = const_cast<unsigned int*>(hs->live.res);
+			res_next = hs->live.res_next;
+			result_error_bits = hs->result_error_bits;
+			vertex_error = ac == 0 ? __uint_as_float_host(result_error_bits) : __uint_as_float_host(hs->vertex_error_bits);
+			if (hs->live.stop != kLoopPrune)
+				break;
+			prune(vertex_error);
 		}
-		MO_CUDA_CHECK(cudaGraphLaunch(loop_.exec, stream));
-		readScalars();
-		takeScale();
-		lp.launches += loop_.body_launches * hs->live.iterations;
-		if (hs->grid_error)
-			throw std::runtime_error(hs->grid_error & 4 ? "pass loop did not converge"
-			                                            : (hs->grid_error & 2 ? "collapse decision round made no progress" : "grid barrier wait limit reached"));
-		passes = int(hs->live.passes);
 		for (int p = 0; p < passes && p < kMaxPassStats; ++p)
 			rr.pass[p] = hs->pstats[p];
-		result_error_bits = hs->result_error_bits;
-		result_count = hs->live.indices;
-		res = const_cast<unsigned int*>(hs->live.res);
 	}
 	else
+	// ---- the pass loop from the host: a launch per phase, read back twice per pass
 	while (result_count > m.target_index_count)
 	{
 		const size_t T = result_count / 3;
@@ -3903,17 +4262,17 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 
 		// adjacency of the current result, welded by remap
 		MO_CUDA_CHECK(cudaMemsetAsync(w.cnt, 0, (V + 1) * 4, stream));
-		MO_LAUNCH(kCountCorners, gridFor(result_count, kThreads), kThreads, 0, stream, res, result_count, w.remap, w.cnt, res_next, nullptr);
+		MO_LAUNCH(kCountCorners, gridFor(result_count, kThreads), kThreads, 0, stream, res, result_count, w.remap, w.cnt, res_next);
 		scanExclusive(w.cnt, w.adj_off, V + 1, nullptr, w.scratch, stream, ss);
-		MO_LAUNCH(kAdjFill, gT, kThreads, 0, stream, res, T, w.remap, w.adj_off, res_next, w.adj, nullptr, I);
+		MO_LAUNCH(kAdjFill, gT, kThreads, 0, stream, res, T, w.remap, w.adj_off, res_next, w.adj, I);
 		if (timed)
 			MO_CUDA_CHECK(cudaEventRecord(ev[3], stream));
 
 		// pick
-		MO_LAUNCH(kPickCount, gT, kThreads, 0, stream, res, T, w.remap, w.kind, w.loop, w.loopback, w.tcnt, pick_codes, nullptr);
+		MO_LAUNCH(kPickCount, gT, kThreads, 0, stream, res, T, w.remap, w.kind, w.loop, w.loopback, w.tcnt, pick_codes);
 		scanExclusive(w.tcnt, w.tcnt, gT, &w.sc->pick_total, w.scratch, stream, ss);
 		MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->pick_trunc, 0xFF, 4, stream));
-		MO_LAUNCH(kPickEmit, gT, kThreads, 0, stream, res, T, pick_codes, w.tcnt, w.sc, w.crec, nullptr);
+		MO_LAUNCH(kPickEmit, gT, kThreads, 0, stream, res, T, pick_codes, w.tcnt, w.sc, w.crec);
 		readScalars();
 		const size_t C = std::min<size_t>(hs->pick_total, hs->pick_trunc);
 		if (timed)
@@ -3923,44 +4282,18 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 
 		// rank + sort
 		MO_LAUNCH(kRank, gridFor(C, kRankThreads), kRankThreads, 0, stream, C, w.crec, w.cring, w.cerr, w.ckind, w.pos, w.vq, w.remap, w.wedge, w.kind, w.loop, w.loopback,
-		    w.adj_off, w.attr, w.aq, w.ag, ac, nullptr);
+		    w.adj_off, w.attr, w.aq, w.ag, ac);
 		if (timed)
 			MO_CUDA_CHECK(cudaEventRecord(ev[5], stream));
-		sortCandidates(w, C, stream, nullptr, ss, sort_items_ ? sort_items_ : keySortItems(C));
+		sortCandidates(w, C, stream, ss, keySortItems(C));
 		if (timed)
 			MO_CUDA_CHECK(cudaEventRecord(ev[6], stream));
 
 		// perform: decisions, stop rules, apply, loop remap and compaction in one cooperative launch
 		const size_t goal = (result_count - m.target_index_count) / 3;
 		{
-			PerformArgs pa;
+			PerformArgs pa = performArgs();
 			pa.count = unsigned(C);
-			pa.crec = w.crec;
-			pa.cring = w.cring;
-			pa.rank = w.rank;
-			pa.skind = w.skind;
-			pa.serr = w.serr;
-			pa.status = w.status;
-			pa.vcount = unsigned(V);
-			pa.minT[0] = w.minT;
-			pa.minT[1] = w.minT + (V + 1);
-			pa.minS = w.minS;
-			pa.cr = w.cr;
-			pa.list[0] = w.act0;
-			pa.list[1] = w.act1;
-			pa.commits = w.commits;
-			pa.adj_off = w.adj_off;
-			pa.adj = w.adj;
-			pa.pos = w.pos;
-			pa.remap = w.remap;
-			pa.wedge = w.wedge;
-			pa.loop = w.loop;
-			pa.loopback = w.loopback;
-			pa.vq = w.vq;
-			pa.aq = w.aq;
-			pa.ag = w.ag;
-			pa.ac = ac;
-			pa.vg = (solve && ac) ? w.vg : nullptr;
 			pa.prev_err_bits = result_error_bits;
 			pa.error_limit = error_limit;
 			pa.goal = goal;
@@ -3970,19 +4303,11 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 			pa.res = res;
 			pa.res_next = res_next;
 			pa.tris = unsigned(T);
-			pa.blk = w.blk;
-			pa.live = nullptr;
-			pa.sc = w.sc;
 			MO_CUDA_CHECK(cudaMemsetAsync(w.sc->bar, 0, sizeof(unsigned int) * 5, stream));
 			MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->cut, 0xFF, 8, stream));
 			MO_CUDA_CHECK(cudaMemsetAsync(&w.sc->done, 0, 12, stream));
 			MO_CUDA_CHECK(cudaMemcpyAsync(&w.sc->result_error_bits, &result_error_bits, 4, cudaMemcpyHostToDevice, stream));
-			unsigned int want = gridFor(std::max(std::max(C, V), T), kPerformThreads);
-			unsigned int blocks = std::max(1u, std::min(perform_blocks_, want));
-			if (tuning_.perform_grid_cap > 0)
-				blocks = std::min(blocks, performGridCap());
-			if (size_t(blocks) * kPerformThreads > kListSlack)
-				throw std::runtime_error("kPerform grid exceeds the candidate list slack");
+			const unsigned int blocks = performGrid(std::max(std::max(C, V), T));
 			void* params[] = {&pa};
 			cudaEvent_t e0 = probeBegin("kPerform", stream);
 			MO_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kPerform, dim3(blocks), dim3(kPerformThreads), params, 0, stream));
@@ -4066,11 +4391,11 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		if (result_count)
 		{
 			MO_LAUNCH(kMarkUpdate, gridFor(result_count, kThreads), kThreads, 0, stream, res, result_count, w.remap, w.vupdate);
-			MO_LAUNCH(kCountCorners, gridFor(result_count, kThreads), kThreads, 0, stream, res, result_count, w.remap, w.cnt, slot, nullptr);
+			MO_LAUNCH(kCountCorners, gridFor(result_count, kThreads), kThreads, 0, stream, res, result_count, w.remap, w.cnt, slot);
 		}
 		scanExclusive(w.cnt, w.adj_off, V + 1, nullptr, w.scratch, stream, ss);
 		if (T)
-			MO_LAUNCH(kAdjFill, gridFor(T, kThreads), kThreads, 0, stream, res, T, w.remap, w.adj_off, slot, w.adj, nullptr, I);
+			MO_LAUNCH(kAdjFill, gridFor(T, kThreads), kThreads, 0, stream, res, T, w.remap, w.adj_off, slot, w.adj, I);
 		const unsigned int gV = gridFor(V, kThreads);
 		{
 			SolveArgs sa;
@@ -4096,7 +4421,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 			sa.sc = w.sc;
 			// co-resident blocks of this kernel (its own register count), as many as the pass kernel's at most
 			unsigned int resident = unsigned(std::max(1, solve_per_sm_ * sms_));
-			unsigned int blocks = std::max(1u, std::min(std::min(perform_blocks_, resident), gV));
+			unsigned int blocks = std::max(1u, std::min(std::min(unsigned(performBlocksPerSMMax() * sms_), resident), gV));
 			MO_CUDA_CHECK(cudaMemsetAsync(w.sc->bar, 0, sizeof(unsigned int) * 5, stream));
 			void* params[] = {&sa};
 			cudaEvent_t e0 = probeBegin("kSolvePositions", stream);

@@ -116,12 +116,12 @@ private:
 // MESHOPTGPU_PERFORM_BLOCKS_PER_SM, MESHOPTGPU_WINDOW_FACTOR and MESHOPTGPU_DEVICE_LOOP).
 struct Tuning
 {
-	int perform_blocks_per_sm = 2;  // resident blocks (512 threads) per SM of the cooperative pass kernel
+	int perform_blocks_per_sm = 0;  // resident blocks (512 threads) per SM of the pass kernels (0: by size)
 	double window_factor = 2.0;     // first decision window = factor * (triangle goal / 2) + 4096
 	int perform_grid_cap = 0;       // at most this many blocks of 256 threads for the pass kernel and the
 	                                // scans (0: no cap); lets concurrent simplifications share the GPU
-	bool device_loop = true;        // run the pass loop as a device-resident CUDA graph (off: one host
-	                                // round trip per pass, needed for per-kernel event timing)
+	bool device_loop = true;        // run the pass loop in one launch (off: a launch per phase from the host
+	                                // and two round trips per pass, as per-kernel event timing needs)
 	static Tuning fromEnvironment();
 };
 
@@ -151,56 +151,21 @@ private:
 	DeviceArena arena_;
 	DeviceArena sparse_arena_; // compact copy of a sparse subset
 	unsigned int* pinned_ = nullptr; // small pinned readback buffer
-	cudaStream_t capture2_ = nullptr; // records the pass body's second branch (the pick)
-	cudaEvent_t fork_ = nullptr, join_ = nullptr; // the branch's fork and join while recording
-	cudaStream_t capture_ = nullptr; // records the device-resident pass loop (the caller's stream may be
-	                                 // the legacy default stream, which cannot capture)
 	unsigned int coop_blocks_ = 1;   // resident blocks of the cooperative pass kernel (occupancy)
-	unsigned int perform_blocks_ = 1;
-	unsigned int sort_items_ = 0;    // candidates per thread of the pass sort's tiles (0: by count)
 	int sms_ = 1;
 	int solve_per_sm_ = 1; // resident blocks of the position solve kernel per SM
 	int clock_khz_ = 0;    // SM clock for the phase counters (queried once: the query costs ~0.6 ms)
 	Tuning tuning_;
-	// The device-resident pass loop's executable graph, kept for the next run of the same shape:
-	// the graph holds workspace pointers (fixed by the arena base and the layout's sizes) and
-	// grid sizes; everything else it reads (targets, counts, the error limit) is on the device.
-	struct LoopGraph
-	{
-		const void* base = nullptr;
-		size_t I = 0, V = 0;
-		int ac = 0;
-		bool solve = false;
-		unsigned int blocks = 0;
-		unsigned int sort_items = 0;
-		unsigned int scan_blocks = 0;         // the one-launch scans' grid cap recorded in the body (0: none)
-		unsigned long long body_launches = 0; // kernels one replay of the body launches
-		cudaGraph_t graph = nullptr;
-		cudaGraphExec_t exec = nullptr;
-	} loop_;
-	void dropLoopGraph();
+	int passBlocksPerSM(size_t index_count) const;
 	unsigned int performGridCap() const; // perform_grid_cap in blocks of the pass kernel
 
 public:
-	void setTuning(const Tuning& t)
-	{
-		tuning_ = t;
-		perform_blocks_ = std::min(coop_blocks_, unsigned(std::max(1, sms_ * t.perform_blocks_per_sm)));
-	}
-	// The launch shape of the pass kernels an autotuner picks: pass-kernel blocks per SM, and the
-	// pass sort's candidates per thread (4, 8 or 16; 0: chosen by the candidate count). Results do
-	// not depend on either.
-	void setPassShape(int perform_blocks_per_sm, unsigned int sort_items)
-	{
-		Tuning t = tuning_;
-		t.perform_blocks_per_sm = perform_blocks_per_sm;
-		setTuning(t);
-		sort_items_ = (sort_items == 4 || sort_items == 8 || sort_items == 16) ? sort_items : 0;
-	}
-	int performBlocksPerSM() const { return tuning_.perform_blocks_per_sm; }
+	void setTuning(const Tuning& t) { tuning_ = t; }
+	// The launch shape an autotuner picks: pass-kernel blocks per SM (0: by size). Results do not depend
+	// on it.
+	void setPassShape(int perform_blocks_per_sm) { tuning_.perform_blocks_per_sm = perform_blocks_per_sm; }
 	// resident blocks per SM of the pass kernel at most (its register count)
 	int performBlocksPerSMMax() const { return int(coop_blocks_ / unsigned(std::max(1, sms_))); }
-	unsigned int sortItems() const { return sort_items_; }
 	const Tuning& tuning() const { return tuning_; }
 };
 

@@ -66,6 +66,50 @@ def test_update_vertex_orders(port, order, amp, ratio):
     assert not _same(got[1], p)
 
 
+@pytest.fixture
+def single_path():
+    mg.set_dropin_batch_limit(0)
+    yield
+    mg.set_dropin_batch_limit()
+
+
+# the pass loop's runs of triangles, vertices and candidates per block and its sort's tiles of 512:
+# fewer than one of each, exactly one, one more, several per block; the last is above the size where
+# two blocks per SM run it (pruning calls are not tuned, so the size decides)
+@pytest.mark.parametrize("nx,ny", [(2, 2), (3, 2), (5, 5), (17, 17), (18, 17), (14, 26), (33, 65), (91, 90), (301, 299), (421, 410)])
+@pytest.mark.parametrize("options", [0, mg.SimplifyPrune | mg.SimplifyLockBorder])
+def test_pass_loop_sizes(port, single_path, nx, ny, options):
+    if nx > 300 and not options & mg.SimplifyPrune:
+        pytest.skip("the two sizes are there for the untuned calls")
+    a = (np.arange(ny - 1)[:, None] * nx + np.arange(nx - 1)[None, :]).reshape(-1)
+    idx = np.stack([a, a + 1, a + nx, a + nx, a + 1, a + nx + 1], 1).reshape(-1).astype(np.uint32)
+    rng = np.random.default_rng(nx * 1000 + ny)
+    y, x = np.meshgrid(np.arange(ny), np.arange(nx), indexing="ij")
+    pos = np.stack([x, y, 0.4 * rng.standard_normal((ny, nx))], -1).reshape(-1, 3).astype(np.float32)
+    for ratio, error in ((0.0, 1.0), (0.3, 2e-2)):
+        target = W.target_count(len(idx), ratio)
+        ref, ref_err = port.simplify("port", idx, pos, target, error, options)
+        for device_loop in (True, False):
+            mg.set_device_loop(device_loop)
+            try:
+                out, err = mg.simplify(idx, pos, target, error, options)
+            finally:
+                mg.set_device_loop(True)
+            assert np.array_equal(out, ref)
+            assert err == ref_err
+
+
+@pytest.mark.parametrize("amp", [0.0, 1e-4])
+def test_pass_loop_equal_keys(port, single_path, amp):
+    """All candidates in a few sort bins: long runs of equal keys across the sorting blocks."""
+    idx, pos = W.heightfield(49, seed=2, amp=amp)
+    target = W.target_count(len(idx), 0.2)
+    ref, ref_err = port.simplify("port", idx, pos, target, 1e-1, mg.SimplifyPrune)
+    out, err = mg.simplify(idx, pos, target, 1e-1, mg.SimplifyPrune)
+    assert np.array_equal(out, ref)
+    assert err == ref_err
+
+
 def _meshlet_groups(case):
     """Groups of the sphere's triangles in file order and the parameters they are cut with."""
     idx, pos, _, _ = W.octa_sphere(6, seed=9)
