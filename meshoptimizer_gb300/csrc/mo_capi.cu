@@ -1660,15 +1660,10 @@ size_t meshoptgpu_optimizeVertexFetchRemapDevice(unsigned int* destination, cons
 		cudaStream_t st = static_cast<cudaStream_t>(stream);
 		unsigned int* scratch = static_cast<unsigned int*>(s.compact_scratch.ensure((vertexOrderScratchWords(index_count, vertex_count) + 64) * 4));
 		unsigned int* counters = scratch + vertexOrderScratchWords(index_count, vertex_count);
-		vertexOrder(destination, indices, index_count, vertex_count, scratch, counters, st);
-		unsigned int h[2];
-		MO_CUDA_CHECK(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, st));
-		MO_CUDA_CHECK(cudaStreamSynchronize(st));
-		probe().collect();
-		if (h[1])
-			throw std::invalid_argument("an index is out of range of vertex_count");
+		vertexOrder(destination, true, indices, index_count, vertex_count, scratch, counters, st);
+		const unsigned int used = takeOrderCount(counters, st);
 		setStatus(meshoptgpu_StatusOk, "");
-		return h[0];
+		return used;
 	}
 	catch (const std::exception& e)
 	{
@@ -1703,21 +1698,12 @@ size_t meshoptgpu_optimizeVertexFetchDevice(void* destination, unsigned int* ind
 			MO_CUDA_CHECK(cudaMemcpyAsync(copy, vertices, copy_bytes, cudaMemcpyDeviceToDevice, st));
 			src = copy;
 		}
-		vertexOrder(order, indices, index_count, vertex_count, scratch, counters, st);
-		unsigned int h[2];
-		MO_CUDA_CHECK(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, st));
-		MO_CUDA_CHECK(cudaStreamSynchronize(st));
-		if (h[1])
-		{
-			probe().collect();
-			throw std::invalid_argument("an index is out of range of vertex_count");
-		}
-		moveVertices(destination, src, vertex_count, vertex_size, order, st);
-		rewriteIndices(indices, index_count, order, st);
-		MO_CUDA_CHECK(cudaStreamSynchronize(st));
-		probe().collect();
+		// the moves are queued behind the order and do nothing if an index is bad, so the call waits once
+		vertexOrder(order, false, indices, index_count, vertex_count, scratch, counters, st);
+		compactVertices(destination, src, vertex_count, vertex_size, indices, index_count, order, vertexOrderList(scratch, vertex_count), counters, st);
+		const unsigned int used = takeOrderCount(counters, st);
 		setStatus(meshoptgpu_StatusOk, "");
-		return h[0];
+		return used;
 	}
 	catch (const std::exception& e)
 	{

@@ -3,15 +3,21 @@
 // and meshopt_generatePositionRemap (src/indexgenerator.cpp:555-578).
 //
 // The reference walks the index buffer once and numbers vertices as they are first seen. Here
-// the same order comes from three data-parallel steps: the first index position of every
-// vertex (atomicMin), a flag at every index position that is a first use, and an exclusive
-// scan of the flags, whose value at a first use is that vertex's new index. The position remap
+// the same order comes from two data-parallel steps: the first index position of every vertex
+// (atomicMin), and a scan over the index positions that are first uses, whose value there is that
+// vertex's new index. Vertices then move from the new order's side, so only used ones are read and
+// neighbouring threads write neighbouring bytes. The position remap
 // is an open-addressing table keyed by position in which the smallest vertex index of each
 // position wins (atomicMin), which is the vertex the reference's sequential insertion keeps.
 #include "mo_vfetch.cuh"
 #include "mo_common.cuh"
+#include "mo_grid.cuh"
 #include "mo_prims.cuh"
 #include "mo_probe.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <stdexcept>
 
 namespace mogpu
 {
@@ -24,13 +30,6 @@ constexpr int kThreads = 256;
 __device__ __forceinline__ size_t gtidv()
 {
 	return (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-}
-
-__global__ void kClearWords(unsigned int* p, size_t n, unsigned int value)
-{
-	size_t i = gtidv();
-	if (i < n)
-		p[i] = value;
 }
 
 // first[v] = smallest index position that references v; out-of-range indices raise *bad
@@ -48,54 +47,84 @@ __global__ void kFirstPosition(const unsigned int* __restrict__ idx, size_t n, s
 	atomicMin(&first[v], (unsigned int)p);
 }
 
-__global__ void kFirstFlag(const unsigned int* __restrict__ idx, size_t n, size_t vcount, const unsigned int* __restrict__ first, unsigned int* __restrict__ flags)
+constexpr unsigned int kOrderTile = kThreads * 4;
+
+// counters: used vertices, bad indices, the grid barrier's two words and its error flag
+constexpr int kCounters = 5;
+
+// order[v] = rank of v's first use among the index positions that are first uses, list[rank] = v: one
+// cooperative launch, each block over a run of tiles, counting them, then (behind the grid barrier)
+// adding up the counts before it and ranking them. A flag per position, its three-launch scan and a
+// pass over all vertices before it moved 16 bytes per index and 8 per vertex more, in five launches.
+__global__ void __launch_bounds__(kThreads) kVertexOrder(const unsigned int* __restrict__ idx, size_t n, size_t vcount, const unsigned int* __restrict__ first,
+    unsigned int* __restrict__ order, unsigned int* __restrict__ list, unsigned int* sums, unsigned int* counters)
 {
-	size_t p = gtidv();
-	if (p >= n)
-		return;
-	unsigned int v = idx[p];
-	flags[p] = (v < vcount && first[v] == (unsigned int)p) ? 1u : 0u;
+	__shared__ unsigned int smem[kThreads / 32 + 1];
+	const size_t tiles = (n + kOrderTile - 1) / kOrderTile, per = (tiles + gridDim.x - 1) / gridDim.x;
+	const size_t t0 = min(tiles, (size_t)blockIdx.x * per), t1 = min(tiles, t0 + per);
+	auto firstUses = [&](size_t t, unsigned int v[4]) {
+		const size_t p = t * kOrderTile + threadIdx.x * 4;
+		unsigned int uses = 0;
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+			v[j] = p + j < n ? idx[p + j] : ~0u;
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+			uses |= (v[j] < vcount && first[v[j]] == (unsigned int)(p + j)) ? 1u << j : 0u;
+		return uses;
+	};
+	unsigned int c = 0, v[4];
+	for (size_t t = t0; t < t1; ++t)
+		c += __popc(firstUses(t, v));
+	unsigned int total;
+	blockExclusiveScan<kThreads>(c, smem, &total);
+	if (threadIdx.x == 0)
+		sums[blockIdx.x] = total;
+	gridBarrierOnce(counters + 2, counters + 4);
+	if (__ldcg(counters + 4))
+		return; // a barrier wait ran out: nothing is written from incomplete sums
+	unsigned int before = 0, base;
+	for (unsigned int q = threadIdx.x; q < blockIdx.x; q += kThreads)
+		before += __ldcg(sums + q);
+	blockExclusiveScan<kThreads>(before, smem, &base);
+	for (size_t t = t0; t < t1; ++t)
+	{
+		const unsigned int uses = firstUses(t, v);
+		__syncthreads(); // every thread has read the previous scan's shared words
+		unsigned int r = base + blockExclusiveScan<kThreads>(__popc(uses), smem, &total);
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+			if (uses >> j & 1u)
+			{
+				order[v[j]] = r;
+				list[r++] = v[j];
+			}
+		base += total;
+	}
+	if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+		counters[0] = base;
 }
 
-// new index of each vertex: the rank of its first use, ~0u when unused
-__global__ void kVertexOrder(const unsigned int* __restrict__ first, const unsigned int* __restrict__ rank, size_t vcount, unsigned int* __restrict__ order)
-{
-	size_t v = gtidv();
-	if (v >= vcount)
-		return;
-	unsigned int f = first[v];
-	order[v] = f == ~0u ? ~0u : rank[f];
-}
-
-__global__ void kRewriteIndices(unsigned int* idx, size_t n, const unsigned int* __restrict__ order)
+// indices to the new order; nothing where an index is bad or the order is incomplete
+__global__ void kRewriteIndices(unsigned int* idx, size_t n, const unsigned int* __restrict__ order, const unsigned int* __restrict__ counters)
 {
 	size_t p = gtidv();
-	if (p < n)
+	if (p < n && !counters[1] && !counters[4])
 		idx[p] = order[idx[p]];
 }
 
-// vertices to their new slots: one thread per 4-byte word (vertex_size a multiple of 4 and
-// both buffers 4-byte aligned) or per byte otherwise
-__global__ void kMoveVertexWords(const unsigned int* __restrict__ src, size_t vcount, size_t words, const unsigned int* __restrict__ order, unsigned int* __restrict__ dst)
+// row r of the new order from vertex list[r], by 2^log_lanes threads per row in units of T (a divisor
+// of the vertex size that both buffers are aligned to)
+template <class T>
+__global__ void kMoveVertices(const T* __restrict__ src, unsigned int units, unsigned int log_lanes, const unsigned int* __restrict__ list,
+    const unsigned int* __restrict__ counters, T* __restrict__ dst)
 {
-	size_t t = gtidv();
-	if (t >= vcount * words)
+	const size_t t = gtidv(), r = t >> log_lanes;
+	if (r >= counters[0] || counters[1] || counters[4])
 		return;
-	size_t v = t / words, w = t - v * words;
-	unsigned int o = order[v];
-	if (o != ~0u)
-		dst[(size_t)o * words + w] = src[t];
-}
-
-__global__ void kMoveVertexBytes(const unsigned char* __restrict__ src, size_t vcount, size_t size, const unsigned int* __restrict__ order, unsigned char* __restrict__ dst)
-{
-	size_t t = gtidv();
-	if (t >= vcount * size)
-		return;
-	size_t v = t / size, b = t - v * size;
-	unsigned int o = order[v];
-	if (o != ~0u)
-		dst[(size_t)o * size + b] = src[t];
+	const size_t from = (size_t)list[r] * units, to = r * units;
+	for (unsigned int u = (unsigned int)t & ((1u << log_lanes) - 1u); u < units; u += 1u << log_lanes)
+		dst[to + u] = src[from + u];
 }
 
 __device__ __forceinline__ unsigned int keyBits(float f)
@@ -169,47 +198,103 @@ size_t alignWords(size_t n)
 
 } // namespace
 
+constexpr unsigned int kOrderBlocksMax = 4096; // words for the blocks' sums
+
+// co-resident blocks of kVertexOrder on the current device, queried once
+unsigned int orderBlocks()
+{
+	constexpr int kDevices = 64;
+	static std::atomic<unsigned int> cache[kDevices];
+	int dev = 0, sms = 0, occ = 0;
+	MO_CUDA_CHECK(cudaGetDevice(&dev));
+	unsigned int c = dev < kDevices ? cache[dev].load(std::memory_order_relaxed) : 0u;
+	if (c)
+		return c;
+	MO_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+	MO_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kVertexOrder, kThreads, 0));
+	c = std::min(kOrderBlocksMax, unsigned(std::max(1, sms) * std::max(1, std::min(occ, 4))));
+	if (dev < kDevices)
+		cache[dev].store(c, std::memory_order_relaxed);
+	return c;
+}
+
 size_t vertexOrderScratchWords(size_t index_count, size_t vertex_count)
 {
-	return alignWords(vertex_count) + alignWords(index_count) + alignWords(scanScratchWords(index_count)) + 64;
+	return alignWords(vertex_count) + alignWords(std::min(index_count, vertex_count)) + kOrderBlocksMax + 64;
 }
 
-void vertexOrder(unsigned int* order, const unsigned int* indices, size_t index_count, size_t vertex_count, unsigned int* scratch, unsigned int* counters,
-    cudaStream_t stream)
+unsigned int* vertexOrderList(unsigned int* scratch, size_t vertex_count)
+{
+	return scratch + alignWords(vertex_count);
+}
+
+void vertexOrder(unsigned int* order, bool mark_unused, const unsigned int* indices, size_t index_count, size_t vertex_count, unsigned int* scratch,
+    unsigned int* counters, cudaStream_t stream)
 {
 	unsigned int* first = scratch;
-	unsigned int* flags = first + alignWords(vertex_count);
-	unsigned int* sscratch = flags + alignWords(index_count);
-	MO_CUDA_CHECK(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned int), stream));
-	if (vertex_count)
-		MO_LAUNCH(kClearWords, gridFor(vertex_count, kThreads), kThreads, 0, stream, first, vertex_count, ~0u);
-	if (index_count)
-	{
-		MO_LAUNCH(kFirstPosition, gridFor(index_count, kThreads), kThreads, 0, stream, indices, index_count, vertex_count, first, &counters[1]);
-		MO_LAUNCH(kFirstFlag, gridFor(index_count, kThreads), kThreads, 0, stream, indices, index_count, vertex_count, first, flags);
-		scanExclusive(flags, flags, index_count, &counters[0], sscratch, stream);
-	}
-	if (vertex_count)
-		MO_LAUNCH(kVertexOrder, gridFor(vertex_count, kThreads), kThreads, 0, stream, first, flags, vertex_count, order);
-}
-
-void rewriteIndices(unsigned int* indices, size_t index_count, const unsigned int* order, cudaStream_t stream)
-{
-	if (index_count)
-		MO_LAUNCH(kRewriteIndices, gridFor(index_count, kThreads), kThreads, 0, stream, indices, index_count, order);
-}
-
-void moveVertices(void* destination, const void* vertices, size_t vertex_count, size_t vertex_size, const unsigned int* order, cudaStream_t stream)
-{
-	if (!vertex_count)
+	unsigned int* list = vertexOrderList(scratch, vertex_count);
+	unsigned int* sums = list + alignWords(std::min(index_count, vertex_count));
+	MO_CUDA_CHECK(cudaMemsetAsync(counters, 0, kCounters * sizeof(unsigned int), stream));
+	if (vertex_count && mark_unused)
+		MO_CUDA_CHECK(cudaMemsetAsync(order, 0xFF, vertex_count * sizeof(unsigned int), stream));
+	if (!index_count)
 		return;
-	bool words = vertex_size % 4 == 0 && reinterpret_cast<uintptr_t>(destination) % 4 == 0 && reinterpret_cast<uintptr_t>(vertices) % 4 == 0;
-	if (words)
-		MO_LAUNCH(kMoveVertexWords, gridFor(vertex_count * (vertex_size / 4), kThreads), kThreads, 0, stream, static_cast<const unsigned int*>(vertices),
-		    vertex_count, vertex_size / 4, order, static_cast<unsigned int*>(destination));
-	else
-		MO_LAUNCH(kMoveVertexBytes, gridFor(vertex_count * vertex_size, kThreads), kThreads, 0, stream, static_cast<const unsigned char*>(vertices),
-		    vertex_count, vertex_size, order, static_cast<unsigned char*>(destination));
+	if (vertex_count)
+		MO_CUDA_CHECK(cudaMemsetAsync(first, 0xFF, vertex_count * sizeof(unsigned int), stream));
+	MO_LAUNCH(kFirstPosition, gridFor(index_count, kThreads), kThreads, 0, stream, indices, index_count, vertex_count, first, &counters[1]);
+	const size_t tiles = (index_count + kOrderTile - 1) / kOrderTile, cap = orderBlocks(), per = (tiles + cap - 1) / cap;
+	const unsigned int blocks = unsigned((tiles + per - 1) / per);
+	const unsigned int* cfirst = first;
+	void* params[] = {(void*)&indices, (void*)&index_count, (void*)&vertex_count, (void*)&cfirst, (void*)&order, (void*)&list, (void*)&sums, (void*)&counters};
+	cudaEvent_t e0 = probeBegin("kVertexOrder", stream);
+	MO_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kVertexOrder, dim3(blocks), dim3(kThreads), params, 0, stream));
+	probeEnd(e0, stream);
+}
+
+unsigned int takeOrderCount(const unsigned int* counters, cudaStream_t stream)
+{
+	unsigned int h[kCounters];
+	MO_CUDA_CHECK(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, stream));
+	MO_CUDA_CHECK(cudaStreamSynchronize(stream));
+	probe().collect();
+	if (h[1])
+		throw std::invalid_argument("an index is out of range of vertex_count");
+	if (h[4])
+		throw std::runtime_error("grid barrier wait limit reached in the vertex order");
+	return h[0];
+}
+
+template <class T>
+void moveUnits(void* destination, const void* vertices, size_t rows, size_t vertex_size, const unsigned int* list, const unsigned int* counters, cudaStream_t stream)
+{
+	const unsigned int units = unsigned(vertex_size / sizeof(T));
+	unsigned int log_lanes = 0;
+	while (log_lanes < 5 && (1u << log_lanes) < units)
+		++log_lanes;
+	MO_LAUNCH(kMoveVertices<T>, gridFor(rows << log_lanes, kThreads), kThreads, 0, stream, static_cast<const T*>(vertices), units, log_lanes, list, counters,
+	    static_cast<T*>(destination));
+}
+
+void compactVertices(void* destination, const void* vertices, size_t vertex_count, size_t vertex_size, unsigned int* indices, size_t index_count,
+    const unsigned int* order, const unsigned int* list, const unsigned int* counters, cudaStream_t stream)
+{
+	if (!index_count)
+		return;
+	// the widest unit that divides the vertices and that both buffers are aligned to
+	const size_t align = vertex_size | reinterpret_cast<uintptr_t>(destination) | reinterpret_cast<uintptr_t>(vertices);
+	const size_t rows = std::min(vertex_count, index_count);
+	if (rows)
+	{
+		if (align % 16 == 0)
+			moveUnits<uint4>(destination, vertices, rows, vertex_size, list, counters, stream);
+		else if (align % 8 == 0)
+			moveUnits<uint2>(destination, vertices, rows, vertex_size, list, counters, stream);
+		else if (align % 4 == 0)
+			moveUnits<unsigned int>(destination, vertices, rows, vertex_size, list, counters, stream);
+		else
+			moveUnits<unsigned char>(destination, vertices, rows, vertex_size, list, counters, stream);
+	}
+	MO_LAUNCH(kRewriteIndices, gridFor(index_count, kThreads), kThreads, 0, stream, indices, index_count, order, counters);
 }
 
 size_t positionRemapScratchWords(size_t vertex_count)

@@ -163,3 +163,45 @@ def test_meshlets_wide_group():
     rm, rv, rt = ML.build_meshlets_flex(idx, pos, 128, 42, 128, 0.0, 2.0, kind="port")
     rv, rt = ML.optimize_meshlets(rm, rv, rt, 1, kind="port")
     assert np.array_equal(m, rm) and np.array_equal(v, rv) and np.array_equal(t, rt)
+
+
+@pytest.mark.parametrize("size,shift", [(1, 0), (3, 1), (4, 0), (6, 2), (8, 8), (8, 4), (12, 0), (16, 0), (16, 8), (20, 4), (48, 0), (132, 0), (256, 0), (256, 1)])
+@pytest.mark.parametrize("corners", [3, 1023, 1026, 8190])
+def test_compaction_units(port, size, shift, corners):
+    """Vertex sizes and alignments of every copy width, index counts around a tile of 1024."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(size * 100 + corners + shift)
+    vc = corners // 2 + 5
+    idx = rng.integers(0, vc, corners).astype(np.uint32)
+    verts = rng.integers(0, 256, (vc, size)).astype(np.uint8)
+    ref_idx, ref_verts, n = port.optimize_vertex_fetch("port", idx, verts)
+    ref_remap, _ = port.optimize_vertex_fetch_remap("port", idx, vc)
+    src = torch.zeros(vc * size + 64, dtype=torch.uint8, device="cuda")
+    src[shift:shift + vc * size] = torch.from_numpy(verts.reshape(-1)).cuda()
+    for in_place in (False, True):
+        di = torch.from_numpy(idx.view(np.int32).copy()).cuda()
+        s = src.clone()
+        d = s if in_place else torch.full_like(s, 7)
+        remap = torch.zeros(vc, dtype=torch.int32, device="cuda")
+        assert mg.optimize_vertex_fetch_remap_device(remap.data_ptr(), di.data_ptr(), corners, vc) == n
+        assert np.array_equal(remap.cpu().numpy().view(np.uint32), ref_remap)
+        assert mg.optimize_vertex_fetch_device(d.data_ptr() + shift, di.data_ptr(), corners, s.data_ptr() + shift, vc, size) == n
+        assert np.array_equal(di.cpu().numpy().view(np.uint32), ref_idx)
+        got = d.cpu().numpy()
+        assert np.array_equal(got[shift:shift + n * size].reshape(n, size), np.asarray(ref_verts).view(np.uint8).reshape(-1, size)[:n])
+        # nothing outside the used rows
+        keep = (s if in_place else torch.full_like(s, 7)).cpu().numpy() if not in_place else src.cpu().numpy()
+        assert np.array_equal(got[:shift], keep[:shift]) and np.array_equal(got[shift + n * size:], keep[shift + n * size:])
+
+
+def test_compaction_bad_index_changes_nothing():
+    torch = pytest.importorskip("torch")
+    idx = np.arange(3000, dtype=np.int32) % 700
+    idx[2999] = 700
+    di = torch.from_numpy(idx.copy()).cuda()
+    src = torch.arange(700 * 16, dtype=torch.int32, device="cuda").to(torch.uint8)
+    d = torch.full_like(src, 9)
+    with pytest.raises(mg.SimplifyError) as e:
+        mg.optimize_vertex_fetch_device(d.data_ptr(), di.data_ptr(), 3000, src.data_ptr(), 700, 16)
+    assert e.value.status == mg.STATUS_INVALID_ARGUMENT
+    assert np.array_equal(di.cpu().numpy(), idx) and bool((d == 9).all())
