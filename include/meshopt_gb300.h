@@ -226,7 +226,7 @@ MESHOPTGPU_API int meshoptgpu_buildMeshletsFlexGroups(unsigned int* meshlets, un
 
 /* Batch launch shape: threads per CTA (128, 256 or 512; 0 = autotune, the default) and the
  * shared-memory budget per CTA in bytes (0 = autotune, the default). The autotuner times every
- * open pair of thread count and budget (64, 104 and 160 KiB) on the first batch of a size class
+ * open pair of thread count and budget (54, 110 and 216 KiB) on the first batch of a size class
  * and keeps the fastest for that class. */
 MESHOPTGPU_API void meshoptgpu_setBatchConfig(int threads, unsigned int smem_bytes);
 

@@ -42,10 +42,17 @@ struct BatchResult
 	unsigned int status; // 0 ok, 2 invalid index, 3 a decision round made no progress
 };
 
-// scratch bytes one mesh needs: without the decision-round state (rounds = false) in shared
-// memory, where it runs when that size fits the launch's budget, else with it in a global slab.
-// A sparse mesh has at most min(index_count, vertex_count) vertices of its own.
-size_t batchWorkspaceBytes(size_t index_count, size_t vertex_count, size_t ac, bool sparse, bool rounds);
+// Memory of one mesh. smem: shared memory it is expected to need beside its attribute rows (rows), which
+// go there too where they fit, else into the CTA's slab; slab: global scratch in which it runs whatever
+// it turns out to need.
+struct BatchBytes
+{
+	size_t smem, rows, slab;
+};
+BatchBytes batchBytes(const BatchDesc& d, bool narrow);
+
+// whether a mesh's ids fit the kernels' 16-bit form
+bool batchNarrow(const BatchDesc& d);
 
 // whether a mesh needs the full-option kernel: a sparse subset (option bit 1), attributes,
 // vertex_lock or Permissive (option bit 5)
@@ -54,11 +61,18 @@ inline bool batchNeedsFull(const BatchDesc& d)
 	return d.ac || d.lock || (d.options & ((1u << 1) | (1u << 5)));
 }
 
-// resident CTAs per SM for a thread count, dynamic shared memory size and kernel form
-int batchBlocksPerSM(int threads, unsigned int smem_bytes, bool full);
+// the kernel's forms (mo_batch_kernel.cuh)
+typedef void (*BatchKernel)(const BatchDesc*, unsigned int, unsigned int*, BatchResult*, char*, size_t, unsigned int);
+BatchKernel batchKernelLean(int threads);
+BatchKernel batchKernelFull(int threads);
+BatchKernel batchKernelWide(bool full);
 
-// full: the instantiation with every option; otherwise the positions-only one
+// resident CTAs per SM for a thread count, dynamic shared memory size and kernel form
+int batchBlocksPerSM(int threads, unsigned int smem_bytes, bool full, bool narrow);
+
+// full: the instantiation with every option; otherwise the positions-only one. narrow: every mesh is
+// narrow. Every CTA has slab_bytes of slabs, at least the largest mesh's.
 void launchBatch(const BatchDesc* d_descs, unsigned int count, unsigned int* d_ticket, BatchResult* d_results, char* d_slabs, size_t slab_bytes,
-    unsigned int smem_bytes, unsigned int blocks, int threads, bool full, cudaStream_t stream);
+    unsigned int smem_bytes, unsigned int blocks, int threads, bool full, bool narrow, cudaStream_t stream);
 
 } // namespace mogpu

@@ -597,7 +597,7 @@ size_t updateHost(unsigned int* indices, size_t index_count, float* vertex_posit
 
 // ---------------------------------------------------------------- batched path
 
-const size_t kBatchSmemDefault = 104 * 1024;    // shared-memory budget per CTA (two CTAs per SM)
+const size_t kBatchSmemDefault = 110 * 1024;    // shared-memory budget per CTA (two CTAs per SM)
 const size_t kBatchSlabTotal = size_t(16) << 30; // global slabs for meshes beyond the budget
 
 struct BatchTuner
@@ -609,8 +609,9 @@ struct BatchTuner
 	std::map<std::pair<int, bool>, std::pair<int, size_t>> shape;
 } g_tuner;
 
-// the shared-memory budgets the batch autotuner times (two, two and one CTAs of 256 threads per SM)
-const size_t kBatchSmemBudgets[3] = {64 * 1024, kBatchSmemDefault, 160 * 1024};
+// the shared-memory budgets the batch autotuner times (four, two and one CTAs per SM; a smaller largest
+// mesh leaves room for more)
+const size_t kBatchSmemBudgets[3] = {54 * 1024, kBatchSmemDefault, 216 * 1024};
 
 int sizeClass(size_t max_index_count)
 {
@@ -676,12 +677,6 @@ BatchDesc makeDesc(const meshoptgpu_BatchMesh& m, const unsigned int* indices, c
 	return d;
 }
 
-// workspace of a batched mesh in shared memory (serial perform) and in a global slab (rounds)
-size_t descWorkspace(const BatchDesc& d, bool rounds)
-{
-	return batchWorkspaceBytes(d.index_count, d.vertex_count, d.ac, (d.options & kOptSparse) != 0, rounds);
-}
-
 // Runs descs (device pointers) through the persistent kernel; results in the same order.
 // attr_of[i] indexes maps.maps for descs[i] (-1: none).
 void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& maps, const std::vector<int>& attr_of, std::vector<BatchResult>& results,
@@ -702,20 +697,25 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		ordered[i] = descs[perm[i]];
 		maxidx = std::max<size_t>(maxidx, ordered[i].index_count);
 	}
-	// a budget's dynamic shared memory (the largest mesh that fits it) and slab size (the largest
-	// that does not): meshes whose workspace fits the launch's shared memory run there
-	auto footprint = [&](size_t budget, unsigned int& smem, size_t& maxslab) {
-		size_t maxfit = 0;
-		maxslab = 0;
-		for (const BatchDesc& d : ordered)
-		{
-			const size_t ws = descWorkspace(d, false);
-			if (ws <= budget)
-				maxfit = std::max(maxfit, ws);
-			else
-				maxslab = std::max(maxslab, descWorkspace(d, true));
-		}
-		smem = unsigned((maxfit + 15) & ~size_t(15));
+	bool full = false, narrow = true;
+	for (const BatchDesc& d : ordered)
+	{
+		full = full || batchNeedsFull(d);
+		narrow = narrow && batchNarrow(d);
+	}
+	std::vector<BatchBytes> bytes(n);
+	size_t maxslab = 0;
+	for (size_t i = 0; i < n; ++i)
+	{
+		bytes[i] = batchBytes(ordered[i], narrow);
+		maxslab = std::max(maxslab, bytes[i].slab);
+	}
+	// a budget's dynamic shared memory: the largest mesh that fits it, with its attribute rows or without
+	auto footprint = [&](size_t budget) {
+		size_t most = 0;
+		for (const BatchBytes& b : bytes)
+			most = std::max(most, b.smem + b.rows <= budget ? b.smem + b.rows : (b.smem <= budget ? b.smem : size_t(0)));
+		return unsigned((most + 15) & ~size_t(15));
 	};
 	const int sms = s.sms;
 
@@ -740,19 +740,13 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	if (nm)
 		MO_CUDA_CHECK(cudaMemcpyAsync(d_maps, hmeta + off_maps, nm * sizeof(BatchAttr), cudaMemcpyHostToDevice, st));
 
-	bool full = false;
-	for (const BatchDesc& d : ordered)
-		full = full || batchNeedsFull(d);
 	auto launch = [&](int threads, size_t budget) {
-		unsigned int smem = 0;
-		size_t maxslab = 0;
-		footprint(budget, smem, maxslab);
-		int per_sm = std::max(1, batchBlocksPerSM(threads, smem, full));
+		const unsigned int smem = footprint(budget);
+		int per_sm = std::max(1, batchBlocksPerSM(threads, smem, full, narrow));
 		unsigned int blocks = unsigned(std::min<size_t>(size_t(per_sm) * sms, n));
-		if (maxslab)
-			blocks = unsigned(std::max<size_t>(1, std::min<size_t>(blocks, kBatchSlabTotal / maxslab)));
-		char* slabs = maxslab ? static_cast<char*>(s.batch_slabs.ensure(size_t(blocks) * maxslab)) : nullptr;
-		launchBatch(d_descs, unsigned(n), d_ticket, d_res, slabs, maxslab, smem, blocks, threads, full, st);
+		blocks = unsigned(std::max<size_t>(1, std::min<size_t>(blocks, kBatchSlabTotal / std::max<size_t>(maxslab, 1))));
+		char* slabs = static_cast<char*>(s.batch_slabs.ensure(size_t(blocks) * maxslab));
+		launchBatch(d_descs, unsigned(n), d_ticket, d_res, slabs, maxslab, smem, blocks, threads, full, narrow, st);
 	};
 
 	int threads = s.batch_threads;
@@ -1072,11 +1066,10 @@ struct ServerImpl
 
 const size_t kServerBudgetDefault = size_t(40) << 30;
 
-// device bytes a request holds while it runs on the batch path (its global slab; meshes that
-// fit shared memory hold none) or on the single-mesh path (its arena)
+// device bytes a request holds while it runs on the batch path (its global slab) or on the single-mesh path (its arena)
 size_t batchReserve(const ServerRequest& r)
 {
-	return descWorkspace(r.desc, false) <= kBatchSmemDefault ? 4096 : descWorkspace(r.desc, true);
+	return std::max<size_t>(4096, batchBytes(r.desc, batchNarrow(r.desc)).slab);
 }
 
 void publish(ServerImpl& S, std::vector<ServerRequest*>& done_reqs, size_t release)
@@ -1119,8 +1112,7 @@ void batchWorker(ServerImpl* S)
 			while (!S->small_q.empty() && take.size() < size_t(S->cfg.max_batch))
 			{
 				ServerRequest* r = S->small_q.front();
-				size_t slab = batchReserve(*r) > 4096 ? batchReserve(*r) : 0;
-				size_t nm = std::max(maxslab, slab);
+				size_t nm = std::max(maxslab, batchReserve(*r));
 				size_t blocks = std::min<size_t>(take.size() + 1, size_t(S->sms) * 4);
 				size_t need = blocks * nm + 4096 * (take.size() + 1);
 				if (S->reserved + need > S->cfg.memory_budget && !take.empty())

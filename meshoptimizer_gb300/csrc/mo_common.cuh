@@ -413,16 +413,16 @@ __device__ __forceinline__ void qreduceAttr(Quadric& Q, const Quadric& A, const 
 	}
 }
 
-// getComplexTarget, :1278-1290
-__device__ __forceinline__ unsigned int complexTarget(unsigned int v, unsigned int target, const unsigned int* remap,
-    const unsigned int* loop, const unsigned int* loopback)
+// getComplexTarget, :1278-1290 (IX: the mesh's index type; all ones: no loop)
+template <class IX>
+__device__ __forceinline__ unsigned int complexTarget(unsigned int v, unsigned int target, const IX* remap, const IX* loop, const IX* loopback)
 {
-	unsigned int r = remap[target];
-	unsigned int lv = loop[v];
-	if (lv != ~0u && remap[lv] == r)
+	const unsigned int r = remap[target];
+	const IX lv = loop[v];
+	if (lv != IX(~0u) && remap[lv] == r)
 		return lv;
-	unsigned int lb = loopback[v];
-	if (lb != ~0u && remap[lb] == r)
+	const IX lb = loopback[v];
+	if (lb != IX(~0u) && remap[lb] == r)
 		return lb;
 	return target;
 }
@@ -434,6 +434,39 @@ __device__ __forceinline__ void atomicMaxNonNegFloat(unsigned int* addr, float v
 	if (!(v == v))
 		return;
 	atomicMax(addr, __float_as_uint(v));
+}
+
+// block-wide exclusive scan of (sum, sum, max) triples; returns the block totals
+__device__ __forceinline__ uint3 blockScan3(unsigned int& t, unsigned int& f, unsigned int& m, unsigned int (*sm)[33])
+{
+	unsigned int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	unsigned int it = t, iff = f, im = m;
+	for (int o = 1; o < 32; o <<= 1)
+	{
+		unsigned int x = __shfl_up_sync(0xffffffffu, it, o), y = __shfl_up_sync(0xffffffffu, iff, o), z = __shfl_up_sync(0xffffffffu, im, o);
+		if (lane >= (unsigned)o)
+			it += x, iff += y, im = max(im, z);
+	}
+	unsigned int pm = __shfl_up_sync(0xffffffffu, im, 1);
+	if (lane == 31)
+		sm[0][w] = it, sm[1][w] = iff, sm[2][w] = im;
+	__syncthreads();
+	// every warp scans the warp totals for itself: no second barrier, no serial loop over the warps
+	const unsigned int nw = blockDim.x / 32;
+	unsigned int x = lane < nw ? sm[0][lane] : 0u, y = lane < nw ? sm[1][lane] : 0u, z = lane < nw ? sm[2][lane] : 0u;
+	for (int o = 1; o < 32; o <<= 1)
+	{
+		const unsigned int a = __shfl_up_sync(0xffffffffu, x, o), b = __shfl_up_sync(0xffffffffu, y, o), c = __shfl_up_sync(0xffffffffu, z, o);
+		if (lane >= (unsigned)o)
+			x += a, y += b, z = max(z, c);
+	}
+	const uint3 tot = make_uint3(__shfl_sync(0xffffffffu, x, 31), __shfl_sync(0xffffffffu, y, 31), __shfl_sync(0xffffffffu, z, 31));
+	const unsigned int before = w ? w - 1 : 0;
+	x = __shfl_sync(0xffffffffu, x, before), y = __shfl_sync(0xffffffffu, y, before), z = __shfl_sync(0xffffffffu, z, before);
+	const unsigned int et = (w ? x : 0u) + it - t, ef = (w ? y : 0u) + iff - f, em = max(w ? z : 0u, lane ? pm : 0u);
+	__syncthreads();
+	t = et, f = ef, m = em;
+	return tot;
 }
 
 } // namespace mogpu

@@ -1703,40 +1703,6 @@ __device__ __forceinline__ void stopTerms(unsigned char st, unsigned char kd, un
 	errc = (commit && e == e) ? errbits : 0u; // NaN never raises result_error
 }
 
-// block-wide exclusive scan of (sum, sum, max) triples; returns the block totals
-__device__ __forceinline__ uint3 blockScan3(unsigned int& t, unsigned int& f, unsigned int& m, unsigned int (*sm)[33])
-{
-	unsigned int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	unsigned int it = t, iff = f, im = m;
-	for (int o = 1; o < 32; o <<= 1)
-	{
-		unsigned int x = __shfl_up_sync(0xffffffffu, it, o), y = __shfl_up_sync(0xffffffffu, iff, o), z = __shfl_up_sync(0xffffffffu, im, o);
-		if (lane >= (unsigned)o)
-			it += x, iff += y, im = max(im, z);
-	}
-	unsigned int pm = __shfl_up_sync(0xffffffffu, im, 1);
-	if (lane == 31)
-		sm[0][w] = it, sm[1][w] = iff, sm[2][w] = im;
-	__syncthreads();
-	if (threadIdx.x == 0)
-	{
-		unsigned int x = 0, y = 0, z = 0;
-		for (unsigned int q = 0; q < blockDim.x / 32; ++q)
-		{
-			unsigned int a = sm[0][q], b = sm[1][q], c = sm[2][q];
-			sm[0][q] = x, sm[1][q] = y, sm[2][q] = z;
-			x += a, y += b, z = max(z, c);
-		}
-		sm[0][32] = x, sm[1][32] = y, sm[2][32] = z;
-	}
-	__syncthreads();
-	unsigned int et = sm[0][w] + it - t, ef = sm[1][w] + iff - f, em = max(sm[2][w], lane ? pm : 0u);
-	uint3 tot = make_uint3(sm[0][32], sm[1][32], sm[2][32]);
-	__syncthreads();
-	t = et, f = ef, m = em;
-	return tot;
-}
-
 __device__ __forceinline__ bool keepTriangle(const unsigned int* res, size_t t, const unsigned int* cr, const unsigned int* remap,
     uint3& out)
 {

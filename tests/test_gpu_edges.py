@@ -205,3 +205,87 @@ def test_compaction_bad_index_changes_nothing():
         mg.optimize_vertex_fetch_device(d.data_ptr(), di.data_ptr(), 3000, src.data_ptr(), 700, 16)
     assert e.value.status == mg.STATUS_INVALID_ARGUMENT
     assert np.array_equal(di.cpu().numpy(), idx) and bool((d == 9).all())
+
+
+def _grid(nx, ny, amp, seed):
+    a = (np.arange(ny - 1)[:, None] * nx + np.arange(nx - 1)[None, :]).reshape(-1)
+    idx = np.stack([a, a + 1, a + nx, a + nx, a + 1, a + nx + 1], 1).reshape(-1).astype(np.uint32)
+    y, x = np.meshgrid(np.arange(ny), np.arange(nx), indexing="ij")
+    z = amp * np.random.default_rng(seed).standard_normal((ny, nx))
+    return idx, np.stack([x, y, z], -1).reshape(-1, 3).astype(np.float32)
+
+
+def _batch_same(port, ms, threads, smem_kb):
+    mg.set_batch_config(threads, smem_kb * 1024)
+    try:
+        res = mg.simplify_batch(ms)
+    finally:
+        mg.set_batch_config(0)
+    for i, (m, (out, err)) in enumerate(zip(ms, res)):
+        ref, ref_err = port.simplify("port", m["indices"], m["positions"], m["target"], m["error"], m.get("options", 0),
+                                     attributes=m.get("attributes"), weights=m.get("weights"), lock=m.get("lock"))
+        assert np.array_equal(out, ref), f"mesh {i}"
+        assert err == ref_err, f"mesh {i}"
+
+
+SHAPES = [(128, 54), (256, 110), (512, 216), (256, 2)]
+
+
+@pytest.mark.parametrize("threads,smem_kb", SHAPES)
+@pytest.mark.parametrize("amp", [0.0, 1e-3, 0.3])
+def test_batch_decision_windows(port, threads, smem_kb, amp):
+    """Passes whose expected window is just below, at and above the one that a warp walks (224: a goal of
+    160 or 161 triangles), flat meshes (more candidates of one sort key than are ranked in place), and
+    passes that run out of candidates or reach the error limit in the middle of a window."""
+    ms = []
+    for nx, ny in ((2, 2), (4, 3), (9, 9), (17, 17), (14, 26)):
+        idx, pos = _grid(nx, ny, amp, nx)
+        tris = len(idx) // 3
+        for removed in (31, 32, 33, 158, 159, 160, 161, 162, 163, 164, tris):
+            if removed <= tris:
+                for error in (1.0, 1e-2):
+                    ms.append(dict(indices=idx, positions=pos, target=3 * (tris - removed), error=error, options=mg.SimplifyErrorAbsolute))
+    _batch_same(port, ms, threads, smem_kb)
+
+
+@pytest.mark.parametrize("threads,smem_kb", SHAPES)
+@pytest.mark.parametrize("count", [1, 8, 9])
+def test_batch_attribute_rows(port, threads, smem_kb, count):
+    """Attribute gradients summed in registers (up to eight, where there is room) and in place."""
+    rng = np.random.default_rng(count)
+    ms = []
+    for nx, ny in ((5, 4), (17, 17), (24, 20)):
+        idx, pos = _grid(nx, ny, 0.1, nx)
+        ms.append(dict(indices=idx, positions=pos, attributes=rng.standard_normal((len(pos), count)).astype(np.float32),
+                       weights=rng.uniform(0.1, 1.0, count).astype(np.float32), target=len(idx) // 12 * 3, error=1.0))
+    _batch_same(port, ms, threads, smem_kb)
+
+
+@pytest.mark.parametrize("threads,smem_kb", SHAPES)
+def test_batch_beyond_estimate(port, threads, smem_kb):
+    """Meshes that need more vertices or candidates than the launch's shared memory was sized for, so that
+    they start there and go on in the slab: a sparse subset of separate triangles (three vertices for each)
+    and of fans, next to ordinary ones."""
+    rng = np.random.default_rng(9)
+    shared = rng.uniform(0, 1, (6000, 3)).astype(np.float32)
+    idx, pos = _grid(17, 17, 0.1, 3)
+    ms = [dict(indices=idx, positions=pos, target=300, error=1.0)]
+    for tris in (64, 300, 700, 1024):
+        soup = rng.permutation(6000)[: 3 * tris].astype(np.uint32)
+        fan = np.stack([np.zeros(tris, np.int64), np.arange(1, tris + 1), np.arange(2, tris + 2)], 1).reshape(-1).astype(np.uint32)
+        for i in (soup, fan):
+            ms.append(dict(indices=i, positions=shared, target=0, error=1.0, options=mg.SimplifySparse))
+            ms.append(dict(indices=i, positions=shared, target=len(i) // 6 * 3, error=1.0, options=mg.SimplifySparse | mg.SimplifyPermissive))
+    _batch_same(port, ms, threads, smem_kb)
+
+
+@pytest.mark.parametrize("indices,vertices", [(60000, 10201), (60003, 10201), (59994, 24000), (59994, 24001)])
+def test_batch_id_width(port, indices, vertices):
+    """The largest meshes with 16-bit ids and the smallest with 32-bit ones, by indices and by vertices."""
+    idx, pos = _grid(101, 101, 0.2, 1)
+    idx = np.concatenate([idx, idx[: max(0, indices - len(idx))]])[:indices]
+    pos = np.concatenate([pos, np.random.default_rng(2).uniform(0, 100, (vertices - len(pos), 3)).astype(np.float32)])
+    ms = [dict(indices=idx, positions=pos, target=W.target_count(len(idx), 0.5), error=1e-1)]
+    small, sp = _grid(9, 9, 0.2, 1)
+    ms.append(dict(indices=small, positions=sp, target=30, error=1.0))
+    _batch_same(port, ms, 512, 110)
