@@ -1594,14 +1594,7 @@ __device__ __forceinline__ void commitOne(const PerformArgs& a, const uint4& cd,
 // (ringDecide) for the waits, the flip test and the commit; and last the candidates that still
 // wait: locked at once if a commit of this round took an endpoint, else marked for the next round.
 
-#ifndef MO_RING_LANES
-#define MO_RING_LANES 8
-#endif
-#ifndef MO_RING_BATCH
-#define MO_RING_BATCH 1
-#endif
-constexpr unsigned int kRingLanes = MO_RING_LANES; // lanes that walk one candidate's one-ring
-constexpr unsigned int kRingBatch = MO_RING_BATCH; // corners per lane in one batch of loads
+constexpr unsigned int kRingCorners = 8; // corners of a one-ring read at a time
 
 enum
 {
@@ -1610,20 +1603,22 @@ enum
 	kRingCommit = 2,
 };
 
-// One walk over the one-ring of r0, by kRingLanes lanes together (all of `mask`; lane sub == 0 of them
+// One walk over the one-ring of r0, by RL lanes together (all of `mask`; lane sub == 0 of them
 // records the decision). If an undecided earlier candidate moves a vertex of the ring, the candidate
 // waits. Otherwise the flip test (hasTriangleFlips :1201-1232) sees the one-ring as moved by earlier
 // commits only, and the candidate is rejected or commits. The whole ring is checked for waits before
 // a flip decides anything: a wait means an earlier decision is still open that may move a vertex the
 // test reads.
-// Bound by dependent L2 round trips: a ring of up to kRingLanes * kRingBatch corners is two of them
-// (its corners, then their marks and positions), and its corners are read side by side. One lane per
-// candidate, two corners at a time, took three or four batches of both. Whole calls, 256^2
-// heightfield / 2M attribute sphere / 20M terrain, in ms: one lane 0.92 / 4.36 / 40.4; 8 lanes x 1
-// corner 0.81 / 4.22 / 39.0; 4 x 2 0.82 / 4.20 / 38.5; 4 x 1 0.84 / 4.26 / 39.2; 2 x 4 (spills)
-// 0.88 / 4.61 / 43.7. With the candidates' lists in shared memory and blocks of 512: 8 x 1
-// 0.75 / 4.06 / 38.3, 4 x 2 0.77 / 4.12 / 38.3.
-template <bool LOOP>
+// Bound by dependent L2 round trips, and by how many loads are in flight for them: a ring of up to
+// kRingCorners corners is three trips (its corners, their marks, the positions of where they are now), and
+// its corners are read side by side, by RL lanes with kRingCorners / RL of them each. Eight lanes are the
+// least latency for one walk; four walk twice the candidates at a time, the better where all SMs have
+// many to walk. Whole calls, 256^2 heightfield / 2M attribute sphere / 20M terrain, in ms: 8 lanes
+// 0.637 / 3.87 / 35.2; 4 lanes 0.655 / 3.82 / 34.8. With the ring's own positions read along with the
+// marks, and again where a vertex had moved: 8 lanes 0.645 / 3.90 / 35.6, 4 lanes 0.67 / 3.97 / 35.4.
+// One lane per candidate (before lists and blocks were as they are) 0.92 / 4.36 / 40.4, 8 lanes 0.81 /
+// 4.22 / 39.0.
+template <bool LOOP, unsigned int RL>
 __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, unsigned int k, const uint4& rec, unsigned int round, unsigned int sub,
     unsigned int mask)
 {
@@ -1633,16 +1628,15 @@ __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, 
 	const uint4 cd = sub == 0 ? ld<LOOP>(a.crec + c) : make_uint4(0, 0, 0, 0); // in flight during the walk
 	const V3 v0 = ldpos(a.pos, r0), v1 = ldpos(a.pos, r1);
 	bool flip = false;
-	constexpr unsigned int FB = kRingBatch;
-	for (unsigned int j0 = b; j0 < e; j0 += FB * kRingLanes)
+	constexpr unsigned int FB = kRingCorners / RL;
+	for (unsigned int j0 = b; j0 < e; j0 += kRingCorners)
 	{
 		uint2 ed[FB];
 		ulonglong2 sx[FB], sy[FB];
-		float4 px[FB], py[FB];
 #pragma unroll
 		for (unsigned int q = 0; q < FB; ++q)
 		{
-			const unsigned int j = j0 + q * kRingLanes + sub;
+			const unsigned int j = j0 + q * RL + sub;
 			ed[q] = j < e ? ld<LOOP>(a.adj + j) : make_uint2(r1, r1); // r1 is in the ring already
 		}
 #pragma unroll
@@ -1650,8 +1644,6 @@ __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, 
 		{
 			sx[q] = __ldcg(reinterpret_cast<const ulonglong2*>(a.minS) + ed[q].x);
 			sy[q] = __ldcg(reinterpret_cast<const ulonglong2*>(a.minS) + ed[q].y);
-			px[q] = __ldg(a.pos + ed[q].x);
-			py[q] = __ldg(a.pos + ed[q].y);
 		}
 		bool wait = false;
 #pragma unroll
@@ -1669,9 +1661,7 @@ __device__ __forceinline__ int ringDecide(const PerformArgs& a, unsigned int c, 
 			const unsigned int vb = mvy ? (unsigned int)sy[q].y : ed[q].y;
 			if (va == r1 || vb == r1 || va == vb)
 				continue;
-			const V3 pa = mvx ? ldpos(a.pos, va) : V3{px[q].x, px[q].y, px[q].z};
-			const V3 pb = mvy ? ldpos(a.pos, vb) : V3{py[q].x, py[q].y, py[q].z};
-			flip |= triFlip(pa, pb, v0, v1);
+			flip |= triFlip(ldpos(a.pos, va), ldpos(a.pos, vb), v0, v1);
 		}
 	}
 	flip = __any_sync(mask, flip);
@@ -2035,7 +2025,7 @@ __device__ __forceinline__ unsigned int countTriangles(const PassLoopArgs& l, bo
 // kept: the triangles of that buffer; cutv: where the stop rules cut (position and rule). LOOP (kPassLoop): the first window's candidates are marked
 // already, and the next pass's counting (countTriangle) is done as the triangles are written: mine
 // becomes the block's run of them.
-template <bool LOOP>
+template <bool LOOP, unsigned int RL>
 __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopArgs* loop, const PassIn& in, GridSum& grid, const PassShared& sh,
     unsigned int& rounds, unsigned int& kept_total, unsigned long long& cutv, BlockTriangles& mine)
 {
@@ -2051,7 +2041,7 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 	const unsigned int G = gridDim.x;
 	const size_t gthreads = (size_t)G * blockDim.x;
 	const unsigned int lane = threadIdx.x & 31;
-	const unsigned int sub = lane & (kRingLanes - 1), ring_mask = (~0u >> (32 - kRingLanes)) << (lane - sub);
+	const unsigned int sub = lane & (RL - 1), ring_mask = (~0u >> (32 - RL)) << (lane - sub);
 	const unsigned int count = in.count, tris = in.tris, round_base = in.round_base;
 	const unsigned long long goal = in.goal;
 	const float error_limit = in.error_limit;
@@ -2184,15 +2174,15 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 				__syncthreads();
 				// stage B: the one-ring's marks, the flip test and the commit, in one walk
 				const unsigned int nB = s_app[1];
-				for (unsigned int base = 0; base < nB; base += blockDim.x / kRingLanes)
+				for (unsigned int base = 0; base < nB; base += blockDim.x / RL)
 				{
-					const unsigned int x = base + threadIdx.x / kRingLanes;
+					const unsigned int x = base + threadIdx.x / RL;
 					int r = kRingFlip;
 					unsigned int c = 0;
 					if (x < nB)
 					{
 						c = s_stage[0][x];
-						r = ringDecide<LOOP>(a, c, ld<LOOP>(a.rank + c), ld<LOOP>(a.cring + c), round, sub, ring_mask);
+						r = ringDecide<LOOP, RL>(a, c, ld<LOOP>(a.rank + c), ld<LOOP>(a.cring + c), round, sub, ring_mask);
 					}
 					append(sub == 0 && r == kRingWaits, c, &s_app[3], s_stage[1]);
 					append(sub == 0 && r == kRingCommit, c, &s_commits, commits);
@@ -2537,7 +2527,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	unsigned int rounds = 0, kept = 0;
 	unsigned long long cutv;
 	BlockTriangles none;
-	const int r = performPass<false>(a, nullptr, in, grid, sh, rounds, kept, cutv, none);
+	const int r = performPass<false, 8>(a, nullptr, in, grid, sh, rounds, kept, cutv, none);
 	if (r == kPassDone && gtid() == 0)
 		sc->tri_total = kept;
 	if (timer && r != kPassFailed)
@@ -2921,7 +2911,7 @@ __global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArg
 			PhaseClock{s_clock}.skip();
 		unsigned int rounds = 0, kept = 0;
 		unsigned long long cutv = 0;
-		const int r = performPass<true>(a.p, &a, in, grid, sh, rounds, kept, cutv, mine);
+		const int r = performPass<true, PER_SM == 1 ? 8 : 4>(a.p, &a, in, grid, sh, rounds, kept, cutv, mine);
 		if (r == kPassFailed)
 			break;
 		const unsigned int cut = cutv == ~0ull ? C : (unsigned int)(cutv >> 2);
