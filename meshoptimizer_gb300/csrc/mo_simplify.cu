@@ -45,6 +45,17 @@ constexpr size_t kPinnedBytes = 16384; // host readback buffer of the scalars bl
 constexpr unsigned int kStageChunk = MO_STAGE_CHUNK; // candidates of a block taken through the decision stages at a time
 constexpr unsigned int kStageItems = MO_STAGE_ITEMS; // candidates per thread in the first decision stage
 
+// A pass that its first window does not end goes on by windows of an eighth of what it has decided, or
+// kWindowStep, or as much again: each costs a set of decision rounds whatever its size, 150 us or so.
+constexpr unsigned int kWindowStep = 1u << 18;
+
+// What a pass did per candidate that its stop rules let it look at: the next one's are about the same.
+struct PassRates
+{
+	float flips; // flip rejections
+	float tris;  // triangles removed; 0 before the first pass
+};
+
 // Where kPassLoop left the pass loop.
 struct LoopState
 {
@@ -54,7 +65,7 @@ struct LoopState
 	unsigned int stop;       // why it ended
 	unsigned int passes;
 	unsigned int round_base;
-	double window_factor;    // the next pass's first decision window, in units of the triangle goal / 2
+	PassRates rates;         // of the last pass
 };
 
 // The sorted positions a pass decides before its stop rules cut grow from pass to pass relative to
@@ -1976,8 +1987,8 @@ struct PassLoopArgs
 	unsigned int max_passes;
 	unsigned int passes;       // done before this launch, and their decision rounds
 	unsigned int round_base;
-	double window_factor;      // of this launch's first pass
-	double window_base;
+	PassRates rates;           // before this launch's first pass
+	double window_factor;      // first window in units of the triangle goal / 2, or 0: predicted
 	float target_error;
 	int absolute;              // target_error is absolute
 	const unsigned int* res;
@@ -2027,7 +2038,7 @@ __device__ __forceinline__ unsigned int countTriangles(const PassLoopArgs& l, bo
 // becomes the block's run of them.
 template <bool LOOP, unsigned int RL>
 __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopArgs* loop, const PassIn& in, GridSum& grid, const PassShared& sh,
-    unsigned int& rounds, unsigned int& kept_total, unsigned long long& cutv, BlockTriangles& mine)
+    unsigned int& rounds, unsigned int& kept_total, unsigned long long& cutv, unsigned int& flips, BlockTriangles& mine)
 {
 	Scalars* sc = a.sc;
 	PhaseClock pc{sh.clock};
@@ -2144,12 +2155,13 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 					for (unsigned int q = 0; q < kStageItems; ++q)
 					{
 						kk[q] = ok[q] ? ld<LOOP>(a.rank + cc[q]) : 0u;
+						ok[q] = ok[q] && (!first || windows == 1 || (kk[q] >= K0 && kk[q] < K1)); // few of a later window's
 						const uint4 rec = ok[q] ? ld<LOOP>(a.cring + cc[q]) : make_uint4(0, 0, 0, 0);
 						ends[q] = make_uint2(rec.x, rec.y);
 					}
 #pragma unroll
 					for (unsigned int q = 0; q < kStageItems; ++q)
-						ok[q] = ok[q] && (!first || (kk[q] >= K0 && kk[q] < K1));
+						ok[q] = ok[q] && (!first || kk[q] < K1);
 					unsigned long long m0[kStageItems], m1[kStageItems];
 #pragma unroll
 					for (unsigned int q = 0; q < kStageItems; ++q)
@@ -2338,7 +2350,7 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		carryF += ww.y;
 		carryM = ww.z;
 		K0 = K1;
-		K1 = (unsigned int)min((unsigned long long)count, 2ull * K1);
+		K1 = (unsigned int)min((unsigned long long)count, (unsigned long long)K1 + max(K1 / 8, min(K1, kWindowStep)));
 	}
 	if (grid.failed())
 		return kPassFailed;
@@ -2388,6 +2400,7 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		}
 	}
 	grid.wait();
+	flips = __ldcg(&sc->invalid); // a barrier is yet to come before the next pass clears it
 	if (timer)
 		pc.lap(kPhApply);
 	rounds = round - round_base;
@@ -2524,10 +2537,10 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	grid.start(reinterpret_cast<unsigned long long*>(sc->bar), &sc->grid_error, s_grid);
 	resetVertices(a);
 	grid.wait();
-	unsigned int rounds = 0, kept = 0;
+	unsigned int rounds = 0, kept = 0, flips = 0;
 	unsigned long long cutv;
 	BlockTriangles none;
-	const int r = performPass<false, 8>(a, nullptr, in, grid, sh, rounds, kept, cutv, none);
+	const int r = performPass<false, 8>(a, nullptr, in, grid, sh, rounds, kept, cutv, flips, none);
 	if (r == kPassDone && gtid() == 0)
 		sc->tri_total = kept;
 	if (timer && r != kPassFailed)
@@ -2595,6 +2608,12 @@ __device__ __forceinline__ unsigned int loopScan(unsigned int v, unsigned int* r
 	return r;
 }
 
+// the least error of a sort key's bin
+__device__ __forceinline__ float binError(unsigned int bin)
+{
+	return bin < kKeyBins ? __uint_as_float(bin << 19) : FLT_MAX;
+}
+
 // Phase 1 of the first pass: even runs of triangles.
 __device__ __forceinline__ BlockTriangles countFirst(const PassLoopArgs& a, const unsigned int* res, unsigned int tris, unsigned int (*sm)[33])
 {
@@ -2621,7 +2640,7 @@ __device__ __forceinline__ BlockTriangles countFirst(const PassLoopArgs& a, cons
 
 // phases 2 to 5: the pass's ranked, sorted candidates and its first window; false when there are none
 // (in.count is 0 then) or the grid failed
-__device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTriangles& mine, double window_factor, PassIn& in, GridSum& grid,
+__device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTriangles& mine, const PassRates& rates, PassIn& in, GridSum& grid,
     unsigned char* smem, unsigned int (*sm)[33])
 {
 	const PerformArgs& p = a.p;
@@ -2703,8 +2722,6 @@ __device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTr
 	in.count = C;
 	if (C == 0 || grid.failed())
 		return false;
-	const double wf = window_factor * double(in.goal / 2) + 4096.0;
-	in.first_window = unsigned(double(C) < wf ? double(C) : wf);
 
 	// ---- 3: adjacency; the candidates ranked; the sorting blocks' key histograms
 	for (unsigned int t = mine.begin + tid; t < mine.end; t += kPerformThreads)
@@ -2777,19 +2794,74 @@ __device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTr
 	}
 	grid.wait();
 
-	// ---- 5: sorted positions, as kKeyScatter gives them; the first window's candidates mark their
-	// endpoints for the first decision round
-	if (B < rows)
+	// ---- 5: the first window; sorted positions, as kKeyScatter gives them; the first window's
+	// candidates mark their endpoints for the first decision round
+	constexpr unsigned int kPer = kKeyBins / kPerformThreads;
+	static_assert(kPer * kPerformThreads == kKeyBins, "bins divide among the threads");
+	unsigned int* const gbase = reinterpret_cast<unsigned int*>(smem);
+	unsigned int tot[kPer], s = 0, dummy;
+#pragma unroll
+	for (unsigned int q = 0; q < kPer; ++q)
+		tot[q] = __ldcg(totals + tid * kPer + q), s += tot[q];
+	const unsigned int bin0 = loopScan(s, sm[0], dummy); // the thread's first bin's start
 	{
-		unsigned int* const gbase = reinterpret_cast<unsigned int*>(smem);
-		unsigned char* const wcnt = smem + kKeyBins * 4; // per key, 16 warps: the step's count
-		constexpr unsigned int kPer = kKeyBins / kPerformThreads;
-		static_assert(kPer * kPerformThreads == kKeyBins, "bins divide among the threads");
-		unsigned int tot[kPer], s = 0;
+		unsigned int* const start = gbase;
+		__shared__ unsigned int s_limit, s_errors;
+		if (tid == 0)
+			s_limit = s_errors = C;
+		unsigned int o = bin0;
 #pragma unroll
 		for (unsigned int q = 0; q < kPer; ++q)
-			tot[q] = __ldcg(totals + tid * kPer + q), s += tot[q];
-		unsigned int dummy, o = loopScan(s, sm[0], dummy);
+		{
+			start[tid * kPer + q] = o;
+			o += tot[q];
+		}
+		__syncthreads();
+		// The window is to end just behind the position at which the stop rules will: every candidate
+		// in it is decided, and a second window costs a set of rounds more. That is the first of: the
+		// first bin beyond the error limit; the first beyond the error goal, with some more flip
+		// rejections per candidate than the last pass had; and as many candidates as removed the
+		// goal's triangles at the last pass's rate, which the cheapest ones exceed. Whole calls with
+		// this, and with 1.5 times what the last pass looked at relative to its goal (2 for the first
+		// pass), in ms: tile of 101 x 67 0.596 and 0.795, 256^2 heightfield 0.622 and 0.639, 2M
+		// attribute sphere 3.80 and 3.82, 20M terrain 32.2 and 34.8 (130M and 184M candidate rounds).
+		const float flips = 1.5f * rates.flips + 0.02f;
+#pragma unroll
+		for (unsigned int q = 0; q < kPer; ++q)
+		{
+			const unsigned int bin = q * kPerformThreads + tid, at = start[bin];
+			if (at == (bin + 1 < kKeyBins ? start[bin + 1] : C))
+				continue;
+			const float least = binError(bin);
+			if (least > in.error_limit)
+				atomicMin(&s_limit, at);
+			const unsigned long long goal_at = in.goal / 2 + (unsigned long long)(flips * float(at));
+			if (goal_at < C)
+			{
+				unsigned int lo = 0, hi = kKeyBins; // lo: the last bin that starts at or before goal_at
+				while (hi - lo > 1)
+				{
+					const unsigned int mid = (lo + hi) / 2;
+					(start[mid] <= goal_at ? lo : hi) = mid;
+				}
+				if (least > 1.5f * binError(lo + 1))
+					atomicMin(&s_errors, at);
+			}
+		}
+		__syncthreads();
+		double window = double(s_errors) + 256;
+		if (rates.tris > 0)
+			window = fmin(window, double(in.goal) / rates.tris + 256);
+		window = fmin(window, double(s_limit) + 1);
+		if (a.window_factor > 0)
+			window = a.window_factor * double(in.goal / 2) + 4096;
+		in.first_window = unsigned(double(C) < window ? double(C) : window);
+		__syncthreads();
+	}
+	if (B < rows)
+	{
+		unsigned char* const wcnt = smem + kKeyBins * 4; // per key, 16 warps: the step's count
+		unsigned int o = bin0;
 #pragma unroll
 		for (unsigned int q = 0; q < kPer; ++q)
 		{
@@ -2887,7 +2959,7 @@ __global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArg
 	unsigned int indices = a.index_count, passes = a.passes, round_base = a.round_base;
 	const unsigned int* res = a.res;
 	unsigned int* res_next = a.res_next;
-	double window_factor = a.window_factor;
+	PassRates rates = a.rates;
 	unsigned int stop = kLoopEnded;
 	BlockTriangles mine;
 	while (indices > a.target)
@@ -2903,15 +2975,14 @@ __global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArg
 		in.res_next = res_next;
 		if (passes == a.passes)
 			mine = countFirst(a, res, tris, sm);
-		if (!preparePass(a, mine, window_factor, in, grid, loop_smem, sm))
+		if (!preparePass(a, mine, rates, in, grid, loop_smem, sm))
 			break;
 		const unsigned int C = in.count;
-		const unsigned long long goal = in.goal;
 		if (timer)
 			PhaseClock{s_clock}.skip();
-		unsigned int rounds = 0, kept = 0;
+		unsigned int rounds = 0, kept = 0, flips = 0;
 		unsigned long long cutv = 0;
-		const int r = performPass<true, PER_SM == 1 ? 8 : 4>(a.p, &a, in, grid, sh, rounds, kept, cutv, mine);
+		const int r = performPass<true, PER_SM == 1 ? 8 : 4>(a.p, &a, in, grid, sh, rounds, kept, cutv, flips, mine);
 		if (r == kPassFailed)
 			break;
 		const unsigned int cut = cutv == ~0ull ? C : (unsigned int)(cutv >> 2);
@@ -2930,7 +3001,8 @@ __global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArg
 			ps.active = (unsigned int)sc->active_sum;
 			ps.windows = sc->windows;
 		}
-		window_factor = nextWindowFactor(a.window_base, goal, evaluated);
+		rates.flips = float(flips) / float(evaluated);
+		rates.tris = float(tris - kept) / float(evaluated);
 		round_base += rounds;
 		passes++;
 		if (r == kPassEmpty)
@@ -2961,7 +3033,7 @@ __global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArg
 		lv.indices = indices;
 		lv.passes = passes;
 		lv.round_base = round_base;
-		lv.window_factor = window_factor;
+		lv.rates = rates;
 		lv.stop = stop;
 	}
 }
@@ -4097,7 +4169,9 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	else if (m.options & kOptPrune)
 		comp_next = FLT_MAX;
 	int passes = 0;
-	double window_factor = tuning_.window_factor; // the first window of the next pass
+	const double window_base = tuning_.window_factor > 0 ? tuning_.window_factor : 2.0;
+	double window_factor = window_base; // the first window of the host loop's next pass
+	PassRates rates{};
 	unsigned int round_base = 0; // decision rounds are numbered across the run (mark tags never repeat)
 
 	// the pass kernel's arguments but for the pass's own values
@@ -4165,7 +4239,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		la.hist = w.scratch;
 		la.target = unsigned(m.target_index_count);
 		la.max_passes = unsigned(I / 3 + 1);
-		la.window_base = tuning_.window_factor;
+		la.window_factor = tuning_.window_factor;
 		la.target_error = m.target_error;
 		la.absolute = (m.options & kOptErrorAbsolute) ? 1 : 0;
 		la.prune = (m.options & kOptPrune) ? 1 : 0;
@@ -4175,7 +4249,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 			la.index_count = unsigned(result_count);
 			la.passes = unsigned(passes);
 			la.round_base = round_base;
-			la.window_factor = window_factor;
+			la.rates = rates;
 			la.res = res;
 			la.res_next = res_next;
 			la.prune_error = comp_next;
@@ -4194,7 +4268,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 				                                            : (hs->grid_error & 2 ? "collapse decision round made no progress" : "grid barrier wait limit reached"));
 			passes = int(hs->live.passes);
 			round_base = hs->live.round_base;
-			window_factor = hs->live.window_factor;
+			rates = hs->live.rates;
 			result_count = hs->live.indices;
 			res = const_cast<unsigned int*>(hs->live.res);
 			res_next = hs->live.res_next;
@@ -4292,7 +4366,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 			ps.active = unsigned(hs->active_sum);
 			ps.windows = hs->windows;
 		}
-		window_factor = nextWindowFactor(tuning_.window_factor, goal, cut < C ? cut + 1 : C);
+		window_factor = nextWindowFactor(window_base, goal, cut < C ? cut + 1 : C);
 		passes++;
 		result_error_bits = hs->result_error_bits;
 		if (hs->done == 0)

@@ -117,7 +117,7 @@ private:
 struct Tuning
 {
 	int perform_blocks_per_sm = 0;  // resident blocks (512 threads) per SM of the pass kernels (0: by size)
-	double window_factor = 2.0;     // first decision window = factor * (triangle goal / 2) + 4096
+	double window_factor = 0;       // first decision window = factor * (triangle goal / 2) + 4096; 0: from the errors and the last pass
 	int perform_grid_cap = 0;       // at most this many blocks of 256 threads for the pass kernel and the
 	                                // scans (0: no cap); lets concurrent simplifications share the GPU
 	bool device_loop = true;        // run the pass loop in one launch (off: a launch per phase from the host

@@ -289,3 +289,20 @@ def test_batch_id_width(port, indices, vertices):
     small, sp = _grid(9, 9, 0.2, 1)
     ms.append(dict(indices=small, positions=sp, target=30, error=1.0))
     _batch_same(port, ms, 512, 110)
+
+
+@pytest.mark.parametrize("factor", ["0.01", "0.3", "60"])
+def test_pass_loop_windows(port, single_path, monkeypatch, factor):
+    """Passes decided in many windows, in a few, and in one that takes every candidate, next to the predicted
+    one of the other tests. The factor is read where a thread's state is made, so each case has a thread."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    monkeypatch.setenv("MESHOPTGPU_WINDOW_FACTOR", factor)
+    for nx, ny, amp, ratio, error in ((17, 17, 0.2, 0.2, 1.0), (120, 90, 0.0, 0.3, 1.0), (301, 299, 0.4, 0.1, 1.0), (301, 299, 0.4, 0.0, 1e-3)):
+        idx, pos = _grid(nx, ny, amp, nx)
+        target = W.target_count(len(idx), ratio)
+        ref, ref_err = port.simplify("port", idx, pos, target, error, mg.SimplifyPrune)
+        with ThreadPoolExecutor(1) as pool:
+            out, err = pool.submit(mg.simplify, idx, pos, target, error, mg.SimplifyPrune).result()
+        assert np.array_equal(out, ref)
+        assert err == ref_err
