@@ -93,6 +93,7 @@ struct Scalars
 	unsigned int probe_fail;
 	unsigned int dup_count;
 	unsigned int capacity;
+	unsigned int rescaled; // blocks of kRescale that are done
 	unsigned long long dual;
 	unsigned int pick_total;
 	unsigned int pick_trunc;
@@ -268,16 +269,6 @@ __global__ void __launch_bounds__(kMinMaxThreads) kMinMaxFinal(const float* __re
 	sc->scale = extent == 0 ? 0.f : 1.f / extent;
 }
 
-__global__ void kRescale(const float4* __restrict__ raw, size_t n, const Scalars* __restrict__ sc, float4* __restrict__ out)
-{
-	size_t i = gtid();
-	if (i >= n)
-		return;
-	float4 p = raw[i];
-	float s = sc->scale;
-	out[i] = make_float4((p.x - sc->minv[0]) * s, (p.y - sc->minv[1]) * s, (p.z - sc->minv[2]) * s, 0.f);
-}
-
 // ---------------------------------------------------------------- setup: position remap
 
 __device__ __forceinline__ unsigned int mix32(unsigned int h)
@@ -301,12 +292,16 @@ __device__ __forceinline__ unsigned int posBits(float f)
 // lowers it to the smallest index with atomicMin. Equal positions hash alike and follow the
 // same probe sequence, and slots are never freed, so all members of a class meet in one slot.
 // Result: remap[i] = smallest index with an equal position (buildPositionRemap :195-214).
-__global__ void kHashInsert(const float4* __restrict__ pos, size_t n, unsigned int* table, unsigned int mask, unsigned int* __restrict__ slot_of, unsigned int* fail)
+// The positions are gathered to rows of four on the way.
+__global__ void kHashInsert(const float* __restrict__ data, size_t stride_f, size_t n, float4* __restrict__ pos, unsigned int* table, unsigned int mask,
+    unsigned int* __restrict__ slot_of, unsigned int* fail)
 {
 	size_t i = gtid();
 	if (i >= n)
 		return;
-	float4 p = pos[i];
+	const float* v = data + i * stride_f;
+	const float4 p = make_float4(v[0], v[1], v[2], 0.f);
+	pos[i] = p;
 	unsigned int h = mix32(posBits(p.x) * 0x9e3779b1u ^ mix32(posBits(p.y) + 0x85ebca6bu) ^ mix32(posBits(p.z) * 0xc2b2ae35u + 1u));
 	unsigned int b = h & mask;
 	for (unsigned int probe = 0; probe <= mask; ++probe)
@@ -322,8 +317,8 @@ __global__ void kHashInsert(const float4* __restrict__ pos, size_t n, unsigned i
 			}
 			cur = prev;
 		}
-		float4 q = pos[cur];
-		if (q.x == p.x && q.y == p.y && q.z == p.z)
+		const float* q = data + (size_t)cur * stride_f;
+		if (q[0] == p.x && q[1] == p.y && q[2] == p.z)
 		{
 			atomicMin(&table[b], (unsigned int)i);
 			slot_of[i] = b;
@@ -335,17 +330,23 @@ __global__ void kHashInsert(const float4* __restrict__ pos, size_t n, unsigned i
 	slot_of[i] = ~0u;
 }
 
+// dups: how many there are (added to; null: not counted)
 __global__ void kHashRemap(const unsigned int* __restrict__ table, const unsigned int* __restrict__ slot_of, size_t n, unsigned int* __restrict__ remap,
-    unsigned int* __restrict__ wedge, unsigned int* __restrict__ dupflag)
+    unsigned int* __restrict__ wedge, unsigned int* __restrict__ dupflag, unsigned int* dups)
 {
 	size_t i = gtid();
-	if (i >= n)
-		return;
-	unsigned int s = slot_of[i];
-	unsigned int r = s == ~0u ? (unsigned int)i : table[s];
-	remap[i] = r;
-	wedge[i] = (unsigned int)i;
-	dupflag[i] = r != i;
+	bool dup = false;
+	if (i < n)
+	{
+		unsigned int s = slot_of[i];
+		unsigned int r = s == ~0u ? (unsigned int)i : table[s];
+		remap[i] = r;
+		wedge[i] = (unsigned int)i;
+		dupflag[i] = dup = r != i;
+	}
+	const unsigned int m = __ballot_sync(0xffffffffu, dup);
+	if (dups && m && (threadIdx.x & 31) == 0)
+		atomicAdd(dups, __popc(m));
 }
 
 // dup vertices sorted by (class, index): wedge[i] = previous member of the class (the
@@ -387,10 +388,10 @@ __global__ void kCountKeys(const unsigned int* __restrict__ idx, const unsigned 
 }
 
 // the corners of every vertex, each corner keeping its slot in its vertex's list; an index of
-// vcount or more is not counted and sets bad. The indices are copied to res on the way (the
+// vcount or more is not counted and sets bad; most: the longest list. The indices are copied to res on the way (the
 // first pass's index buffer).
 __global__ void kCountCornerLists(const unsigned int* __restrict__ idx, size_t n, size_t vcount, unsigned int* __restrict__ cnt,
-    unsigned int* __restrict__ slot, unsigned int* bad, unsigned int* __restrict__ res)
+    unsigned int* __restrict__ slot, unsigned int* bad, unsigned int* __restrict__ res, unsigned int* most)
 {
 	const size_t i = gtid();
 	if (i - (threadIdx.x & 31) >= n)
@@ -412,29 +413,13 @@ __global__ void kCountCornerLists(const unsigned int* __restrict__ idx, size_t n
 	if (valid && lane == leader)
 		base = atomicAdd(&cnt[v], __popc(peers));
 	base = __shfl_sync(0xffffffffu, base, leader);
+	const unsigned int at = base + __popc(peers & ((1u << lane) - 1u));
 	if (valid)
-		slot[i] = base + __popc(peers & ((1u << lane) - 1u));
-}
-
-// the largest count of corners[v] = off[v+1] - off[v]
-__global__ void kMaxDegree(const unsigned int* __restrict__ off, size_t n, unsigned int* out)
-{
-	__shared__ unsigned int wmax[32];
-	size_t i = gtid();
-	unsigned int d = i < n ? off[i + 1] - off[i] : 0u;
-	for (int o = 16; o > 0; o >>= 1)
-		d = max(d, __shfl_down_sync(0xffffffffu, d, o));
-	if ((threadIdx.x & 31) == 0)
-		wmax[threadIdx.x >> 5] = d;
-	__syncthreads();
-	if (threadIdx.x < 32)
-	{
-		d = threadIdx.x < blockDim.x / 32 ? wmax[threadIdx.x] : 0u;
-		for (int o = 16; o > 0; o >>= 1)
-			d = max(d, __shfl_down_sync(0xffffffffu, d, o));
-		if (threadIdx.x == 0 && d)
-			atomicMax(out, d); // one atomic per block
-	}
+		slot[i] = at;
+	// the vertex's last corner has the largest slot
+	const unsigned int longest = __reduce_max_sync(0xffffffffu, valid ? at + 1 : 0u);
+	if (lane == 0 && longest > *most) // an old value costs an atomic, no more
+		atomicMax(most, longest);
 }
 
 // vertex -> corner lists: every corner into its vertex's range at the slot its count gave it
@@ -457,11 +442,8 @@ __global__ void kCornerFill(const unsigned int* __restrict__ idx, const unsigned
 constexpr unsigned int kCornerSortMax = 64;
 constexpr unsigned int kCornerRegs = 16; // lists up to this long are sorted in registers
 
-__global__ void kCornerSort(const unsigned int* __restrict__ off, size_t n, unsigned int* csr)
+__device__ __forceinline__ void sortCorners(const unsigned int* __restrict__ off, size_t v, unsigned int* csr)
 {
-	size_t v = gtid();
-	if (v >= n)
-		return;
 	const unsigned int b = off[v], e = off[v + 1];
 	if (e - b <= kCornerRegs)
 	{
@@ -522,12 +504,9 @@ constexpr unsigned int kFillBatch = MO_FILL_BATCH; // corners whose loads kFillQ
 // openout (stored in loop) and openinc (stored in loopback) of classifyVertices :370-396,
 // from the vertex's own raw half-edge list: ~0u for none, the unique open neighbour, or the
 // vertex itself for several / a degenerate triangle.
-__global__ void kOpenEdges(const unsigned int* __restrict__ idx, const unsigned int* __restrict__ off, const unsigned int* __restrict__ csr, size_t n,
+__device__ __forceinline__ void openEdges(const unsigned int* __restrict__ idx, const unsigned int* __restrict__ off, const unsigned int* csr, size_t vi,
     unsigned int* __restrict__ loop, unsigned int* __restrict__ loopback)
 {
-	size_t vi = gtid();
-	if (vi >= n)
-		return;
 	unsigned int v = (unsigned int)vi;
 	unsigned int b = off[v], e = off[v + 1];
 	if (e - b <= kOpenEdgesRegs)
@@ -601,6 +580,25 @@ __global__ void kOpenEdges(const unsigned int* __restrict__ idx, const unsigned 
 		}
 	loop[v] = degen ? v : (outc == 0 ? ~0u : (outc == 1 ? outt : v));
 	loopback[v] = degen ? v : (inc == 0 ? ~0u : (inc == 1 ? ins : v));
+}
+
+__global__ void kOpenEdges(const unsigned int* __restrict__ idx, const unsigned int* __restrict__ off, const unsigned int* csr, size_t n,
+    unsigned int* __restrict__ loop, unsigned int* __restrict__ loopback)
+{
+	const size_t v = gtid();
+	if (v < n)
+		openEdges(idx, off, csr, v, loop, loopback);
+}
+
+// the same after sorting the vertex's list
+__global__ void kCornerSort(const unsigned int* __restrict__ idx, const unsigned int* __restrict__ off, unsigned int* csr, size_t n,
+    unsigned int* __restrict__ loop, unsigned int* __restrict__ loopback)
+{
+	const size_t v = gtid();
+	if (v >= n)
+		return;
+	sortCorners(off, v, csr);
+	openEdges(idx, off, csr, v, loop, loopback);
 }
 
 // classifyVertices :405-471 for the primary vertex i
@@ -1073,17 +1071,21 @@ __global__ void kFillAttributeQuadrics(const unsigned int* __restrict__ idx, con
 			ag[(size_t)v * count + k] = G[k];
 }
 
-// boundEdgeCollapses :1292-1308 numerator: sum of degrees of manifold and seam vertices (one
-// global add per block: the adds all go to one address)
-__global__ void __launch_bounds__(kThreads) kDualCount(const unsigned int* __restrict__ off, const unsigned char* __restrict__ kind, size_t n,
-    unsigned long long* dual)
+// The rescaled positions (rescalePositions :544-603), and boundEdgeCollapses :1292-1308: the sum of degrees
+// of manifold and seam vertices (one global add per block: the adds all go to one address), from which the
+// last block gets the capacity.
+__global__ void __launch_bounds__(kThreads) kRescale(const float4* __restrict__ raw, size_t n, Scalars* sc, float4* __restrict__ out,
+    const unsigned int* __restrict__ off, const unsigned char* __restrict__ kind, size_t index_count)
 {
 	__shared__ unsigned int wsum[kThreads / 32];
 	size_t i = gtid();
 	unsigned int d = 0;
 	if (i < n)
 	{
-		unsigned char k = kind[i];
+		const float4 p = raw[i];
+		const float s = sc->scale;
+		out[i] = make_float4((p.x - sc->minv[0]) * s, (p.y - sc->minv[1]) * s, (p.z - sc->minv[2]) * s, 0.f);
+		const unsigned char k = kind[i];
 		d = (k == kManifold || k == kSeam) ? (off[i + 1] - off[i]) : 0;
 	}
 	for (int o = 16; o > 0; o >>= 1)
@@ -1097,14 +1099,11 @@ __global__ void __launch_bounds__(kThreads) kDualCount(const unsigned int* __res
 		for (int q = 0; q < kThreads / 32; ++q)
 			b += wsum[q];
 		if (b)
-			atomicAdd(dual, b);
+			atomicAdd(&sc->dual, b);
+		__threadfence();
+		if (atomicAdd(&sc->rescaled, 1u) == gridDim.x - 1)
+			sc->capacity = (unsigned int)((index_count - atomicAdd(&sc->dual, 0ull) / 2) + 3);
 	}
-}
-
-__global__ void kCapacity(size_t index_count, Scalars* sc)
-{
-	if (threadIdx.x == 0 && blockIdx.x == 0)
-		sc->capacity = (unsigned int)((index_count - sc->dual / 2) + 3);
 }
 
 // ---------------------------------------------------------------- pass: adjacency
@@ -3939,18 +3938,16 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 
 	MO_CUDA_CHECK(cudaMemsetAsync(w.sc, 0, sizeof(Scalars), stream));
 
-	// ---- setup
+	// ---- setup: a chain of kernels of 3 to 14 us on a 256^2 heightfield, as long in their launches as in
+	// their work, so that what can ride along with another kernel does (the gather, the counts of duplicates
+	// and of the longest list, the capacity, the sort of a vertex's corners): 17 launches to 12, 624 us to 605
 	const unsigned int gV = gridFor(V, kThreads), gI = gridFor(I, kThreads);
-	if (V)
-		MO_LAUNCH(kGatherPositions, gV, kThreads, 0, stream, m.positions, m.positions_stride / 4, V, w.pos_raw);
-
-	// position remap + wedges
+	// positions, their remap + wedges
 	MO_CUDA_CHECK(cudaMemsetAsync(w.table, 0xFF, size_t(w.hash_mask + 1) * 4, stream));
 	if (V)
 	{
-		MO_LAUNCH(kHashInsert, gV, kThreads, 0, stream, w.pos_raw, V, w.table, w.hash_mask, w.slot, &w.sc->probe_fail);
-		MO_LAUNCH(kHashRemap, gV, kThreads, 0, stream, w.table, w.slot, V, w.remap, w.wedge, w.flags);
-		scanExclusive(w.flags, w.flags, V, &w.sc->dup_count, w.scratch, stream, ss);
+		MO_LAUNCH(kHashInsert, gV, kThreads, 0, stream, m.positions, m.positions_stride / 4, V, w.pos_raw, w.table, w.hash_mask, w.slot, &w.sc->probe_fail);
+		MO_LAUNCH(kHashRemap, gV, kThreads, 0, stream, w.table, w.slot, V, w.remap, w.wedge, w.cnt, &w.sc->dup_count);
 	}
 	// vertex -> corner lists in corner order: raw (classification, attribute quadrics) and
 	// remapped (position quadrics). Their offsets and largest degrees come before the host read
@@ -3965,11 +3962,8 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	if (m.indices_ready)
 		MO_CUDA_CHECK(cudaStreamWaitEvent(stream, m.indices_ready, 0));
 	if (I)
-		MO_LAUNCH(kCountCornerLists, gI, kThreads, 0, stream, m.indices, I, V, w.off_raw, slot_raw, &w.sc->bad_index, w.res0);
+		MO_LAUNCH(kCountCornerLists, gI, kThreads, 0, stream, m.indices, I, V, w.off_raw, slot_raw, &w.sc->bad_index, w.res0, &w.sc->max_degree);
 	scanExclusive(w.off_raw, w.off_raw, V + 1, nullptr, w.scratch, stream, ss);
-	if (V)
-		MO_LAUNCH(kMaxDegree, gV, kThreads, 0, stream, w.off_raw, V, &w.sc->max_degree);
-	// flags now hold offsets; recompute flags from remap in the compaction kernel
 	readScalars();
 	if (hs->bad_index)
 		throw std::invalid_argument("index out of range of vertex_count");
@@ -3978,8 +3972,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	const size_t D = hs->dup_count;
 	if (D)
 	{
-		// rebuild the dup flags (the scan consumed them) into cnt, then compact
-		MO_LAUNCH(kHashRemap, gV, kThreads, 0, stream, w.table, w.slot, V, w.remap, w.wedge, w.cnt);
+		scanExclusive(w.cnt, w.flags, V, nullptr, w.scratch, stream, ss);
 		MO_LAUNCH(kCompactFlagged, gV, kThreads, 0, stream, w.cnt, w.flags, w.remap, V, w.keys_b, w.vals_b);
 		radixSortPairs(w.keys_b, w.vals_b, w.keys_a, w.vals_a, w.cerr, reinterpret_cast<unsigned int*>(w.crec), D, bitsFor(V), w.scratch, stream, ss);
 		MO_LAUNCH(kWedgeLink, gridFor(D, kThreads), kThreads, 0, stream, w.keys_a, w.vals_a, D, w.wedge);
@@ -3992,7 +3985,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		if (I && V)
 		{
 			MO_LAUNCH(kCornerFill, gI, kThreads, 0, stream, w.res0, nullptr, I, w.off_raw, slot_raw, w.csr_raw);
-			MO_LAUNCH(kCornerSort, gV, kThreads, 0, stream, w.off_raw, V, w.csr_raw);
+			MO_LAUNCH(kCornerSort, gV, kThreads, 0, stream, w.res0, w.off_raw, w.csr_raw, V, w.loop, w.loopback);
 		}
 	}
 	else
@@ -4000,11 +3993,12 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		// a vertex with many corners: a stable radix sort by vertex
 		radixSortPairs(w.res0, nullptr, w.keys_a, w.csr_raw, w.keys_b, w.vals_b, I, vbits, w.scratch, stream, ss);
 	}
+	if (V && (!I || hs->max_degree > kCornerSortMax))
+		MO_LAUNCH(kOpenEdges, gV, kThreads, 0, stream, w.res0, w.off_raw, w.csr_raw, V, w.loop, w.loopback);
 
 	// classification
 	if (V)
 	{
-		MO_LAUNCH(kOpenEdges, gV, kThreads, 0, stream, w.res0, w.off_raw, w.csr_raw, V, w.loop, w.loopback);
 		MO_LAUNCH(kClassify, gV, kThreads, 0, stream, V, w.remap, w.wedge, w.loop, w.loopback, w.kind);
 		if (m.options & kOptPermissive)
 		{
@@ -4026,8 +4020,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	unsigned int mmb = gridFor((V + per - 1) / per, kMinMaxThreads);
 	MO_LAUNCH(kMinMaxPartial, mmb, kMinMaxThreads, 0, stream, w.pos_raw, V, per, w.partial);
 	MO_LAUNCH(kMinMaxFinal, 1, kMinMaxThreads, 0, stream, w.partial, mmb, w.sc);
-	if (V)
-		MO_LAUNCH(kRescale, gV, kThreads, 0, stream, w.pos_raw, V, w.sc, w.pos);
+	MO_LAUNCH(kRescale, gridFor(std::max<size_t>(V, 1), kThreads), kThreads, 0, stream, w.pos_raw, V, w.sc, w.pos, w.off_raw, w.kind, I);
 	if (ac && V)
 	{
 		if (m.attributes_ready)
@@ -4069,9 +4062,6 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		radixSortPairs(w.comp, nullptr, w.keys_a, w.vals_a, w.keys_b, w.vals_b, V, bitsFor(comp_count ? comp_count - 1 : 0), w.scratch, stream, ss);
 		MO_LAUNCH(kMeasureComponents, gridFor(comp_count, kMeasureWarps), kMeasureWarps * 32, 0, stream, comp_count, w.comp_off, w.vals_a, w.pos, w.comp_err);
 	}
-	if (V)
-		MO_LAUNCH(kDualCount, gV, kThreads, 0, stream, w.off_raw, w.kind, V, &w.sc->dual);
-	MO_LAUNCH(kCapacity, 1, 32, 0, stream, I, w.sc);
 	MO_CUDA_CHECK(cudaGetLastError());
 
 	// The one-launch pass loop (below) takes no host values from setup, so it is queued behind it and the
