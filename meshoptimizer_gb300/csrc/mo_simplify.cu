@@ -376,17 +376,6 @@ __global__ void kCompactFlagged(const unsigned int* __restrict__ flags, const un
 
 // ---------------------------------------------------------------- setup: CSR
 
-__global__ void kCountKeys(const unsigned int* __restrict__ idx, const unsigned int* __restrict__ remap, size_t n, unsigned int* __restrict__ cnt)
-{
-	size_t i = gtid();
-	if (i >= n)
-		return;
-	unsigned int v = idx[i];
-	if (remap)
-		v = remap[v];
-	atomicAdd(&cnt[v], 1u);
-}
-
 // the corners of every vertex, each corner keeping its slot in its vertex's list; an index of
 // vcount or more is not counted and sets bad; most: the longest list. The indices are copied to res on the way (the
 // first pass's index buffer).
@@ -3349,73 +3338,98 @@ __global__ void kComponentIds(size_t n, const unsigned int* __restrict__ remap, 
 	comp[i] = rootrank[r];
 }
 
-// center = average position (sums in vertex order, as measureComponents), radius^2 = max
-// squared distance; one warp per component over its vertices sorted by (component, index).
-// Bound by the sum's chain of dependent adds, one per vertex and axis: the lanes gather a tile of
-// positions through shared memory while lanes 0-2 add the tile before it, one axis each. One thread
-// per component paid two dependent loads per vertex instead: a 188k-triangle scan of 23 pieces, whole
-// call 4.19 ms then, 2.12 ms now.
-constexpr unsigned int kMeasureWarps = 4;
-constexpr unsigned int kMeasureItems = 8; // positions of a tile per lane
-__global__ void __launch_bounds__(kMeasureWarps * 32) kMeasureComponents(size_t ncomp, const unsigned int* __restrict__ off,
-    const unsigned int* __restrict__ verts, const float4* __restrict__ pos, float* __restrict__ err)
+// where each component's vertices start in the list sorted by (component, index); every component has some
+__global__ void kComponentStarts(const unsigned int* __restrict__ sorted, size_t n, size_t ncomp, unsigned int* __restrict__ start)
 {
-	constexpr unsigned int kTile = 32 * kMeasureItems;
-	__shared__ float tile[kMeasureWarps][3][kTile];
-	const unsigned int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	const size_t c = (size_t)blockIdx.x * kMeasureWarps + w;
-	if (c >= ncomp)
+	const size_t i = gtid();
+	if (i >= n)
 		return;
-	const unsigned int b = off[c], e = off[c + 1];
+	if (i == 0 || sorted[i] != sorted[i - 1])
+		start[sorted[i]] = (unsigned int)i;
+	if (i == 0)
+		start[ncomp] = (unsigned int)n;
+}
+
+// center = average position (sums in vertex order, as measureComponents), radius^2 = max
+// squared distance; one block of T threads per component over its vertices sorted by (component, index).
+// Bound by the sum's chain of dependent adds, one per vertex and axis: the block gathers a tile of
+// positions through shared memory while its threads 0-2 add the tile before it, one axis each, four
+// positions a load. A block of one warp where components are small (many of them share an SM), of 256
+// threads where they have kMeasureWide vertices or more on average (few tiles, gathered faster).
+// A 188k-triangle scan of 23 pieces, whole call: one thread per component, with two dependent loads per
+// vertex, 4.19 ms; a warp, 2.12 (163 us in this kernel, of 1.27 ms since other steps); a block, and the
+// starts from the sorted list where they were counted with atomics, 1.13.
+constexpr size_t kMeasureWide = 512;
+template <unsigned int T>
+__global__ void __launch_bounds__(T) kMeasureComponents(const unsigned int* __restrict__ off, const unsigned int* __restrict__ verts,
+    const float4* __restrict__ pos, float* __restrict__ err)
+{
+	constexpr unsigned int kMeasureThreads = T, kMeasureItems = T == 32 ? 8 : 4; // positions of a tile per thread
+	constexpr unsigned int kTile = kMeasureThreads * kMeasureItems;
+	__shared__ float4 tile[2][3][kTile / 4];
+	__shared__ float s_center[3], s_far[kMeasureThreads / 32];
+	const unsigned int tid = threadIdx.x;
+	const unsigned int b = off[blockIdx.x], e = off[blockIdx.x + 1];
 	float4 p[kMeasureItems];
 	auto gather = [&](unsigned int base) {
 		unsigned int v[kMeasureItems];
 #pragma unroll
 		for (unsigned int q = 0; q < kMeasureItems; ++q)
 		{
-			const unsigned int j = base + q * 32 + lane;
+			const unsigned int j = base + q * kMeasureThreads + tid;
 			v[q] = j < e ? verts[j] : ~0u;
 		}
 #pragma unroll
 		for (unsigned int q = 0; q < kMeasureItems; ++q)
 			p[q] = v[q] != ~0u ? __ldg(pos + v[q]) : make_float4(0.f, 0.f, 0.f, 0.f);
 	};
-	float sum = 0.f; // of this lane's axis
+	float sum = 0.f; // of this thread's axis
+	unsigned int turn = 0;
 	gather(b);
-	for (unsigned int base = b; base < e; base += kTile)
+	for (unsigned int base = b; base < e; base += min(kTile, e - base), turn ^= 1)
 	{
-		__syncwarp();
+		float* const to = reinterpret_cast<float*>(tile[turn]);
 #pragma unroll
 		for (unsigned int q = 0; q < kMeasureItems; ++q)
 		{
-			tile[w][0][q * 32 + lane] = p[q].x;
-			tile[w][1][q * 32 + lane] = p[q].y;
-			tile[w][2][q * 32 + lane] = p[q].z;
+			to[q * kMeasureThreads + tid] = p[q].x;
+			to[kTile + q * kMeasureThreads + tid] = p[q].y;
+			to[2 * kTile + q * kMeasureThreads + tid] = p[q].z;
 		}
-		__syncwarp();
+		__syncthreads(); // and the tile before last is added
 		const unsigned int m = min(kTile, e - base);
 		gather(base + m); // the next tile's, in flight while this one is added
-		if (lane < 3)
+		if (tid < 3)
 		{
-			const float* t = tile[w][lane];
-#pragma unroll 8
-			for (unsigned int j = 0; j < m; ++j)
-				sum += t[j];
+			const float4* t = tile[turn][tid];
+#pragma unroll 4
+			for (unsigned int j = 0; j < m / 4; ++j)
+			{
+				const float4 x = t[j];
+				sum += x.x;
+				sum += x.y;
+				sum += x.z;
+				sum += x.w;
+			}
+			for (unsigned int j = m & ~3u; j < m; ++j)
+				sum += reinterpret_cast<const float*>(t)[j];
 		}
 	}
 	// the reference counts in float, which stops at 2^24
 	const float sw = float(min(e - b, 1u << 24));
 	const float iw = sw == 0.f ? 0.f : 1.f / sw;
-	sum *= iw;
-	const float sx = __shfl_sync(0xffffffffu, sum, 0), sy = __shfl_sync(0xffffffffu, sum, 1), sz = __shfl_sync(0xffffffffu, sum, 2);
+	if (tid < 3)
+		s_center[tid] = sum * iw;
+	__syncthreads();
+	const float sx = s_center[0], sy = s_center[1], sz = s_center[2];
 	float r2 = 0.f;
-	for (unsigned int base = b; base < e; base += kTile)
+	for (unsigned int base = b; base < e; base += min(kTile, e - base))
 	{
 		gather(base);
 #pragma unroll
 		for (unsigned int q = 0; q < kMeasureItems; ++q)
 		{
-			if (base + q * 32 + lane >= e)
+			if (q * kMeasureThreads + tid >= e - base)
 				continue;
 			float dx = p[q].x - sx, dy = p[q].y - sy, dz = p[q].z - sz;
 			float r = dx * dx + dy * dy + dz * dz;
@@ -3425,8 +3439,15 @@ __global__ void __launch_bounds__(kMeasureWarps * 32) kMeasureComponents(size_t 
 	// NaN distances are skipped above, so the maximum has no order
 	for (int o = 16; o > 0; o >>= 1)
 		r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, o));
-	if (lane == 0)
-		err[c] = r2;
+	if ((tid & 31) == 0)
+		s_far[tid / 32] = r2;
+	__syncthreads();
+	if (tid == 0)
+	{
+		for (unsigned int q = 1; q < kMeasureThreads / 32; ++q)
+			r2 = fmaxf(r2, s_far[q]);
+		err[blockIdx.x] = r2;
+	}
 }
 
 __global__ void kMinFloat(const float* __restrict__ v, size_t n, unsigned int* out)
@@ -4056,11 +4077,12 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		MO_LAUNCH(kComponentIds, gV, kThreads, 0, stream, V, w.remap, w.parent, w.fill, w.comp);
 		readScalars();
 		comp_count = hs->dup_count;
-		MO_CUDA_CHECK(cudaMemsetAsync(w.cnt, 0, (comp_count + 1) * 4, stream));
-		MO_LAUNCH(kCountKeys, gV, kThreads, 0, stream, w.comp, nullptr, V, w.cnt);
-		scanExclusive(w.cnt, w.comp_off, comp_count + 1, nullptr, w.scratch, stream, ss);
 		radixSortPairs(w.comp, nullptr, w.keys_a, w.vals_a, w.keys_b, w.vals_b, V, bitsFor(comp_count ? comp_count - 1 : 0), w.scratch, stream, ss);
-		MO_LAUNCH(kMeasureComponents, gridFor(comp_count, kMeasureWarps), kMeasureWarps * 32, 0, stream, comp_count, w.comp_off, w.vals_a, w.pos, w.comp_err);
+		MO_LAUNCH(kComponentStarts, gV, kThreads, 0, stream, w.keys_a, V, comp_count, w.comp_off);
+		if (V >= comp_count * kMeasureWide)
+			MO_LAUNCH(kMeasureComponents<256>, unsigned(comp_count), 256, 0, stream, w.comp_off, w.vals_a, w.pos, w.comp_err);
+		else
+			MO_LAUNCH(kMeasureComponents<32>, unsigned(comp_count), 32, 0, stream, w.comp_off, w.vals_a, w.pos, w.comp_err);
 	}
 	MO_CUDA_CHECK(cudaGetLastError());
 

@@ -306,3 +306,17 @@ def test_pass_loop_windows(port, single_path, monkeypatch, factor):
             out, err = pool.submit(mg.simplify, idx, pos, target, error, mg.SimplifyPrune).result()
         assert np.array_equal(out, ref)
         assert err == ref_err
+
+
+@pytest.mark.parametrize("sizes", [(1022, 1024, 1026), (2046, 2048, 2050, 4), (6000, 510), (4,) * 300, (2050,) + (4,) * 40], ids=lambda s: f"{len(s)}x{s[0]}")
+def test_prune_component_blocks(port, sizes):
+    """Component radii around the block's tile of 1,024 vertices (512 and more per component on average), and
+    many small components with one warp each, also with a large one among them."""
+    idx, pos = _strips(sizes, len(sizes))
+    opt = mg.SimplifyPrune | mg.SimplifyLockBorder
+    for target in (0, W.target_count(len(idx), 0.5)):
+        for error in (1e-2, 1e-1, 1.0):
+            ref, ref_err = port.simplify("port", idx, pos, target, error, opt)
+            out, err = mg.simplify(idx, pos, target, error, opt)
+            assert np.array_equal(out, ref)
+            assert err == ref_err
