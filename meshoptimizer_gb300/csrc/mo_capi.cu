@@ -1066,10 +1066,12 @@ struct ServerImpl
 
 const size_t kServerBudgetDefault = size_t(40) << 30;
 
-// device bytes a request holds while it runs on the batch path (its global slab) or on the single-mesh path (its arena)
-size_t batchReserve(const ServerRequest& r)
+// device bytes a request holds while it runs on the batch path (its global slab; a mesh that is expected to
+// run in shared memory is never too large for the budget) or on the single-mesh path (its arena)
+size_t batchReserve(const ServerRequest& r, size_t budget)
 {
-	return std::max<size_t>(4096, batchBytes(r.desc, batchNarrow(r.desc)).slab);
+	const BatchBytes b = batchBytes(r.desc, batchNarrow(r.desc));
+	return std::max<size_t>(4096, b.smem + b.rows <= kBatchSmemDefault ? std::min(b.slab, budget) : b.slab);
 }
 
 void publish(ServerImpl& S, std::vector<ServerRequest*>& done_reqs, size_t release)
@@ -1102,7 +1104,7 @@ void batchWorker(ServerImpl* S)
 			S->cv_work.wait(lk, [&] {
 				if (S->stop)
 					return true;
-				return !S->small_q.empty() && S->reserved + batchReserve(*S->small_q.front()) <= S->cfg.memory_budget;
+				return !S->small_q.empty() && S->reserved + batchReserve(*S->small_q.front(), S->cfg.memory_budget) <= S->cfg.memory_budget;
 			});
 			if (S->stop && S->small_q.empty())
 				return;
@@ -1112,7 +1114,7 @@ void batchWorker(ServerImpl* S)
 			while (!S->small_q.empty() && take.size() < size_t(S->cfg.max_batch))
 			{
 				ServerRequest* r = S->small_q.front();
-				size_t nm = std::max(maxslab, batchReserve(*r));
+				size_t nm = std::max(maxslab, batchReserve(*r, S->cfg.memory_budget));
 				size_t blocks = std::min<size_t>(take.size() + 1, size_t(S->sms) * 4);
 				size_t need = blocks * nm + 4096 * (take.size() + 1);
 				if (S->reserved + need > S->cfg.memory_budget && !take.empty())
@@ -1807,7 +1809,7 @@ long long meshoptgpu_serverSubmit(meshoptgpu_Server* server, const meshoptgpu_Ba
 	// memory or a global slab); larger ones, and the options the batch kernel does not have,
 	// take the multi-CTA single-mesh path
 	bool large = S->cfg.plain || mesh->index_count > S->cfg.large_index_count || (mesh->options & ~kBatchOptions);
-	r->reserve = large ? Simplifier::workspaceBytes(mesh->index_count, mesh->vertex_count, r->desc.ac) : batchReserve(*r);
+	r->reserve = large ? Simplifier::workspaceBytes(mesh->index_count, mesh->vertex_count, r->desc.ac) : batchReserve(*r, S->cfg.memory_budget);
 	if (r->reserve > S->cfg.memory_budget)
 	{
 		setStatus(meshoptgpu_StatusOutOfMemory, "request needs more device scratch than the server's memory budget");

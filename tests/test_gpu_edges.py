@@ -320,3 +320,21 @@ def test_prune_component_blocks(port, sizes):
             out, err = mg.simplify(idx, pos, target, error, opt)
             assert np.array_equal(out, ref)
             assert err == ref_err
+
+
+@pytest.mark.parametrize("budget", [16 << 10, 64 << 10, 1 << 20])
+def test_server_small_budget(port, budget):
+    """Meshes that run in shared memory are taken however small the memory budget, one after another."""
+    torch = pytest.importorskip("torch")
+    idx, pos = _grid(17, 17, 0.1, 3)
+    di, dp = torch.from_numpy(idx.view(np.int32)).cuda(), torch.from_numpy(pos).cuda()
+    outs = [torch.empty(len(idx), dtype=torch.int32, device="cuda") for _ in range(20)]
+    torch.cuda.synchronize()
+    ref, ref_err = port.simplify("port", idx, pos, 300, 1.0, 0)
+    with mg.Server(memory_budget=budget) as srv:
+        tickets = [srv.submit(di.data_ptr(), len(idx), dp.data_ptr(), len(pos), 300, 1.0, 0, o.data_ptr()) for o in outs]
+        for t, o in zip(tickets, outs):
+            status, n, err, _ = srv.wait(t)
+            assert status == 0
+            assert np.array_equal(o[:n].cpu().numpy().view(np.uint32), ref)
+            assert err == ref_err
