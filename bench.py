@@ -740,7 +740,7 @@ def bench_single(args, mg, torch, c, dist=None, world=1, rank=0, local=0, roofli
     total_ms = sum(a.elapsed_time(b) for a, b in ev)
 
     # per-launch CUDA-event timing of the roofline kernel: the same steps replayed with the
-    # host-driven pass loop (events cannot be recorded inside the device-resident loop's graph)
+    # host-driven pass loop (the device-resident loop is one launch)
     k_launches = k_ms = host_loop_ms = 0
     if roofline:
         mg.set_device_loop(False)
@@ -850,7 +850,7 @@ def bench_single(args, mg, torch, c, dist=None, world=1, rank=0, local=0, roofli
                 "algorithmic_bytes_per_launch": int(bytes_per_launch), "unit_definition": KPERFORM_BYTES_DEFINITION,
                 "share_of_step": round(k_ms / host_loop_ms, 4) if host_loop_ms else None,
                 "kernel_timing": "CUDA events around every launch on its stream, over the same steps replayed with the host-driven "
-                                 "pass loop (the timed steps run the device-resident loop, whose graph cannot hold events)"}
+                                 "pass loop (the timed steps run the device-resident loop, one launch for all passes)"}
         tr = kernel_traffic(args.kernel, c["name"])
         if tr:
             roof["traffic"] = tr["dram_bytes_per_launch"]
