@@ -15,6 +15,7 @@
 // triangles 1.43 ms, now 0.96; 2,048 groups of 1,024 triangles with attributes 3.67 ms, now 1.88.
 #pragma once
 
+#include <cmath>
 #include <type_traits>
 
 #include "mo_common.cuh"
@@ -221,13 +222,12 @@ __host__ __device__ inline size_t rowBytes(size_t V, size_t ac)
 // its perimeter's (1,024 triangles: 560; 589 are allowed for), and its capacity (boundEdgeCollapses) is
 // about two thirds of its indices. A mesh that needs more than the launch's shared memory runs in the
 // slab.
-__host__ __device__ inline size_t expectedVertices(size_t I, size_t bound, bool sparse)
+inline size_t expectedVertices(size_t I, size_t bound, bool sparse)
 {
-	size_t root = 1;
-	while (root * root < I)
-		++root;
-	const size_t v = I / 6 + root * 5 / 4 + 8;
-	return sparse && v < bound ? v : bound;
+	if (!sparse)
+		return bound;
+	const size_t v = I / 6 + size_t(std::sqrt(double(I))) * 5 / 4 + 10;
+	return v < bound ? v : bound;
 }
 
 __host__ __device__ inline size_t expectedCapacity(size_t I)

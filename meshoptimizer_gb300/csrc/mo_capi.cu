@@ -803,8 +803,8 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		}
 	}
 	launch(threads, budget);
-	std::vector<BatchResult> tmp(n);
-	MO_CUDA_CHECK(cudaMemcpyAsync(tmp.data(), d_res, n * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
+	const BatchResult* tmp = reinterpret_cast<const BatchResult*>(hmeta + off_res);
+	MO_CUDA_CHECK(cudaMemcpyAsync(hmeta + off_res, d_res, n * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
 	MO_CUDA_CHECK(cudaStreamSynchronize(st));
 	probe().collect();
 	for (size_t i = 0; i < n; ++i)
