@@ -604,9 +604,10 @@ def set_dropin_batch_limit(max_index_count=DROPIN_BATCH_LIMIT):
 
 
 def probe_barrier_wait(once=False, blocks=8, wait_limit=4096):
-    """meshoptgpu_probeBarrierWait: (status, timed_out) of a grid barrier that one block never reaches."""
+    """meshoptgpu_probeBarrierWait: (status, timed_out) of a grid barrier that one block never reaches
+    (once=2: the pass kernels' barrier)."""
     flag = C.c_uint(0)
-    st = int(load().meshoptgpu_probeBarrierWait(int(bool(once)), int(blocks), int(wait_limit), C.byref(flag)))
+    st = int(load().meshoptgpu_probeBarrierWait(2 if once == 2 else int(bool(once)), int(blocks), int(wait_limit), C.byref(flag)))
     return st, int(flag.value)
 
 

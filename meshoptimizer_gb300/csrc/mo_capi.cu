@@ -1906,7 +1906,7 @@ int meshoptgpu_probeBarrierWait(int once, unsigned int blocks, unsigned int wait
 		s.ensure();
 		if (blocks < 2 || blocks > coopScanCapacity() || wait_limit == 0 || wait_limit > (1u << 20) || !timed_out)
 			throw std::invalid_argument("probeBarrierWait: blocks must be 2..resident blocks, wait_limit 1..2^20, timed_out non-null");
-		*timed_out = probeBarrierWait(once, blocks, wait_limit, s.stream);
+		*timed_out = probeBarrierWait(once == 2 ? 2 : once != 0, blocks, wait_limit, s.stream);
 		setStatus(meshoptgpu_StatusOk, "");
 		return meshoptgpu_StatusOk;
 	}

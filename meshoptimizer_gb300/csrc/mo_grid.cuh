@@ -16,6 +16,8 @@ namespace mogpu
 constexpr unsigned int kBarrierSpinLimit = 1u << 25; // x >= 32 ns sleep (or an L2 round trip): seconds, never reached in a normal run
 constexpr unsigned int kBarrierSleepNs = MO_BARRIER_SLEEP_NS; // between polls
 
+constexpr unsigned int kBarrierErrorPolls = 1u << 10;         // polls between looks at the error flag
+
 // an arrival that publishes everything the block wrote before it (the block barrier ahead of it
 // orders the other threads' writes before this thread's release)
 __device__ __forceinline__ unsigned int arriveRelease(unsigned int* p)
@@ -87,9 +89,10 @@ struct GridSum
 			unsigned long long v;
 			asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;" : "=l"(v) : "l"(w), "l"(1ull | (unsigned long long)add << 32) : "memory");
 			const unsigned int target = ((unsigned int)v / gridDim.x + 1) * gridDim.x;
-			const unsigned int failed = __ldcg(err); // another block's, seen one barrier later at most
-			unsigned int spins = 0, out = 0;
-			for (;;)
+			// once a wait has run out anywhere, barriers are arrived at and not waited for: a block that
+			// never comes costs the others one limit, not one for every barrier until they return
+			unsigned int out = s[3] | __ldcg(err), spins = 0;
+			while (!out)
 			{
 				asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
 				if ((int)((unsigned int)v - target) >= 0)
@@ -98,20 +101,22 @@ struct GridSum
 				{
 					atomicOr(err, 1u);
 					out = 1;
-					break;
 				}
+				else if (spins % kBarrierErrorPolls == 0)
+					out = __ldcg(err);
 				if (kBarrierSleepNs)
 					__nanosleep(kBarrierSleepNs);
 			}
 			const unsigned int sum = (unsigned int)(v >> 32);
 			s[2] = sum - s[phase & 1];
 			s[phase & 1] = sum;
-			s[3] = failed | out;
+			s[3] = out;
 		}
 		++phase;
 		__syncthreads();
 		return s[2];
 	}
+	// a wait has run out: what the barriers should have ordered is not to be read any more
 	__device__ __forceinline__ bool failed() const { return s[3] != 0; }
 };
 

@@ -294,31 +294,47 @@ __global__ void __launch_bounds__(kSortThreads, 5) kRadixScatter(const unsigned 
 
 } // namespace
 
-// The bounded waits of both grid barriers, made to run out: block 0 never arrives, so every
+// The bounded waits of the grid barriers, made to run out: block 0 never arrives, so every
 // other block waits `limit` times, records the error and leaves. Nothing faults or hangs.
-__global__ void kBarrierWaitProbe(unsigned int* words, unsigned int limit, int once)
+// words: the barrier's (the first four), the error flag, and what went wrong in mode 2: a block that did
+// not see the failure, or that waited at a later barrier.
+__global__ void kBarrierWaitProbe(unsigned int* words, unsigned int limit, int mode)
 {
 	if (blockIdx.x == 0)
 		return;
-	if (once)
-		gridBarrierOnce(words, words + 2, limit);
+	if (mode == 2)
+	{
+		__shared__ unsigned int s_grid[4];
+		GridSum grid;
+		grid.start(reinterpret_cast<unsigned long long*>(words), words + 4, s_grid);
+		grid.wait(blockIdx.x, limit);
+		const bool seen = grid.failed();
+		const long long t = clock64();
+		grid.wait(blockIdx.x, 1u << 16);
+		grid.wait(0, 1u << 16);
+		// two waits would take 4 million cycles and more, two arrivals a few thousand
+		if (!seen || !grid.failed() || clock64() - t > (1ll << 20))
+			atomicOr(words + 5, 2u);
+	}
+	else if (mode)
+		gridBarrierOnce(words, words + 4, limit);
 	else
-		gridBarrier(words, words + 2, limit);
+		gridBarrier(words, words + 4, limit);
 }
 
-unsigned int probeBarrierWait(int once, unsigned int blocks, unsigned int limit, cudaStream_t stream)
+unsigned int probeBarrierWait(int mode, unsigned int blocks, unsigned int limit, cudaStream_t stream)
 {
 	unsigned int* words = nullptr;
-	MO_CUDA_CHECK(cudaMalloc(&words, 4 * sizeof(unsigned int)));
-	unsigned int err = 0;
+	MO_CUDA_CHECK(cudaMalloc(&words, 6 * sizeof(unsigned int)));
+	unsigned int err[2] = {0, 0};
 	try
 	{
-		MO_CUDA_CHECK(cudaMemsetAsync(words, 0, 4 * sizeof(unsigned int), stream));
-		void* params[] = {(void*)&words, (void*)&limit, (void*)&once};
+		MO_CUDA_CHECK(cudaMemsetAsync(words, 0, 6 * sizeof(unsigned int), stream));
+		void* params[] = {(void*)&words, (void*)&limit, (void*)&mode};
 		cudaEvent_t e0 = probeBegin("kBarrierWaitProbe", stream);
 		MO_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kBarrierWaitProbe, dim3(blocks), dim3(kScanThreads), params, 0, stream));
 		probeEnd(e0, stream);
-		MO_CUDA_CHECK(cudaMemcpyAsync(&err, words + 2, sizeof(err), cudaMemcpyDeviceToHost, stream));
+		MO_CUDA_CHECK(cudaMemcpyAsync(err, words + 4, sizeof(err), cudaMemcpyDeviceToHost, stream));
 		MO_CUDA_CHECK(cudaStreamSynchronize(stream));
 	}
 	catch (...)
@@ -327,7 +343,7 @@ unsigned int probeBarrierWait(int once, unsigned int blocks, unsigned int limit,
 		throw;
 	}
 	MO_CUDA_CHECK(cudaFree(words));
-	return err;
+	return err[0] | err[1];
 }
 
 constexpr int kMaxDevices = 64;

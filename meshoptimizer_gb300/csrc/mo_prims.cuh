@@ -90,10 +90,11 @@ struct ScanSync
 	                             // concurrent callers on other streams can be resident beside it
 };
 
-// Runs the grid barrier (once != 0: the single-use one) with one of `blocks` blocks never
-// arriving and a wait limit of `limit` polls; returns the error flag the waiting blocks set
-// (1 when the bounded wait ran out, as it must). For tests of the failure path.
-unsigned int probeBarrierWait(int once, unsigned int blocks, unsigned int limit, cudaStream_t stream);
+// Runs a grid barrier (mode 0: the position solve's, 1: the single-use one, 2: the pass kernels') with
+// one of `blocks` blocks never arriving and a wait limit of `limit` polls; returns the error flag the
+// waiting blocks set (1 when the bounded wait ran out, as it must; in mode 2 with 2 added if a block did
+// not see that, or waited at a later barrier all the same). For tests of the failure path.
+unsigned int probeBarrierWait(int mode, unsigned int blocks, unsigned int limit, cudaStream_t stream);
 
 // Blocks a single-launch scan may use on the current device (all resident at once); queried
 // once per device and cached.

@@ -2090,6 +2090,8 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 					markCandidate(a, k, ld<LOOP>(a.cring + c), round + 1);
 			}
 			grid.wait();
+			if (grid.failed())
+				return kPassFailed;
 		}
 		if (timer)
 			pc.lap(windows == 1 ? kPhInit : kPhMarks);
@@ -2108,7 +2110,7 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		while (n)
 		{
 			++round;
-			if (++guard > count + 1 || grid.failed())
+			if (++guard > count + 1)
 				break;
 			active_sum += n;
 			const unsigned int* cur = a.list[round & 1] + region;
@@ -2235,6 +2237,8 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 			__syncthreads(); // the counter's reset is seen when the block had no candidates
 			nb = s_app[0];
 			const unsigned int nn = grid.wait(nb);
+			if (grid.failed())
+				return kPassFailed;
 			if (timer)
 			{
 				long long before = pc.last();
@@ -2258,8 +2262,6 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 			first = false;
 			listed = list_next;
 		}
-		if (grid.failed())
-			return kPassFailed;
 
 		// ---- stop rules over [K0, K1): block chunks, thread sub-chunks, carried prefix
 		const unsigned int len = K1 - K0;
@@ -2279,6 +2281,8 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		if (threadIdx.x == 0)
 			a.blk[blockIdx.x] = make_uint4(tot.x, tot.y, tot.z, 0);
 		grid.wait();
+		if (grid.failed())
+			return kPassFailed;
 		// every block adds up the block totals itself: those before it (with the carry of earlier
 		// windows) and, for the next window's carry, all of them
 		unsigned int bT = 0, bF = 0, bM = carryM, wT = 0, wF = 0, wM = carryM;
@@ -2332,7 +2336,9 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		grid.wait();
 		if (timer)
 			pc.lap(kPhStop);
-		if (__ldcg(&sc->cut) != ~0ull || K1 == count || grid.failed())
+		if (grid.failed())
+			return kPassFailed;
+		if (__ldcg(&sc->cut) != ~0ull || K1 == count)
 			break;
 		carryT += ww.x;
 		carryF += ww.y;
@@ -2340,8 +2346,6 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		K0 = K1;
 		K1 = (unsigned int)min((unsigned long long)count, (unsigned long long)K1 + max(K1 / 8, min(K1, kWindowStep)));
 	}
-	if (grid.failed())
-		return kPassFailed;
 
 	// ---- apply the committed prefix. Commits are independent (no two share an endpoint), so
 	// any order gives the same result: each block applies its own commits (pick order, so their
@@ -2388,6 +2392,8 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		}
 	}
 	grid.wait();
+	if (grid.failed())
+		return kPassFailed;
 	flips = __ldcg(&sc->invalid); // a barrier is yet to come before the next pass clears it
 	if (timer)
 		pc.lap(kPhApply);
@@ -2398,8 +2404,6 @@ __device__ __forceinline__ int performPass(const PerformArgs& a, const PassLoopA
 		sc->active_sum = active_sum;
 		sc->windows = windows;
 	}
-	if (grid.failed())
-		return kPassFailed;
 	if (__ldcg(&sc->done) == 0)
 		return kPassEmpty;
 
@@ -2649,6 +2653,8 @@ __device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTr
 		sc->invalid = 0;
 	}
 	grid.wait();
+	if (grid.failed())
+		return false;
 
 	// ---- 2: the block's vertices' lists, at a place taken with one add; its candidates
 	const unsigned int vper = (p.vcount + G - 1) / G;
@@ -2746,6 +2752,8 @@ __device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTr
 			a.hist[(size_t)B * kKeyBins + b] = bins[b];
 	}
 	grid.wait();
+	if (grid.failed())
+		return false;
 
 	// ---- 4: every bin's counts as prefixes over the rows, and its total: 32 bins per block, a run of
 	// rows per warp
@@ -2781,6 +2789,8 @@ __device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTr
 		}
 	}
 	grid.wait();
+	if (grid.failed())
+		return false;
 
 	// ---- 5: the first window; sorted positions, as kKeyScatter gives them; the first window's
 	// candidates mark their endpoints for the first decision round

@@ -41,3 +41,21 @@ def test_barrier_probe_rejects_bad_arguments():
         args.update(kw)
         st, _ = mg.probe_barrier_wait(**args)
         assert st == mg.STATUS_INVALID_ARGUMENT, kw
+
+
+def test_pass_barrier_wait_runs_out_and_reports(port):
+    """The pass kernels' barrier, which carries a sum: the blocks see the failure as they leave, and those
+    that reach later barriers do not wait there again."""
+    for blocks in (2, 16, 152):
+        st, timed_out = mg.probe_barrier_wait(once=2, blocks=blocks, wait_limit=4096)
+        assert st == mg.STATUS_OK
+        assert timed_out == 1
+    idx, pos = W.heightfield(48, seed=7)
+    target = W.target_count(len(idx), 0.25)
+    mg.set_dropin_batch_limit(0)
+    try:
+        out, err = mg.simplify(idx, pos, target, 1e-2)
+    finally:
+        mg.set_dropin_batch_limit()
+    ref, ref_err = port.simplify("port", idx, pos, target, 1e-2, 0)
+    assert np.array_equal(out, ref)
