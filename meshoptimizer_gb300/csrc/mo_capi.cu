@@ -1564,6 +1564,8 @@ int meshoptgpu_buildMeshletsFlexGroups(unsigned int* meshlets, unsigned int* mes
 			bad = "group " + std::to_string(g) + ": fewer meshlet rows than meshopt_buildMeshletsBound(index_count, max_vertices, min_triangles)";
 		else if (n >= (size_t(1) << 31))
 			bad = "group " + std::to_string(g) + ": index count must be below 2^31";
+		else if (n && (!vertex_count || !vertex_positions)) // the kernel reads vertex 0 in the place of a bad index
+			bad = "an index is out of range of vertex_count";
 	}
 	if (!bad.empty())
 	{
