@@ -48,6 +48,11 @@ constexpr unsigned int kStageItems = MO_STAGE_ITEMS; // candidates per thread in
 // A pass that its first window does not end goes on by windows of an eighth of what it has decided, or
 // kWindowStep, or as much again: each costs a set of decision rounds whatever its size, 150 us or so.
 constexpr unsigned int kWindowStep = 1u << 18;
+// The first pass's first window at most, of the goal's triangles and beyond. Planes of 256^2 / 512^2
+// vertices to 90%, whole calls in ms: no bound 3.66 / 13.5; 1 2.28 / 4.56, 1.5 2.56 / 5.68, 2 2.80 / 3.30,
+// 3 3.25 / 4.26. Curved and noisy meshes need 0.5 to 1.
+constexpr double kFirstWindowGoals = 2.0;
+constexpr unsigned int kFirstWindowSlack = 4096;
 
 // What a pass did per candidate that its stop rules let it look at: the next one's are about the same.
 struct PassRates
@@ -2848,8 +2853,9 @@ __device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTr
 		}
 		__syncthreads();
 		double window = double(s_errors) + 256;
-		if (rates.tris > 0)
-			window = fmin(window, double(in.goal) / rates.tris + 256);
+		// the error goal says nothing where most errors are alike (a plane's are all zero), so the first
+		// pass, which has no rate yet, is bounded by its goal
+		window = fmin(window, rates.tris > 0 ? double(in.goal) / rates.tris + 256 : kFirstWindowGoals * double(in.goal) + kFirstWindowSlack);
 		window = fmin(window, double(s_limit) + 1);
 		if (a.window_factor > 0)
 			window = a.window_factor * double(in.goal / 2) + 4096;

@@ -338,3 +338,18 @@ def test_server_small_budget(port, budget):
             assert status == 0
             assert np.array_equal(o[:n].cpu().numpy().view(np.uint32), ref)
             assert err == ref_err
+
+
+@pytest.mark.parametrize("ratio", [0.99, 0.9, 0.5])
+def test_first_window_of_a_plane(port, single_path, ratio):
+    """All errors are zero: the first pass decides about as many candidates as it has triangles to remove,
+    not all of them."""
+    idx, pos = _grid(257, 257, 0.0, 1)
+    target = W.target_count(len(idx), ratio)
+    ref, ref_err = port.simplify("port", idx, pos, target, 1e-2, 0)
+    for _ in range(2):  # the first call of a size class may time launch shapes
+        out, err = mg.simplify(idx, pos, target, 1e-2, 0)
+    assert np.array_equal(out, ref)
+    assert err == ref_err
+    goal = (len(idx) - target) // 3
+    assert mg.last_round_trace()[0][0] <= min(2 * goal + 4096, mg.last_pass_stats()[0]["candidates"])
