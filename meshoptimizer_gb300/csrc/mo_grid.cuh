@@ -90,27 +90,30 @@ struct GridSum
 			asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;" : "=l"(v) : "l"(w), "l"(1ull | (unsigned long long)add << 32) : "memory");
 			const unsigned int target = ((unsigned int)v / gridDim.x + 1) * gridDim.x;
 			// once a wait has run out anywhere, barriers are arrived at and not waited for: a block that
-			// never comes costs the others one limit, not one for every barrier until they return
-			unsigned int out = s[3] | __ldcg(err), spins = 0;
-			while (!out)
+			// never comes costs the others one limit, not one for every barrier until they return. The
+			// flag's load is in flight during the first poll.
+			const unsigned int failed = s[3] | __ldcg(err);
+			unsigned int spins = 0, out = 0;
+			for (;;)
 			{
 				asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
-				if ((int)((unsigned int)v - target) >= 0)
+				if ((int)((unsigned int)v - target) >= 0 || out)
 					break;
+				out = failed;
 				if (++spins > limit)
 				{
 					atomicOr(err, 1u);
 					out = 1;
 				}
 				else if (spins % kBarrierErrorPolls == 0)
-					out = __ldcg(err);
+					out |= __ldcg(err);
 				if (kBarrierSleepNs)
 					__nanosleep(kBarrierSleepNs);
 			}
 			const unsigned int sum = (unsigned int)(v >> 32);
 			s[2] = sum - s[phase & 1];
 			s[phase & 1] = sum;
-			s[3] = out;
+			s[3] = failed | out;
 		}
 		++phase;
 		__syncthreads();
