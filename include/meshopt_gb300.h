@@ -227,7 +227,9 @@ MESHOPTGPU_API int meshoptgpu_buildMeshletsFlexGroups(unsigned int* meshlets, un
 /* Batch launch shape: threads per CTA (128, 256 or 512; 0 = autotune, the default) and the
  * shared-memory budget per CTA in bytes (0 = autotune, the default). The autotuner times every
  * open pair of thread count and budget (54, 110 and 216 KiB) on the first batch of a size class
- * and keeps the fastest for that class. */
+ * and keeps the fastest for that class. Meshes of more than 60,000 indices or 24,000 vertices (of
+ * their own, where they are sparse subsets) are larger than any budget; they run in global memory,
+ * always with 512 threads, in a launch beside the others'. */
 MESHOPTGPU_API void meshoptgpu_setBatchConfig(int threads, unsigned int smem_bytes);
 
 /* Drop-in calls (meshopt_simplify, meshopt_simplifyWithAttributes, meshoptgpu_simplifyDevice)
@@ -245,6 +247,9 @@ MESHOPTGPU_API void meshoptgpu_setBatchConfig(int threads, unsigned int smem_byt
  * mode, Prune or debug bit) times the candidates on its own mesh. MESHOPTGPU_AUTOTUNE=0 in the
  * environment turns both tuners off (fixed defaults). */
 MESHOPTGPU_API void meshoptgpu_setDropinBatchLimit(size_t max_index_count);
+
+/* Where the meshes of the calling thread's last batched call ran (either pointer may be NULL). */
+MESHOPTGPU_API void meshoptgpu_getLastBatchPlacement(size_t* in_shared_memory, size_t* in_global_memory);
 
 /* The autotuner's choices for meshes of index_count indices (with attributes or not), on the
  * current device: out4[0] pass-kernel blocks per SM, out4[1] 0 (the pass sort's tile follows the

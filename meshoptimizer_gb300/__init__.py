@@ -53,6 +53,7 @@ EXPORTS = [
     "meshoptgpu_optimizeVertexFetchRemapDevice", "meshoptgpu_optimizeVertexFetchDevice", "meshoptgpu_generatePositionRemapDevice",
     "meshoptgpu_simplifyGroups", "meshoptgpu_buildMeshletsFlexGroups", "meshoptgpu_setDropinBatchLimit", "meshoptgpu_setDeviceLoop",
     "meshoptgpu_probeBarrierWait",
+    "meshoptgpu_getLastBatchPlacement",
 ]
 
 
@@ -595,6 +596,13 @@ def set_batch_config(threads=0, smem_bytes=0):
 
 
 DROPIN_BATCH_LIMIT = 2 ** 64 - 1  # the library's default: the route is autotuned per size class
+
+
+def last_batch_placement():
+    """(meshes in shared memory, meshes in global memory) of the calling thread's last batched call."""
+    a, b = C.c_size_t(0), C.c_size_t(0)
+    load().meshoptgpu_getLastBatchPlacement(C.byref(a), C.byref(b))
+    return int(a.value), int(b.value)
 
 
 def set_dropin_batch_limit(max_index_count=DROPIN_BATCH_LIMIT):

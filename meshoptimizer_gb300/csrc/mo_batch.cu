@@ -9,11 +9,6 @@
 namespace mogpu
 {
 
-bool batchNarrow(const BatchDesc& d)
-{
-	return narrowMesh(d.index_count, localVertexBound(d.index_count, d.vertex_count, (d.options & kOptSparse) != 0));
-}
-
 template <class IX>
 BatchBytes bytesOf(const BatchDesc& d)
 {

@@ -39,8 +39,9 @@ struct BatchResult
 	unsigned int index_count;
 	float result_error;
 	unsigned int passes;
-	unsigned int status; // 0 ok, 2 invalid index, 3 a decision round made no progress
+	unsigned int status; // 0 ok, 2 invalid index, 3 a decision round made no progress; + kBatchInSlab
 };
+constexpr unsigned int kBatchInSlab = 0x100; // the mesh ran in its CTA's slab
 
 // Memory of one mesh. smem: shared memory it is expected to need beside its attribute rows (rows), which
 // go there too where they fit, else into the CTA's slab; slab: global scratch in which it runs whatever
@@ -51,8 +52,15 @@ struct BatchBytes
 };
 BatchBytes batchBytes(const BatchDesc& d, bool narrow);
 
-// whether a mesh's ids fit the kernels' 16-bit form
-bool batchNarrow(const BatchDesc& d);
+// whether a mesh's ids fit the kernels' 16-bit form: its indices, and its (local) vertices, of which a
+// sparse mesh (option bit 1) has one per index at most
+constexpr size_t kNarrowIndices = 60000;
+constexpr size_t kNarrowVertices = 24000; // their table has at most 32,768 slots
+inline bool batchNarrow(const BatchDesc& d)
+{
+	const bool few = d.vertex_count <= kNarrowVertices || ((d.options & (1u << 1)) && d.index_count <= kNarrowVertices);
+	return d.index_count <= kNarrowIndices && few;
+}
 
 // whether a mesh needs the full-option kernel: a sparse subset (option bit 1), attributes,
 // vertex_lock or Permissive (option bit 5)

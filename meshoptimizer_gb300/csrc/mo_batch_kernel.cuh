@@ -55,8 +55,6 @@ constexpr unsigned int kSortKeys = 2560;  // values of sortKey
 // 510 triangles 1.17 / 1.12 / 1.07 / 1.00 / 1.02 / 1.01 ms; 2,048 groups of 1,024 triangles 1.92 / 1.89 /
 // 1.90 / 1.90 / 1.99 / 2.05 ms.
 constexpr unsigned int kWalk = 224;
-constexpr size_t kNarrowIndices = 60000;  // indices of a mesh with 16-bit ids at most
-constexpr size_t kNarrowVertices = 24000; // and its (local) vertices: their table has at most 32,768 slots
 
 template <class IX>
 struct CtaWork
@@ -107,11 +105,6 @@ __host__ __device__ inline size_t hashBucketsFor(size_t count)
 __host__ __device__ inline size_t localVertexBound(size_t I, size_t vertex_count, bool sparse)
 {
 	return sparse ? (I < vertex_count ? I : vertex_count) : vertex_count;
-}
-
-__host__ __device__ inline bool narrowMesh(size_t I, size_t V)
-{
-	return I <= kNarrowIndices && V <= kNarrowVertices;
 }
 
 // Memory handed out front to back; what lies past the limit is not to be used (ok() is false then), and
@@ -404,6 +397,7 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 	unsigned int* const red = s_red;
 	typedef typename Pair2<IX>::T IX2;
 	constexpr IX kNone = IX(~0u); // no loop, no slot
+	constexpr unsigned int kWhere = FAST ? 0u : kBatchInSlab;
 	const unsigned int tid = threadIdx.x;
 	const unsigned int I = d.index_count;
 	const float* P = d.positions;
@@ -435,7 +429,7 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 	if (s_flag)
 	{
 		if (tid == 0)
-			*out = BatchResult{I, 0.f, 0, 2};
+			*out = BatchResult{I, 0.f, 0, 2u | kWhere};
 		for (unsigned int i = tid; i < I; i += NT)
 			d.out[i] = d.indices[i];
 		return true;
@@ -1644,7 +1638,7 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 	for (unsigned int i = tid; i < result_count; i += NT)
 		d.out[i] = src(w.idx[i]);
 	if (tid == 0)
-		*out = BatchResult{result_count, sqrtf(result_error) * error_scale, passes, s_stall ? 3u : 0u};
+		*out = BatchResult{result_count, sqrtf(result_error) * error_scale, passes, (s_stall ? 3u : 0u) | kWhere};
 	return true;
 }
 
@@ -1670,8 +1664,8 @@ __global__ void __launch_bounds__(NT, (kBatchWarps<NT, FULL>) * 32 / NT) kBatch(
 		if (job >= count)
 			break;
 		const BatchDesc d = descs[job];
-		// in shared memory, its attribute rows there or in the slab; where that is too small (meshes with
-		// 32-bit ids always are too large), in the slab
+		// in shared memory, its attribute rows there or in the slab; where that is too small, in the slab (a
+		// mesh that needs 32-bit ids is larger than any shared memory)
 		const size_t bound = localVertexBound(d.index_count, d.vertex_count, FULL && (d.options & kOptSparse) != 0);
 		const size_t rows = FULL && d.ac ? rowBytes<IX>(bound, d.ac) : 0;
 		bool done = false;

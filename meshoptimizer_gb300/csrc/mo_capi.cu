@@ -109,6 +109,18 @@ struct ThreadState
 	// only slow the first inputs down). Events: positions, attributes, indices copied.
 	cudaStream_t copy_stream = nullptr;
 	cudaEvent_t copy_done[3] = {nullptr, nullptr, nullptr};
+	// the second launch of a batch whose meshes need both forms of the kernel
+	cudaStream_t batch_stream = nullptr;
+	cudaEvent_t batch_event = nullptr;
+	size_t batch_in_shared = 0, batch_in_slab = 0; // meshes of the last batch by where they ran
+
+	void ensureBatchStream()
+	{
+		if (!batch_stream)
+			MO_CUDA_CHECK(cudaStreamCreateWithFlags(&batch_stream, cudaStreamNonBlocking));
+		if (!batch_event)
+			MO_CUDA_CHECK(cudaEventCreateWithFlags(&batch_event, cudaEventDisableTiming));
+	}
 
 	void ensureCopyStreams()
 	{
@@ -119,7 +131,7 @@ struct ThreadState
 				MO_CUDA_CHECK(cudaEventCreateWithFlags(&copy_done[i], cudaEventDisableTiming));
 	}
 
-	void releaseCopyStreams()
+	void releaseStreams()
 	{
 		for (int i = 0; i < 3; ++i)
 		{
@@ -130,12 +142,18 @@ struct ThreadState
 		if (copy_stream)
 			cudaStreamDestroy(copy_stream);
 		copy_stream = nullptr;
+		if (batch_event)
+			cudaEventDestroy(batch_event);
+		batch_event = nullptr;
+		if (batch_stream)
+			cudaStreamDestroy(batch_stream);
+		batch_stream = nullptr;
 	}
 
 	~ThreadState()
 	{
 		simplifier.reset();
-		releaseCopyStreams();
+		releaseStreams();
 		if (stream)
 			cudaStreamDestroy(stream);
 	}
@@ -147,7 +165,7 @@ struct ThreadState
 		if (simplifier && device == dev)
 			return;
 		simplifier.reset();
-		releaseCopyStreams();
+		releaseStreams();
 		if (stream)
 			cudaStreamDestroy(stream);
 		stream = nullptr;
@@ -679,61 +697,70 @@ BatchDesc makeDesc(const meshoptgpu_BatchMesh& m, const unsigned int* indices, c
 
 // Runs descs (device pointers) through the persistent kernel; results in the same order.
 // attr_of[i] indexes maps.maps for descs[i] (-1: none).
+// Meshes whose ids need 32 bits run in a launch of their own, beside the others': that form has no
+// shared-memory path, and one such mesh in a batch would take it from all others (4,096 meshes of 384
+// triangles and one of 24,100 vertices that uses 221 of them: 3.43 ms in one launch).
 void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& maps, const std::vector<int>& attr_of, std::vector<BatchResult>& results,
     cudaStream_t st)
 {
 	const size_t n = descs.size();
 	results.assign(n, BatchResult{0, 0.f, 0, 0});
+	s.batch_in_shared = s.batch_in_slab = 0;
 	if (n == 0)
 		return;
-	// largest meshes first so the queue's tail is short; results are mapped back below
+	// the wide meshes, then the others, each with the largest first so the queue's tail is short; results
+	// are mapped back below
 	std::vector<unsigned int> perm(n);
+	size_t wide = 0;
 	{
 		// by eighths of a power of two: one counting pass, where a sort of 4,096 took 0.1 ms of the call
-		auto size = [&](size_t i) {
-			unsigned int e = 0;
-			for (size_t v = size_t(descs[i].index_count) + 8; v >= 16; v >>= 1)
-				++e;
-			return 511 - std::min<size_t>(511, size_t(e) * 8 + ((size_t(descs[i].index_count) + 8) >> e) - 8);
-		};
-		size_t start[513] = {};
+		constexpr size_t kSizes = 512;
+		std::vector<unsigned short> place(n);
+		size_t start[2 * kSizes + 1] = {};
 		for (size_t i = 0; i < n; ++i)
-			++start[size(i) + 1];
-		for (size_t k = 0; k < 512; ++k)
+		{
+			const size_t v = size_t(descs[i].index_count) + 8;
+			const unsigned int e = 60 - __builtin_clzll(v); // v >> e is 8 to 15
+			const size_t size = size_t(e) * 8 + (v >> e) - 8;
+			place[i] = (unsigned short)(kSizes - 1 - std::min(kSizes - 1, size) + (batchNarrow(descs[i]) ? kSizes : 0));
+			++start[place[i] + 1];
+		}
+		for (size_t k = 0; k < 2 * kSizes; ++k)
 			start[k + 1] += start[k];
+		wide = start[kSizes];
 		for (size_t i = 0; i < n; ++i)
-			perm[start[size(i)]++] = (unsigned int)i;
+			perm[start[place[i]]++] = (unsigned int)i;
 	}
 	std::vector<BatchDesc> ordered(n);
-	size_t maxidx = 0;
-	for (size_t i = 0; i < n; ++i)
-	{
-		ordered[i] = descs[perm[i]];
-		maxidx = std::max<size_t>(maxidx, ordered[i].index_count);
-	}
-	bool full = false, narrow = true;
-	for (const BatchDesc& d : ordered)
-	{
-		full = full || batchNeedsFull(d);
-		narrow = narrow && batchNarrow(d);
-	}
 	std::vector<BatchBytes> bytes(n);
-	size_t maxslab = 0;
-	for (size_t i = 0; i < n; ++i)
+	struct Part // the meshes of one form of the kernel
 	{
-		bytes[i] = batchBytes(ordered[i], narrow);
-		maxslab = std::max(maxslab, bytes[i].slab);
-	}
+		size_t first, count;
+		bool narrow, full;
+		size_t slab, max_index_count;
+		int threads;
+		size_t budget;
+	} parts[2] = {{0, wide, false, false, 0, 0, 0, 0}, {wide, n - wide, true, false, 0, 0, 0, 0}};
+	for (Part& p : parts)
+		for (size_t i = p.first; i < p.first + p.count; ++i)
+		{
+			ordered[i] = descs[perm[i]];
+			bytes[i] = batchBytes(ordered[i], p.narrow);
+			p.full = p.full || batchNeedsFull(ordered[i]);
+			p.slab = std::max(p.slab, bytes[i].slab);
+			p.max_index_count = std::max<size_t>(p.max_index_count, ordered[i].index_count);
+		}
 	// a budget's dynamic shared memory: the largest mesh that fits it, with its attribute rows or without
-	auto footprint = [&](size_t budget) {
+	auto footprint = [&](const Part& p, size_t budget) {
 		size_t most = 0;
-		for (const BatchBytes& b : bytes)
-			most = std::max(most, b.smem + b.rows <= budget ? b.smem + b.rows : (b.smem <= budget ? b.smem : size_t(0)));
+		if (p.narrow)
+			for (size_t i = p.first; i < p.first + p.count; ++i)
+				most = std::max(most, bytes[i].smem + bytes[i].rows <= budget ? bytes[i].smem + bytes[i].rows : (bytes[i].smem <= budget ? bytes[i].smem : size_t(0)));
 		return unsigned((most + 15) & ~size_t(15));
 	};
 	const int sms = s.sms;
 
-	// device metadata: descriptors, results, the ticket, the attribute maps; descriptors and
+	// device metadata: descriptors, results, the tickets, the attribute maps; descriptors and
 	// maps go up in one copy from pinned staging
 	const size_t nm = maps.maps.size();
 	const size_t off_res = align256(n * sizeof(BatchDesc)), off_ticket = off_res + align256(n * sizeof(BatchResult));
@@ -754,75 +781,117 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	if (nm)
 		MO_CUDA_CHECK(cudaMemcpyAsync(d_maps, hmeta + off_maps, nm * sizeof(BatchAttr), cudaMemcpyHostToDevice, st));
 
-	auto launch = [&](int threads, size_t budget) {
-		const unsigned int smem = footprint(budget);
-		int per_sm = std::max(1, batchBlocksPerSM(threads, smem, full, narrow));
-		unsigned int blocks = unsigned(std::min<size_t>(size_t(per_sm) * sms, n));
-		blocks = unsigned(std::max<size_t>(1, std::min<size_t>(blocks, kBatchSlabTotal / std::max<size_t>(maxslab, 1))));
-		char* slabs = static_cast<char*>(s.batch_slabs.ensure(size_t(blocks) * maxslab));
-		launchBatch(d_descs, unsigned(n), d_ticket, d_res, slabs, maxslab, smem, blocks, threads, full, narrow, st);
+	auto slabBlocks = [&](const Part& p, int threads, unsigned int smem) {
+		const int per_sm = std::max(1, batchBlocksPerSM(threads, smem, p.full, p.narrow));
+		const size_t blocks = std::min<size_t>(size_t(per_sm) * sms, p.count);
+		return unsigned(std::max<size_t>(1, std::min<size_t>(blocks, kBatchSlabTotal / std::max<size_t>(p.slab, 1))));
+	};
+	auto launch = [&](const Part& p, int threads, unsigned int smem, unsigned int blocks, char* slabs, cudaStream_t on) {
+		launchBatch(d_descs + p.first, unsigned(p.count), d_ticket + (p.narrow ? 1 : 0), d_res + p.first, slabs, p.slab, smem, blocks, threads, p.full, p.narrow, on);
 	};
 
-	int threads = s.batch_threads;
-	size_t budget = s.batch_smem ? s.batch_smem : kBatchSmemDefault;
-	if (threads == 0 || s.batch_smem == 0)
+	for (Part& p : parts)
 	{
+		if (!p.count)
+			continue;
+		p.threads = s.batch_threads;
+		p.budget = s.batch_smem ? s.batch_smem : kBatchSmemDefault;
+		if (!p.narrow || (p.threads && s.batch_smem))
+			continue; // the 32-bit form has one shape
 		// the block size and the shared-memory budget the caller left open are autotuned per size
 		// class: the first batch of a class times every candidate pair on its own meshes
 		// (identical results) and keeps the fastest
-		const std::pair<int, bool> cls(sizeClass(maxidx), n > size_t(sms));
-		bool known = false;
+		const std::pair<int, bool> cls(sizeClass(p.max_index_count), p.count > size_t(sms));
 		{
 			std::lock_guard<std::mutex> g(g_tuner.lock);
 			auto it = g_tuner.shape.find(cls);
 			if (it != g_tuner.shape.end())
 			{
-				threads = threads ? threads : it->second.first;
-				budget = s.batch_smem ? budget : it->second.second;
-				known = true;
+				p.threads = p.threads ? p.threads : it->second.first;
+				p.budget = s.batch_smem ? p.budget : it->second.second;
+				continue;
 			}
 		}
-		if (!known)
+		cudaEvent_t e0, e1;
+		MO_CUDA_CHECK(cudaEventCreate(&e0));
+		MO_CUDA_CHECK(cudaEventCreate(&e1));
+		float best = 1e30f;
+		int best_t = p.threads ? p.threads : 256;
+		size_t best_b = p.budget;
+		for (int t : {128, 256, 512})
 		{
-			cudaEvent_t e0, e1;
-			MO_CUDA_CHECK(cudaEventCreate(&e0));
-			MO_CUDA_CHECK(cudaEventCreate(&e1));
-			float best = 1e30f;
-			int best_t = threads ? threads : 256;
-			size_t best_b = budget;
-			for (int t : {128, 256, 512})
+			if (p.threads && t != p.threads)
+				continue;
+			for (size_t b : kBatchSmemBudgets)
 			{
-				if (threads && t != threads)
+				if (s.batch_smem && b != s.batch_smem)
 					continue;
-				for (size_t b : kBatchSmemBudgets)
-				{
-					if (s.batch_smem && b != s.batch_smem)
-						continue;
-					MO_CUDA_CHECK(cudaEventRecord(e0, st));
-					launch(t, b);
-					MO_CUDA_CHECK(cudaEventRecord(e1, st));
-					MO_CUDA_CHECK(cudaEventSynchronize(e1));
-					float ms = 0;
-					MO_CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
-					if (ms < best)
-						best = ms, best_t = t, best_b = b;
-				}
+				const unsigned int smem = footprint(p, b), blocks = slabBlocks(p, t, smem);
+				char* slabs = static_cast<char*>(s.batch_slabs.ensure(size_t(blocks) * p.slab));
+				MO_CUDA_CHECK(cudaEventRecord(e0, st));
+				launch(p, t, smem, blocks, slabs, st);
+				MO_CUDA_CHECK(cudaEventRecord(e1, st));
+				MO_CUDA_CHECK(cudaEventSynchronize(e1));
+				float ms = 0;
+				MO_CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
+				if (ms < best)
+					best = ms, best_t = t, best_b = b;
 			}
-			cudaEventDestroy(e0);
-			cudaEventDestroy(e1);
-			threads = best_t;
-			budget = best_b;
-			std::lock_guard<std::mutex> g(g_tuner.lock);
-			g_tuner.shape[cls] = std::make_pair(threads, budget);
+		}
+		cudaEventDestroy(e0);
+		cudaEventDestroy(e1);
+		p.threads = best_t;
+		p.budget = best_b;
+		std::lock_guard<std::mutex> g(g_tuner.lock);
+		g_tuner.shape[cls] = std::make_pair(best_t, best_b);
+	}
+
+	// both parts at once, the wide one from a stream of its own
+	unsigned int smem[2] = {0, 0}, blocks[2] = {0, 0};
+	size_t slab_bytes[2] = {0, 0};
+	for (int q = 0; q < 2; ++q)
+		if (parts[q].count)
+		{
+			smem[q] = footprint(parts[q], parts[q].budget);
+			blocks[q] = slabBlocks(parts[q], parts[q].threads, smem[q]);
+			slab_bytes[q] = align256(size_t(blocks[q]) * parts[q].slab);
+		}
+	char* slabs = static_cast<char*>(s.batch_slabs.ensure(slab_bytes[0] + slab_bytes[1]));
+	const bool both = parts[0].count && parts[1].count;
+	if (both)
+	{
+		s.ensureBatchStream();
+		MO_CUDA_CHECK(cudaEventRecord(s.batch_event, st));
+		MO_CUDA_CHECK(cudaStreamWaitEvent(s.batch_stream, s.batch_event, 0));
+	}
+	try
+	{
+		if (parts[0].count)
+			launch(parts[0], parts[0].threads, smem[0], blocks[0], slabs, both ? s.batch_stream : st);
+		if (parts[1].count)
+			launch(parts[1], parts[1].threads, smem[1], blocks[1], slabs + slab_bytes[0], st);
+		if (both)
+		{
+			MO_CUDA_CHECK(cudaEventRecord(s.batch_event, s.batch_stream));
+			MO_CUDA_CHECK(cudaStreamWaitEvent(st, s.batch_event, 0));
 		}
 	}
-	launch(threads, budget);
+	catch (...)
+	{
+		if (both)
+			cudaStreamSynchronize(s.batch_stream); // the caller's buffers are its own again when the call returns
+		throw;
+	}
 	const BatchResult* tmp = reinterpret_cast<const BatchResult*>(hmeta + off_res);
 	MO_CUDA_CHECK(cudaMemcpyAsync(hmeta + off_res, d_res, n * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
 	MO_CUDA_CHECK(cudaStreamSynchronize(st));
 	probe().collect();
 	for (size_t i = 0; i < n; ++i)
-		results[perm[i]] = tmp[i];
+	{
+		BatchResult& r = results[perm[i]] = tmp[i];
+		++(r.status & kBatchInSlab ? s.batch_in_slab : s.batch_in_shared);
+		r.status &= ~kBatchInSlab;
+	}
 }
 
 // argument checks of a batched mesh: those of meshopt_simplifyEdge (:2348-2357), then the
@@ -1880,6 +1949,15 @@ void meshoptgpu_setBatchConfig(int threads, unsigned int smem_bytes)
 void meshoptgpu_setDropinBatchLimit(size_t max_index_count)
 {
 	state().dropin_batch_limit = max_index_count;
+}
+
+void meshoptgpu_getLastBatchPlacement(size_t* in_shared_memory, size_t* in_global_memory)
+{
+	const ThreadState& s = state();
+	if (in_shared_memory)
+		*in_shared_memory = s.batch_in_shared;
+	if (in_global_memory)
+		*in_global_memory = s.batch_in_slab;
 }
 
 int meshoptgpu_setDeviceLoop(int enabled)

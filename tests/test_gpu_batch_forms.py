@@ -1,0 +1,70 @@
+"""The batch kernel's forms and where meshes run: batches that need several, bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+import meshoptimizer_gb300 as mg
+from meshoptimizer_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    from meshoptimizer_gb300 import build
+
+    build.build()
+    mg.load()
+
+
+def _grid(nx, ny, amp, seed):
+    a = (np.arange(ny - 1)[:, None] * nx + np.arange(nx - 1)[None, :]).reshape(-1)
+    idx = np.stack([a, a + 1, a + nx, a + nx, a + 1, a + nx + 1], 1).reshape(-1).astype(np.uint32)
+    y, x = np.meshgrid(np.arange(ny), np.arange(nx), indexing="ij")
+    z = amp * np.random.default_rng(seed).standard_normal((ny, nx))
+    return idx, np.stack([x, y, z], -1).reshape(-1, 3).astype(np.float32)
+
+
+def _same(port, ms, res):
+    seen = {}
+    for i, (m, (out, err)) in enumerate(zip(ms, res)):
+        key = (id(m["indices"]), id(m["positions"]), id(m.get("attributes")), m["target"], m["error"], m.get("options", 0))
+        if key not in seen:
+            seen[key] = port.simplify("port", m["indices"], m["positions"], m["target"], m["error"], m.get("options", 0),
+                                      attributes=m.get("attributes"), weights=m.get("weights"), lock=m.get("lock"))
+        ref, ref_err = seen[key]
+        assert np.array_equal(out, ref), f"mesh {i}"
+        assert err == ref_err, f"mesh {i}"
+
+
+def _small(count, attributes=0, nx=13, ny=11):
+    rng = np.random.default_rng(count + attributes)
+    distinct = []
+    for k in range(8):
+        idx, pos = _grid(nx, ny, 0.1, k)
+        m = dict(indices=idx, positions=pos, target=len(idx) // 6 * 3, error=1.0)
+        if attributes:
+            m.update(attributes=rng.standard_normal((len(pos), attributes)).astype(np.float32),
+                     weights=rng.uniform(0.1, 1.0, attributes).astype(np.float32))
+        distinct.append(m)
+    return [distinct[i % 8] for i in range(count)]
+
+
+@pytest.mark.parametrize("count,attributes", [(1, 0), (8, 3), (2000, 0), (700, 2)])
+def test_batch_with_wide_meshes(port, count, attributes):
+    """Small meshes stay in shared memory next to one of many indices and one over a large vertex buffer."""
+    ms = _small(count, attributes)
+    idx, pos = _grid(104, 101, 0.2, 3)
+    assert len(idx) > 60000
+    wide = [dict(indices=idx, positions=pos, target=len(idx) // 6 * 3, error=1.0)]
+    few, fp = _grid(13, 11, 0.1, 0)
+    far = np.concatenate([fp, np.random.default_rng(2).uniform(0, 100, (24100 - len(fp), 3)).astype(np.float32)])
+    wide.append(dict(indices=few, positions=far, target=len(few) // 6 * 3, error=1.0))
+    for at in (0, count // 2, count):  # wherever they stand in the batch
+        batch = ms[:at] + wide + ms[at:]
+        for _ in range(2):  # with the size class's trials and without
+            res = mg.simplify_batch(batch)
+            assert mg.last_batch_placement() == (count, 2)
+        _same(port, batch, res)
+    res = mg.simplify_batch(wide)
+    assert mg.last_batch_placement() == (0, 2)
+    _same(port, wide, res)
