@@ -621,10 +621,12 @@ const size_t kBatchSlabTotal = size_t(16) << 30; // global slabs for meshes beyo
 struct BatchTuner
 {
 	std::mutex lock;
-	// (size class, the batch has more meshes than SMs) -> fastest (threads per CTA, shared-memory budget
-	// per CTA): a mesh that has an SM to itself wants many threads, a batch that fills the GPU many CTAs
-	// (4,096 groups with what their size class's single meshes had been given: 2.09 ms against 1.43)
-	std::map<std::pair<int, bool>, std::pair<int, size_t>> shape;
+	// (device, size class, the batch has more meshes than SMs, full form) -> fastest (threads per CTA,
+	// shared-memory budget per CTA): a mesh that has an SM to itself wants many threads, a batch that fills
+	// the GPU many CTAs (4,096 groups with what their size class's single meshes had been given: 2.09 ms
+	// against 1.43), and the lean and full forms differ in registers (4,096 meshes of 384 triangles with
+	// five attributes, with what positions-only ones had been given: 2.63 ms against 1.66)
+	std::map<std::tuple<int, int, bool, bool>, std::pair<int, size_t>> shape;
 } g_tuner;
 
 // the shared-memory budgets the batch autotuner times (four, two and one CTAs per SM; a smaller largest
@@ -801,7 +803,7 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		// the block size and the shared-memory budget the caller left open are autotuned per size
 		// class: the first batch of a class times every candidate pair on its own meshes
 		// (identical results) and keeps the fastest
-		const std::pair<int, bool> cls(sizeClass(p.max_index_count), p.count > size_t(sms));
+		const auto cls = std::make_tuple(s.device, sizeClass(p.max_index_count), p.count > size_t(sms), p.full);
 		{
 			std::lock_guard<std::mutex> g(g_tuner.lock);
 			auto it = g_tuner.shape.find(cls);
@@ -822,12 +824,16 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		{
 			if (p.threads && t != p.threads)
 				continue;
+			bool loaded = false; // a form's first launch also loads its code
 			for (size_t b : kBatchSmemBudgets)
 			{
 				if (s.batch_smem && b != s.batch_smem)
 					continue;
 				const unsigned int smem = footprint(p, b), blocks = slabBlocks(p, t, smem);
 				char* slabs = static_cast<char*>(s.batch_slabs.ensure(size_t(blocks) * p.slab));
+				if (!loaded)
+					launch(p, t, smem, blocks, slabs, st);
+				loaded = true;
 				MO_CUDA_CHECK(cudaEventRecord(e0, st));
 				launch(p, t, smem, blocks, slabs, st);
 				MO_CUDA_CHECK(cudaEventRecord(e1, st));
@@ -2032,8 +2038,9 @@ int meshoptgpu_getTuning(size_t index_count, size_t attribute_count, int* out4)
 	}
 	{
 		std::lock_guard<std::mutex> g(g_tuner.lock);
-		if (!g_tuner.shape.empty())
-			out4[3] = int(g_tuner.shape.rbegin()->second.second / 1024);
+		for (const auto& it : g_tuner.shape) // in order of the size class
+			if (std::get<0>(it.first) == dev)
+				out4[3] = int(it.second.second / 1024);
 	}
 	return found;
 }

@@ -1,4 +1,8 @@
 """The batch kernel's forms and where meshes run: batches that need several, bit for bit against the oracle."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -68,3 +72,27 @@ def test_batch_with_wide_meshes(port, count, attributes):
     res = mg.simplify_batch(wide)
     assert mg.last_batch_placement() == (0, 2)
     _same(port, wide, res)
+
+
+def test_tuned_per_form():
+    """A batch with attributes is timed itself, also after a positions-only one of its size class (in a
+    process of its own: what is timed is kept for the process)."""
+    code = """
+import sys
+sys.path[:0] = [%r, %r]
+import test_gpu_batch_forms as T
+import meshoptimizer_gb300 as mg
+
+def launches(ms):
+    n = mg.launch_count()
+    mg.simplify_batch(ms)
+    return mg.launch_count() - n
+
+lean, full = T._small(400), T._small(400, 3)
+first, again, other, once = launches(lean), launches(lean), launches(full), launches(full)
+assert first > 3 and again == 1 and other > 3 and once == 1, (first, again, other, once)
+assert mg.tuning(len(lean[0]["indices"]))["batch_smem_kib"] in (54, 110, 216)
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", code % (here, os.path.dirname(here))], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
