@@ -119,7 +119,8 @@ struct GridSum
 		__syncthreads();
 		return s[2];
 	}
-	// a wait has run out: what the barriers should have ordered is not to be read any more
+	// a wait has run out: what the barriers should have ordered is not to be read any more, and the block
+	// arrives at one more barrier at most (with two, it would complete the one that a slower block waits at)
 	__device__ __forceinline__ bool failed() const { return s[3] != 0; }
 };
 

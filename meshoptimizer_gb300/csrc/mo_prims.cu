@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kSortThreads, 5) kRadixScatter(const unsigned 
 // The bounded waits of the grid barriers, made to run out: block 0 never arrives, so every
 // other block waits `limit` times, records the error and leaves. Nothing faults or hangs.
 // words: the barrier's (the first four), the error flag, and what went wrong in mode 2: a block that did
-// not see the failure, or that waited at a later barrier.
+// not see the failure, or that waited at the next barrier.
 __global__ void kBarrierWaitProbe(unsigned int* words, unsigned int limit, int mode)
 {
 	if (blockIdx.x == 0)
@@ -311,8 +311,7 @@ __global__ void kBarrierWaitProbe(unsigned int* words, unsigned int limit, int m
 		const bool seen = grid.failed();
 		const long long t = clock64();
 		grid.wait(blockIdx.x, 1u << 16);
-		grid.wait(0, 1u << 16);
-		// two waits would take 4 million cycles and more, two arrivals a few thousand
+		// a wait would take 4 million cycles and more, an arrival a few thousand
 		if (!seen || !grid.failed() || clock64() - t > (1ll << 20))
 			atomicOr(words + 5, 2u);
 	}

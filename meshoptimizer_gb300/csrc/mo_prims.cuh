@@ -93,7 +93,7 @@ struct ScanSync
 // Runs a grid barrier (mode 0: the position solve's, 1: the single-use one, 2: the pass kernels') with
 // one of `blocks` blocks never arriving and a wait limit of `limit` polls; returns the error flag the
 // waiting blocks set (1 when the bounded wait ran out, as it must; in mode 2 with 2 added if a block did
-// not see that, or waited at a later barrier all the same). For tests of the failure path.
+// not see that, or waited at the next barrier all the same). For tests of the failure path.
 unsigned int probeBarrierWait(int mode, unsigned int blocks, unsigned int limit, cudaStream_t stream);
 
 // Blocks a single-launch scan may use on the current device (all resident at once); queried

@@ -44,8 +44,8 @@ def test_barrier_probe_rejects_bad_arguments():
 
 
 def test_pass_barrier_wait_runs_out_and_reports(port):
-    """The pass kernels' barrier, which carries a sum: the blocks see the failure as they leave, and those
-    that reach later barriers do not wait there again."""
+    """The pass kernels' barrier, which carries a sum: the blocks see the failure as they leave, and do
+    not wait at the next barrier."""
     for blocks in (2, 16, 152):
         st, timed_out = mg.probe_barrier_wait(once=2, blocks=blocks, wait_limit=4096)
         assert st == mg.STATUS_OK
