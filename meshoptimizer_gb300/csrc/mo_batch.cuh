@@ -39,9 +39,10 @@ struct BatchResult
 	unsigned int index_count;
 	float result_error;
 	unsigned int passes;
-	unsigned int status; // 0 ok, 2 invalid index, 3 a decision round made no progress; + kBatchInSlab
+	unsigned int status; // 0 ok, 2 invalid index, 3 a decision round made no progress; and the bits below
 };
 constexpr unsigned int kBatchInSlab = 0x100; // the mesh ran in its CTA's slab
+constexpr unsigned int kBatchBeyond = 0x200; // it had more vertices or a larger capacity than expected
 
 // Memory of one mesh. smem: shared memory it is expected to need beside its attribute rows (rows), which
 // go there too where they fit, else into the CTA's slab; slab: global scratch in which it runs whatever

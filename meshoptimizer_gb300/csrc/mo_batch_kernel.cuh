@@ -214,8 +214,9 @@ __host__ __device__ inline size_t rowBytes(size_t V, size_t ac)
 
 // What a mesh is expected to need: a square patch of a surface has one vertex for two triangles and half
 // its perimeter's (1,024 triangles: 560; 589 are allowed for), and its capacity (boundEdgeCollapses) is
-// about two thirds of its indices. A mesh that needs more than the launch's shared memory runs in the
-// slab.
+// about two thirds of its indices (all of them where every edge is on a border). A mesh that needs more
+// than the launch's shared memory runs in the slab, after its setup up to there; where many do, launches
+// are sized for the most a mesh can need.
 inline size_t expectedVertices(size_t I, size_t bound, bool sparse)
 {
 	if (!sparse)
@@ -227,6 +228,13 @@ inline size_t expectedVertices(size_t I, size_t bound, bool sparse)
 __host__ __device__ inline size_t expectedCapacity(size_t I)
 {
 	return I - I * 3 / 10 + 16;
+}
+
+// whether a mesh had more vertices or a larger capacity than that
+__device__ inline bool beyondExpected(unsigned int V, unsigned int I, unsigned int cap, bool sparse)
+{
+	const unsigned int x = V > I / 6 + 10 ? V - I / 6 - 10 : 0u; // beside 1.25 times the root of I
+	return cap > expectedCapacity(I) || (sparse && (unsigned long long)x * x * 16 > 25ull * I);
 }
 
 // ---------------------------------------------------------------- block helpers
@@ -1638,7 +1646,7 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 	for (unsigned int i = tid; i < result_count; i += NT)
 		d.out[i] = src(w.idx[i]);
 	if (tid == 0)
-		*out = BatchResult{result_count, sqrtf(result_error) * error_scale, passes, (s_stall ? 3u : 0u) | kWhere};
+		*out = BatchResult{result_count, sqrtf(result_error) * error_scale, passes, (s_stall ? 3u : 0u) | kWhere | (beyondExpected(V, I, s_cap, sparse) ? kBatchBeyond : 0u)};
 	return true;
 }
 

@@ -618,15 +618,36 @@ size_t updateHost(unsigned int* indices, size_t index_count, float* vertex_posit
 const size_t kBatchSmemDefault = 110 * 1024;    // shared-memory budget per CTA (two CTAs per SM)
 const size_t kBatchSlabTotal = size_t(16) << 30; // global slabs for meshes beyond the budget
 
+// threads per CTA, shared-memory budget per CTA, and whether the shared memory under that budget is sized
+// for the most a mesh can need rather than for what it is expected to
+struct BatchShape
+{
+	int threads = 0;
+	size_t budget = 0;
+	bool sure = false;
+};
+
+// The fastest shapes of a class: for meshes as expected, and for batches with many that need more (ribbons
+// and separate quads, whose edges are borders; flat shaded groups, with three vertices per triangle), which
+// shared memory sized by the expectation sends to the slab after their setup or part of it. What the
+// class's last batch was like says which one is next. 4,096 ribbons of 120 / 200 triangles 1.44 / 2.01 ms
+// by the expectation and 0.82 / 1.04 by the most they can need; flat groups of 60 / 200 triangles 0.80 /
+// 1.75 and 0.57 / 0.96.
+struct BatchShapes
+{
+	BatchShape as_expected, beyond;
+	bool timed_beyond = false, last_beyond = false;
+};
+
 struct BatchTuner
 {
 	std::mutex lock;
-	// (device, size class, the batch has more meshes than SMs, full form) -> fastest (threads per CTA,
-	// shared-memory budget per CTA): a mesh that has an SM to itself wants many threads, a batch that fills
-	// the GPU many CTAs (4,096 groups with what their size class's single meshes had been given: 2.09 ms
-	// against 1.43), and the lean and full forms differ in registers (4,096 meshes of 384 triangles with
-	// five attributes, with what positions-only ones had been given: 2.63 ms against 1.66)
-	std::map<std::tuple<int, int, bool, bool>, std::pair<int, size_t>> shape;
+	// (device, size class, the batch has more meshes than SMs, full form) -> fastest shape: a mesh that has
+	// an SM to itself wants many threads, a batch that fills the GPU many CTAs (4,096 groups with what their
+	// size class's single meshes had been given: 2.09 ms against 1.43), and the lean and full forms differ
+	// in registers (4,096 meshes of 384 triangles with five attributes, with what positions-only ones had
+	// been given: 2.63 ms against 1.66)
+	std::map<std::tuple<int, int, bool, bool>, BatchShapes> shape;
 } g_tuner;
 
 // the shared-memory budgets the batch autotuner times (four, two and one CTAs per SM; a smaller largest
@@ -742,7 +763,8 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		size_t slab, max_index_count;
 		int threads;
 		size_t budget;
-	} parts[2] = {{0, wide, false, false, 0, 0, 0, 0}, {wide, n - wide, true, false, 0, 0, 0, 0}};
+		bool sure;
+	} parts[2] = {{0, wide, false, false, 0, 0, 0, 0, false}, {wide, n - wide, true, false, 0, 0, 0, 0, false}};
 	for (Part& p : parts)
 		for (size_t i = p.first; i < p.first + p.count; ++i)
 		{
@@ -752,12 +774,17 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 			p.slab = std::max(p.slab, bytes[i].slab);
 			p.max_index_count = std::max<size_t>(p.max_index_count, ordered[i].index_count);
 		}
-	// a budget's dynamic shared memory: the largest mesh that fits it, with its attribute rows or without
-	auto footprint = [&](const Part& p, size_t budget) {
+	// a budget's dynamic shared memory: the largest mesh that fits it, with its attribute rows or without, by
+	// what meshes are expected to need or (sure) by the most they can
+	auto footprint = [&](const Part& p, size_t budget, bool sure) {
 		size_t most = 0;
 		if (p.narrow)
 			for (size_t i = p.first; i < p.first + p.count; ++i)
-				most = std::max(most, bytes[i].smem + bytes[i].rows <= budget ? bytes[i].smem + bytes[i].rows : (bytes[i].smem <= budget ? bytes[i].smem : size_t(0)));
+			{
+				const BatchBytes& b = bytes[i];
+				const size_t all = sure ? b.slab : b.smem + b.rows;
+				most = std::max(most, all <= budget ? all : (b.smem <= budget ? b.smem : size_t(0)));
+			}
 		return unsigned((most + 15) & ~size_t(15));
 	};
 	const int sms = s.sms;
@@ -792,6 +819,20 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		launchBatch(d_descs + p.first, unsigned(p.count), d_ticket + (p.narrow ? 1 : 0), d_res + p.first, slabs, p.slab, smem, blocks, threads, p.full, p.narrow, on);
 	};
 
+	auto readResults = [&](const Part& p) {
+		BatchResult* const r = reinterpret_cast<BatchResult*>(hmeta + off_res) + p.first;
+		MO_CUDA_CHECK(cudaMemcpyAsync(r, d_res + p.first, p.count * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
+		MO_CUDA_CHECK(cudaStreamSynchronize(st));
+		return r;
+	};
+	auto manyBeyond = [](const BatchResult* r, size_t count) {
+		size_t beyond = 0;
+		for (size_t i = 0; i < count; ++i)
+			beyond += (r[i].status & kBatchBeyond) != 0;
+		return beyond > count / 16;
+	};
+	bool tuned = false;
+	std::tuple<int, int, bool, bool> cls;
 	for (Part& p : parts)
 	{
 		if (!p.count)
@@ -803,53 +844,76 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		// the block size and the shared-memory budget the caller left open are autotuned per size
 		// class: the first batch of a class times every candidate pair on its own meshes
 		// (identical results) and keeps the fastest
-		const auto cls = std::make_tuple(s.device, sizeClass(p.max_index_count), p.count > size_t(sms), p.full);
+		tuned = true;
+		cls = std::make_tuple(s.device, sizeClass(p.max_index_count), p.count > size_t(sms), p.full);
+		BatchShapes shapes;
+		bool known = false;
 		{
 			std::lock_guard<std::mutex> g(g_tuner.lock);
 			auto it = g_tuner.shape.find(cls);
 			if (it != g_tuner.shape.end())
-			{
-				p.threads = p.threads ? p.threads : it->second.first;
-				p.budget = s.batch_smem ? p.budget : it->second.second;
-				continue;
-			}
+				shapes = it->second, known = true;
 		}
-		cudaEvent_t e0, e1;
-		MO_CUDA_CHECK(cudaEventCreate(&e0));
-		MO_CUDA_CHECK(cudaEventCreate(&e1));
-		float best = 1e30f;
-		int best_t = p.threads ? p.threads : 256;
-		size_t best_b = p.budget;
-		for (int t : {128, 256, 512})
-		{
-			if (p.threads && t != p.threads)
-				continue;
-			bool loaded = false; // a form's first launch also loads its code
-			for (size_t b : kBatchSmemBudgets)
-			{
-				if (s.batch_smem && b != s.batch_smem)
-					continue;
-				const unsigned int smem = footprint(p, b), blocks = slabBlocks(p, t, smem);
+		auto trials = [&](bool sure) {
+			BatchShape best = sure ? shapes.as_expected : BatchShape{p.threads ? p.threads : 256, p.budget, false};
+			cudaEvent_t e0, e1;
+			MO_CUDA_CHECK(cudaEventCreate(&e0));
+			MO_CUDA_CHECK(cudaEventCreate(&e1));
+			auto timed = [&](const BatchShape& c, bool warm) {
+				const unsigned int smem = footprint(p, c.budget, c.sure), blocks = slabBlocks(p, c.threads, smem);
 				char* slabs = static_cast<char*>(s.batch_slabs.ensure(size_t(blocks) * p.slab));
-				if (!loaded)
-					launch(p, t, smem, blocks, slabs, st);
-				loaded = true;
-				MO_CUDA_CHECK(cudaEventRecord(e0, st));
-				launch(p, t, smem, blocks, slabs, st);
-				MO_CUDA_CHECK(cudaEventRecord(e1, st));
-				MO_CUDA_CHECK(cudaEventSynchronize(e1));
-				float ms = 0;
-				MO_CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
-				if (ms < best)
-					best = ms, best_t = t, best_b = b;
+				if (warm)
+					launch(p, c.threads, smem, blocks, slabs, st);
+				float least = 1e30f;
+				for (int rep = 0; rep < (p.count > size_t(sms) ? 1 : 3); ++rep) // short launches: the fastest of three
+				{
+					MO_CUDA_CHECK(cudaEventRecord(e0, st));
+					launch(p, c.threads, smem, blocks, slabs, st);
+					MO_CUDA_CHECK(cudaEventRecord(e1, st));
+					MO_CUDA_CHECK(cudaEventSynchronize(e1));
+					float ms = 0;
+					MO_CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
+					least = std::min(least, ms);
+				}
+				return least;
+			};
+			float best_ms = sure ? timed(best, false) : 1e30f;
+			for (int t : {128, 256, 512})
+			{
+				if (p.threads && t != p.threads)
+					continue;
+				bool warm = true; // a form's first launch also loads its code
+				for (size_t b : kBatchSmemBudgets)
+				{
+					if ((s.batch_smem && b != s.batch_smem) || (sure && footprint(p, b, true) <= footprint(p, b, false)))
+						continue;
+					const BatchShape c{t, b, sure};
+					const float ms = timed(c, warm);
+					warm = false;
+					if (ms < best_ms)
+						best_ms = ms, best = c;
+				}
 			}
+			cudaEventDestroy(e0);
+			cudaEventDestroy(e1);
+			return best;
+		};
+		if (!known)
+		{
+			shapes.as_expected = trials(false);
+			shapes.last_beyond = manyBeyond(readResults(p), p.count);
 		}
-		cudaEventDestroy(e0);
-		cudaEventDestroy(e1);
-		p.threads = best_t;
-		p.budget = best_b;
+		if (shapes.last_beyond && !shapes.timed_beyond)
+		{
+			shapes.beyond = trials(true);
+			shapes.timed_beyond = true;
+		}
+		const BatchShape use = shapes.last_beyond && shapes.timed_beyond ? shapes.beyond : shapes.as_expected;
+		p.threads = p.threads ? p.threads : use.threads;
+		p.budget = s.batch_smem ? p.budget : use.budget;
+		p.sure = use.sure;
 		std::lock_guard<std::mutex> g(g_tuner.lock);
-		g_tuner.shape[cls] = std::make_pair(best_t, best_b);
+		g_tuner.shape[cls] = shapes;
 	}
 
 	// both parts at once, the wide one from a stream of its own
@@ -858,7 +922,7 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	for (int q = 0; q < 2; ++q)
 		if (parts[q].count)
 		{
-			smem[q] = footprint(parts[q], parts[q].budget);
+			smem[q] = footprint(parts[q], parts[q].budget, parts[q].sure);
 			blocks[q] = slabBlocks(parts[q], parts[q].threads, smem[q]);
 			slab_bytes[q] = align256(size_t(blocks[q]) * parts[q].slab);
 		}
@@ -892,11 +956,17 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	MO_CUDA_CHECK(cudaMemcpyAsync(hmeta + off_res, d_res, n * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
 	MO_CUDA_CHECK(cudaStreamSynchronize(st));
 	probe().collect();
+	if (tuned)
+	{
+		const bool beyond = manyBeyond(tmp + parts[1].first, parts[1].count);
+		std::lock_guard<std::mutex> g(g_tuner.lock);
+		g_tuner.shape[cls].last_beyond = beyond;
+	}
 	for (size_t i = 0; i < n; ++i)
 	{
 		BatchResult& r = results[perm[i]] = tmp[i];
 		++(r.status & kBatchInSlab ? s.batch_in_slab : s.batch_in_shared);
-		r.status &= ~kBatchInSlab;
+		r.status &= ~(kBatchInSlab | kBatchBeyond);
 	}
 }
 
@@ -2009,7 +2079,7 @@ int meshoptgpu_getBatchThreads(void)
 	if (s.batch_threads)
 		return s.batch_threads;
 	std::lock_guard<std::mutex> g(g_tuner.lock);
-	return g_tuner.shape.empty() ? 0 : g_tuner.shape.rbegin()->second.first;
+	return g_tuner.shape.empty() ? 0 : g_tuner.shape.rbegin()->second.as_expected.threads;
 }
 
 int meshoptgpu_getTuning(size_t index_count, size_t attribute_count, int* out4)
@@ -2040,7 +2110,7 @@ int meshoptgpu_getTuning(size_t index_count, size_t attribute_count, int* out4)
 		std::lock_guard<std::mutex> g(g_tuner.lock);
 		for (const auto& it : g_tuner.shape) // in order of the size class
 			if (std::get<0>(it.first) == dev)
-				out4[3] = int(it.second.second / 1024);
+				out4[3] = int(it.second.as_expected.budget / 1024);
 	}
 	return found;
 }

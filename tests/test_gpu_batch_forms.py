@@ -96,3 +96,70 @@ assert mg.tuning(len(lean[0]["indices"]))["batch_smem_kib"] in (54, 110, 216)
     here = os.path.dirname(os.path.abspath(__file__))
     r = subprocess.run([sys.executable, "-c", code % (here, os.path.dirname(here))], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def _ribbon(tris, seed):
+    return _grid(tris // 2 + 1, 2, 0.1, seed)
+
+
+def _quads(count, seed):
+    """Separate quads: every vertex is on a border."""
+    p = np.random.default_rng(seed).random((count, 1, 3)) * 10 + np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [1, 1, 0.1]])[None]
+    idx = (np.arange(count)[:, None] * 4 + np.array([0, 1, 2, 2, 1, 3])[None]).reshape(-1)
+    return idx.astype(np.uint32), p.reshape(-1, 3).astype(np.float32)
+
+
+@pytest.mark.parametrize("tris", [2, 40, 128, 200])
+def test_open_meshes_in_shared_memory(port, tris):
+    """Meshes whose vertices are mostly on borders have a larger capacity than expected; after a batch of
+    them, the next one's shared memory is sized for it."""
+    for make in (_ribbon, lambda t, s: _quads(t // 2, s)):
+        distinct = []
+        for k in range(4):
+            idx, pos = make(tris, k)
+            distinct.append(dict(indices=idx, positions=pos, target=len(idx) // 6 * 3, error=1.0))
+        ms = [distinct[i % 4] for i in range(600)]
+        for _ in range(2):
+            res = mg.simplify_batch(ms)
+        assert mg.last_batch_placement() == (len(ms), 0)
+        _same(port, ms, res)
+    # and back: ordinary meshes of the same number of indices
+    idx, pos = _grid(11, tris // 20 + 1, 0.1, 1)
+    ms = [dict(indices=idx, positions=pos, target=len(idx) // 6 * 3, error=1.0)] * 600
+    for _ in range(2):
+        _same(port, ms, mg.simplify_batch(ms))
+
+
+@pytest.mark.parametrize("attributes", [0, 2])
+@pytest.mark.parametrize("tris", [20, 120, 240])
+def test_unshared_sparse_groups_in_shared_memory(port, tris, attributes):
+    """Sparse groups with three vertices per triangle (flat shaded): more than a surface's share of them. A
+    process of its own, so that this kind is the first of its size class."""
+    code = """
+import sys
+sys.path[:0] = [%r, %r, %r]
+import numpy as np
+import oracle
+import test_gpu_batch_forms as T
+import meshoptimizer_gb300 as mg
+
+idx, pos = T._grid(11, %d // 20 + 1, 0.1, 1)
+n, count, attributes = len(idx), 300, %d
+flat = np.concatenate([pos[idx] + [20 * (i %% 8), 0, 0] for i in range(count)]).astype(np.float32)
+at = np.random.default_rng(1).standard_normal((len(flat), max(attributes, 1))).astype(np.float32)
+ms = []
+for i in range(count):
+    m = dict(indices=(np.arange(n) + n * i).astype(np.uint32), positions=flat, target=n // 6 * 3, error=1.0, options=mg.SimplifySparse)
+    if attributes:
+        m.update(attributes=at, weights=np.full(attributes, 0.3, np.float32))
+    ms.append(m)
+for _ in range(2):
+    res = mg.simplify_batch(ms)
+assert mg.last_batch_placement() == (count, 0), mg.last_batch_placement()
+T._same(oracle, ms[:20], res[:20])
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    root = os.path.dirname(here)
+    r = subprocess.run([sys.executable, "-c", code % (here, root, os.path.join(root, "oracle"), tris, attributes)], capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
