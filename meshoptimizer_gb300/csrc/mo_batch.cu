@@ -2,6 +2,7 @@
 // mesh needs, and the launch.
 #include "mo_batch_kernel.cuh"
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -17,7 +18,7 @@ BatchBytes bytesOf(const BatchDesc& d)
 	BatchBytes b;
 	b.smem = hotBytes<IX>(I, V, bound, expectedCapacity(I), sparse);
 	b.rows = rowBytes<IX>(V, d.ac);
-	b.slab = rowBytes<IX>(bound, d.ac) + hotBytes<IX>(I, bound, bound, I + 4, sparse);
+	b.slab = rowBytes<IX>(bound, d.ac) + hotBytes<IX>(I, bound, bound, std::max(I + 4, expectedCapacity(I)), sparse);
 	return b;
 }
 

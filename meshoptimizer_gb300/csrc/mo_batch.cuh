@@ -39,14 +39,14 @@ struct BatchResult
 	unsigned int index_count;
 	float result_error;
 	unsigned int passes;
-	unsigned int status; // 0 ok, 2 invalid index, 3 a decision round made no progress; and the bits below
+	unsigned int status; // 0 ok, 2 invalid index, 3 a decision round made no progress, 4 its scratch was too small; and the bits below
 };
 constexpr unsigned int kBatchInSlab = 0x100; // the mesh ran in its CTA's slab
 constexpr unsigned int kBatchBeyond = 0x200; // it had more vertices or a larger capacity than expected
 
 // Memory of one mesh. smem: shared memory it is expected to need beside its attribute rows (rows), which
-// go there too where they fit, else into the CTA's slab; slab: global scratch in which it runs whatever
-// it turns out to need.
+// go there too where they fit, else into the CTA's slab; slab: memory of either kind in which it runs
+// whatever it turns out to need.
 struct BatchBytes
 {
 	size_t smem, rows, slab;
@@ -80,7 +80,7 @@ BatchKernel batchKernelWide(bool full);
 int batchBlocksPerSM(int threads, unsigned int smem_bytes, bool full, bool narrow);
 
 // full: the instantiation with every option; otherwise the positions-only one. narrow: every mesh is
-// narrow. Every CTA has slab_bytes of slabs, at least the largest mesh's.
+// narrow. Every CTA has slab_bytes of slabs, the largest mesh's at least, or none where smem_bytes are that.
 void launchBatch(const BatchDesc* d_descs, unsigned int count, unsigned int* d_ticket, BatchResult* d_results, char* d_slabs, size_t slab_bytes,
     unsigned int smem_bytes, unsigned int blocks, int threads, bool full, bool narrow, cudaStream_t stream);
 

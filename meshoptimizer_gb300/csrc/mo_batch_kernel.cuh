@@ -519,9 +519,11 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 	auto src = [&](unsigned int i) { return sparse ? w.back[i] : i; };
 	if (FULL && ac)
 	{
-		Region with = mem;
+		Region with = mem, rest = mem;
 		carveRows(w, with, V, ac);
-		if (FAST && with.off + hotBytes<IX>(0, 0, 0, expectedCapacity(I), false) <= with.limit)
+		rest.off = with.off;
+		carveCandidates(w, rest, expectedCapacity(I));
+		if (FAST && rest.ok())
 			mem = with;
 		else
 		{
@@ -1675,7 +1677,8 @@ __global__ void __launch_bounds__(NT, (kBatchWarps<NT, FULL>) * 32 / NT) kBatch(
 		// in shared memory, its attribute rows there or in the slab; where that is too small, in the slab (a
 		// mesh that needs 32-bit ids is larger than any shared memory)
 		const size_t bound = localVertexBound(d.index_count, d.vertex_count, FULL && (d.options & kOptSparse) != 0);
-		const size_t rows = FULL && d.ac ? rowBytes<IX>(bound, d.ac) : 0;
+		// (a launch without slabs has shared memory for the most any of its meshes can need)
+		const size_t rows = FULL && d.ac ? min(rowBytes<IX>(bound, d.ac), slab_bytes) : 0;
 		bool done = false;
 		if constexpr (sizeof(IX) == 2)
 		{
@@ -1683,7 +1686,9 @@ __global__ void __launch_bounds__(NT, (kBatchWarps<NT, FULL>) * 32 / NT) kBatch(
 			__syncthreads();
 		}
 		if (!done)
-			simplifyMesh<NT, FULL, IX, false>(d, &results[job], Region(slab + rows, slab_bytes - rows), Region(slab, rows));
+			done = simplifyMesh<NT, FULL, IX, false>(d, &results[job], Region(slab + rows, slab_bytes - rows), Region(slab, rows));
+		if (!done && threadIdx.x == 0)
+			results[job] = BatchResult{0, 0.f, 0, 4};
 		__syncthreads();
 	}
 }

@@ -113,6 +113,7 @@ struct ThreadState
 	cudaStream_t batch_stream = nullptr;
 	cudaEvent_t batch_event = nullptr;
 	size_t batch_in_shared = 0, batch_in_slab = 0; // meshes of the last batch by where they ran
+	size_t batch_slab_limit = ~size_t(0); // bytes of slabs a batch may allocate where its meshes can do without (the server's)
 
 	void ensureBatchStream()
 	{
@@ -810,14 +811,35 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	if (nm)
 		MO_CUDA_CHECK(cudaMemcpyAsync(d_maps, hmeta + off_maps, nm * sizeof(BatchAttr), cudaMemcpyHostToDevice, st));
 
-	auto slabBlocks = [&](const Part& p, int threads, unsigned int smem) {
-		const int per_sm = std::max(1, batchBlocksPerSM(threads, smem, p.full, p.narrow));
-		const size_t blocks = std::min<size_t>(size_t(per_sm) * sms, p.count);
-		return unsigned(std::max<size_t>(1, std::min<size_t>(blocks, kBatchSlabTotal / std::max<size_t>(p.slab, 1))));
+	// a launch: shared memory per CTA, the CTAs, and each one's slab, if a mesh may need one. Where the slabs
+	// would exceed the limit, shared memory is for the most that every mesh of up to kBatchSmemDefault can
+	// need, which are then sure to need no slab.
+	struct Plan
+	{
+		unsigned int smem, blocks;
+		size_t slab;
 	};
-	auto launch = [&](const Part& p, int threads, unsigned int smem, unsigned int blocks, char* slabs, cudaStream_t on) {
-		launchBatch(d_descs + p.first, unsigned(p.count), d_ticket + (p.narrow ? 1 : 0), d_res + p.first, slabs, p.slab, smem, blocks, threads, p.full, p.narrow, on);
+	auto plan = [&](const Part& p, const BatchShape& c, size_t limit) {
+		Plan r{footprint(p, c.budget, c.sure), 0, 0};
+		r.slab = p.slab > r.smem ? p.slab : 0;
+		if (r.slab > limit && p.narrow)
+		{
+			for (size_t i = p.first; i < p.first + p.count; ++i)
+				if (bytes[i].slab <= kBatchSmemDefault)
+					r.smem = std::max(r.smem, unsigned((bytes[i].slab + 15) & ~size_t(15)));
+			r.slab = p.slab > r.smem ? p.slab : 0;
+		}
+		const int per_sm = std::max(1, batchBlocksPerSM(c.threads, r.smem, p.full, p.narrow));
+		size_t blocks = std::min<size_t>(size_t(per_sm) * sms, p.count);
+		if (r.slab)
+			blocks = std::max<size_t>(1, std::min(blocks, limit / r.slab));
+		r.blocks = unsigned(blocks);
+		return r;
 	};
+	auto launch = [&](const Part& p, int threads, const Plan& r, char* slabs, cudaStream_t on) {
+		launchBatch(d_descs + p.first, unsigned(p.count), d_ticket + (p.narrow ? 1 : 0), d_res + p.first, slabs, r.slab, r.smem, r.blocks, threads, p.full, p.narrow, on);
+	};
+	const size_t limit = std::min(s.batch_slab_limit, kBatchSlabTotal);
 
 	auto readResults = [&](const Part& p) {
 		BatchResult* const r = reinterpret_cast<BatchResult*>(hmeta + off_res) + p.first;
@@ -844,7 +866,6 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		// the block size and the shared-memory budget the caller left open are autotuned per size
 		// class: the first batch of a class times every candidate pair on its own meshes
 		// (identical results) and keeps the fastest
-		tuned = true;
 		cls = std::make_tuple(s.device, sizeClass(p.max_index_count), p.count > size_t(sms), p.full);
 		BatchShapes shapes;
 		bool known = false;
@@ -860,15 +881,15 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 			MO_CUDA_CHECK(cudaEventCreate(&e0));
 			MO_CUDA_CHECK(cudaEventCreate(&e1));
 			auto timed = [&](const BatchShape& c, bool warm) {
-				const unsigned int smem = footprint(p, c.budget, c.sure), blocks = slabBlocks(p, c.threads, smem);
-				char* slabs = static_cast<char*>(s.batch_slabs.ensure(size_t(blocks) * p.slab));
+				const Plan r = plan(p, c, limit);
+				char* slabs = r.slab ? static_cast<char*>(s.batch_slabs.ensure(r.blocks * r.slab)) : nullptr;
 				if (warm)
-					launch(p, c.threads, smem, blocks, slabs, st);
+					launch(p, c.threads, r, slabs, st);
 				float least = 1e30f;
 				for (int rep = 0; rep < (p.count > size_t(sms) ? 1 : 3); ++rep) // short launches: the fastest of three
 				{
 					MO_CUDA_CHECK(cudaEventRecord(e0, st));
-					launch(p, c.threads, smem, blocks, slabs, st);
+					launch(p, c.threads, r, slabs, st);
 					MO_CUDA_CHECK(cudaEventRecord(e1, st));
 					MO_CUDA_CHECK(cudaEventSynchronize(e1));
 					float ms = 0;
@@ -898,12 +919,14 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 			cudaEventDestroy(e1);
 			return best;
 		};
+		if (!known && p.slab > limit) // no room for slabs: shapes cannot be told apart, and nothing is kept
+			continue;
 		if (!known)
 		{
 			shapes.as_expected = trials(false);
 			shapes.last_beyond = manyBeyond(readResults(p), p.count);
 		}
-		if (shapes.last_beyond && !shapes.timed_beyond)
+		if (shapes.last_beyond && !shapes.timed_beyond && p.slab <= limit)
 		{
 			shapes.beyond = trials(true);
 			shapes.timed_beyond = true;
@@ -912,22 +935,24 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		p.threads = p.threads ? p.threads : use.threads;
 		p.budget = s.batch_smem ? p.budget : use.budget;
 		p.sure = use.sure;
+		tuned = true;
 		std::lock_guard<std::mutex> g(g_tuner.lock);
 		g_tuner.shape[cls] = shapes;
 	}
 
 	// both parts at once, the wide one from a stream of its own
-	unsigned int smem[2] = {0, 0}, blocks[2] = {0, 0};
+	const bool both = parts[0].count && parts[1].count;
+	Plan plans[2] = {};
 	size_t slab_bytes[2] = {0, 0};
-	for (int q = 0; q < 2; ++q)
+	for (int q = 1; q >= 0; --q) // the narrow part's slabs, if any, leave the rest of the limit to the wide one
 		if (parts[q].count)
 		{
-			smem[q] = footprint(parts[q], parts[q].budget, parts[q].sure);
-			blocks[q] = slabBlocks(parts[q], parts[q].threads, smem[q]);
-			slab_bytes[q] = align256(size_t(blocks[q]) * parts[q].slab);
+			const BatchShape c{parts[q].threads, parts[q].budget, parts[q].sure};
+			const size_t share = both && q == 1 ? limit / 2 : limit - std::min(limit, slab_bytes[1]);
+			plans[q] = plan(parts[q], c, share);
+			slab_bytes[q] = align256(plans[q].blocks * plans[q].slab);
 		}
-	char* slabs = static_cast<char*>(s.batch_slabs.ensure(slab_bytes[0] + slab_bytes[1]));
-	const bool both = parts[0].count && parts[1].count;
+	char* slabs = slab_bytes[0] + slab_bytes[1] ? static_cast<char*>(s.batch_slabs.ensure(slab_bytes[0] + slab_bytes[1])) : nullptr;
 	if (both)
 	{
 		s.ensureBatchStream();
@@ -937,9 +962,9 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	try
 	{
 		if (parts[0].count)
-			launch(parts[0], parts[0].threads, smem[0], blocks[0], slabs, both ? s.batch_stream : st);
+			launch(parts[0], parts[0].threads, plans[0], slabs, both ? s.batch_stream : st);
 		if (parts[1].count)
-			launch(parts[1], parts[1].threads, smem[1], blocks[1], slabs + slab_bytes[0], st);
+			launch(parts[1], parts[1].threads, plans[1], slabs + slab_bytes[0], st);
 		if (both)
 		{
 			MO_CUDA_CHECK(cudaEventRecord(s.batch_event, s.batch_stream));
@@ -993,8 +1018,8 @@ bool smallMeshOnBatch(ThreadState& s, const MeshDesc& m, unsigned int* d_out, cu
 	runBatch(s, descs, maps, attr_of, res, st);
 	if (res[0].status == 2)
 		throw std::invalid_argument("index out of range of vertex_count");
-	if (res[0].status == 3)
-		throw std::runtime_error("collapse decision round made no progress");
+	if (res[0].status)
+		throw std::runtime_error(res[0].status == 3 ? "collapse decision round made no progress" : "batch scratch too small");
 	s.last = RunResult();
 	s.last.index_count = res[0].index_count;
 	s.last.result_error = res[0].result_error;
@@ -1182,12 +1207,12 @@ int finishBatch(const std::vector<BatchResult>& res, size_t* counts, float* erro
 		if (errors)
 			errors[i] = res[i].result_error;
 		if (res[i].status)
-			status = res[i].status == 3 ? meshoptgpu_StatusCudaError : meshoptgpu_StatusInvalidArgument;
+			status = res[i].status >= 3 ? meshoptgpu_StatusCudaError : meshoptgpu_StatusInvalidArgument;
 	}
 	if (status == meshoptgpu_StatusInvalidArgument)
 		setStatus(status, "a batched mesh has an index out of range of its vertex_count");
 	else if (status != meshoptgpu_StatusOk)
-		setStatus(status, "a batched mesh's decision round made no progress");
+		setStatus(status, "a batched mesh's decision round made no progress, or its scratch was too small");
 	else
 		setStatus(meshoptgpu_StatusOk, "");
 	return status;
@@ -1200,7 +1225,7 @@ struct ServerRequest
 	BatchDesc desc;
 	std::vector<float> weights; // attribute weights, copied at submission
 	size_t index_count = 0, vertex_count = 0;
-	size_t reserve = 0;
+	size_t reserve = 0, slab = 0;
 	std::chrono::steady_clock::time_point submitted, completed;
 	bool done = false;
 	int status = meshoptgpu_StatusOk;
@@ -1225,12 +1250,11 @@ struct ServerImpl
 
 const size_t kServerBudgetDefault = size_t(40) << 30;
 
-// device bytes a request holds while it runs on the batch path (its global slab; a mesh that is expected to
-// run in shared memory is never too large for the budget) or on the single-mesh path (its arena)
-size_t batchReserve(const ServerRequest& r, size_t budget)
+// device bytes a request holds while it runs on the batch path: a slab, or for a mesh that shared memory
+// holds whatever it needs, no more than its share of the batch's descriptors and results
+size_t batchReserve(size_t slab)
 {
-	const BatchBytes b = batchBytes(r.desc, batchNarrow(r.desc));
-	return std::max<size_t>(4096, b.smem + b.rows <= kBatchSmemDefault ? std::min(b.slab, budget) : b.slab);
+	return slab <= kBatchSmemDefault ? 4096 : slab;
 }
 
 void publish(ServerImpl& S, std::vector<ServerRequest*>& done_reqs, size_t release)
@@ -1263,26 +1287,30 @@ void batchWorker(ServerImpl* S)
 			S->cv_work.wait(lk, [&] {
 				if (S->stop)
 					return true;
-				return !S->small_q.empty() && S->reserved + batchReserve(*S->small_q.front(), S->cfg.memory_budget) <= S->cfg.memory_budget;
+				return !S->small_q.empty() && S->reserved + S->small_q.front()->reserve <= S->cfg.memory_budget;
 			});
 			if (S->stop && S->small_q.empty())
 				return;
 			// continuous batching: everything that arrived since this worker last launched, in
 			// arrival order, while the memory budget and the batch limit allow
-			size_t maxslab = 0;
+			size_t least = 0, most = 0; // a CTA's slab: where shared memory may be too small, and for all
 			while (!S->small_q.empty() && take.size() < size_t(S->cfg.max_batch))
 			{
 				ServerRequest* r = S->small_q.front();
-				size_t nm = std::max(maxslab, batchReserve(*r, S->cfg.memory_budget));
-				size_t blocks = std::min<size_t>(take.size() + 1, size_t(S->sms) * 4);
-				size_t need = blocks * nm + 4096 * (take.size() + 1);
-				if (S->reserved + need > S->cfg.memory_budget && !take.empty())
+				const size_t nl = std::max(least, r->slab <= kBatchSmemDefault ? size_t(0) : r->slab);
+				const size_t blocks = std::min<size_t>(take.size() + 1, size_t(S->sms) * 4);
+				if (S->reserved + blocks * nl + 4096 * (take.size() + 1) > S->cfg.memory_budget && !take.empty())
 					break;
-				maxslab = nm;
-				reserve = need;
+				least = nl;
+				most = std::max(most, r->slab);
 				take.push_back(r);
 				S->small_q.pop_front();
 			}
+			// slabs for all where there is room: shared memory can then be sized by what meshes are expected
+			// to need, for more CTAs per SM
+			const size_t blocks = std::min<size_t>(take.size(), size_t(S->sms) * 4), fixed = 4096 * take.size();
+			ts.batch_slab_limit = blocks * (S->reserved + blocks * most + fixed <= S->cfg.memory_budget ? most : least);
+			reserve = ts.batch_slab_limit + fixed;
 			S->reserved += reserve;
 			S->peak_reserved = std::max(S->peak_reserved, S->reserved);
 			S->inflight += take.size();
@@ -1970,7 +1998,9 @@ long long meshoptgpu_serverSubmit(meshoptgpu_Server* server, const meshoptgpu_Ba
 	// memory or a global slab); larger ones, and the options the batch kernel does not have,
 	// take the multi-CTA single-mesh path
 	bool large = S->cfg.plain || mesh->index_count > S->cfg.large_index_count || (mesh->options & ~kBatchOptions);
-	r->reserve = large ? Simplifier::workspaceBytes(mesh->index_count, mesh->vertex_count, r->desc.ac) : batchReserve(*r, S->cfg.memory_budget);
+	if (!large)
+		r->slab = batchBytes(r->desc, batchNarrow(r->desc)).slab;
+	r->reserve = large ? Simplifier::workspaceBytes(mesh->index_count, mesh->vertex_count, r->desc.ac) : batchReserve(r->slab);
 	if (r->reserve > S->cfg.memory_budget)
 	{
 		setStatus(meshoptgpu_StatusOutOfMemory, "request needs more device scratch than the server's memory budget");

@@ -98,6 +98,35 @@ assert mg.tuning(len(lean[0]["indices"]))["batch_smem_kib"] in (54, 110, 216)
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("budget", [8 << 10, 16 << 10, 200 << 10, 4 << 20])
+def test_server_budget_bounds_what_it_holds(port, budget):
+    """Requests that shared memory holds whatever they need hold no slab where the budget has no room for
+    one, and go on together; one that may need a slab larger than the budget is refused."""
+    torch = pytest.importorskip("torch")
+    idx, pos = _grid(17, 17, 0.1, 3)
+    di, dp = torch.from_numpy(idx.view(np.int32)).cuda(), torch.from_numpy(pos).cuda()
+    # a sparse group may use a vertex per index
+    gi, gp = _grid(33, 33, 0.1, 5)
+    ga = torch.zeros(len(gp) * 8, dtype=torch.float32, device="cuda")
+    gd, gv = torch.from_numpy(gi.view(np.int32)).cuda(), torch.from_numpy(np.concatenate([gp] * 6)).cuda()
+    outs = [torch.empty(max(len(idx), len(gi)), dtype=torch.int32, device="cuda") for _ in range(60)]
+    torch.cuda.synchronize()
+    ref, ref_err = port.simplify("port", idx, pos, 300, 1.0, 0)
+    with mg.Server(memory_budget=budget) as srv:
+        tickets = [srv.submit(di.data_ptr(), len(idx), dp.data_ptr(), len(pos), 300, 1.0, 0, o.data_ptr()) for o in outs]
+        if budget < 1 << 20:
+            with pytest.raises(mg.SimplifyError) as e:
+                srv.submit(gd.data_ptr(), len(gi), gv.data_ptr(), len(gp) * 6, 300, 1.0, mg.SimplifySparse, outs[0].data_ptr(),
+                           d_attributes=ga.data_ptr(), attr_stride=32, weights=np.ones(8, np.float32))
+            assert e.value.status == mg.STATUS_OUT_OF_MEMORY
+        for t, o in zip(tickets, outs):
+            status, n, err, _ = srv.wait(t)
+            assert status == 0
+            assert np.array_equal(o[:n].cpu().numpy().view(np.uint32), ref)
+            assert err == ref_err
+        assert srv.stats()["peak_reserved"] <= budget
+
+
 def _ribbon(tris, seed):
     return _grid(tris // 2 + 1, 2, 0.1, seed)
 
