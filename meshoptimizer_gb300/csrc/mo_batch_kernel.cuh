@@ -55,6 +55,10 @@ constexpr unsigned int kSortKeys = 2560;  // values of sortKey
 // 510 triangles 1.17 / 1.12 / 1.07 / 1.00 / 1.02 / 1.01 ms; 2,048 groups of 1,024 triangles 1.92 / 1.89 /
 // 1.90 / 1.90 / 1.99 / 2.05 ms.
 constexpr unsigned int kWalk = 224;
+// Where a walk hands over to the rounds, if the stop rules let it come so far (most candidates' flips are
+// rejected). One mesh of 16,700 triangles that looks at 15,000 candidates in each of two passes to remove
+// 100 triangles: 14.7 ms with a walk to their end, 4.8 so.
+constexpr unsigned int kWalkEnd = 2 * kWalk;
 
 template <class IX>
 struct CtaWork
@@ -422,6 +426,7 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 	__shared__ unsigned int s_cap, s_count, s_trunc, s_done, s_errbits, s_stall;
 	__shared__ unsigned long long s_cut;
 	__shared__ unsigned int s_sums[3][33];
+	__shared__ unsigned int s_walk[4]; // sorted positions walked, and the stop rules' terms up to there
 
 	if (tid == 0)
 		s_flag = 0, s_stall = 0;
@@ -1115,12 +1120,12 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 			blockDigitPass<NT>(w.cerr, (const IX*)w.sort_tmp, w.order, C, 8, w.hist, red);
 		}
 		// perform (performEdgeCollapses :1498-1636). A pass that is expected to look at few candidates is
-		// walked in sorted order by one warp, four flip tests at a time; a longer one goes in block-level
-		// decision rounds: a candidate is decided once nothing earlier in sorted order can change its
-		// outcome (the rule of the multi-CTA path's performPass), over a window of sorted order that grows
-		// until the stop rules fire; the stop rules are a prefix scan of the decisions. A warp keeps the
-		// undecided ones of every NT / 32nd position, so a round needs two barriers only: marks are
-		// complete, decisions are complete.
+		// walked in sorted order by one warp, four flip tests at a time; a longer one, and what a walk has not
+		// come to by kWalkEnd, goes in block-level decision rounds: a candidate is decided once nothing earlier
+		// in sorted order can change its outcome (the rule of the multi-CTA path's performPass), over a window
+		// of sorted order that grows until the stop rules fire; the stop rules are a prefix scan of the
+		// decisions. A warp keeps the undecided ones of every NT / 32nd position, so a round needs two barriers
+		// only: marks are complete, decisions are complete.
 		typedef typename Pair2<IX>::Mark Mark;
 		constexpr unsigned int kTagShift = sizeof(Mark) * 4;
 		constexpr Mark kFree = Mark(~0ull);
@@ -1162,13 +1167,15 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 		};
 		// the window a pass is expected to need
 		const unsigned int window = (unsigned int)min((unsigned long long)C, 2ull * (goal / 2) + 64ull);
+		if (tid == 0)
+			s_walk[0] = 0, s_walk[1] = 0, s_walk[2] = 0, s_walk[3] = __float_as_uint(result_error);
 		if (window <= kWalk)
 		{
 			if (warp == 0)
 			{
-				unsigned int T = 0, F = 0, M = __float_as_uint(result_error);
+				unsigned int T = 0, F = 0, M = __float_as_uint(result_error), base = 0;
 				bool stopped = false;
-				for (unsigned int base = 0; base < C && !stopped; base += 32)
+				for (; base < min(C, kWalkEnd) && !stopped; base += 32)
 				{
 					unsigned int i0 = 0, i1 = 0, r0 = 0, r1 = 0, eb = 0;
 					if (base + lane < C)
@@ -1279,10 +1286,12 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 						__syncwarp();
 					}
 				}
+				if (lane == 0)
+					s_walk[0] = stopped ? C : base, s_walk[1] = T, s_walk[2] = F, s_walk[3] = M;
 			}
-			__syncthreads();
 		}
-		else
+		__syncthreads();
+		if (s_walk[0] < C)
 		{
 			// rounds are numbered within the pass, which sets all marks free: a pass has at most a round per
 			// candidate, and later rounds' tags are smaller
@@ -1293,8 +1302,8 @@ __device__ bool simplifyMesh(const BatchDesc& d, BatchResult* out, Region mem, R
 				atomicMin(&w.minT[r1], m);
 				atomicMin(&w.minS[r0], m);
 			};
-			unsigned int carryT = 0, carryF = 0, carryM = __float_as_uint(result_error);
-			unsigned int K0 = 0, K1 = min(C, max(window, (unsigned int)NT));
+			unsigned int carryT = s_walk[1], carryF = s_walk[2], carryM = s_walk[3];
+			unsigned int K0 = s_walk[0], K1 = min(C, max(max(window, 2 * K0), (unsigned int)NT));
 			for (;;)
 			{
 				// the warp's undecided candidates: beyond 32 a list in the warp's share of sort_tmp, then one per lane

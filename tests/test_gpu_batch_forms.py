@@ -192,3 +192,61 @@ T._same(oracle, ms[:20], res[:20])
     r = subprocess.run([sys.executable, "-c", code % (here, root, os.path.join(root, "oracle"), tris, attributes)], capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def _stars(count):
+    """A lattice of 1,682 triangles, and flat stars whose centres cannot move anywhere: ten candidates each of
+    no error, all of whose flips are rejected before the lattice's candidates are looked at."""
+    idx, pos = _grid(30, 30, 0.3, 1)
+    a = np.arange(10) * np.pi / 5
+    rad = np.where(np.arange(10) % 2, 0.15, 1.0)
+    ring = np.concatenate([[[0, 0, 0]], np.stack([rad * np.cos(a), rad * np.sin(a), 0 * a], 1)])
+    fan = np.stack([np.zeros(10, int), 1 + np.arange(10), 1 + (np.arange(10) + 1) % 10], 1).reshape(-1)
+    centre = np.stack([np.arange(count) % 64 * 3.0, np.arange(count) // 64 * 3.0, np.full(count, 5.0)], 1)
+    si = (np.arange(count)[:, None] * 11 + fan[None]).reshape(-1) + len(pos)
+    sp = (centre[:, None] + ring[None]).reshape(-1, 3)
+    return np.concatenate([idx, si]).astype(np.uint32), np.concatenate([pos, sp]).astype(np.float32)
+
+
+@pytest.mark.parametrize("threads,smem_kb", [(128, 54), (256, 110), (512, 216)])
+@pytest.mark.parametrize("count", [10, 22, 41, 42, 45, 60, 300])
+def test_walks_that_hand_over(port, count, threads, smem_kb):
+    """Passes that are walked in sorted order and end before, at and after the position where the rounds take
+    over (448), with the stop rules' terms carried over."""
+    idx, pos = _stars(count)
+    opt = mg.SimplifyErrorAbsolute | mg.SimplifyLockBorder
+    ms = [dict(indices=idx, positions=pos, target=len(idx) - 3 * goal, error=err, options=opt)
+          for goal in (1, 10, 40, 100, 150, 160) for err in (1e9, 0.05)]
+    mg.set_batch_config(threads, smem_kb * 1024)
+    try:
+        res = mg.simplify_batch(ms)
+    finally:
+        mg.set_batch_config(0)
+    _same(port, ms, res)
+
+
+def test_walk_costs_no_more_than_rounds():
+    """15,000 rejected candidates before the first that counts, with a goal that is walked (100 triangles) and
+    one that goes in rounds (200): the kernel's times are alike (a walk to the end took several times more)."""
+    torch = pytest.importorskip("torch")
+    idx, pos = _stars(1500)
+    di, dp = torch.from_numpy(idx.view(np.int32)).cuda(), torch.from_numpy(pos).cuda()
+    out = torch.empty_like(di)
+    times = {}
+    mg.set_batch_config(256, 110 * 1024)
+    try:
+        for goal in (100, 200):
+            d = mg.BatchDescriptors([dict(d_indices=di.data_ptr(), index_count=len(idx), d_positions=dp.data_ptr(), vertex_count=len(pos),
+                                          target=len(idx) - 3 * goal, error=1e9, options=mg.SimplifyErrorAbsolute | mg.SimplifyLockBorder,
+                                          d_destination=out.data_ptr())])
+            for _ in range(2):
+                mg.simplify_batch_device(d)
+            mg.set_kernel_profile("kBatch")
+            for _ in range(5):
+                mg.simplify_batch_device(d)
+            n, ms = mg.kernel_profile()
+            mg.set_kernel_profile(None)
+            times[goal] = ms / n
+    finally:
+        mg.set_batch_config(0)
+    assert times[100] < 1.25 * times[200], times
