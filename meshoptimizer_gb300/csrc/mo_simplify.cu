@@ -3367,17 +3367,18 @@ __global__ void kComponentStarts(const unsigned int* __restrict__ sorted, size_t
 }
 
 // center = average position (sums in vertex order, as measureComponents), radius^2 = max
-// squared distance; one block of T threads per component over its vertices sorted by (component, index).
+// squared distance; a block of T threads for a component, over its vertices sorted by (component, index).
 // Bound by the sum's chain of dependent adds, one per vertex and axis: the block gathers a tile of
 // positions through shared memory while its threads 0-2 add the tile before it, one axis each, four
-// positions a load. A block of one warp where components are small (many of them share an SM), of 256
-// threads where they have kMeasureWide vertices or more on average (few tiles, gathered faster).
+// positions a load. A block of one warp for small components (many of them share an SM), of 256 threads for
+// those of kMeasureWide vertices or more (few tiles, gathered faster).
 // A 188k-triangle scan of 23 pieces, whole call: one thread per component, with two dependent loads per
 // vertex, 4.19 ms; a warp, 2.12 (163 us in this kernel, of 1.27 ms since other steps); a block, and the
-// starts from the sorted list where they were counted with atomics, 1.13.
-constexpr size_t kMeasureWide = 512;
+// starts from the sorted list where they were counted with atomics, 1.13. A piece of 90,000 vertices among
+// 3,000 / 60,000 specks: whole calls 1.66 ms by one warp, 1.33 and 1.37 by a block.
+constexpr unsigned int kMeasureWide = 512;
 template <unsigned int T>
-__global__ void __launch_bounds__(T) kMeasureComponents(const unsigned int* __restrict__ off, const unsigned int* __restrict__ verts,
+__device__ __forceinline__ void measureComponent(unsigned int component, const unsigned int* __restrict__ off, const unsigned int* __restrict__ verts,
     const float4* __restrict__ pos, float* __restrict__ err)
 {
 	constexpr unsigned int kMeasureThreads = T, kMeasureItems = T == 32 ? 8 : 4; // positions of a tile per thread
@@ -3385,7 +3386,7 @@ __global__ void __launch_bounds__(T) kMeasureComponents(const unsigned int* __re
 	__shared__ float4 tile[2][3][kTile / 4];
 	__shared__ float s_center[3], s_far[kMeasureThreads / 32];
 	const unsigned int tid = threadIdx.x;
-	const unsigned int b = off[blockIdx.x], e = off[blockIdx.x + 1];
+	const unsigned int b = off[component], e = off[component + 1];
 	float4 p[kMeasureItems];
 	auto gather = [&](unsigned int base) {
 		unsigned int v[kMeasureItems];
@@ -3462,7 +3463,41 @@ __global__ void __launch_bounds__(T) kMeasureComponents(const unsigned int* __re
 	{
 		for (unsigned int q = 1; q < kMeasureThreads / 32; ++q)
 			r2 = fmaxf(r2, s_far[q]);
-		err[blockIdx.x] = r2;
+		err[component] = r2;
+	}
+}
+
+// one component per block; in blocks of a warp, those of kMeasureWide vertices or more are left to
+// kMeasureWideComponents
+template <unsigned int T>
+__global__ void __launch_bounds__(T) kMeasureComponents(const unsigned int* __restrict__ off, const unsigned int* __restrict__ verts,
+    const float4* __restrict__ pos, float* __restrict__ err)
+{
+	if (T == 32 && off[blockIdx.x + 1] - off[blockIdx.x] >= kMeasureWide)
+		return;
+	measureComponent<T>(blockIdx.x, off, verts, pos, err);
+}
+
+// the components of kMeasureWide vertices or more, wherever they are among the others: a block looks
+// through every gridDim.x-th component, so that neighbouring ones go to different blocks
+__global__ void __launch_bounds__(256) kMeasureWideComponents(const unsigned int* __restrict__ off, size_t count, const unsigned int* __restrict__ verts,
+    const float4* __restrict__ pos, float* __restrict__ err)
+{
+	__shared__ unsigned int found, wide[256];
+	for (size_t base = 0; base * gridDim.x + blockIdx.x < count; base += 256)
+	{
+		if (threadIdx.x == 0)
+			found = 0;
+		__syncthreads();
+		const size_t c = (base + threadIdx.x) * gridDim.x + blockIdx.x;
+		if (c < count && off[c + 1] - off[c] >= kMeasureWide)
+			wide[atomicAdd(&found, 1u)] = (unsigned int)c;
+		__syncthreads();
+		for (unsigned int i = 0; i < found; ++i)
+		{
+			measureComponent<256>(wide[i], off, verts, pos, err);
+			__syncthreads(); // its shared memory is the next one's
+		}
 	}
 }
 
@@ -4095,10 +4130,16 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 		comp_count = hs->dup_count;
 		radixSortPairs(w.comp, nullptr, w.keys_a, w.vals_a, w.keys_b, w.vals_b, V, bitsFor(comp_count ? comp_count - 1 : 0), w.scratch, stream, ss);
 		MO_LAUNCH(kComponentStarts, gV, kThreads, 0, stream, w.keys_a, V, comp_count, w.comp_off);
+		// few components with less than kMeasureWide vertices where that is their average: blocks of 256 for all
 		if (V >= comp_count * kMeasureWide)
 			MO_LAUNCH(kMeasureComponents<256>, unsigned(comp_count), 256, 0, stream, w.comp_off, w.vals_a, w.pos, w.comp_err);
 		else
+		{
 			MO_LAUNCH(kMeasureComponents<32>, unsigned(comp_count), 32, 0, stream, w.comp_off, w.vals_a, w.pos, w.comp_err);
+			if (V >= kMeasureWide)
+				MO_LAUNCH(kMeasureWideComponents, unsigned(std::min<size_t>(comp_count, size_t(sms_) * 2)), 256, 0, stream, w.comp_off, comp_count, w.vals_a, w.pos,
+				    w.comp_err);
+		}
 	}
 	MO_CUDA_CHECK(cudaGetLastError());
 

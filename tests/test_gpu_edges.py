@@ -353,3 +353,43 @@ def test_first_window_of_a_plane(port, single_path, ratio):
     assert err == ref_err
     goal = (len(idx) - target) // 3
     assert mg.last_round_trace()[0][0] <= min(2 * goal + 4096, mg.last_pass_stats()[0]["candidates"])
+
+
+@pytest.mark.parametrize("sizes", [(510,) + (4,) * 400, (512,) + (4,) * 400, (4,) * 400 + (514, 4, 4000), (600,) * 40 + (4,) * 700, (4,) * 127], ids=lambda s: f"{len(s)}x{max(s)}")
+def test_prune_wide_among_small(port, sizes):
+    """Large components among many small ones: each is measured by the block its own size asks for."""
+    idx, pos = _strips(sizes, len(sizes))
+    opt = mg.SimplifyPrune | mg.SimplifyLockBorder
+    for target in (0, W.target_count(len(idx), 0.5)):
+        for error in (1e-2, 1e-1):
+            ref, ref_err = port.simplify("port", idx, pos, target, error, opt)
+            out, err = mg.simplify(idx, pos, target, error, opt)
+            assert np.array_equal(out, ref)
+            assert err == ref_err
+
+
+def test_prune_large_component_among_specks():
+    """A body's radius takes about as long with thousands of specks around it as alone."""
+    torch = pytest.importorskip("torch")
+    idx, pos = _grid(300, 300, 0.05, 3)
+    speck = np.array([0, 1, 2, 2, 1, 3])
+    corner = np.array([[0, 0, 0], [0.1, 0, 0], [0, 0.1, 0], [0.1, 0.1, 0]])
+    times = {}
+    for count in (0, 3000):
+        si = (np.arange(count)[:, None] * 4 + speck[None]).reshape(-1) + len(pos)
+        sp = (np.random.default_rng(3).random((count, 1, 3)) * 300 + corner[None]).reshape(-1, 3)
+        di = torch.from_numpy(np.concatenate([idx, si]).astype(np.uint32).view(np.int32)).cuda()
+        dp = torch.from_numpy(np.concatenate([pos, sp]).astype(np.float32)).cuda()
+        out = torch.empty_like(di)
+
+        def call():
+            mg.simplify_device(out.data_ptr(), di.data_ptr(), len(di), dp.data_ptr(), len(dp), 12, len(idx) // 12 * 3, 1e-2,
+                               mg.SimplifyPrune | mg.SimplifyLockBorder)
+
+        call()
+        mg.set_kernel_profile("kMeasure")
+        for _ in range(5):
+            call()
+        times[count] = mg.kernel_profile()[1]
+        mg.set_kernel_profile(None)
+    assert times[3000] < 1.3 * times[0], times
