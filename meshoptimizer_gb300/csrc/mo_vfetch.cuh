@@ -12,7 +12,7 @@ namespace mogpu
 size_t vertexOrderScratchWords(size_t index_count, size_t vertex_count);
 
 // order[v] = new index of vertex v in order of first use by indices; mark_unused: ~0u if unused (else
-// left as it is). The scratch keeps the vertices in their new order (vertexOrderList). counters: 5
+// left as it is, and the scratch keeps the vertices in their new order, vertexOrderList). counters: 5
 // device words, read by takeOrderCount.
 void vertexOrder(unsigned int* order, bool mark_unused, const unsigned int* indices, size_t index_count, size_t vertex_count, unsigned int* scratch,
     unsigned int* counters, cudaStream_t stream);

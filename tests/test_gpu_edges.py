@@ -393,3 +393,26 @@ def test_prune_large_component_among_specks():
         times[count] = mg.kernel_profile()[1]
         mg.set_kernel_profile(None)
     assert times[3000] < 1.3 * times[0], times
+
+
+@pytest.mark.parametrize("corners", [608 * 1024 * 2 + 3, 608 * 1024 * 16 + 1023, 608 * 1024 * 17 + 1026])
+def test_compaction_many_tiles(corners):
+    """Several tiles per block of the vertex order, around the 16 whose first uses a block keeps."""
+    torch = pytest.importorskip("torch")
+    corners = corners // 3 * 3
+    vc = 500_003
+    g = torch.Generator(device="cuda").manual_seed(corners)
+    di = torch.randint(0, vc, (corners,), generator=g, dtype=torch.int32, device="cuda")
+    src = torch.arange(vc, dtype=torch.int32, device="cuda")
+    # the first position of every vertex, and its rank among them
+    first = torch.full((vc,), corners, dtype=torch.int64, device="cuda").scatter_reduce_(0, di.long(), torch.arange(corners, device="cuda"), "amin")
+    used = first < corners
+    want = torch.full((vc,), -1, dtype=torch.int32, device="cuda")
+    want[torch.argsort(first)[: int(used.sum())]] = torch.arange(int(used.sum()), dtype=torch.int32, device="cuda")
+    remap = torch.zeros(vc, dtype=torch.int32, device="cuda")
+    assert mg.optimize_vertex_fetch_remap_device(remap.data_ptr(), di.data_ptr(), corners, vc) == int(used.sum())
+    assert torch.equal(remap, want)
+    dst, new = torch.full_like(src, -7), di.clone()
+    assert mg.optimize_vertex_fetch_device(dst.data_ptr(), new.data_ptr(), corners, src.data_ptr(), vc, 4) == int(used.sum())
+    assert torch.equal(new, want[di.long()])
+    assert torch.equal(dst[: int(used.sum())], torch.argsort(first)[: int(used.sum())].int()) and bool((dst[int(used.sum()):] == -7).all())
