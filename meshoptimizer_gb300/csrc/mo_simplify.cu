@@ -3818,6 +3818,11 @@ Simplifier::Simplifier(int device) : device_(device)
 // kPassLoop.
 constexpr size_t kOnePerSmMax = 1000000;
 
+// The pass loop's blocks at least: a mesh of a few triangles still has 2,560 sort bins in 80 groups a pass.
+// Calls on 5^2 / 8^2 / 12^2 quads in us with one block 512 / 640 / 489, 4: 350 / 435 / 442, 8: 325 / 400 /
+// 417, 16: 317 / 400 / 415, 32: 312 / 387 / 405.
+constexpr unsigned int kMinPassBlocks = 32;
+
 int Simplifier::passBlocksPerSM(size_t index_count) const
 {
 	if (tuning_.perform_blocks_per_sm > 0)
@@ -4279,7 +4284,7 @@ RunResult Simplifier::run(const MeshDesc& m, unsigned int* d_out, cudaStream_t s
 	// the grid of the pass kernels for up to n items in a phase
 	const int per_sm = passBlocksPerSM(I);
 	auto performGrid = [&](size_t n) {
-		unsigned int blocks = std::max(1u, std::min(unsigned(per_sm * sms_), gridFor(n, kPerformThreads)));
+		unsigned int blocks = std::min(unsigned(per_sm * sms_), std::max(kMinPassBlocks, gridFor(n, kPerformThreads)));
 		if (tuning_.perform_grid_cap > 0)
 			blocks = std::min(blocks, performGridCap());
 		if (size_t(blocks) * kPerformThreads > kListSlack)

@@ -416,3 +416,26 @@ def test_compaction_many_tiles(corners):
     assert mg.optimize_vertex_fetch_device(dst.data_ptr(), new.data_ptr(), corners, src.data_ptr(), vc, 4) == int(used.sum())
     assert torch.equal(new, want[di.long()])
     assert torch.equal(dst[: int(used.sum())], torch.argsort(first)[: int(used.sum())].int()) and bool((dst[int(used.sum()):] == -7).all())
+
+
+def test_small_mesh_takes_no_longer(single_path):
+    """A mesh of 128 triangles on the single-mesh path against one of 2,048: a pass has work that does not
+    shrink with the mesh, which more than one block shares."""
+    torch = pytest.importorskip("torch")
+    times = {}
+    for nx in (9, 33):
+        idx, pos = _grid(nx, nx, 0.05, 3)
+        di, dp = torch.from_numpy(idx.view(np.int32)).cuda(), torch.from_numpy(pos).cuda()
+        out = torch.empty_like(di)
+
+        def call():
+            mg.simplify_device(out.data_ptr(), di.data_ptr(), len(di), dp.data_ptr(), len(dp), 12, len(idx) // 12 * 3, 1e-2, 0)
+
+        call()
+        call()
+        mg.set_kernel_profile("kPassLoop")
+        for _ in range(5):
+            call()
+        times[nx] = mg.kernel_profile()[1] / 5
+        mg.set_kernel_profile(None)
+    assert times[9] < 1.15 * times[33], times
