@@ -71,12 +71,13 @@ struct GridSum
 {
 	unsigned long long* word; // global, two words
 	unsigned int* err;
-	unsigned int* s;    // shared: [0], [1] the words' sums so far, [2] this barrier's total, [3] the error flag
+	unsigned int* s;    // shared, 16-byte aligned: [0], [1] the words' sums so far, [2] this barrier's total, [3] the error flag
 	unsigned int phase; // barriers passed
+	unsigned int bad;   // the error flag at the last one
 
 	__device__ void start(unsigned long long* w, unsigned int* e, unsigned int* sh)
 	{
-		word = w, err = e, s = sh, phase = 0;
+		word = w, err = e, s = sh, phase = 0, bad = 0;
 		if (threadIdx.x == 0)
 			s[0] = s[1] = s[2] = s[3] = 0;
 	}
@@ -92,7 +93,7 @@ struct GridSum
 			// once a wait has run out anywhere, barriers are arrived at and not waited for: a block that
 			// never comes costs the others one limit, not one for every barrier until they return. The
 			// flag's load is in flight during the first poll.
-			const unsigned int failed = s[3] | __ldcg(err);
+			const unsigned int failed = bad | __ldcg(err);
 			unsigned int spins = 0, out = 0;
 			for (;;)
 			{
@@ -117,11 +118,13 @@ struct GridSum
 		}
 		++phase;
 		__syncthreads();
-		return s[2];
+		const uint2 r = *reinterpret_cast<const uint2*>(s + 2);
+		bad = r.y;
+		return r.x;
 	}
 	// a wait has run out: what the barriers should have ordered is not to be read any more, and the block
 	// arrives at one more barrier at most (with two, it would complete the one that a slower block waits at)
-	__device__ __forceinline__ bool failed() const { return s[3] != 0; }
+	__device__ __forceinline__ bool failed() const { return bad != 0; }
 };
 
 // A grid barrier that a cooperative launch passes once, leaving its two words zero for the next

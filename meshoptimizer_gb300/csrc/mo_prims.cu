@@ -304,7 +304,7 @@ __global__ void kBarrierWaitProbe(unsigned int* words, unsigned int limit, int m
 		return;
 	if (mode == 2)
 	{
-		__shared__ unsigned int s_grid[4];
+		__shared__ __align__(16) unsigned int s_grid[4];
 		GridSum grid;
 		grid.start(reinterpret_cast<unsigned long long*>(words), words + 4, s_grid);
 		grid.wait(blockIdx.x, limit);

@@ -2521,7 +2521,7 @@ __global__ void __launch_bounds__(kPerformThreads, MO_PERFORM_MIN_BLOCKS) kPerfo
 	__shared__ unsigned int s_app[5];
 	__shared__ unsigned int s_stage[2][kStageChunk];
 	__shared__ unsigned int s_list[kStageChunk];
-	__shared__ unsigned int s_grid[4];
+	__shared__ __align__(16) unsigned int s_grid[4];
 	__shared__ long long s_clock[10];
 	__shared__ unsigned int sm[3][33];
 	Scalars* sc = a.sc;
@@ -2946,7 +2946,7 @@ __global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArg
 {
 	extern __shared__ __align__(16) unsigned char loop_smem[];
 	__shared__ unsigned int s_app[5];
-	__shared__ unsigned int s_grid[4];
+	__shared__ __align__(16) unsigned int s_grid[4];
 	__shared__ long long s_clock[10];
 	__shared__ unsigned int sm[3][33];
 	Scalars* sc = a.p.sc;
