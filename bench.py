@@ -39,10 +39,10 @@ sys.path.insert(0, ROOT)
 
 from meshoptimizer_gb300 import workloads as W  # noqa: E402
 
-# Algorithmic bytes of the dominant kernel, kPerform (one cooperative launch per pass): the
-# compulsory traffic of a pass, every array it must touch read (and written where it changes)
-# once, from the per-pass counters the library reports (T triangles of the pass, V vertices of
-# the buffer; a mesh of T triangles uses about T / 2 of them):
+# Algorithmic bytes of a pass from its ranked candidates to the next pass's index buffer (kPerform,
+# and the last phases of a pass in kPassLoop): the compulsory traffic, every array it must touch
+# read (and written where it changes) once, from the per-pass counters the library reports (T
+# triangles of the pass, V vertices of the buffer; a mesh of T triangles uses about T / 2 of them):
 #   candidate records  42 B per evaluated candidate (pick records 16 + 16, sorted position 4,
 #                      error bits 4, kind 1, decision 1): every candidate up to the stop cut
 #                      is decided
@@ -65,7 +65,22 @@ KPERFORM_BYTES_DEFINITION = ("kperform_bytes(): 42 B per evaluated candidate, 52
                              "144 B per commit + (144 + 48 a) B with a attributes")
 
 
-# Per-pass byte model of the whole pass (attribute path included), for the per-phase GB/s of
+# Algorithmic bytes of a whole pass in kPassLoop, the dominant kernel (one cooperative launch for all
+# passes): 64 B per triangle before perform (corner slots written and read 24, indices 12, adjacency
+# written 24, pick codes written and read 4), 8 B per vertex (list starts and counts), 81 B per
+# candidate (picked 16, ranked 16 read and 32 written, sorted 8 read and 9 written), the rows of the
+# used vertices that rank reads (pass_phase_bytes), and perform's.
+def passloop_bytes(p, vertices, next_triangles, attributes=0):
+    T = p["triangles"]
+    rows = 77 + (48 + 20 * attributes if attributes else 0)
+    return 64 * T + 8 * vertices + 81 * p["candidates"] + rows * (T // 2) + kperform_bytes(p, vertices, next_triangles, attributes)
+
+
+PASSLOOP_BYTES_DEFINITION = ("passloop_bytes(), summed over the launch's passes: kperform_bytes() and 64 B per triangle, 8 B per vertex, 81 B per "
+                             "candidate, 77 + 48 + 20 a B per used vertex (a attributes; 77 without)")
+
+
+# Per-pass byte model of the host-driven loop's phases (attribute path included), for the per-phase GB/s of
 # the stress line: adjacency 12 B per input triangle (indices) + 24 B per triangle (corner records
 # written) + 8 B per vertex (counts and offsets); pick 12 B per triangle + 12 B per candidate
 # written; rank 12 B per candidate read + 37 B per candidate written + the rows of the used
@@ -739,11 +754,12 @@ def bench_single(args, mg, torch, c, dist=None, world=1, rank=0, local=0, roofli
     launches = mg.launch_count() - launches0
     total_ms = sum(a.elapsed_time(b) for a, b in ev)
 
-    # per-launch CUDA-event timing of the roofline kernel: the same steps replayed with the
-    # host-driven pass loop (the device-resident loop is one launch)
-    k_launches = k_ms = host_loop_ms = 0
+    # per-launch CUDA-event timing of the roofline kernel: the same steps replayed (kPassLoop is one launch
+    # per step; the kernels of the host-driven pass loop need that loop)
+    k_launches = k_ms = replay_ms = 0
+    in_loop = args.kernel.startswith("kPassLoop")
     if roofline:
-        mg.set_device_loop(False)
+        mg.set_device_loop(in_loop)
         step()
         mg.set_kernel_profile(args.kernel)
         kev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
@@ -756,7 +772,7 @@ def bench_single(args, mg, torch, c, dist=None, world=1, rank=0, local=0, roofli
         k_launches, k_ms = mg.kernel_profile()
         mg.set_kernel_profile(None)
         mg.set_device_loop(True)
-        host_loop_ms = sum(a.elapsed_time(b) for a, b in kev)
+        replay_ms = sum(a.elapsed_time(b) for a, b in kev)
     from meshoptimizer_gb300 import replicas
 
     rate, secs, _ = replicas.aggregate(total_ms / 1e3, float(c["tris"] * args.steps), dist=dist, device=dev)
@@ -764,13 +780,15 @@ def bench_single(args, mg, torch, c, dist=None, world=1, rank=0, local=0, roofli
     value = rate / 1e6
     gpu_out = out[:n_out].cpu().numpy().view(np.uint32)
 
-    # per-pass and per-phase view of one more run (not timed for the value)
+    # the passes and rounds of one more step, and the phases of one with the host-driven loop (not timed for
+    # the value)
+    step()
+    passes = mg.last_pass_stats()
+    trace = mg.last_round_trace()
     mg.set_timing(True)
     step()
     phases = mg.last_phase_times()
-    passes = mg.last_pass_stats()
     pass_phases = mg.last_pass_phase_times()
-    trace = mg.last_round_trace()
     mg.set_timing(False)
 
     # end to end through the drop-in C ABI with pinned host buffers
@@ -841,16 +859,17 @@ def bench_single(args, mg, torch, c, dist=None, world=1, rank=0, local=0, roofli
     nxt = [p["triangles"] for p in passes[1:]] + [int(n_out) // 3]
     if k_launches:
         avg_ms = k_ms / k_launches
-        bytes_run = sum(kperform_bytes(p, V, t, ac_used) for p, t in zip(passes, nxt))
-        bytes_per_launch = bytes_run / max(len(passes), 1)
+        of_pass = passloop_bytes if in_loop else kperform_bytes
+        bytes_run = sum(of_pass(p, V, t, ac_used) for p, t in zip(passes, nxt))
+        bytes_per_launch = bytes_run / (1 if in_loop else max(len(passes), 1))
         achieved = bytes_per_launch / (avg_ms / 1e3) / 1e9 if avg_ms > 0 else 0
         roof = {"bound": "hbm", "kernel": args.kernel, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "peak_source": peak_kind, "traffic": None,
                 "avg_launch_us": round(1e3 * avg_ms, 2), "launches": k_launches,
-                "algorithmic_bytes_per_launch": int(bytes_per_launch), "unit_definition": KPERFORM_BYTES_DEFINITION,
-                "share_of_step": round(k_ms / host_loop_ms, 4) if host_loop_ms else None,
-                "kernel_timing": "CUDA events around every launch on its stream, over the same steps replayed with the host-driven "
-                                 "pass loop (the timed steps run the device-resident loop, one launch for all passes)"}
+                "algorithmic_bytes_per_launch": int(bytes_per_launch), "unit_definition": PASSLOOP_BYTES_DEFINITION if in_loop else KPERFORM_BYTES_DEFINITION,
+                "share_of_step": round(k_ms / replay_ms, 4) if replay_ms else None,
+                "kernel_timing": "CUDA events around every launch on its stream, over the same steps replayed" +
+                                 ("" if in_loop else " with the host-driven pass loop (the timed steps run all passes in one launch)")}
         tr = kernel_traffic(args.kernel, c["name"])
         if tr:
             roof["traffic"] = tr["dram_bytes_per_launch"]
@@ -874,10 +893,10 @@ def bench_single(args, mg, torch, c, dist=None, world=1, rank=0, local=0, roofli
         "config": {"workload": c["name"], "input_tris": c["tris"], "output_tris": int(n_out) // 3, "target_index_count": c["target"],
                    "target_error": c["error"], "options": c["options"], "attributes": ac, "result_error": err,
                    "l2": "flushed between steps (512 MiB write, outside the timed events)", "parallelism": f"replicas{world}",
-                   "autotuned": {"perform_blocks_per_sm": tuned["perform_blocks_per_sm"], "sort_items_per_thread": tuned["sort_items"]}},
+                   "autotuned": {"perform_blocks_per_sm": tuned["perform_blocks_per_sm"]}},
         "e2e": e2e, "roofline": roof, "cpu_baseline": cpu, "bit_exact_vs_oracle": bit_exact, "error_vs_fp64_oracle": fp64,
         "clocks": clocks.summary(), "gpu_launches": int(launches),
-        "phases_ms": {k: round(v, 3) for k, v in phases.items()},
+        "phases_ms": {k: round(v, 3) for k, v in phases.items()}, "phases_of": "one step with the host-driven pass loop, a launch per phase",
         "passes": [{k: p[k] for k in ("triangles", "candidates", "evaluated", "done", "rounds", "active", "windows")} for p in passes],
         "round_trace_us": [[n, round(t, 1)] for n, t in trace[:64]],
     }
@@ -905,7 +924,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="gb300", choices=["gb300", "reference"])
     ap.add_argument("--workload", default="sphere_attr_2m", choices=sorted(WORKLOADS))
-    ap.add_argument("--kernel", default="kPerform", help="kernel whose CUDA-event time gives the roofline line")
+    ap.add_argument("--kernel", default="kPassLoop", help="kernel whose CUDA-event time gives the roofline line (kPassLoop, or kPerform of the host-driven pass loop)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-extras", action="store_true", help="skip the groups, serving, cluster-LOD and heightfield summaries of the default line")
