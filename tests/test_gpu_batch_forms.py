@@ -250,3 +250,72 @@ def test_walk_costs_no_more_than_rounds():
     finally:
         mg.set_batch_config(0)
     assert times[100] < 1.25 * times[200], times
+
+
+def _odd_values(kind, nx, ny, seed):
+    """A lattice some of whose errors are not finite: attributes that are infinite, whose squares overflow or
+    that are NaN, or positions that are NaN."""
+    rng = np.random.default_rng(seed)
+    idx, pos = _grid(nx, ny, 0.1, seed)
+    attr = rng.standard_normal((len(pos), 3)).astype(np.float32)
+    at = rng.permutation(len(pos))[: max(1, len(pos) // 9)]
+    value = {"inf": np.inf, "huge": 1e25, "nan": np.nan, "mixed": np.nan, "nan_position": 0.0, "all_inf": np.inf}[kind]
+    if kind == "nan_position":
+        pos[at[: max(1, len(at) // 4)], 1] = np.nan
+    elif kind == "all_inf":
+        attr[:] = rng.choice([-np.inf, np.inf], attr.shape)
+    else:
+        attr[at, rng.integers(0, 3, len(at))] = value
+        if kind == "mixed":
+            attr[at[::2], 0], attr[at[1::3], 1] = np.inf, -1e25
+    return dict(indices=idx, positions=pos, attributes=attr, weights=np.array([0.5, 1.0, 0.25], np.float32))
+
+
+ODD = ["inf", "huge", "nan", "mixed", "nan_position", "all_inf"]
+
+
+@pytest.mark.parametrize("threads,smem_kb", [(128, 54), (256, 110), (512, 216), (256, 2)])
+@pytest.mark.parametrize("kind", ODD)
+def test_odd_values_in_batches(port, kind, threads, smem_kb):
+    """Infinite and NaN errors in the walk, the rounds, the stop rules and the sort."""
+    ms = []
+    for nx, ny in ((3, 3), (9, 8), (17, 17), (26, 23)):
+        m = _odd_values(kind, nx, ny, nx)
+        tris = len(m["indices"]) // 3
+        for removed in sorted({1, tris // 4, min(150, tris // 2), tris // 2, tris}):
+            for error in (1e-2, 3e38, np.inf):
+                for opt in (0, mg.SimplifyErrorAbsolute):
+                    ms.append(dict(m, target=3 * (tris - removed), error=error, options=opt))
+    mg.set_batch_config(threads, smem_kb * 1024)
+    try:
+        res = mg.simplify_batch(ms)
+    finally:
+        mg.set_batch_config(0)
+    for i, (m, (out, err)) in enumerate(zip(ms, res)):
+        ref, ref_err = port.simplify("port", m["indices"], m["positions"], m["target"], m["error"], m["options"], attributes=m["attributes"],
+                                     weights=m["weights"])
+        assert np.array_equal(out, ref), f"mesh {i}"
+        assert err == ref_err or (np.isnan(err) and np.isnan(ref_err)), f"mesh {i}"
+
+
+@pytest.mark.parametrize("kind", ODD)
+def test_odd_values_in_the_pass_loop(port, kind):
+    """The same on the single-mesh path, whose first window is predicted from the errors."""
+    mg.set_dropin_batch_limit(0)
+    try:
+        for nx, ny in ((9, 8), (40, 37), (120, 97)):
+            m = _odd_values(kind, nx, ny, nx)
+            tris = len(m["indices"]) // 3
+            for removed in (tris // 50 + 1, tris // 2, tris):
+                for error in (1e-2, np.inf):
+                    for prune in (0, mg.SimplifyPrune):
+                        if prune and kind == "nan_position":
+                            continue
+                        target = 3 * (tris - removed)
+                        ref, ref_err = port.simplify("port", m["indices"], m["positions"], target, error, prune, attributes=m["attributes"],
+                                                     weights=m["weights"])
+                        out, err = mg.simplify(m["indices"], m["positions"], target, error, prune, attributes=m["attributes"], weights=m["weights"])
+                        assert np.array_equal(out, ref)
+                        assert err == ref_err or (np.isnan(err) and np.isnan(ref_err))
+    finally:
+        mg.set_dropin_batch_limit()
