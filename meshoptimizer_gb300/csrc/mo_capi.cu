@@ -719,6 +719,12 @@ BatchDesc makeDesc(const meshoptgpu_BatchMesh& m, const unsigned int* indices, c
 	return d;
 }
 
+// whether a mesh's output leaves its indices as they are, so that the call can be repeated
+bool apart(const unsigned int* out, const unsigned int* indices, size_t index_count)
+{
+	return std::less_equal<const unsigned int*>()(out + index_count, indices) || std::less_equal<const unsigned int*>()(indices + index_count, out);
+}
+
 // Runs descs (device pointers) through the persistent kernel; results in the same order.
 // attr_of[i] indexes maps.maps for descs[i] (-1: none).
 // Meshes whose ids need 32 bits run in a launch of their own, beside the others': that form has no
@@ -764,14 +770,16 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		size_t slab, max_index_count;
 		int threads;
 		size_t budget;
-		bool sure;
-	} parts[2] = {{0, wide, false, false, 0, 0, 0, 0, false}, {wide, n - wide, true, false, 0, 0, 0, 0, false}};
+		bool sure, repeatable;
+	} parts[2] = {{0, wide, false, false, 0, 0, 0, 0, false, true}, {wide, n - wide, true, false, 0, 0, 0, 0, false, true}};
 	for (Part& p : parts)
 		for (size_t i = p.first; i < p.first + p.count; ++i)
 		{
 			ordered[i] = descs[perm[i]];
 			bytes[i] = batchBytes(ordered[i], p.narrow);
 			p.full = p.full || batchNeedsFull(ordered[i]);
+			const BatchDesc& d = ordered[i]; // in place: its indices are its output after a launch
+			p.repeatable = p.repeatable && apart(d.out, d.indices, d.index_count);
 			p.slab = std::max(p.slab, bytes[i].slab);
 			p.max_index_count = std::max<size_t>(p.max_index_count, ordered[i].index_count);
 		}
@@ -865,7 +873,7 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 			continue; // the 32-bit form has one shape
 		// the block size and the shared-memory budget the caller left open are autotuned per size
 		// class: the first batch of a class times every candidate pair on its own meshes
-		// (identical results) and keeps the fastest
+		// (identical results; not with meshes simplified in place) and keeps the fastest
 		cls = std::make_tuple(s.device, sizeClass(p.max_index_count), p.count > size_t(sms), p.full);
 		BatchShapes shapes;
 		bool known = false;
@@ -919,14 +927,17 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 			cudaEventDestroy(e1);
 			return best;
 		};
-		if (!known && p.slab > limit) // no room for slabs: shapes cannot be told apart, and nothing is kept
+		// trials need meshes that a launch leaves as they are, and room for slabs: else the shape that is
+		// known, or the default, which is not kept
+		const bool trial = p.repeatable && p.slab <= limit;
+		if (!known && !trial)
 			continue;
 		if (!known)
 		{
 			shapes.as_expected = trials(false);
 			shapes.last_beyond = manyBeyond(readResults(p), p.count);
 		}
-		if (shapes.last_beyond && !shapes.timed_beyond && p.slab <= limit)
+		if (shapes.last_beyond && !shapes.timed_beyond && trial)
 		{
 			shapes.beyond = trials(true);
 			shapes.timed_beyond = true;
@@ -1055,7 +1066,7 @@ std::tuple<int, int, int> shapeKey(const ThreadState& s, const MeshDesc& m)
 
 bool repeatable(const ThreadState& s, const MeshDesc& m, const unsigned int* d_out)
 {
-	return s.autotune && !s.timing && static_cast<const void*>(d_out) != static_cast<const void*>(m.indices) &&
+	return s.autotune && !s.timing && apart(d_out, m.indices, m.index_count) &&
 	       !(m.options & (kOptPrune | kOptInternalDebug | kOptInternalSolve)) && m.index_count > m.target_index_count;
 }
 

@@ -319,3 +319,54 @@ def test_odd_values_in_the_pass_loop(port, kind):
                         assert err == ref_err or (np.isnan(err) and np.isnan(ref_err))
     finally:
         mg.set_dropin_batch_limit()
+
+
+@pytest.mark.parametrize("call", ["device", "batch", "groups"])
+def test_in_place_as_the_first_call(call):
+    """Destinations may alias indices, also in the first call of a size class, whose shapes would be timed on
+    its meshes (a process of its own)."""
+    code = """
+import sys
+sys.path[:0] = [%r, %r, %r]
+import numpy as np, torch
+import oracle
+import test_gpu_batch_forms as T
+import meshoptimizer_gb300 as mg
+
+call = %r
+idx, pos = T._grid(17, 13, 0.1, 1)
+target = len(idx) // 6 * 3
+dp = torch.from_numpy(pos).cuda()
+count = {"device": 1, "batch": 40, "groups": 40}[call]
+d = torch.from_numpy(np.tile(idx.view(np.int32), count)).cuda()
+opt = mg.SimplifySparse if call == "groups" else 0
+if call == "device":
+    n, err = mg.simplify_device(d.data_ptr(), d.data_ptr(), len(idx), dp.data_ptr(), len(pos), 12, target, 1.0)
+    counts, errs = [n], [err]
+elif call == "batch":
+    at = [d.data_ptr() + 4 * len(idx) * i for i in range(count)]
+    counts, errs = mg.simplify_batch_device([dict(d_indices=p, index_count=len(idx), d_positions=dp.data_ptr(), vertex_count=len(pos), target=target,
+                                                  error=1.0, d_destination=p) for p in at])
+else:
+    # every group uses every position, so all are locked but for one group's: one group, many separate vertex copies
+    posn = np.concatenate([pos + [0, 0, 50 * i] for i in range(count)]).astype(np.float32)
+    ii = np.concatenate([idx + len(pos) * i for i in range(count)]).astype(np.uint32)
+    d = torch.from_numpy(ii.view(np.int32)).cuda()
+    dp = torch.from_numpy(posn).cuda()
+    remap = torch.arange(len(posn), dtype=torch.int32, device="cuda")
+    locks = torch.zeros(len(posn), dtype=torch.uint8, device="cuda")
+    off = np.arange(count + 1) * len(idx)
+    counts, errs = mg.simplify_groups_device(d.data_ptr(), d.data_ptr(), off, dp.data_ptr(), len(posn), 12, remap.data_ptr(), locks.data_ptr(),
+                                             [target] * count, 1.0, 0)
+got = d.cpu().numpy().view(np.uint32)
+for i in range(count):
+    p, base = (pos, 0) if call != "groups" else (posn[len(pos) * i:len(pos) * (i + 1)], len(pos) * i)
+    ref, ref_err = oracle.simplify("port", idx, np.ascontiguousarray(p), target, 1.0, opt)
+    out = got[len(idx) * i:len(idx) * i + int(counts[i])]
+    assert np.array_equal(out, ref + np.uint32(base)), i
+    assert errs[i] == np.float32(ref_err), i
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    root = os.path.dirname(here)
+    r = subprocess.run([sys.executable, "-c", code % (here, root, os.path.join(root, "oracle"), call)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
