@@ -1902,8 +1902,8 @@ struct PhaseClock
 
 #ifndef MO_PERFORM_THREADS
 // threads per block of the pass kernel: fewer blocks arrive at each grid barrier. 256^2 heightfield /
-// 2M attribute sphere / 20M terrain in ms: 256 threads 0.76 / 4.04 / 38.7, 512 0.75 / 4.06 / 38.3,
-// 1024 (4 lanes x 2 corners) 0.81 / 4.33 / 38.7
+// 2M attribute sphere / 20M terrain in ms, with a launch per pass: 256 threads 0.76 / 4.04 / 38.7, 512
+// 0.75 / 4.06 / 38.3, 1024 (4 lanes x 2 corners) 0.81 / 4.33 / 38.7
 #define MO_PERFORM_THREADS 512
 #endif
 #ifndef MO_PERFORM_MIN_BLOCKS
@@ -2932,10 +2932,11 @@ __device__ __forceinline__ bool preparePass(const PassLoopArgs& a, const BlockTr
 }
 
 // PER_SM: resident blocks per SM it is compiled for (1: 128 registers, no spills; 2: twice the warps).
-// Whole calls with 1 / 2, in ms: heightfields of 40^2 0.56 / 0.58, 256^2 0.66 / 0.69, 400^2 0.84 / 0.84,
-// 560^2 1.15 / 1.08, 1100^2 3.25 / 2.61; attribute spheres of 131k triangles 1.18 / 1.21, 524k 2.25 /
-// 2.20, 2M 5.26 / 3.96; 20M terrain 46.3 / 35.9. A graph of per-phase kernels (recorded once, looping
-// on the device) took 0.63, 0.75, 0.90, 1.16, 2.64; 1.30, 2.36, 4.02; 36.4.
+// Whole calls with 1 / 2, in ms: heightfields of 40^2 0.36 / 0.38, 256^2 0.60 / 0.67, 400^2 0.77 / 0.78,
+// 560^2 1.08 / 1.00, 1100^2 3.12 / 2.41; attribute spheres of 131k triangles 0.82 / 0.90, 524k 1.91 /
+// 1.89, 2M 5.06 / 3.75; 20M terrain 42.1 / 31.8. (When it was written, and with a graph of per-phase
+// kernels in its place: 256^2 0.66 and 0.75, 1100^2 2.61 and 2.64, 2M sphere 3.96 and 4.02, terrain 35.9
+// and 36.4.)
 template <int PER_SM>
 __global__ void __launch_bounds__(kPerformThreads, PER_SM) kPassLoop(PassLoopArgs a)
 {
@@ -3173,7 +3174,7 @@ __device__ __forceinline__ bool solveRing(const SolveArgs& a, unsigned int i)
 // (a change always queues its readers), so the order inside a round does not matter.
 // Bound by the latency of a few grid-wide rounds. Waiting for lower neighbours to be final instead
 // took one round per link of the longest index-ordered chain, hundreds on a row-ordered
-// lattice: 131k-triangle globe, whole call 9.18 ms then, 1.46 ms now.
+// lattice: 131k-triangle globe, whole call 9.18 ms then, 1.46 ms so (0.94 with the steps since).
 __global__ void __launch_bounds__(kThreads) kSolvePositions(SolveArgs a)
 {
 	Scalars* sc = a.sc;
