@@ -849,18 +849,7 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	};
 	const size_t limit = std::min(s.batch_slab_limit, kBatchSlabTotal);
 
-	auto readResults = [&](const Part& p) {
-		BatchResult* const r = reinterpret_cast<BatchResult*>(hmeta + off_res) + p.first;
-		MO_CUDA_CHECK(cudaMemcpyAsync(r, d_res + p.first, p.count * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
-		MO_CUDA_CHECK(cudaStreamSynchronize(st));
-		return r;
-	};
-	auto manyBeyond = [](const BatchResult* r, size_t count) {
-		size_t beyond = 0;
-		for (size_t i = 0; i < count; ++i)
-			beyond += (r[i].status & kBatchBeyond) != 0;
-		return beyond > count / 16;
-	};
+	auto many = [](size_t beyond, size_t count) { return beyond > count / 16; };
 	bool tuned = false;
 	std::tuple<int, int, bool, bool> cls;
 	for (Part& p : parts)
@@ -935,7 +924,10 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 		if (!known)
 		{
 			shapes.as_expected = trials(false);
-			shapes.last_beyond = manyBeyond(readResults(p), p.count);
+			BatchResult* const seen = reinterpret_cast<BatchResult*>(hmeta + off_res) + p.first;
+			MO_CUDA_CHECK(cudaMemcpyAsync(seen, d_res + p.first, p.count * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
+			MO_CUDA_CHECK(cudaStreamSynchronize(st));
+			shapes.last_beyond = many(std::count_if(seen, seen + p.count, [](const BatchResult& r) { return (r.status & kBatchBeyond) != 0; }), p.count);
 		}
 		if (shapes.last_beyond && !shapes.timed_beyond && trial)
 		{
@@ -992,17 +984,22 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 	MO_CUDA_CHECK(cudaMemcpyAsync(hmeta + off_res, d_res, n * sizeof(BatchResult), cudaMemcpyDeviceToHost, st));
 	MO_CUDA_CHECK(cudaStreamSynchronize(st));
 	probe().collect();
-	if (tuned)
-	{
-		const bool beyond = manyBeyond(tmp + parts[1].first, parts[1].count);
-		std::lock_guard<std::mutex> g(g_tuner.lock);
-		g_tuner.shape[cls].last_beyond = beyond;
-	}
+	size_t slab = 0, beyond = 0;
 	for (size_t i = 0; i < n; ++i)
 	{
-		BatchResult& r = results[perm[i]] = tmp[i];
-		++(r.status & kBatchInSlab ? s.batch_in_slab : s.batch_in_shared);
-		r.status &= ~(kBatchInSlab | kBatchBeyond);
+		const unsigned int where = tmp[i].status;
+		slab += where / kBatchInSlab & 1;
+		beyond += i >= wide ? where / kBatchBeyond & 1 : 0;
+		BatchResult& r = results[perm[i]];
+		r = tmp[i];
+		r.status = where & 0xff;
+	}
+	s.batch_in_slab = slab;
+	s.batch_in_shared = n - slab;
+	if (tuned)
+	{
+		std::lock_guard<std::mutex> g(g_tuner.lock);
+		g_tuner.shape[cls].last_beyond = many(beyond, parts[1].count);
 	}
 }
 

@@ -370,3 +370,22 @@ for i in range(count):
     root = os.path.dirname(here)
     r = subprocess.run([sys.executable, "-c", code % (here, root, os.path.join(root, "oracle"), call)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("threads,smem_kb", [(128, 54), (512, 216), (256, 2)])
+def test_windows_that_the_error_limit_ends(port, threads, smem_kb):
+    """Passes with many triangles to remove that the error limit ends after none, a few (walked: up to 31) and
+    more candidates, up to all of them, and limits of zero and infinity."""
+    ms = []
+    for nx, ny, amp in ((17, 17, 0.1), (26, 23, 0.02), (40, 21, 0.0)):
+        idx, pos = _grid(nx, ny, amp, nx)
+        attr = np.random.default_rng(nx).standard_normal((len(pos), 2)).astype(np.float32)
+        for error in [0.0, np.inf] + [float(10.0 ** (-e / 6)) for e in range(6, 30)]:
+            for extra in (dict(), dict(options=mg.SimplifyRegularize), dict(attributes=attr, weights=np.full(2, 0.1, np.float32))):
+                ms.append(dict(dict(indices=idx, positions=pos, target=0, error=error), **extra))
+    mg.set_batch_config(threads, smem_kb * 1024)
+    try:
+        res = mg.simplify_batch(ms)
+    finally:
+        mg.set_batch_config(0)
+    _same(port, ms, res)
