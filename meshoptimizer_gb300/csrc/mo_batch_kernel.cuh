@@ -12,7 +12,7 @@
 // apart from the code for a mesh in the CTA's slab of global memory, so that its loads are shared-memory
 // loads (as generic ones they made the whole kernel 10 to 20% slower). Measured with 32-bit ids in memory
 // addressed generically, the mesh in shared memory only where the largest fits whole: 4,096 meshes of 510
-// triangles 1.43 ms and 0.86 since (the kernel alone 0.54); 2,048 groups of 1,024 triangles with attributes
+// triangles 1.43 ms and 0.82 since (the kernel alone 0.53); 2,048 groups of 1,024 triangles with attributes
 // 3.67 ms and 1.88.
 #pragma once
 
