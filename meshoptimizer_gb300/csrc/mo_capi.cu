@@ -895,7 +895,8 @@ void runBatch(ThreadState& s, std::vector<BatchDesc>& descs, const AttrMaps& map
 				}
 				return least;
 			};
-			float best_ms = sure ? timed(best, false) : 1e30f;
+			// a shape for the most a mesh can need is taken unless it is clearly the slower: it runs no setup twice
+			float best_ms = sure ? 1.1f * timed(best, false) : 1e30f;
 			for (int t : {128, 256, 512})
 			{
 				if (p.threads && t != p.threads)
